@@ -573,7 +573,7 @@ def run_b200(args):
             else:
                 alg = mean_distinct * 2 * TENSOR_BYTES + B * H * 4 + B * K * M * 4
                 kname = ("q4_gemm_tc_kernel<fused> (tcgen05 gate/up + GeGLU)" if tc_mode
-                         else "q4_tile16_kernel<2,TT> / q4_fused_expert_kernel (gate/up + GeGLU)")
+                         else "q4_batch_kernel<2,RL> / q4_fused_expert_kernel (gate/up + GeGLU)")
                 if fmt == "nvfp4":
                     # the class brackets the whole NVFP4 expert phase of a layer (five launches)
                     alg = mean_distinct * 3 * TENSOR_BYTES + B * H * 4 + B * K * (2 * H + 4 * M) * 4

@@ -390,7 +390,7 @@ typedef struct SaltB200Nvfp4Buffers {
     const uint8_t *chain_codes, *chain_scales;
 } SaltB200Nvfp4Buffers;
 int salt_b200_stack_nvfp4_buffers(void *stack, SaltB200Nvfp4Buffers *out);
-/* Batches of up to 4 tokens run gate/up, GeGLU and down of all selected experts in ONE launch
+/* The experts of ONE token run gate/up, GeGLU and down in one launch
  * (one persistent block per SM, weights of both phases in flight from the start; the reference
  * runs the three projections as separate calls, models/gemma4-26b-a4b/src/gemma4_text.c:7971-7997).
  * A forward pass of ONE token over affine-Q4 layers goes further: level 1 (the default) runs each layer

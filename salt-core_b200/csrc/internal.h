@@ -15,7 +15,6 @@ struct Q4Job;
 cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes);
 
 // ---- q4_kernels.cu -------------------------------------------------------
-bool q4_tile_supported(int C);
 // Runs every job (all share C and nmat).  njobs_dev (device int, may be null)
 // bounds the live jobs when the count is only known on the device; blocks past
 // it exit at once.  `aligned` promises 16-byte aligned tensors and x rows.
@@ -25,17 +24,21 @@ bool q4_tile_supported(int C);
 cudaError_t launch_q4_jobs(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
                            int nmat, bool aligned, cudaStream_t stream, int pdl = -1);
 
+// ---- q4_batch_kernels.cu -----------------------------------------------------
+// The same jobs for groups of several tokens (aligned tensors, C a multiple of 64).
+constexpr int Q4_PASS_TOKENS = 4;        // tokens that share one dequantisation
+bool q4_batch_supported(int C, int nmat);
+cudaError_t launch_q4_batch(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
+                            int nmat, cudaStream_t stream, int pdl);
+
 // ---- q4_fused_decode.cu ------------------------------------------------------
 // Decode-sized expert execution in one launch (gate | up -> GeGLU -> down).
 constexpr int FUSED_MAX_JOBS = 32;       // expert groups per launch
-constexpr int FUSED_MAX_TOKENS = 4;      // activation rows per launch (and tokens per group)
-struct FusedJob {
+struct FusedJob {      // one token per expert
     const uint8_t* v[3];                       // packed values of gate, up, down (16-byte aligned)
     const uint32_t* t[3];                      // their derived tables: (scale bf16 << 16) | bias bf16 per group, [rows][C / 64]
-    int32_t x_row[FUSED_MAX_TOKENS];           // activation row of each token of the group
-    int32_t g0;                                // first grouped row (GeGLU rows and output rows g0, g0 + 1, ...)
-    int32_t ntok;
-    int32_t lit, pad;                          // lit bit k: tensor k has a scale that needs the two-rounding dequantisation
+    int32_t g0;                                // grouped row (of the GeGLU values and of the output)
+    int32_t lit, pad[2];                          // lit bit k: tensor k has a scale that needs the two-rounding dequantisation
 };
 // Builds the derived tables of n_experts expert slots (gate | up | down, each values | scales | biases).
 // words: [n_experts][3][groups] (groups = R * C / 64 of one tensor); flags: [n_experts].
@@ -46,17 +49,16 @@ struct FusedArgs {
     const int* n_jobs_dev;       // live jobs (device)
     int n_jobs_max;
     int* done;                   // [n_jobs_max] arrival counters, zero at launch
-    const float* x;              // [n_x][x_stride] activation rows
-    int x_stride, n_x;
+    const float* x;              // [H] activation row
     float* chain;                // [grouped rows][M]
     float* out;                  // [grouped rows][H]
     int H, M;
     int jobs_per_round;          // filled in by the launcher
     int* status;
 };
-struct FusedLaunch { int grid, jobs_per_round, tt; size_t smem; };
+struct FusedLaunch { int grid, jobs_per_round; size_t smem; };
 // Whether the fused kernel serves this geometry on the current device (and how it would be launched).
-bool q4_fused_plan(int H, int M, int n_x, int n_jobs_max, FusedLaunch* out);
+bool q4_fused_plan(int H, int M, int n_jobs_max, FusedLaunch* out);
 // Launched as a programmatic dependent launch; jobs, counters and x come from the previous kernel.
 cudaError_t launch_q4_fused(const FusedArgs& args, cudaStream_t stream);
 
@@ -88,7 +90,7 @@ struct alignas(16) LayerDecodeArgs {
 bool q4_layer_decode_plan(int H, int M, int E, int topk, int n_jobs_max, FusedLaunch* out);
 cudaError_t launch_q4_layer_decode(const LayerDecodeArgs& args, int n_jobs_max, cudaStream_t stream);
 // All layers in one launch: d_layers [n_layers] arguments in device memory (f.jobs_per_round = the value of
-// q4_layer_decode_jobs_per_round, f.n_x = 1), d_done [n_layers] arrival counters, zero at launch.
+// q4_layer_decode_jobs_per_round), d_done [n_layers] arrival counters, zero at launch.
 cudaError_t launch_q4_stack_decode(const LayerDecodeArgs* d_layers, int n_layers, int* d_done, int H, int M, int E, int topk,
                                    int n_jobs_max, cudaStream_t stream);
 int q4_layer_decode_jobs_per_round(int H, int M, int E, int topk, int n_jobs_max);
@@ -275,8 +277,9 @@ struct MoePlanArgs {
     const float* x;              // [rows][hidden] layer input
     float* chain;                // [jobs][inter] grouped GeGLU output
     float* grouped_out;          // [jobs][hidden] grouped down output
-    Q4Job* gateup_jobs;          // [E]
-    Q4Job* down_jobs;            // [E]
+    int pass_tokens;             // 0: one job per expert group; else one per pass of at most this many of its tokens
+    Q4Job* gateup_jobs;          // [E], or [E + jobs / pass_tokens]
+    Q4Job* down_jobs;
     // optional: descriptors and zeroed arrival counters of the fused decode kernel
     // (the first FUSED_MAX_JOBS local groups; the caller only uses them when there can be no more)
     FusedJob* fused_jobs;        // [FUSED_MAX_JOBS] or null

@@ -84,7 +84,7 @@ struct Stack {
     CUtensorMap fp4_x_gu[3], fp4_x_dn[3];      // packed activations as [2J][H/2] and as [J][M/2]
     CUtensorMap fp4_xs_gu[3], fp4_xs_dn[3];    // their block scales as [2J][H/16] and as [J][M/16]
     bool fp4_maps_ok = false;
-    int fused_decode = 1;                      // 0: phase kernels; 1: one-launch expert kernel (B <= 4) and one launch per decode layer (B = 1); 2: all layers of a B = 1 pass in one launch (measured slower than 1)
+    int fused_decode = 1;                      // one token: 0 phase kernels; 1 one-launch expert kernel and one launch per decode layer; 2 all layers of a pass in one launch (measured slower than 1)
     void *xh = nullptr, *xl = nullptr, *chain_h = nullptr, *chain_l = nullptr;   // fp16 operands (hi, lo) of the tensor-core path
     bool tc_ready = false;                     // tensor maps built and the geometry fits the single-precision tensor-core kernel
     bool tc_split_ready = false;               // ... and the hi + lo form
@@ -201,7 +201,8 @@ int salt_b200_stack_create(int max_tokens, int hidden, int inter, int n_experts,
               dev_alloc(&s->io_out, T * hidden) && dev_alloc(&s->selected, J) &&
               dev_alloc(&s->group_offsets, (size_t)n_experts + 1) && dev_alloc(&s->g2c, J) &&
               dev_alloc(&s->c2g, J) && dev_alloc(&s->counters, 4) && dev_alloc(&s->status, 1) &&
-              dev_alloc(&s->gateup_jobs, (size_t)n_experts) && dev_alloc(&s->down_jobs, (size_t)n_experts) &&
+              dev_alloc(&s->gateup_jobs, (size_t)n_experts + J / Q4_PASS_TOKENS) &&
+              dev_alloc(&s->down_jobs, (size_t)n_experts + J / Q4_PASS_TOKENS) &&
               dev_alloc(&s->fused_jobs, (size_t)FUSED_MAX_JOBS) && dev_alloc(&s->fused_done, (size_t)FUSED_MAX_JOBS) &&
               dev_alloc(&s->grouped_alt, (size_t)topk * hidden) && dev_alloc(&s->weights_alt, (size_t)topk) &&
               dev_alloc((uint16_t**)&s->xh, J * hidden) && dev_alloc((uint16_t**)&s->chain_h, J * inter) &&
@@ -461,17 +462,26 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
     a.hidden = H; a.inter = M; a.x = d_x; a.chain = s->chain; a.grouped_out = s->grouped_out;
     a.gateup_jobs = s->gateup_jobs; a.down_jobs = s->down_jobs; a.status = s->status;
     const int local = s->expert_end - s->expert_begin;
-    const int njobs_max = jobs < local ? jobs : local;
+    int njobs_max = jobs < local ? jobs : local;
     // decode batches: gate/up, GeGLU and down of all selected experts in one launch
     const bool fused = !l.nvfp4 && s->fused_decode && !(flags & (SB_EXPERTS_TENSOR_CORE | SB_EXPERTS_TENSOR_CORE_SINGLE |
                                                      SB_EXPERTS_TWO_LAUNCHES)) &&
-                       B <= FUSED_MAX_TOKENS && njobs_max <= FUSED_MAX_JOBS &&
+                       B == 1 && njobs_max <= FUSED_MAX_JOBS &&
                        ((((uintptr_t)d_x) | ((uintptr_t)l.pool) | l.expert_stride) & 15) == 0 &&
-                       q4_fused_plan(H, M, B, njobs_max, nullptr);
+                       q4_fused_plan(H, M, njobs_max, nullptr);
     if (fused) {
         a.fused_jobs = s->fused_jobs; a.fused_done = s->fused_done;
         a.fused_tables = l.sb_tables - (size_t)s->expert_begin * 6 * a.group_bytes;
         a.fused_lit = l.lit_flags - s->expert_begin;
+    }
+    // exact projections: one job per pass of the batch kernel instead of one per group
+    const bool exact_q4 = !l.nvfp4 && !fused && !(flags & (SB_EXPERTS_TENSOR_CORE | SB_EXPERTS_TENSOR_CORE_SINGLE));
+    if (exact_q4 && B > Q4_PASS_TOKENS && q4_batch_supported(H, 2) && q4_batch_supported(M, 1)) {
+        const int passes_max = std::min(jobs, local + jobs / Q4_PASS_TOKENS);
+        if (passes_max <= 65535) {                          // the grid's y extent
+            a.pass_tokens = Q4_PASS_TOKENS;
+            njobs_max = passes_max;
+        }
     }
     {
         Timed t(s, KC_PLAN, st);
@@ -528,16 +538,15 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
         FusedArgs f;
         memset(&f, 0, sizeof f);
         f.jobs = s->fused_jobs; f.n_jobs_dev = s->counters; f.n_jobs_max = njobs_max; f.done = s->fused_done;
-        f.x = d_x; f.x_stride = H; f.n_x = B; f.chain = s->chain; f.out = s->grouped_out; f.H = H; f.M = M;
+        f.x = d_x; f.chain = s->chain; f.out = s->grouped_out; f.H = H; f.M = M;
         f.status = s->status;
         Timed t(s, KC_GATE_UP, st);
         if (!cuda_ok(launch_q4_fused(f, st), "fused experts")) return -1;
         count_launches(3);
         return 0;
     }
-    // tokens per expert group: at most B (the tile kernels loop over a group's tokens and use the bound
-    // only to pick their token block; the any-shape kernel takes one grid row per token)
-    const int tok_hint = B;
+    // tokens per job: at most B, or those of a pass
+    const int tok_hint = a.pass_tokens ? a.pass_tokens : B;
     if (flags & (SB_EXPERTS_TENSOR_CORE | SB_EXPERTS_TENSOR_CORE_SINGLE)) {
         const bool split = (flags & SB_EXPERTS_TENSOR_CORE) != 0;
         if (!s->tc_ready || !l.q4_tc_ok || (split && !s->tc_split_ready)) {
@@ -1038,7 +1047,6 @@ static int forward_decode_layers(Stack* s, int first, int count, const float* d_
         a.value_bytes = elems / 2; a.group_bytes = elems / 64 * 2; a.tensor_bytes = a.value_bytes + 2 * a.group_bytes;
         if (stacked) {
             a.f.jobs_per_round = q4_layer_decode_jobs_per_round(H, M, s->n_experts, K, n_jobs_max);
-            a.f.n_x = 1;
             s->h_layer_args[(size_t)i] = a;
             continue;
         }

@@ -6,14 +6,13 @@
 //   L_j = ((((0 + acc[j]) + acc[j+4]) + ...) + acc[j+28]),  j = 0..3
 //   y   = fl(fl(L0 + L2) + fl(L1 + L3))
 //
-// Thread mapping: sixteen adjacent lanes share a weight row; lane v = tid & 15 owns the
-// accumulators 2v and 2v + 1, i.e. the two nibbles of byte v of every 32-column step (16 packed
-// bytes), so "accumulator c mod 32, columns ascending" is a sequential loop per lane and the
-// canonical fold is a chain through the sixteen lanes.  Each lane keeps two weight rows (gate +
-// up of the same output row, or two rows of one matrix) so the activation values it loads are
-// used twice, and TT tokens share one dequantisation.  Dequantisation and the products are
-// issued as sm_100 packed pairs (add/mul/fma.rn.f32x2): each half of a pair is an independent
-// IEEE round-to-nearest operation.
+// tile16_steps below is the inner loop of the one-token kernels (q4_fused_decode.cu): sixteen adjacent
+// lanes share a weight row; lane v = tid & 15 owns the accumulators 2v and 2v + 1, i.e. the two nibbles
+// of byte v of every 32-column step (16 packed bytes), so "accumulator c mod 32, columns ascending" is a
+// sequential loop per lane and the canonical fold is a chain through the sixteen lanes.  Each lane keeps
+// two weight rows (gate + up of the same output row, or two rows of one matrix).  Products are issued as
+// sm_100 packed pairs (add/mul/fma.rn.f32x2): each half of a pair is an independent IEEE
+// round-to-nearest operation.  Several tokens per weight row: q4_batch_kernels.cu.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -108,12 +107,6 @@ __device__ __forceinline__ void product_then_add(f32x2& acc, f32x2 d, f32x2 x, f
     acc = add2(acc, fma2(d, x, negzero));
 }
 
-// ---- the tile kernel: 16 lanes per row ----------------------------------------------
-// A row's 32 accumulators are spread over sixteen adjacent lanes (lane v = tid & 15 holds
-// acc[2v], acc[2v + 1], i.e. one packed byte per 32-column step).  An earlier form with eight
-// lanes per row (four accumulators each, half the warps) ran decode at the same speed and
-// batches of 64 tokens 1.4x slower.
-
 // One packed byte (two nibbles) as exact floats.
 template <bool LIT>
 __device__ __forceinline__ f32x2 dequant2(uint32_t b, const NibbleMagic& mg, f32x2 ss, f32x2 bb) {
@@ -153,27 +146,6 @@ __device__ __forceinline__ void tile16_steps(const NibbleMagic& mg, const uint8_
                 product_then_add(accB[tt], dB, xv, nz);
             }
         }
-    }
-}
-
-template <int TT, bool LIT>
-__device__ __forceinline__ void tile16_run(const NibbleMagic& mg, int s_begin, int s_end, const uint8_t* wA,
-                                           const uint8_t* wB, const uint32_t* tA, const uint32_t* tB,
-                                           const float* sX, int x_pitch, f32x2 (&accA)[TT], f32x2 (&accB)[TT],
-                                           f32x2 nz) {
-    int st = s_begin;
-    constexpr int BLK = 8;
-    for (; st + BLK <= s_end; st += BLK) {
-        const float* xs[TT];
-#pragma unroll
-        for (int tt = 0; tt < TT; tt++) xs[tt] = sX + tt * x_pitch + st * 32;
-        tile16_steps<TT, LIT, BLK>(mg, wA + st * 16, wB + st * 16, tA + (st >> 1), tB + (st >> 1), xs, accA, accB, nz);
-    }
-    for (; st + 2 <= s_end; st += 2) {
-        const float* xs[TT];
-#pragma unroll
-        for (int tt = 0; tt < TT; tt++) xs[tt] = sX + tt * x_pitch + st * 32;
-        tile16_steps<TT, LIT, 2>(mg, wA + st * 16, wB + st * 16, tA + (st >> 1), tB + (st >> 1), xs, accA, accB, nz);
     }
 }
 

@@ -55,7 +55,7 @@ struct FusedGeom {
     size_t off_dn, off_sgu, off_sdn, off_x, off_chain, off_jobs, off_bars, total;
 };
 
-static __host__ __device__ __forceinline__ FusedGeom fused_geom(int H, int M, int tt, int slots) {
+static __host__ __device__ __forceinline__ FusedGeom fused_geom(int H, int M, int slots) {
     FusedGeom g;
     g.gu_rb = H >> 1; g.gu_stride = fused_row_stride(g.gu_rb); g.gu_gpr = H >> 6;
     g.dn_rb = M >> 1; g.dn_stride = g.dn_rb; g.dn_gpr = M >> 6;      // dense: the block's down rows arrive as one copy
@@ -67,8 +67,8 @@ static __host__ __device__ __forceinline__ FusedGeom fused_geom(int H, int M, in
     g.off_dn = o;    o += (size_t)g.dn_cap * g.dn_stride;
     g.off_sgu = o;   o += (size_t)2 * g.gu_sc_cap;       // scale | bias words of the gate rows, of the up rows
     g.off_sdn = o;   o += (size_t)g.dn_sc_cap;           // scale | bias words of the down rows
-    g.off_x = o;     o += (size_t)tt * H * 4;
-    g.off_chain = o; o += (size_t)2 * tt * M * 4;
+    g.off_x = o;     o += (size_t)H * 4;
+    g.off_chain = o; o += (size_t)2 * M * 4;
     g.off_jobs = o;  o += (size_t)FUSED_MAX_JOBS * sizeof(FusedJob);
     g.off_bars = o;  o += (size_t)(slots / 2 * FUSED_GU_CHUNKS + 4) * 8;   // gate/up barriers per warp and chunk, x, scales, down
     g.total = o;
@@ -106,22 +106,18 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     return v;
 }
 
-// One lane's two rows for the NT tokens of its job: the dot products in the reference order
+// One lane's two rows of its job: the dot products in the reference order
 // (tile16_steps: sixteen lanes per row, lane v owns accumulators 2v and 2v + 1) and the canonical
 // fold.  The rarely needed two-rounding form (a scale so large that q*s could overflow) is
 // rolled up, so that it adds little to the code the SM has to fetch.
-template <int NT>
 __device__ __forceinline__ bool fused_slot(const NibbleMagic& mg, bool lit, int steps, const uint8_t* wA,
                                            const uint8_t* wB, const uint32_t* tA, const uint32_t* tB,
-                                           const float* const (&xrow)[NT], int v, float (&yA)[NT], float (&yB)[NT],
-                                           f32x2 nz, uint64_t* chunk_bars, uint32_t parity, int chunk_steps) {
-    // the two row slots of a warp may belong to jobs with different token counts (or one of them
-    // may be empty): the fold only involves the slot's own sixteen lanes
+                                           const float* x, int v, float& yA, float& yB, f32x2 nz,
+                                           uint64_t* chunk_bars, uint32_t parity, int chunk_steps) {
+    // one of the two row slots of a warp may be empty: the fold only involves the slot's own sixteen lanes
     const uint32_t half_mask = 0xffffu << (threadIdx.x & 16);
     bool timeout = false;
-    f32x2 accA[NT], accB[NT];
-#pragma unroll
-    for (int tt = 0; tt < NT; tt++) { accA[tt] = pack2(0.0f, 0.0f); accB[tt] = pack2(0.0f, 0.0f); }
+    f32x2 accA[1] = {pack2(0.0f, 0.0f)}, accB[1] = {pack2(0.0f, 0.0f)};
     // the rows arrive in chunks of chunk_steps steps (chunk_bars: one barrier per chunk; null: all here)
 #pragma unroll 1
     for (int c0 = 0; c0 < steps; c0 += chunk_steps) {
@@ -131,33 +127,24 @@ __device__ __forceinline__ bool fused_slot(const NibbleMagic& mg, bool lit, int 
         if (lit) {
 #pragma unroll 1
             for (; st + 2 <= c1; st += 2) {
-                const float* xs[NT];
-#pragma unroll
-                for (int tt = 0; tt < NT; tt++) xs[tt] = xrow[tt] + st * 32;
-                tile16_steps<NT, true, 2>(mg, wA + st * 16, wB + st * 16, tA + (st >> 1), tB + (st >> 1), xs, accA, accB, nz);
+                const float* const xs[1] = {x + st * 32};
+                tile16_steps<1, true, 2>(mg, wA + st * 16, wB + st * 16, tA + (st >> 1), tB + (st >> 1), xs, accA, accB, nz);
             }
         } else {
 #pragma unroll 1
             for (; st + 8 <= c1; st += 8) {
-                const float* xs[NT];
-#pragma unroll
-                for (int tt = 0; tt < NT; tt++) xs[tt] = xrow[tt] + st * 32;
-                tile16_steps<NT, false, 8>(mg, wA + st * 16, wB + st * 16, tA + (st >> 1), tB + (st >> 1), xs, accA, accB, nz);
+                const float* const xs[1] = {x + st * 32};
+                tile16_steps<1, false, 8>(mg, wA + st * 16, wB + st * 16, tA + (st >> 1), tB + (st >> 1), xs, accA, accB, nz);
             }
 #pragma unroll 1
             for (; st + 2 <= c1; st += 2) {
-                const float* xs[NT];
-#pragma unroll
-                for (int tt = 0; tt < NT; tt++) xs[tt] = xrow[tt] + st * 32;
-                tile16_steps<NT, false, 2>(mg, wA + st * 16, wB + st * 16, tA + (st >> 1), tB + (st >> 1), xs, accA, accB, nz);
+                const float* const xs[1] = {x + st * 32};
+                tile16_steps<1, false, 2>(mg, wA + st * 16, wB + st * 16, tA + (st >> 1), tB + (st >> 1), xs, accA, accB, nz);
             }
         }
     }
-#pragma unroll
-    for (int tt = 0; tt < NT; tt++) {
-        yA[tt] = fold_row_hexadecants(accA[tt], v, half_mask);
-        yB[tt] = fold_row_hexadecants(accB[tt], v, half_mask);
-    }
+    yA = fold_row_hexadecants(accA[0], v, half_mask);
+    yB = fold_row_hexadecants(accB[0], v, half_mask);
     return timeout;
 }
 
@@ -175,7 +162,7 @@ template <int NROWS, int IT>
 struct TableRegs { uint32_t w[NROWS][IT]; };
 
 // Shared-memory views of a block (see fused_geom).
-template <int TT, int SLOTS>
+template <int SLOTS>
 struct FusedSmem {
     static constexpr int NT = 16 * SLOTS, NW = SLOTS / 2;
     uint8_t *sGU, *sDN, *sSG, *sSD;
@@ -187,8 +174,8 @@ struct FusedSmem {
         sDN = smem + G.off_dn;                        // [dn_cap] down rows, dense
         sSG = smem + G.off_sgu;                       // [2][gu_sc_cap] (scale << 16) | bias words of the gate / up rows
         sSD = smem + G.off_sdn;                       // [dn_sc_cap] the same for the down rows
-        sX = (float*)(smem + G.off_x);                // [TT][H] the call's activation rows
-        sC = (float*)(smem + G.off_chain);            // [2 jobs][TT][M] GeGLU rows of the down phase
+        sX = (float*)(smem + G.off_x);                // [H] the call's activation row
+        sC = (float*)(smem + G.off_chain);            // [2 jobs][M] GeGLU rows of the down phase
         sJ = (FusedJob*)(smem + G.off_jobs);
         bar_gu = (uint64_t*)(smem + G.off_bars);      // [NW][FUSED_GU_CHUNKS] packed gate/up rows of a warp, by chunk
         bar_x = bar_gu + NW * FUSED_GU_CHUNKS;        // activations
@@ -210,8 +197,8 @@ struct FusedSmem {
 // The expert phases of a block for the n_jobs descriptors in S.sJ (barriers initialised, the block
 // synchronised).  x_resident: S.sX already holds the activation rows; otherwise they are copied from
 // a.x.  Returns true when a bounded wait ran out.  Every thread of the block must call.
-template <int TT, int SLOTS>
-__device__ __forceinline__ bool fused_expert_rounds(const FusedArgs& a, const FusedGeom& G, const FusedSmem<TT, SLOTS>& S,
+template <int SLOTS>
+__device__ __forceinline__ bool fused_expert_rounds(const FusedArgs& a, const FusedGeom& G, const FusedSmem<SLOTS>& S,
                                                     int n_jobs, bool x_resident, ScaleRange* s_rg, ScaleRange* s_rd) {
     constexpr int NT = 16 * SLOTS;
     const int H = a.H, M = a.M;
@@ -325,8 +312,8 @@ __device__ __forceinline__ bool fused_expert_rounds(const FusedArgs& a, const Fu
     if (warp == 0) issue_scales(R);
     if (tid == 0) {
         if (!x_resident) {
-            mbar_expect_tx(bar_x, (uint32_t)(a.n_x * H * 4));
-            for (int t = 0; t < a.n_x; t++) bulk_g2s(sX + (size_t)t * H, a.x + (size_t)t * a.x_stride, (uint32_t)(H * 4), bar_x);
+            mbar_expect_tx(bar_x, (uint32_t)(H * 4));
+            bulk_g2s(sX, a.x, (uint32_t)(H * 4), bar_x);
         }
     }
     __syncthreads();               // s_rg / s_rd are published, the small requests are queued
@@ -346,35 +333,11 @@ __device__ __forceinline__ bool fused_expert_rounds(const FusedArgs& a, const Fu
             const uint32_t* tA = table_row(s_rg, sSG, G.gu_sc_cap, 0, jl - R.gu_lo / M, row, G.gu_gpr);
             const uint32_t* tB = table_row(s_rg, sSG, G.gu_sc_cap, 1, jl - R.gu_lo / M, row, G.gu_gpr);
             const bool lit_gu = (jb.lit & 3) != 0;
-            const int ntok = jb.ntok;
             float* crow = a.chain + (size_t)jb.g0 * M + row;
-            if (TT >= 4 && ntok >= 3) {
-                constexpr int N = TT >= 4 ? 4 : 1;
-                const float* xr[N];
-                float yA[N], yB[N];
-#pragma unroll
-                for (int t = 0; t < N; t++) xr[t] = sX + (size_t)jb.x_row[min(t, ntok - 1)] * H + 2 * v;
-                timeout |= fused_slot<N>(mg, lit_gu, H >> 5, wA, wB, tA, tB, xr, v, yA, yB, nz, bar_gu + warp * FUSED_GU_CHUNKS, ph_gu & 1, gu_chunk_steps);
-                if (v == 0)
-#pragma unroll
-                    for (int t = 0; t < N; t++)
-                        if (t < ntok) crow[(size_t)t * M] = __fmul_rn(gelu_tanh_exact(yA[t]), yB[t]);
-            } else if (TT >= 2 && ntok == 2) {
-                constexpr int N = TT >= 2 ? 2 : 1;
-                const float* xr[N];
-                float yA[N], yB[N];
-#pragma unroll
-                for (int t = 0; t < N; t++) xr[t] = sX + (size_t)jb.x_row[min(t, ntok - 1)] * H + 2 * v;
-                timeout |= fused_slot<N>(mg, lit_gu, H >> 5, wA, wB, tA, tB, xr, v, yA, yB, nz, bar_gu + warp * FUSED_GU_CHUNKS, ph_gu & 1, gu_chunk_steps);
-                if (v == 0)
-#pragma unroll
-                    for (int t = 0; t < N; t++) crow[(size_t)t * M] = __fmul_rn(gelu_tanh_exact(yA[t]), yB[t]);
-            } else {
-                const float* xr[1] = {sX + (size_t)jb.x_row[0] * H + 2 * v};
-                float yA[1], yB[1];
-                timeout |= fused_slot<1>(mg, lit_gu, H >> 5, wA, wB, tA, tB, xr, v, yA, yB, nz, bar_gu + warp * FUSED_GU_CHUNKS, ph_gu & 1, gu_chunk_steps);
-                if (v == 0) crow[0] = __fmul_rn(gelu_tanh_exact(yA[0]), yB[0]);
-            }
+            float y_gate, y_up;
+            timeout |= fused_slot(mg, lit_gu, H >> 5, wA, wB, tA, tB, sX + 2 * v, v, y_gate, y_up, nz,
+                                  bar_gu + warp * FUSED_GU_CHUNKS, ph_gu & 1, gu_chunk_steps);
+            if (v == 0) *crow = __fmul_rn(gelu_tanh_exact(y_gate), y_up);
         }
         __syncwarp();
         if (gu_rows_w > 0) ph_gu++;    // this warp's chunk barriers have all completed a phase
@@ -407,10 +370,9 @@ __device__ __forceinline__ bool fused_expert_rounds(const FusedArgs& a, const Fu
         __syncthreads();
         for (int j = dja; j <= djb; j++) {
             const FusedJob& jb = sJ[R.j0 + j];
-            const int n = jb.ntok * M;                      // the job's GeGLU rows are contiguous
             const float* src = a.chain + (size_t)jb.g0 * M;
-            float* dstc = sC + (size_t)(j - dja) * TT * M;
-            for (int i = tid * 4; i < n; i += NT * 4) *(float4*)(dstc + i) = __ldcg((const float4*)(src + i));
+            float* dstc = sC + (size_t)(j - dja) * M;
+            for (int i = tid * 4; i < M; i += NT * 4) *(float4*)(dstc + i) = __ldcg((const float4*)(src + i));
         }
         if (!fused_mbar_wait(bar_dn, r & 1)) timeout = true;
         __syncthreads();
@@ -426,36 +388,11 @@ __device__ __forceinline__ bool fused_expert_rounds(const FusedArgs& a, const Fu
             const uint32_t* tA = table_row(s_rd, sSD, G.dn_sc_cap, 0, jl - dja, row, G.dn_gpr);
             const uint32_t* tB = tA + G.dn_gpr;
             const bool lit_dn = (jb.lit & 4) != 0;
-            const float* cbase = sC + (size_t)(jl - dja) * TT * M + 2 * v;
-            const int ntok = jb.ntok;
+            const float* cbase = sC + (size_t)(jl - dja) * M + 2 * v;
             float* orow = a.out + (size_t)jb.g0 * H + row;
-            if (TT >= 4 && ntok >= 3) {
-                constexpr int N = TT >= 4 ? 4 : 1;
-                const float* xr[N];
-                float yA[N], yB[N];
-#pragma unroll
-                for (int t = 0; t < N; t++) xr[t] = cbase + (size_t)min(t, ntok - 1) * M;
-                fused_slot<N>(mg, lit_dn, M >> 5, wA, wB, tA, tB, xr, v, yA, yB, nz, nullptr, 0, M >> 5);
-                if (v == 0)
-#pragma unroll
-                    for (int t = 0; t < N; t++)
-                        if (t < ntok) *(float2*)(orow + (size_t)t * H) = make_float2(yA[t], yB[t]);
-            } else if (TT >= 2 && ntok == 2) {
-                constexpr int N = TT >= 2 ? 2 : 1;
-                const float* xr[N];
-                float yA[N], yB[N];
-#pragma unroll
-                for (int t = 0; t < N; t++) xr[t] = cbase + (size_t)t * M;
-                fused_slot<N>(mg, lit_dn, M >> 5, wA, wB, tA, tB, xr, v, yA, yB, nz, nullptr, 0, M >> 5);
-                if (v == 0)
-#pragma unroll
-                    for (int t = 0; t < N; t++) *(float2*)(orow + (size_t)t * H) = make_float2(yA[t], yB[t]);
-            } else {
-                const float* xr[1] = {cbase};
-                float yA[1], yB[1];
-                fused_slot<1>(mg, lit_dn, M >> 5, wA, wB, tA, tB, xr, v, yA, yB, nz, nullptr, 0, M >> 5);
-                if (v == 0) *(float2*)orow = make_float2(yA[0], yB[0]);
-            }
+            float y0, y1;
+            fused_slot(mg, lit_dn, M >> 5, wA, wB, tA, tB, cbase, v, y0, y1, nz, nullptr, 0, M >> 5);
+            if (v == 0) *(float2*)orow = make_float2(y0, y1);
         }
         __syncthreads();               // the block is done with this round's down rows and tables
         if (r + 1 < rounds && warp == 0) {
@@ -470,12 +407,12 @@ __device__ __forceinline__ bool fused_expert_rounds(const FusedArgs& a, const Fu
     return timeout;
 }
 
-template <int TT, int SLOTS>
+template <int SLOTS>
 __global__ void __launch_bounds__(16 * SLOTS, 1) q4_fused_expert_kernel(FusedArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int NT = 16 * SLOTS;
-    const FusedGeom G = fused_geom(a.H, a.M, TT, SLOTS);
-    FusedSmem<TT, SLOTS> S(smem, G);
+    const FusedGeom G = fused_geom(a.H, a.M, SLOTS);
+    FusedSmem<SLOTS> S(smem, G);
     __shared__ int s_njobs;
     __shared__ ScaleRange s_rg[2], s_rd[2];                // the (up to two) job segments of the block's shares
     const int tid = threadIdx.x;
@@ -494,7 +431,7 @@ __global__ void __launch_bounds__(16 * SLOTS, 1) q4_fused_expert_kernel(FusedArg
     __syncthreads();               // barriers initialised, jobs and count in shared memory
     const int n_jobs = s_njobs;
     if (n_jobs == 0) return;
-    const bool timeout = fused_expert_rounds<TT, SLOTS>(a, G, S, n_jobs, false, s_rg, s_rd);
+    const bool timeout = fused_expert_rounds<SLOTS>(a, G, S, n_jobs, false, s_rg, s_rd);
     if (timeout && a.status) atomicOr(a.status, SB_ERR_TIMEOUT);
 }
 
@@ -545,8 +482,8 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
                                                   int* my_done) {
     constexpr int SLOTS = LAYER_SLOTS, NT = 16 * SLOTS, NV = LAYER_NV;
     const int H = a.f.H, M = a.f.M, E = a.E, K = a.topk;
-    const FusedGeom G = fused_geom(H, M, 1, SLOTS);
-    FusedSmem<1, SLOTS> S(smem, G);
+    const FusedGeom G = fused_geom(H, M, SLOTS);
+    FusedSmem<SLOTS> S(smem, G);
     const LayerScratch L = layer_scratch(H, E, K);
     float* const fsm = (float*)smem;
     float* const sq = fsm + L.sq;                 // squares / products for the in-order chains
@@ -780,9 +717,8 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
                 fj.v[k] = base + (size_t)k * a.tensor_bytes;
                 fj.t[k] = (const uint32_t*)(tb + (size_t)k * 2 * a.group_bytes);
             }
-            fj.lit = s_lit[e]; fj.pad = 0;
-            for (int t = 0; t < FUSED_MAX_TOKENS; t++) fj.x_row[t] = 0;
-            fj.g0 = j; fj.ntok = 1;              // one token: grouped order = rank order (experts ascending)
+            fj.lit = s_lit[e];
+            fj.g0 = j;                           // one token: grouped order = rank order (experts ascending)
             S.sJ[slot] = fj;
         }
         if (j == 0) s_njobs = min(total, FUSED_MAX_JOBS);
@@ -802,7 +738,7 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
     }
     __syncthreads();                // jobs published; the scratch is dead: the weight rows may land on it
     const int n_jobs = s_njobs;
-    if (n_jobs > 0) timeout |= fused_expert_rounds<1, SLOTS>(a.f, G, S, n_jobs, true, s_rg, s_rd);
+    if (n_jobs > 0) timeout |= fused_expert_rounds<SLOTS>(a.f, G, S, n_jobs, true, s_rg, s_rd);
     if (timeout && a.f.status) atomicOr(a.f.status, SB_ERR_TIMEOUT);
     if (STACKED) {
         __syncthreads();            // all of this block's rows of the layer are written, its shared memory is free
@@ -880,17 +816,14 @@ DeviceInfo* device_info() {
     return d;
 }
 constexpr size_t FUSED_SMEM_LIMIT = 227 * 1024 - 3072;   // dynamic part: the opt-in maximum less the kernel's static variables
-int fused_tt(int n_x) { return n_x <= 1 ? 1 : (n_x == 2 ? 2 : 4); }
-int fused_slots(int tt) { return tt == 1 ? 40 : 32; }
 }  // namespace
 
-bool q4_fused_plan(int H, int M, int n_x, int n_jobs_max, FusedLaunch* out) {
+bool q4_fused_plan(int H, int M, int n_jobs_max, FusedLaunch* out) {
     DeviceInfo* d = device_info();
-    if (!d || H < 64 || M < 64 || (H & 63) || (M & 63) || n_x < 1 || n_x > 4 || n_jobs_max < 1 ||
-        n_jobs_max > FUSED_MAX_JOBS)
+    if (!d || H < 64 || M < 64 || (H & 63) || (M & 63) || n_jobs_max < 1 || n_jobs_max > FUSED_MAX_JOBS)
         return false;
-    const int tt = fused_tt(n_x), slots = fused_slots(tt);
-    const FusedGeom g = fused_geom(H, M, tt, slots);
+    const int slots = LAYER_SLOTS;
+    const FusedGeom g = fused_geom(H, M, slots);
     if (g.total > FUSED_SMEM_LIMIT) return false;
     const int grid = d->sms;
     // most jobs per round whose shares fit the block: ceil(J*M/grid) <= slots, ceil(J*H/grid) <= dn_cap
@@ -903,34 +836,27 @@ bool q4_fused_plan(int H, int M, int n_x, int n_jobs_max, FusedLaunch* out) {
         jmax = J;
     }
     if (jmax < 1) return false;
-    if (out) { out->grid = grid; out->jobs_per_round = jmax; out->tt = tt; out->smem = g.total; }
+    if (out) { out->grid = grid; out->jobs_per_round = jmax; out->smem = g.total; }
     return true;
-}
-
-template <int TT, int SLOTS>
-static cudaError_t launch_fused_t(FusedArgs& a, const FusedLaunch& L, cudaStream_t stream) {
-    cudaError_t e = ensure_dynamic_smem((const void*)q4_fused_expert_kernel<TT, SLOTS>, FUSED_SMEM_LIMIT);
-    if (e != cudaSuccess) return e;
-    return launch_pdl(q4_fused_expert_kernel<TT, SLOTS>, dim3(L.grid), dim3(16 * SLOTS), L.smem, stream, a);
 }
 
 cudaError_t launch_q4_fused(const FusedArgs& args, cudaStream_t stream) {
     FusedLaunch L;
-    if (!q4_fused_plan(args.H, args.M, args.n_x, args.n_jobs_max, &L)) return cudaErrorInvalidValue;
-    if ((((uintptr_t)args.x) & 15) || ((args.x_stride * 4) & 15)) return cudaErrorInvalidValue;
+    if (!q4_fused_plan(args.H, args.M, args.n_jobs_max, &L)) return cudaErrorInvalidValue;
+    if (((uintptr_t)args.x) & 15) return cudaErrorInvalidValue;
     FusedArgs a = args;
     a.jobs_per_round = L.jobs_per_round;
-    if (L.tt == 1) return launch_fused_t<1, 40>(a, L, stream);
-    if (L.tt == 2) return launch_fused_t<2, 32>(a, L, stream);
-    return launch_fused_t<4, 32>(a, L, stream);
+    cudaError_t e = ensure_dynamic_smem((const void*)q4_fused_expert_kernel<LAYER_SLOTS>, FUSED_SMEM_LIMIT);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(q4_fused_expert_kernel<LAYER_SLOTS>, dim3(L.grid), dim3(16 * LAYER_SLOTS), L.smem, stream, a);
 }
 
 bool q4_layer_decode_plan(int H, int M, int E, int topk, int n_jobs_max, FusedLaunch* out) {
     FusedLaunch L;
-    if (!q4_fused_plan(H, M, 1, n_jobs_max, &L) || L.tt != 1 || H > 16 * LAYER_SLOTS * LAYER_NV || (H & 3) || E < 1 ||
+    if (!q4_fused_plan(H, M, n_jobs_max, &L) || H > 16 * LAYER_SLOTS * LAYER_NV || (H & 3) || E < 1 ||
         E > 1024 || topk < 1 || topk > 64 || topk > E)
         return false;
-    const FusedGeom g = fused_geom(H, M, 1, LAYER_SLOTS);
+    const FusedGeom g = fused_geom(H, M, LAYER_SLOTS);
     if ((size_t)layer_scratch(H, E, topk).end * 4 > g.off_sgu) return false;    // the scratch overlays the weight rows only
     if (out) *out = L;
     return true;
@@ -958,7 +884,6 @@ cudaError_t launch_q4_layer_decode(const LayerDecodeArgs& args, int n_jobs_max, 
     if (e != cudaSuccess) return e;
     LayerDecodeArgs a = args;
     a.f.jobs_per_round = L.jobs_per_round;
-    a.f.n_x = 1;
     return launch_pdl(q4_layer_decode_kernel, dim3(L.grid), dim3(16 * LAYER_SLOTS), L.smem, stream, a);
 }
 

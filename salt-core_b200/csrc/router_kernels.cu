@@ -854,6 +854,27 @@ cudaError_t launch_router_topk(const float* logits, const float* per_expert_scal
     return cudaGetLastError();
 }
 
+// The two projection jobs of grouped rows [g0, g0 + cnt) of expert e.
+static __device__ __forceinline__ void write_expert_jobs(const MoePlanArgs& a, int e, int g0, int cnt, int slot) {
+    const uint8_t* base = a.pool + (size_t)e * a.expert_stride;
+    Q4Job gu;
+    gu.vals = base; gu.scales = base + a.value_bytes; gu.biases = base + a.value_bytes + a.group_bytes;
+    gu.vals2 = base + a.tensor_bytes; gu.scales2 = gu.vals2 + a.value_bytes;
+    gu.biases2 = gu.scales2 + a.group_bytes;
+    gu.x = a.x; gu.y = a.chain + (size_t)g0 * a.inter;
+    gu.x_rows = a.grouped_to_canonical + g0; gu.x_div = a.topk;
+    gu.R = a.inter; gu.C = a.hidden; gu.ntok = cnt; gu.x_stride = a.hidden; gu.y_stride = a.inter;
+    a.gateup_jobs[slot] = gu;
+    Q4Job dn;
+    dn.vals = base + 2 * a.tensor_bytes; dn.scales = dn.vals + a.value_bytes;
+    dn.biases = dn.scales + a.group_bytes;
+    dn.vals2 = nullptr; dn.scales2 = nullptr; dn.biases2 = nullptr;
+    dn.x = a.chain + (size_t)g0 * a.inter; dn.y = a.grouped_out + (size_t)g0 * a.hidden;
+    dn.x_rows = nullptr; dn.x_div = 1;
+    dn.R = a.hidden; dn.C = a.inter; dn.ntok = cnt; dn.x_stride = a.inter; dn.y_stride = a.hidden;
+    a.down_jobs[slot] = dn;
+}
+
 // ---- grouping ---------------------------------------------------------------
 // Stable counting sort of the selections by expert (src/tensorops.c:239-289,
 // src/moe_group.c:83-161): grouped order = expert ascending, then canonical
@@ -965,36 +986,56 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(MoePlanArgs a) {
     }
     if (a.fused_done != nullptr && threadIdx.x < FUSED_MAX_JOBS) a.fused_done[threadIdx.x] = 0;
     __syncthreads();               // the placement is complete: the descriptors below read it back
+    if (a.pass_tokens > 0) {
+        // one job per pass of up to pass_tokens tokens, the largest passes first: their cost is proportional to
+        // their tokens, and with whole groups as jobs the SMs that drew the popular experts finished last (B = 64:
+        // a third of the SM time idle)
+        __shared__ int s_class[32];
+        int* first = hist;         // [E] job index of the expert's first full pass
+        int* rest = hist + E;      // [E] ... of its last, shorter one
+        const int P = a.pass_tokens;   // < 32
+        if (threadIdx.x < 32) s_class[threadIdx.x] = 0;
+        __syncthreads();
+        for (int e = threadIdx.x; e < E; e += blockDim.x)
+            if (act[e] >= 0) {
+                const int cnt = offs[e + 1] - offs[e];
+                if (cnt / P) atomicAdd(&s_class[0], cnt / P);
+                if (cnt % P) atomicAdd(&s_class[P - cnt % P], 1);
+            }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int run = 0;
+            for (int k = 0; k < P; k++) { const int c = s_class[k]; s_class[k] = run; run += c; }
+            *a.n_active = run;
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < E; e += blockDim.x)
+            if (act[e] >= 0) {
+                const int cnt = offs[e + 1] - offs[e];
+                if (cnt / P) first[e] = atomicAdd(&s_class[0], cnt / P);
+                if (cnt % P) rest[e] = atomicAdd(&s_class[P - cnt % P], 1);
+            }
+        __syncthreads();
+        for (int e = warp; e < E; e += 32) {
+            if (act[e] < 0) continue;
+            const int cnt = offs[e + 1] - offs[e];
+            for (int p = lane; p * P < cnt; p += 32)
+                write_expert_jobs(a, e, offs[e] + p * P, min(P, cnt - p * P), (p + 1) * P <= cnt ? first[e] + p : rest[e]);
+        }
+        return;
+    }
     // job descriptors for the local, non-empty experts (ascending expert order)
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
         const int slot = act[e];
         if (slot < 0) continue;
         const int g0 = offs[e], cnt = offs[e + 1] - offs[e];
-        const uint8_t* base = a.pool + (size_t)e * a.expert_stride;
-        Q4Job gu;
-        gu.vals = base; gu.scales = base + a.value_bytes; gu.biases = base + a.value_bytes + a.group_bytes;
-        gu.vals2 = base + a.tensor_bytes; gu.scales2 = gu.vals2 + a.value_bytes;
-        gu.biases2 = gu.scales2 + a.group_bytes;
-        gu.x = a.x; gu.y = a.chain + (size_t)g0 * a.inter;
-        gu.x_rows = a.grouped_to_canonical + g0; gu.x_div = a.topk;
-        gu.R = a.inter; gu.C = a.hidden; gu.ntok = cnt; gu.x_stride = a.hidden; gu.y_stride = a.inter;
-        a.gateup_jobs[slot] = gu;
-        Q4Job dn;
-        dn.vals = base + 2 * a.tensor_bytes; dn.scales = dn.vals + a.value_bytes;
-        dn.biases = dn.scales + a.group_bytes;
-        dn.vals2 = nullptr; dn.scales2 = nullptr; dn.biases2 = nullptr;
-        dn.x = a.chain + (size_t)g0 * a.inter; dn.y = a.grouped_out + (size_t)g0 * a.hidden;
-        dn.x_rows = nullptr; dn.x_div = 1;
-        dn.R = a.hidden; dn.C = a.inter; dn.ntok = cnt; dn.x_stride = a.inter; dn.y_stride = a.hidden;
-        a.down_jobs[slot] = dn;
+        write_expert_jobs(a, e, g0, cnt, slot);
         if (a.fused_jobs != nullptr && slot < FUSED_MAX_JOBS) {
             FusedJob fj;
-            fj.v[0] = gu.vals; fj.v[1] = gu.vals2; fj.v[2] = dn.vals;
+            for (int k = 0; k < 3; k++) fj.v[k] = a.pool + (size_t)e * a.expert_stride + k * a.tensor_bytes;
             for (int k = 0; k < 3; k++)
                 fj.t[k] = (const uint32_t*)(a.fused_tables + ((size_t)e * 6 + 2 * k) * a.group_bytes);
-            for (int t = 0; t < FUSED_MAX_TOKENS; t++)
-                fj.x_row[t] = a.grouped_to_canonical[g0 + min(t, cnt - 1)] / a.topk;
-            fj.g0 = g0; fj.ntok = cnt; fj.lit = a.fused_lit[e]; fj.pad = 0;
+            fj.g0 = g0; fj.lit = a.fused_lit[e];
             a.fused_jobs[slot] = fj;
         }
     }
@@ -1011,7 +1052,7 @@ __global__ void __launch_bounds__(512) moe_plan_small_kernel(MoePlanArgs a) {
     const int E = a.n_experts;
     pdl_wait();                    // the logits come from the previous kernel
     pdl_launch_dependents();
-    __shared__ int s_sel[32], s_first[32], s_g2c[32];
+    __shared__ int s_sel[32], s_first[32];
     if (a.fused_done != nullptr && threadIdx.x < FUSED_MAX_JOBS) a.fused_done[threadIdx.x] = 0;
     {
         float* tk = (float*)sp;
@@ -1039,7 +1080,6 @@ __global__ void __launch_bounds__(512) moe_plan_small_kernel(MoePlanArgs a) {
         if (e >= 0) {
             a.grouped_to_canonical[before] = lane;
             a.canonical_to_grouped[lane] = before;
-            s_g2c[before] = lane;
         }
         s_sel[lane] = e;
         s_first[lane] = (e >= 0 && first) ? 1 : 0;
@@ -1059,31 +1099,13 @@ __global__ void __launch_bounds__(512) moe_plan_small_kernel(MoePlanArgs a) {
         a.group_offsets[e] = e < E ? lt : valid;
         if (e == E || eq == 0 || e < a.expert_begin || e >= a.expert_end) continue;
         const int g0 = lt, cnt = eq;
-        const uint8_t* base = a.pool + (size_t)e * a.expert_stride;
-        Q4Job gu;
-        gu.vals = base; gu.scales = base + a.value_bytes; gu.biases = base + a.value_bytes + a.group_bytes;
-        gu.vals2 = base + a.tensor_bytes; gu.scales2 = gu.vals2 + a.value_bytes;
-        gu.biases2 = gu.scales2 + a.group_bytes;
-        gu.x = a.x; gu.y = a.chain + (size_t)g0 * a.inter;
-        gu.x_rows = a.grouped_to_canonical + g0; gu.x_div = a.topk;
-        gu.R = a.inter; gu.C = a.hidden; gu.ntok = cnt; gu.x_stride = a.hidden; gu.y_stride = a.inter;
-        a.gateup_jobs[slot] = gu;
-        Q4Job dn;
-        dn.vals = base + 2 * a.tensor_bytes; dn.scales = dn.vals + a.value_bytes;
-        dn.biases = dn.scales + a.group_bytes;
-        dn.vals2 = nullptr; dn.scales2 = nullptr; dn.biases2 = nullptr;
-        dn.x = a.chain + (size_t)g0 * a.inter; dn.y = a.grouped_out + (size_t)g0 * a.hidden;
-        dn.x_rows = nullptr; dn.x_div = 1;
-        dn.R = a.hidden; dn.C = a.inter; dn.ntok = cnt; dn.x_stride = a.inter; dn.y_stride = a.hidden;
-        a.down_jobs[slot] = dn;
+        write_expert_jobs(a, e, g0, cnt, slot);
         if (a.fused_jobs != nullptr && slot < FUSED_MAX_JOBS) {
             FusedJob fj;
-            fj.v[0] = gu.vals; fj.v[1] = gu.vals2; fj.v[2] = dn.vals;
+            for (int k = 0; k < 3; k++) fj.v[k] = a.pool + (size_t)e * a.expert_stride + k * a.tensor_bytes;
             for (int k = 0; k < 3; k++)
                 fj.t[k] = (const uint32_t*)(a.fused_tables + ((size_t)e * 6 + 2 * k) * a.group_bytes);
-            for (int t = 0; t < FUSED_MAX_TOKENS; t++)
-                fj.x_row[t] = s_g2c[g0 + min(t, cnt - 1)] / a.topk;
-            fj.g0 = g0; fj.ntok = cnt; fj.lit = a.fused_lit[e]; fj.pad = 0;
+            fj.g0 = g0; fj.lit = a.fused_lit[e];
             a.fused_jobs[slot] = fj;
         }
     }

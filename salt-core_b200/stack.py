@@ -109,7 +109,7 @@ class MoeStack:
         return tuple(int(v or 0) for v in b)
 
     def set_fused_decode(self, enable):
-        """Batches of up to 4 tokens: one-launch expert kernel (default) or the two-launch form."""
+        """Single tokens: one-launch kernels (default) or the two-launch form."""
         level = int(enable)                                   # 0 phase kernels, 1 one launch per layer, 2 one per pass
         return self.lib.salt_b200_stack_set_fused_decode(self.handle, level)
 

@@ -573,12 +573,12 @@ def run_b200(args):
             else:
                 alg = mean_distinct * 2 * TENSOR_BYTES + B * H * 4 + B * K * M * 4
                 kname = ("q4_gemm_tc_kernel<fused> (tcgen05 gate/up + GeGLU)" if tc_mode
-                         else "q4_batch_kernel<2,RL> / q4_fused_expert_kernel (gate/up + GeGLU)")
+                         else "batch_kernel<Q4, 2> / q4_fused_expert_kernel (gate/up + GeGLU)")
                 if fmt == "nvfp4":
                     # the class brackets the whole NVFP4 expert phase of a layer (five launches)
                     alg = mean_distinct * 3 * TENSOR_BYTES + B * H * 4 + B * K * (2 * H + 4 * M) * 4
-                    kname = ("NVFP4 expert phase of a layer: plan, activation quantise-dequantise, nvfp4_tile_kernel "
-                             "gate + up, GeGLU + quantise-dequantise, nvfp4_tile_kernel down (five launches)")
+                    kname = ("NVFP4 expert phase of a layer: plan, activation quantise-dequantise, batch_kernel "
+                             "gate + up, GeGLU + quantise-dequantise, batch_kernel down (five launches)")
                     if tc_mode:
                         kname = ("NVFP4 expert phase of a layer: plan, activation quantise, nvfp4_gemm_tc_kernel "
                                  "(tcgen05.mma.kind::mxf4nvf4 block-scaled) gate + up, GeGLU + quantise, "

@@ -1,4 +1,5 @@
-// Affine-Q4 projections of jobs of any number of tokens, exact (the reference row DAG of q4_core.cuh).
+// Affine-Q4 and NVFP4 projections of jobs of any number of tokens, exact (the reference row DAG of q4_core.cuh; NVFP4:
+// reference src/nvfp4.c:157-192, the same 32 accumulators over dequantised activations).
 //
 // What bounds this work is not HBM: a weight element costs one product and one add per token (the reference
 // rounds between them, so they cannot fuse), and at decode batches the activations that feed those two
@@ -11,7 +12,8 @@
 //     row, and the activations of the tokens of the pass), filled by 16-byte cp.async; the weight rows of a stage
 //     are 128 bytes apart and their 16-byte pieces are permuted by the row index, so the four rows a warp reads
 //     together never share a bank.
-//   * (scale << 16) | bias words of all rows of the tile are interleaved once per tile.
+//   * Q4: (scale << 16) | bias words of all rows of the tile are interleaved once per tile.  NVFP4: the block scales
+//     of a chunk travel with it and index the 256 products fl(E4M3 code * global scale).
 //   * A block takes up to four tokens of the group (its pass), with code specialised for 1, 2, 3 and 4; the passes of
 //     a large group are blocks of their own, so that popular experts do not finish last.
 //   * Dequantisation: a nibble masked at bits 16..19 (12..15) and OR-ed with the exponent of 2^7 (2^11) IS the
@@ -23,7 +25,9 @@
 // What bounds it now: issue cycles.  A packed or a logic operation holds a scheduler for two cycles; per row, lane and
 // 32-column step a token takes 16 of them, the dequantisation 20.  Measured (hidden 2816, inter 704, 128 experts,
 // top-8; gate/up + down of a layer): 64 tokens 698 -> 438 us, 16 tokens 274 -> 175 us, 6 tokens 140 -> 98 us against
-// two rows per lane and whole groups as blocks; 2 tokens 50 us, where one persistent launch for both phases took 51.
+// two rows per lane and whole groups as blocks; 2 tokens 46 us, where one persistent launch for both phases took 51.
+// NVFP4 (hidden 5120, inter 1536, 64 experts, top-4; expert phase of a layer): 1 token 71 -> 51 us, 16 tokens 640 -> 291.
+#include "fp4_core.cuh"
 #include "internal.h"
 #include "pdl.cuh"
 #include "q4_core.cuh"
@@ -42,26 +46,34 @@ constexpr int MAX_T = Q4_PASS_TOKENS;       // tokens per pass
 constexpr int FOLD_BYTES = 4 * 8 * 16;       // fold area of a warp's four rows: eight float4 each
 constexpr int WARPS = 4, NT = 32 * WARPS;
 
-// Shared memory of a block: ring of stages | fold areas (one per warp) | scale-bias table.  The raw scales and
-// biases land where the last stage and the fold areas will be; they are gone before either is used.
+enum { FMT_Q4 = 0, FMT_FP4 = 1 };
+enum { STEP_Q4 = 0, STEP_Q4_LITERAL = 1, STEP_FP4 = 2 };   // dequantisation of the inner loop
+
+// Shared memory of a block: ring of stages | fold areas (one per warp) | table.  Stage: 128 bytes of every weight row,
+// 256 columns of every token and, for NVFP4, 16 block scales of every row.  Table: (scale << 16) | bias words of the
+// rows, or the 256 products fl(E4M3 code * global scale).  The raw Q4 scales and biases land where the last stage and
+// the fold areas will be; they are gone before either is used.
 struct BatchGeom {
     int rows, tpitch, raw_pitch, raw_block;
-    uint32_t stage_bytes, fold_off, table_off, raw_off, smem;
+    uint32_t x_off, sc_off, stage_bytes, fold_off, table_off, raw_off, smem;
 };
-__host__ __device__ inline BatchGeom batch_geom(int C, int nmat, int rl, int stages) {
-    const int warps = WARPS;
+__host__ __device__ inline BatchGeom batch_geom(int fmt, int C, int nmat, int rl) {
     BatchGeom g;
-    g.rows = warps * 4 * rl;
+    g.rows = WARPS * 4 * rl;
     g.tpitch = (C >> 6) + ((C >> 6) % 16 == 0 ? 1 : 0);   // the four rows a warp reads together fall in different banks
     g.raw_pitch = C >> 5;                   // bytes of bf16 scales per row
     g.raw_block = (g.rows / nmat * g.raw_pitch + 15) & ~15;
-    g.stage_bytes = (uint32_t)(g.rows * CH_BYTES + MAX_T * CH_COLS * 4);
-    g.fold_off = g.stage_bytes * stages;
-    g.raw_off = g.stage_bytes * (stages - 1);
-    const uint32_t fold_end = g.fold_off + (uint32_t)(warps * rl * FOLD_BYTES);
-    const uint32_t raw_end = g.raw_off + (uint32_t)(2 * nmat * g.raw_block);
+    g.x_off = (uint32_t)(g.rows * CH_BYTES);
+    g.sc_off = g.x_off + MAX_T * CH_COLS * 4;
+    g.stage_bytes = g.sc_off + (fmt == FMT_FP4 ? (uint32_t)g.rows * 16 : 0u);
+    g.fold_off = g.stage_bytes * STAGES;
+    g.raw_off = g.stage_bytes * (STAGES - 1);
+    const uint32_t fold_end = g.fold_off + (uint32_t)(WARPS * rl * FOLD_BYTES);
+    const uint32_t raw_end = fmt == FMT_FP4 ? 0u : g.raw_off + (uint32_t)(2 * nmat * g.raw_block);
     g.table_off = fold_end > raw_end ? fold_end : raw_end;
-    g.smem = g.table_off + (uint32_t)(g.rows * g.tpitch * 4);
+    const uint32_t table = fmt == FMT_FP4 ? 1024u : (uint32_t)(g.rows * g.tpitch * 4);
+    const uint32_t out = (uint32_t)(MAX_T * g.rows * 4);    // the results of a block pass through the table's space
+    g.smem = g.table_off + (table > out ? table : out);
     return g;
 }
 
@@ -124,6 +136,38 @@ __device__ __forceinline__ void group_step(const uint8_t* w, uint32_t o0, uint32
     }
 }
 
+// Two 32-column steps of NVFP4 rows: w = fl(code * fl(scale * global)), one scale per 16 columns.  The hardware decodes
+// the code 8 as -0 where the reference's table has +0 (src/nvfp4.c:19-23): as a weight that cannot change a result (the
+// product is a zero of either sign, and an accumulator that starts at +0 never becomes -0).
+template <int RL, int T>
+__device__ __forceinline__ void group_step_fp4(const uint8_t* w, uint32_t o0, uint32_t o1, const uint8_t* sc, const float* lut,
+                                               const float* x, f32x2 (&acc)[RL][T][2], f32x2 nz) {
+    constexpr int ISTEP = RL == 4 ? 8 : 16;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+        f32x2 x01[T], x23[T];
+#pragma unroll
+        for (int t = 0; t < T; t++) {
+            const ulonglong2 xv = *(const ulonglong2*)(x + t * CH_COLS + half * 32);
+            x01[t] = xv.x;
+            x23[t] = xv.y;
+        }
+#pragma unroll
+        for (int i = 0; i < RL; i++) {
+            const uint32_t h = *(const uint16_t*)(w + (half ? o1 : o0) + i * ISTEP * CH_BYTES);
+            const float s = lut[sc[i * ISTEP * 16 + 2 * half]];
+            float c[4];
+            e2m1x4(h, c);
+            const f32x2 d01 = pack2(__fmul_rn(c[0], s), __fmul_rn(c[1], s)), d23 = pack2(__fmul_rn(c[2], s), __fmul_rn(c[3], s));
+#pragma unroll
+            for (int t = 0; t < T; t++) {
+                product_then_add(acc[i][t][0], d01, x01[t], nz);
+                product_then_add(acc[i][t][1], d23, x23[t], nz);
+            }
+        }
+    }
+}
+
 // The lane's global row of shared row `sr` (NMAT == 2: sixteen gate rows, then the same sixteen up rows, and so on).
 template <int NMAT>
 __device__ __forceinline__ int tile_row(int sr) {
@@ -132,11 +176,12 @@ __device__ __forceinline__ int tile_row(int sr) {
 
 // Fold and store one pass of T tokens.  acc[i]: shared row sr0 + ISTEP i, tokens t.
 template <int NMAT, int RL, int T>
-__device__ __forceinline__ void finish_pass(const Q4Job& jb, int r0, int nvalid, int tb, float4* fold, int sr0,
-                                            const f32x2 (&acc)[RL][T][2]) {
+__device__ __forceinline__ void finish_pass(const Q4Job& jb, int r0, int nvalid, int tb, float4* fold, float* out,
+                                            int sr0, const f32x2 (&acc)[RL][T][2]) {
     constexpr int LPR = 8 / RL, ISTEP = RL == 4 ? 8 : 16;    // lanes per row of the warp
+    static_assert(RL == 2 || RL == 4, "half of a lane's rows are gate rows, the others the up rows of the same outputs");
     const int lane = threadIdx.x & 31, u = lane & 7, lrow = lane >> 3;
-    const int rr = lane / LPR, par = lane % LPR;             // this lane runs chains par, par + LPR, ... of row rr
+    const int rr = lane / LPR, par = lane % LPR;             // this lane runs chain par and, with two lanes, par + 2
     float y[T];
 #pragma unroll
     for (int t = 0; t < T; t++) {
@@ -180,12 +225,16 @@ __device__ __forceinline__ void finish_pass(const Q4Job& jb, int r0, int nvalid,
         if (tok < T && row < nvalid && (LPR == 2 || lane < 16))
             jb.y[(size_t)(tb + tok) * jb.y_stride + r0 + row] = __fmul_rn(gelu_tanh_exact(gate), up);
     } else {
+        // through the (now unused) table, so that whole lines leave the block: the rows may be in host memory
+        constexpr int ROWS = WARPS * 4 * RL;
         const int row = sr_w + ISTEP * (rr >> 2) + (rr & 3);
-        if (row < nvalid) {
+        __syncthreads();
 #pragma unroll
-            for (int t = 0; t < T; t++)
-                if (t % LPR == par) jb.y[(size_t)(tb + t) * jb.y_stride + r0 + row] = y[t];
-        }
+        for (int t = 0; t < T; t++)
+            if (t % LPR == par) out[t * ROWS + row] = y[t];
+        __syncthreads();
+        for (int i = threadIdx.x; i < T * ROWS; i += NT)
+            if (i % ROWS < nvalid) jb.y[(size_t)(tb + i / ROWS) * jb.y_stride + r0 + i % ROWS] = out[i];
     }
 }
 
@@ -195,14 +244,14 @@ __device__ __forceinline__ void finish_pass(const Q4Job& jb, int r0, int nvalid,
 template <int NMAT, int RL>
 struct Loader {
     static constexpr int RSTEP = NT / 8, ROWS = WARPS * 4 * RL;
-    static_assert(RSTEP == 16, "even k = gate rows, odd k = up rows");
+    static_assert(RSTEP == 16 && ROWS % 16 == 0, "even k = gate rows, odd k = up rows");
     const Q4Job& jb;                 // in shared memory, as are the activation rows: registers are what is short
     const float* const* rows;        // [ntok]
     const uint8_t* src;              // this thread's piece of chunk 0 in its first row
-    int below, ch, ntok, steps;      // rows below the first one; next chunk
+    int r0, below, ch, ntok, steps;  // first row of the tile; rows below this thread's first one; next chunk
 
-    __device__ __forceinline__ Loader(const Q4Job& j, const float* const* rows_, int r0, int C, int ntok_)
-        : jb(j), rows(rows_), ch(0), ntok(ntok_), steps(C >> 5) {
+    __device__ __forceinline__ Loader(const Q4Job& j, const float* const* rows_, int r0_, int C, int ntok_)
+        : jb(j), rows(rows_), r0(r0_), ch(0), ntok(ntok_), steps(C >> 5) {
         const int row = min(r0 + (int)(threadIdx.x >> 3), jb.R - 1);
         below = jb.R - 1 - row;
         src = jb.vals + (size_t)row * (C >> 1) + (threadIdx.x & 7) * 16;
@@ -220,17 +269,34 @@ struct Loader {
             cp_async16(dst + k * RSTEP * CH_BYTES, p + (size_t)(down * steps) * 16 + (NMAT == 2 && (k & 1) ? second : 0));
         }
     }
+    __device__ __forceinline__ void block_scales(uint8_t* stage) const {    // NVFP4: 16 per row and chunk
+        if (threadIdx.x < ROWS) {
+            const int row = min(r0 + (int)threadIdx.x, jb.R - 1);
+            cp_async16(stage + threadIdx.x * 16, jb.scales + (size_t)row * (steps * 2) + ch * 16);
+        }
+    }
     __device__ __forceinline__ void activations(uint8_t* stage) const {
 #pragma unroll
         for (int k = 0; k < (MAX_T * 64 + NT - 1) / NT; k++) {
             const int idx = threadIdx.x + k * NT, t = idx >> 6, pc = idx & 63;
             if (t < ntok && pc < (steps - ch * CH_STEPS) * 8)
-                cp_async16(stage + ROWS * CH_BYTES + idx * 16, rows[t] + ch * CH_COLS + pc * 4);
+                cp_async16(stage + idx * 16, rows[t] + ch * CH_COLS + pc * 4);
         }
     }
 };
 
-template <int NMAT, int RL, int T, bool LIT>
+template <int FMT, int NMAT, int RL>
+__device__ __forceinline__ void load_chunk(Loader<NMAT, RL>& ld, const BatchGeom& G, uint8_t* stage) {
+    if (ld.more()) {
+        ld.weights(stage);
+        ld.activations(stage + G.x_off);
+        if (FMT == FMT_FP4) ld.block_scales(stage + G.sc_off);
+        ld.ch++;
+    }
+    cp_async_commit();
+}
+
+template <int NMAT, int RL, int T, int STEP>
 __device__ __forceinline__ void run_pass(const Q4Job& jb, Loader<NMAT, RL>& ld, const BatchGeom& G, uint8_t* smem,
                                          int r0, int nvalid, int tb) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, u = lane & 7, lrow = lane >> 3;
@@ -249,18 +315,10 @@ __device__ __forceinline__ void run_pass(const Q4Job& jb, Loader<NMAT, RL>& ld, 
     for (int ch = 0; ch < nch; ch++) {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
         __syncthreads();                                    // the chunk has landed; everyone is done with the one before
-        {
-            const int fill = slot == 0 ? STAGES - 1 : slot - 1;
-            if (ld.more()) {
-                ld.weights(smem + fill * G.stage_bytes);
-                ld.activations(smem + fill * G.stage_bytes);
-                ld.ch++;
-            }
-            cp_async_commit();
-        }
-        const uint8_t* w = smem + slot * G.stage_bytes + sr0 * CH_BYTES + 2 * u;
-        const float* x = (const float*)(smem + slot * G.stage_bytes + WARPS * 4 * RL * CH_BYTES) + 4 * u;
-        const uint32_t* tg = tab + ch * (CH_COLS / 64);
+        load_chunk<STEP == STEP_FP4 ? FMT_FP4 : FMT_Q4, NMAT, RL>(ld, G, smem + (slot == 0 ? STAGES - 1 : slot - 1) * G.stage_bytes);
+        const uint8_t* stage = smem + slot * G.stage_bytes;
+        const uint8_t* w = stage + sr0 * CH_BYTES + 2 * u;
+        const float* x = (const float*)(stage + G.x_off) + 4 * u;
         const int live = min(CH_STEPS, steps - ch * CH_STEPS);
         // (one quantisation group per iteration: the four pass sizes of a layer's groups run side by side on an SM, and
         // with whole chunks unrolled their code did not fit the instruction cache)
@@ -268,26 +326,32 @@ __device__ __forceinline__ void run_pass(const Q4Job& jb, Loader<NMAT, RL>& ld, 
 #pragma unroll 2
         for (int g = 0; g < live / 2; g++) {
             const uint32_t o = ((uint32_t)g << 5) ^ r16;
-            group_step<RL, T, LIT>(w, o, o ^ 16u, tg + g, ISTEP * G.tpitch, x + g * 64, acc, m11, m7, nz);
+            if constexpr (STEP == STEP_FP4)
+                group_step_fp4<RL, T>(w, o, o ^ 16u, stage + G.sc_off + sr0 * 16 + 4 * g + (u >> 2),
+                                      (const float*)(smem + G.table_off), x + g * 64, acc, nz);
+            else
+                group_step<RL, T, STEP == STEP_Q4_LITERAL>(w, o, o ^ 16u, tab + ch * (CH_COLS / 64) + g, ISTEP * G.tpitch,
+                                                           x + g * 64, acc, m11, m7, nz);
         }
         slot = slot + 1 == STAGES ? 0 : slot + 1;
     }
-    finish_pass<NMAT, RL, T>(jb, r0, nvalid, tb, (float4*)(smem + G.fold_off + warp * RL * FOLD_BYTES), sr0, acc);
+    finish_pass<NMAT, RL, T>(jb, r0, nvalid, tb, (float4*)(smem + G.fold_off + warp * RL * FOLD_BYTES),
+                             (float*)(smem + G.table_off), sr0, acc);
 }
 
-template <int NMAT, int RL, bool LIT>
+template <int NMAT, int RL, int STEP>
 __device__ __forceinline__ void run_tokens(const Q4Job& jb, Loader<NMAT, RL>& ld, const BatchGeom& G, uint8_t* smem,
                                            int r0, int nvalid, int tb) {
-    if (ld.ntok == 4) run_pass<NMAT, RL, 4, LIT>(jb, ld, G, smem, r0, nvalid, tb);
-    else if (ld.ntok == 3) run_pass<NMAT, RL, 3, LIT>(jb, ld, G, smem, r0, nvalid, tb);
-    else if (ld.ntok == 2) run_pass<NMAT, RL, 2, LIT>(jb, ld, G, smem, r0, nvalid, tb);
-    else run_pass<NMAT, RL, 1, LIT>(jb, ld, G, smem, r0, nvalid, tb);
+    if (ld.ntok == 4) run_pass<NMAT, RL, 4, STEP>(jb, ld, G, smem, r0, nvalid, tb);
+    else if (ld.ntok == 3) run_pass<NMAT, RL, 3, STEP>(jb, ld, G, smem, r0, nvalid, tb);
+    else if (ld.ntok == 2) run_pass<NMAT, RL, 2, STEP>(jb, ld, G, smem, r0, nvalid, tb);
+    else run_pass<NMAT, RL, 1, STEP>(jb, ld, G, smem, r0, nvalid, tb);
 }
 
-// blockIdx: row tile, job, pass of the job's tokens
-template <int NMAT, int RL>
+// blockIdx: row tile, job (entry of the live list if there is one), pass of the job's tokens
+template <int FMT, int NMAT, int RL>
 __global__ void __launch_bounds__(NT, RL == 4 ? 4 : 6)
-q4_batch_kernel(const Q4Job* __restrict__ jobs, const int* __restrict__ njobs_dev, int C, int jobs_early) {
+batch_kernel(const void* __restrict__ jobs, const int* __restrict__ live, const int* __restrict__ njobs_dev, int C, int jobs_early) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int ROWS = 4 * RL * WARPS, ROWS_A = ROWS / NMAT;
     // jobs_early: the job table was written at least two launches back, so everything except the activation rows
@@ -299,35 +363,50 @@ q4_batch_kernel(const Q4Job* __restrict__ jobs, const int* __restrict__ njobs_de
     const int njobs_live = njobs_dev != nullptr ? __ldcg(njobs_dev) : 0x7fffffff;
     if ((int)blockIdx.y >= njobs_live) return;
     __shared__ __align__(16) Q4Job jb;
-    if (threadIdx.x < sizeof(Q4Job) / 16) ((uint4*)&jb)[threadIdx.x] = __ldcg((const uint4*)(jobs + blockIdx.y) + threadIdx.x);
+    float wg = 0.0f;
+    if (FMT == FMT_FP4) {                                   // the same descriptor in the shared form
+        const Fp4Job& f = ((const Fp4Job*)jobs)[live != nullptr ? live[blockIdx.y] : (int)blockIdx.y];
+        wg = f.wg;
+        if (threadIdx.x == 0) {
+            jb.vals = f.codes; jb.scales = f.scales; jb.x = f.x; jb.y = f.y; jb.x_rows = nullptr;
+            jb.R = f.R; jb.ntok = f.ntok; jb.x_stride = f.x_stride; jb.y_stride = f.y_stride;
+        }
+    } else if (threadIdx.x < sizeof(Q4Job) / 16) {
+        ((uint4*)&jb)[threadIdx.x] = __ldcg((const uint4*)((const Q4Job*)jobs + blockIdx.y) + threadIdx.x);
+    }
     __syncthreads();
     const int r0 = blockIdx.x * ROWS_A, tb = blockIdx.z * MAX_T;
     if (r0 >= jb.R || tb >= jb.ntok) return;
     const int nvalid = min(ROWS_A, jb.R - r0), tid = threadIdx.x;
-    const BatchGeom G = batch_geom(C, NMAT, RL, STAGES);
+    const BatchGeom G = batch_geom(FMT, C, NMAT, RL);
     __shared__ const float* x_row[MAX_T];
     Loader<NMAT, RL> ld(jb, x_row, r0, C, min(MAX_T, jb.ntok - tb));
 
-    // first stages: weights, raw scales and biases, then (after the dependency) activations
+    // first stages: weights and scales, then (after the dependency) activations
     ld.weights(smem);
+    if (FMT == FMT_FP4) {
+        ld.block_scales(smem + G.sc_off);
+        for (int c = tid; c < 256; c += NT) ((float*)(smem + G.table_off))[c] = __fmul_rn(e4m3_decode((uint32_t)c), wg);
+    } else {
 #pragma unroll
-    for (int m = 0; m < NMAT; m++) {
-        const uint8_t* gs = (m == 0 ? jb.scales : jb.scales2) + (size_t)r0 * G.raw_pitch;
-        const uint8_t* gb = m == 0 ? jb.biases : jb.biases2;
-        uint8_t* ds = smem + G.raw_off + 2 * m * G.raw_block;
-        uint8_t* db = ds + G.raw_block;
-        const int total = nvalid * G.raw_pitch, full = total >> 4;
-        if (gb) gb += (size_t)r0 * G.raw_pitch;
-        for (int p = tid; p < full; p += NT) {
-            cp_async16(ds + p * 16, gs + p * 16);
-            if (gb) cp_async16(db + p * 16, gb + p * 16);
+        for (int m = 0; m < NMAT; m++) {
+            const uint8_t* gs = (m == 0 ? jb.scales : jb.scales2) + (size_t)r0 * G.raw_pitch;
+            const uint8_t* gb = m == 0 ? jb.biases : jb.biases2;
+            uint8_t* ds = smem + G.raw_off + 2 * m * G.raw_block;
+            uint8_t* db = ds + G.raw_block;
+            const int total = nvalid * G.raw_pitch, full = total >> 4;
+            if (gb) gb += (size_t)r0 * G.raw_pitch;
+            for (int p = tid; p < full; p += NT) {
+                cp_async16(ds + p * 16, gs + p * 16);
+                if (gb) cp_async16(db + p * 16, gb + p * 16);
+            }
+            for (int i = (full << 4) + 2 * tid; i < total; i += 2 * NT) {
+                *(uint16_t*)(ds + i) = *(const uint16_t*)(gs + i);
+                if (gb) *(uint16_t*)(db + i) = *(const uint16_t*)(gb + i);
+            }
+            if (!gb)
+                for (int i = tid; i < G.raw_block / 4; i += NT) ((uint32_t*)db)[i] = 0u;
         }
-        for (int i = (full << 4) + 2 * tid; i < total; i += 2 * NT) {
-            *(uint16_t*)(ds + i) = *(const uint16_t*)(gs + i);
-            if (gb) *(uint16_t*)(db + i) = *(const uint16_t*)(gb + i);
-        }
-        if (!gb)
-            for (int i = tid; i < G.raw_block / 4; i += NT) ((uint32_t*)db)[i] = 0u;
     }
     if (jobs_early) {
         pdl_wait();
@@ -338,23 +417,18 @@ q4_batch_kernel(const Q4Job* __restrict__ jobs, const int* __restrict__ njobs_de
         x_row[tid] = jb.x + (size_t)row * jb.x_stride;
     }
     __syncthreads();
-    ld.activations(smem);
+    ld.activations(smem + G.x_off);
     ld.ch++;
     cp_async_commit();
 #pragma unroll
-    for (int k = 1; k < STAGES - 1; k++) {
-        if (ld.more()) {
-            ld.weights(smem + k * G.stage_bytes);
-            ld.activations(smem + k * G.stage_bytes);
-            ld.ch++;
-        }
-        cp_async_commit();
-    }
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
-    __syncthreads();
-    // interleave scales and biases; does any group need the two-rounding dequantisation?
-    int lit = 0;
-    {
+    for (int k = 1; k < STAGES - 1; k++) load_chunk<FMT, NMAT, RL>(ld, G, smem + k * G.stage_bytes);
+    if constexpr (FMT == FMT_FP4) {
+        run_tokens<NMAT, RL, STEP_FP4>(jb, ld, G, smem, r0, nvalid, tb);
+    } else {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();
+        // interleave scales and biases; does any group need the two-rounding dequantisation?
+        int lit = 0;
         uint32_t* table = (uint32_t*)(smem + G.table_off);
         const int gpr = C >> 6;
         for (int sr = tid >> 3; sr < ROWS; sr += NT / 8) {
@@ -372,43 +446,54 @@ q4_batch_kernel(const Q4Job* __restrict__ jobs, const int* __restrict__ njobs_de
                 table[sr * G.tpitch + g] = (hs << 16) | hb;
             }
         }
+        lit = __syncthreads_or(lit);
+        if (lit) run_tokens<NMAT, RL, STEP_Q4_LITERAL>(jb, ld, G, smem, r0, nvalid, tb);
+        else run_tokens<NMAT, RL, STEP_Q4>(jb, ld, G, smem, r0, nvalid, tb);
     }
-    lit = __syncthreads_or(lit);
-    if (lit) run_tokens<NMAT, RL, true>(jb, ld, G, smem, r0, nvalid, tb);
-    else run_tokens<NMAT, RL, false>(jb, ld, G, smem, r0, nvalid, tb);
 }
 
-template <int NMAT, int RL>
-cudaError_t launch_batch(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
-                         cudaStream_t stream, int pdl) {
-    const BatchGeom G = batch_geom(C, NMAT, RL, STAGES);
-    cudaError_t e = ensure_dynamic_smem((const void*)q4_batch_kernel<NMAT, RL>, G.smem);
+template <int FMT, int NMAT, int RL>
+cudaError_t launch_batch(const void* jobs, int njobs_max, const int* live, const int* njobs_dev, int max_rows, int max_tok,
+                         int C, cudaStream_t stream, int pdl) {
+    const BatchGeom G = batch_geom(FMT, C, NMAT, RL);
+    cudaError_t e = ensure_dynamic_smem((const void*)batch_kernel<FMT, NMAT, RL>, G.smem);
     if (e != cudaSuccess) return e;
     constexpr int ROWS_A = 4 * RL * WARPS / NMAT;
     const dim3 grid((max_rows + ROWS_A - 1) / ROWS_A, njobs_max, (max_tok + MAX_T - 1) / MAX_T);
     if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
     if (pdl >= 0)
-        return launch_pdl(q4_batch_kernel<NMAT, RL>, grid, dim3(NT), (size_t)G.smem, stream, jobs, njobs_dev, C, pdl);
-    q4_batch_kernel<NMAT, RL><<<grid, NT, G.smem, stream>>>(jobs, njobs_dev, C, 0);
+        return launch_pdl(batch_kernel<FMT, NMAT, RL>, grid, dim3(NT), (size_t)G.smem, stream, jobs, live, njobs_dev, C, pdl);
+    batch_kernel<FMT, NMAT, RL><<<grid, NT, G.smem, stream>>>(jobs, live, njobs_dev, C, 0);
     return cudaGetLastError();
 }
 
+// Rows per lane.  Four need a quarter of the shared loads per product; two make twice as many blocks, which start and
+// end more evenly: better below about thirteen blocks per SM (2 tokens of the layer above 76 -> 72 us; one 4096 x 4096
+// row product from the host 62 -> 51).  One row per lane was slower still.  `blocks`: of four rows per lane.
+bool two_rows_per_lane(long blocks) { return blocks < 13 * 148; }
+
 }  // namespace
 
-bool q4_batch_supported(int C, int nmat) { return C >= 64 && (C % 64) == 0 && batch_geom(C, nmat, 4, STAGES).smem <= 225 * 1024; }
+bool q4_batch_supported(int C, int nmat) { return C >= 64 && (C % 64) == 0 && batch_geom(FMT_Q4, C, nmat, 4).smem <= 225 * 1024; }
 
 cudaError_t launch_q4_batch(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
                             int nmat, cudaStream_t stream, int pdl) {
-    // Four rows per lane need a quarter of the shared loads per product; two rows per lane make twice the blocks.
-    // Below about thirteen blocks per SM (three rounds of the four resident ones) the shorter blocks win: they start
-    // and end more evenly (2 tokens of the layer above 76 -> 72 us, one 4096 x 4096 row product from the host 62 -> 51).
     const long blocks = (long)((max_rows + 64 / nmat - 1) / (64 / nmat)) * njobs_max * ((max_tok + MAX_T - 1) / MAX_T);
-    if (blocks < 13 * 148) {
-        if (nmat == 2) return launch_batch<2, 2>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, pdl);
-        return launch_batch<1, 2>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, pdl);
-    }
-    if (nmat == 2) return launch_batch<2, 4>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, pdl);
-    return launch_batch<1, 4>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, pdl);
+    const bool two = two_rows_per_lane(blocks);
+#define SB_BATCH(NM, RL) launch_batch<FMT_Q4, NM, RL>(jobs, njobs_max, nullptr, njobs_dev, max_rows, max_tok, C, stream, pdl)
+    if (nmat == 2) return two ? SB_BATCH(2, 2) : SB_BATCH(2, 4);
+    return two ? SB_BATCH(1, 2) : SB_BATCH(1, 4);
+#undef SB_BATCH
+}
+
+bool fp4_batch_supported(int C) { return C >= 256 && (C % 256) == 0; }
+
+cudaError_t launch_fp4_batch(const Fp4Job* jobs, int njobs_max, const int* live, const int* n_live, int max_rows, int max_tok,
+                             int C, cudaStream_t stream) {
+    const long blocks = (long)((max_rows + 63) / 64) * njobs_max * ((max_tok + MAX_T - 1) / MAX_T);
+    return two_rows_per_lane(blocks)
+               ? launch_batch<FMT_FP4, 1, 2>(jobs, njobs_max, live, n_live, max_rows, max_tok, C, stream, 0)
+               : launch_batch<FMT_FP4, 1, 4>(jobs, njobs_max, live, n_live, max_rows, max_tok, C, stream, 0);
 }
 
 }  // namespace sb

@@ -24,12 +24,16 @@ cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes);
 cudaError_t launch_q4_jobs(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
                            int nmat, bool aligned, cudaStream_t stream, int pdl = -1);
 
-// ---- q4_batch_kernels.cu -----------------------------------------------------
-// The same jobs for groups of several tokens (aligned tensors, C a multiple of 64).
+// ---- batch_kernels.cu --------------------------------------------------------
+// The same jobs for aligned tensors with C a multiple of 64, and NVFP4 jobs with C a multiple of 256.
+struct Fp4Job;
 constexpr int Q4_PASS_TOKENS = 4;        // tokens that share one dequantisation
 bool q4_batch_supported(int C, int nmat);
 cudaError_t launch_q4_batch(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
                             int nmat, cudaStream_t stream, int pdl);
+bool fp4_batch_supported(int C);
+cudaError_t launch_fp4_batch(const Fp4Job* jobs, int njobs_max, const int* live, const int* n_live, int max_rows, int max_tok,
+                             int C, cudaStream_t stream);
 
 // ---- q4_fused_decode.cu ------------------------------------------------------
 // Decode-sized expert execution in one launch (gate | up -> GeGLU -> down).
@@ -201,8 +205,7 @@ cudaError_t launch_nvfp4_gemm_tc(const Fp4TcJob* jobs, int njobs, int R, int C, 
 // live / n_live (optional, device): indices of the jobs that have tokens and their number; njobs is then the
 // largest number of such jobs the call can have, and the grid spans only that many
 cudaError_t launch_nvfp4_jobs(const Fp4Job* jobs, int njobs, int max_rows, int max_tok, int C, bool aligned,
-                              cudaStream_t stream, const int* live = nullptr, const int* n_live = nullptr,
-                              int typical_tok = 0);
+                              cudaStream_t stream, const int* live = nullptr, const int* n_live = nullptr);
 
 // ---- router_kernels.cu ---------------------------------------------------
 // Device-side error word: 0 = ok; set (never cleared) by kernels that meet a

@@ -517,19 +517,17 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
         if (flags & SB_EXPERTS_TENSOR_CORE_SINGLE) return -1;
         Timed t(s, KC_GATE_UP, st);
         const int live_max = std::min(s->expert_end - s->expert_begin, jobs);   // experts that can have tokens
-        const int typical = std::max(1, (jobs + E - 1) / E);                    // selections per expert, evenly routed
         if (!cuda_ok(launch_nvfp4_moe_plan(s->group_offsets, E, s->expert_begin, s->expert_end, jobs, l.fp4_experts, H, M,
                                            s->fp4_dq_gu, s->fp4_gate, s->fp4_up, s->fp4_dq_dn, s->grouped_out,
                                            s->fp4_gu_jobs, s->fp4_dn_jobs, s->fp4_ig_gu, s->fp4_ig_dn, st, nullptr, nullptr,
                                            s->fp4_live), "nvfp4 plan") ||
             !cuda_ok(launch_nvfp4_qdq(d_x, 2 * jobs, H, s->fp4_ig_gu, s->fp4_packed, s->fp4_scales, s->fp4_dq_gu,
                                       s->status, st, s->g2c, jobs, K), "nvfp4 qdq x") ||
-            !cuda_ok(launch_nvfp4_jobs(s->fp4_gu_jobs, 2 * live_max, M, B, H, true, st, s->fp4_live + 2, s->fp4_live,
-                                       typical), "nvfp4 gate/up") ||
+            !cuda_ok(launch_nvfp4_jobs(s->fp4_gu_jobs, 2 * live_max, M, B, H, true, st, s->fp4_live + 2, s->fp4_live), "nvfp4 gate/up") ||
             !cuda_ok(launch_nvfp4_qdq(s->fp4_gate, jobs, M, s->fp4_ig_dn, s->fp4_packed, s->fp4_scales, s->fp4_dq_dn,
                                       s->status, st, nullptr, 1, 1, s->fp4_up), "nvfp4 geglu + qdq") ||
             !cuda_ok(launch_nvfp4_jobs(s->fp4_dn_jobs, live_max, H, B, M, true, st, s->fp4_live + 2 + 2 * E,
-                                       s->fp4_live + 1, typical), "nvfp4 down"))
+                                       s->fp4_live + 1), "nvfp4 down"))
             return -1;
         count_launches(6);
         return 0;

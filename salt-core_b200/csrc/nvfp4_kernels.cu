@@ -3,15 +3,16 @@
 //
 //   nvfp4_qdq_kernel     dynamic group-16 activation quantise -> dequantise
 //                        (salt_nvfp4_quantize_input_reference, nvfp4.c:82-130)
-//   nvfp4_tile_kernel    W4A4 projection on the dequantised activations with the
-//                        canonical 32-accumulator order (nvfp4.c:173-192, 157-171)
-//   nvfp4_generic_kernel any C that is a multiple of 16
+//   nvfp4_generic_kernel W4A4 projection on the dequantised activations with the canonical
+//                        32-accumulator order (nvfp4.c:173-192, 157-171), any C that is a
+//                        multiple of 16; multiples of 256 take batch_kernels.cu
 //
 // The encoders are arithmetic instead of the reference's nearest-code searches:
 // "nearest, ties to the even code" over a monotone code table is round-to-
 // nearest-even in that format (checked against the searches in the tests).
 #include <algorithm>
 
+#include "fp4_core.cuh"
 #include "internal.h"
 #include "pdl.cuh"
 #include "q4_core.cuh"
@@ -20,16 +21,6 @@ namespace sb {
 
 static __device__ __forceinline__ void flag_status(int* status, int bit) {
     if (status) atomicOr(status, bit);
-}
-
-// E4M3FN decode (nvfp4.c:25-39) for the finite codes.
-__device__ __forceinline__ float e4m3_decode(uint32_t code) {
-    const uint32_t ex = (code >> 3) & 15u, man = code & 7u;
-    float v;
-    if (ex == 0) v = __fmul_rn((float)man, 0.001953125f);
-    else if (ex == 15 && man == 7) v = __int_as_float(0x7fc00000);
-    else v = __uint_as_float(((ex + 120u) << 23) | (man << 20));
-    return (code & 0x80u) ? -v : v;
 }
 
 // E4M3FN encode of a finite value in [0, 448] (nvfp4.c:41-63): nearest code,
@@ -151,171 +142,6 @@ cudaError_t launch_nvfp4_qdq(const float* x, int rows, int C, const float* ig_ro
     if (dequant) return geglu_up ? SB_QDQ(true, true) : SB_QDQ(true, false);
     return geglu_up ? SB_QDQ(false, true) : SB_QDQ(false, false);     // the tensor-core consumer reads codes and scales only
 #undef SB_QDQ
-}
-
-// Four E2M1 codes of one half-word as floats, by the hardware conversion (two codes -> f16x2, exact: every E2M1
-// value is an f16).  It decodes the code 8 as -0 where the reference's table has +0 (src/nvfp4.c:19-23): as a
-// WEIGHT that cannot change a result - the product is a zero of either sign, and an accumulator that starts
-// at +0 never becomes -0 (x + (-0) = x, +0 + (-0) = +0) - so the dot-product kernels may use it; the
-// quantise-dequantise kernel, whose decoded values are output, keeps the table form.
-__device__ __forceinline__ void e2m1x4(uint32_t h, f32x2& w01, f32x2& w23) {
-    uint32_t p0, p1;
-    asm("{ .reg .b8 b0, b1;\n\t"
-        "mov.b16 {b0, b1}, %2;\n\t"
-        "cvt.rn.f16x2.e2m1x2 %0, b0;\n\t"
-        "cvt.rn.f16x2.e2m1x2 %1, b1; }\n"
-        : "=r"(p0), "=r"(p1)
-        : "h"((unsigned short)h));
-    float f0, f1, f2, f3;
-    asm("{ .reg .b16 l, u;\n\t"
-        "mov.b32 {l, u}, %2;\n\t"
-        "cvt.f32.f16 %0, l;\n\t"
-        "cvt.f32.f16 %1, u; }\n"
-        : "=f"(f0), "=f"(f1)
-        : "r"(p0));
-    asm("{ .reg .b16 l, u;\n\t"
-        "mov.b32 {l, u}, %2;\n\t"
-        "cvt.f32.f16 %0, l;\n\t"
-        "cvt.f32.f16 %1, u; }\n"
-        : "=f"(f2), "=f"(f3)
-        : "r"(p1));
-    w01 = pack2(f0, f1);
-    w23 = pack2(f2, f3);
-}
-
-// Tile kernel: 16 weight rows per block, eight lanes per row, lane octant u owns accumulators
-// 4u..4u+3 (same mapping as the Q4 kernel).  RPL = rows per lane group: 2 (64 threads, lane rows r and r + 8:
-// one activation load serves two rows - batches) or 1 (128 threads: twice the warps on the same shared
-// memory, which is what a one-token pass, bound by latency, wants).
-// Requires C % 256 == 0 and 16-byte aligned operands.
-template <int TT, int RPL>
-__global__ void __launch_bounds__(128 / RPL)
-nvfp4_tile_kernel(const Fp4Job* __restrict__ jobs, int C, const int* __restrict__ live, const int* __restrict__ n_live) {
-    constexpr int NTH = 128 / RPL;
-    extern __shared__ __align__(16) uint8_t smem[];
-    pdl_wait();                    // jobs, live list and activations come from the kernels before this one
-    pdl_launch_dependents();
-    // with a list of the jobs that have tokens the grid only spans those (a decode step touches 4 of 64 experts)
-    if (live != nullptr && (int)blockIdx.y >= *n_live) return;
-    const Fp4Job jb = jobs[live != nullptr ? live[blockIdx.y] : blockIdx.y];
-    const int r0 = blockIdx.x * 16;
-    if (r0 >= jb.R || jb.ntok < 1) return;
-    const int tid = threadIdx.x, u = tid & 7, pr = tid >> 3;
-    const int nvalid = min(16, jb.R - r0);
-    const int row_bytes = C >> 1, w_stride = row_bytes + 16;
-    const int sc_row = C >> 4, sc_stride = sc_row + 16;
-    const int steps = C >> 5;
-    int chunk_steps = 8, nch = (steps + 7) / 8;
-    if (nch > 15) {
-        chunk_steps = (((steps + 14) / 15) + 1) & ~1;
-        nch = (steps + chunk_steps - 1) / chunk_steps;
-    }
-    uint8_t* sW = smem;                                 // [16][w_stride]
-    uint8_t* sS = sW + 16 * w_stride;                   // [16][sc_stride]
-    float* sTbl = (float*)(sS + 16 * sc_stride);        // [256] fl(e4m3(code) * wg)
-    float* sX = sTbl + 256;                             // [TT][C]
-
-    auto issue_x = [&](int tb) {
-        const int ppr = C >> 2;
-        for (int p = tid; p < TT * ppr; p += NTH) {
-            const int tt = p / ppr, pc = p - tt * ppr;
-            const int tok = min(tb + tt, jb.ntok - 1);
-            cp_async16(sX + tt * C + pc * 4, jb.x + (size_t)tok * jb.x_stride + pc * 4);
-        }
-    };
-    issue_x(0);
-    {
-        const int ppr = sc_row >> 4;
-        for (int p = tid; p < nvalid * ppr; p += NTH) {
-            const int rr = p / ppr, pc = p - rr * ppr;
-            cp_async16(sS + rr * sc_stride + pc * 16, jb.scales + (size_t)(r0 + rr) * sc_row + pc * 16);
-        }
-    }
-    for (int ch = 0; ch < nch; ch++) {
-        const int s_begin = ch * chunk_steps;
-        const int cs = min(chunk_steps, steps - s_begin);
-        for (int p = tid; p < 16 * cs; p += NTH) {
-            const int rr = p / cs, pc = p - rr * cs;
-            const int grow = min(r0 + rr, jb.R - 1);
-            cp_async16(sW + rr * w_stride + (s_begin + pc) * 16,
-                       jb.codes + (size_t)grow * row_bytes + (s_begin + pc) * 16);
-        }
-        cp_async_commit();
-    }
-    for (int c = tid; c < 256; c += NTH) sTbl[c] = __fmul_rn(e4m3_decode((uint32_t)c), jb.wg);
-
-    const uint8_t* wA = sW + pr * w_stride + 2 * u;
-    const uint8_t* wB = sW + (RPL == 2 ? pr + 8 : pr) * w_stride + 2 * u;
-    const uint8_t* scA = sS + pr * sc_stride + (u >> 2);
-    const uint8_t* scB = sS + (RPL == 2 ? pr + 8 : pr) * sc_stride + (u >> 2);
-    const float* xs = sX + 4 * u;
-    const f32x2 nz = pack2u(c_neg_zero, c_neg_zero);
-
-    for (int tb = 0; tb < jb.ntok; tb += TT) {
-        if (tb > 0) {
-            __syncthreads();
-            issue_x(tb);
-            cp_async_commit();
-            cp_async_wait_dyn(0);
-            __syncthreads();
-        }
-        // accumulators 4u .. 4u + 3 of each row as two packed pairs (add.rn.f32x2 = two independent roundings)
-        f32x2 accA[TT][2], accB[TT][2];
-#pragma unroll
-        for (int tt = 0; tt < TT; tt++)
-#pragma unroll
-            for (int j = 0; j < 2; j++) { accA[tt][j] = pack2(0.0f, 0.0f); accB[tt][j] = pack2(0.0f, 0.0f); }
-        for (int ch = 0; ch < nch; ch++) {
-            if (tb == 0) {
-                cp_async_wait_dyn(nch - 1 - ch);
-                __syncthreads();
-            }
-            const int s_begin = ch * chunk_steps;
-            const int s_end = min(s_begin + chunk_steps, steps);
-#pragma unroll 2
-            for (int st = s_begin; st < s_end; st++) {
-                const float sa = sTbl[scA[2 * st]];
-                const uint32_t hA = *(const uint16_t*)(wA + st * 16);
-                f32x2 a01, a23, b01, b23;
-                e2m1x4(hA, a01, a23);
-                const f32x2 ssa = pack2(sa, sa);
-                a01 = mul2(a01, ssa); a23 = mul2(a23, ssa);
-                if (RPL == 2) {
-                    const float sb_ = sTbl[scB[2 * st]];
-                    const uint32_t hB = *(const uint16_t*)(wB + st * 16);
-                    e2m1x4(hB, b01, b23);
-                    const f32x2 ssb = pack2(sb_, sb_);
-                    b01 = mul2(b01, ssb); b23 = mul2(b23, ssb);
-                }
-#pragma unroll
-                for (int tt = 0; tt < TT; tt++) {
-                    const ulonglong2 xv = *(const ulonglong2*)(xs + tt * C + st * 32);
-                    // the product as fma(w, x, -0): exactly fl(w * x), and an add that the assembler cannot
-                    // contract with it into one fused multiply-add (it would with a plain mul.f32x2)
-                    accA[tt][0] = add2(accA[tt][0], fma2(a01, xv.x, nz));
-                    accA[tt][1] = add2(accA[tt][1], fma2(a23, xv.y, nz));
-                    if (RPL == 2) {
-                        accB[tt][0] = add2(accB[tt][0], fma2(b01, xv.x, nz));
-                        accB[tt][1] = add2(accB[tt][1], fma2(b23, xv.y, nz));
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int tt = 0; tt < TT; tt++) {
-            float fa[4], fb[4];
-            unpack2(accA[tt][0], fa[0], fa[1]); unpack2(accA[tt][1], fa[2], fa[3]);
-            unpack2(accB[tt][0], fb[0], fb[1]); unpack2(accB[tt][1], fb[2], fb[3]);
-            const float y0 = fold_row_octants(fa, u);
-            const float y1 = RPL == 2 ? fold_row_octants(fb, u) : 0.0f;
-            const int tok = tb + tt;
-            if (u == 7 && tok < jb.ntok) {
-                float* yrow = jb.y + (size_t)tok * jb.y_stride;
-                if (pr < nvalid) yrow[r0 + pr] = y0;
-                if (RPL == 2 && pr + 8 < nvalid) yrow[r0 + pr + 8] = y1;
-            }
-        }
-    }
 }
 
 // Any C (multiple of 16), any alignment: one warp per (row, token), lane l owns
@@ -440,33 +266,10 @@ cudaError_t launch_nvfp4_moe_plan(const int* group_offsets, int E, int expert_be
                       tc_dn, live);
 }
 
-static size_t fp4_smem(int C, int tt) {
-    return (size_t)16 * (C / 2 + 16) + (size_t)16 * (C / 16 + 16) + 256 * sizeof(float) + (size_t)tt * C * sizeof(float);
-}
-
-template <int TT>
-static cudaError_t launch_fp4_tile(const Fp4Job* jobs, int njobs, int max_rows, int C, cudaStream_t stream,
-                                   const int* live, const int* n_live) {
-    {
-        cudaError_t e = ensure_dynamic_smem((const void*)nvfp4_tile_kernel<TT, (TT == 1 ? 1 : 2)>, (size_t)(200 * 1024));
-        if (e != cudaSuccess) return e;
-    }
-    dim3 grid((max_rows + 15) / 16, njobs);
-    constexpr int RPL = TT == 1 ? 1 : 2;
-    return launch_pdl(nvfp4_tile_kernel<TT, RPL>, grid, dim3(128 / RPL), fp4_smem(C, TT), stream, jobs, C, live, n_live);
-}
-
 cudaError_t launch_nvfp4_jobs(const Fp4Job* jobs, int njobs, int max_rows, int max_tok, int C, bool aligned,
-                              cudaStream_t stream, const int* live, const int* n_live, int typical_tok) {
+                              cudaStream_t stream, const int* live, const int* n_live) {
     if (njobs < 1 || max_rows < 1 || max_tok < 1) return cudaSuccess;
-    if (aligned && (C % 256) == 0) {
-        // tokens per pass: sized for the typical group, not the largest possible one - a wider pass stages that
-        // many activation rows in shared memory and costs resident blocks when most groups hold one token
-        const int tt = typical_tok > 0 ? std::min(typical_tok, max_tok) : max_tok;
-        if (tt >= 3 && fp4_smem(C, 4) <= 200 * 1024) return launch_fp4_tile<4>(jobs, njobs, max_rows, C, stream, live, n_live);
-        if (tt >= 2 && fp4_smem(C, 2) <= 200 * 1024) return launch_fp4_tile<2>(jobs, njobs, max_rows, C, stream, live, n_live);
-        if (fp4_smem(C, 1) <= 200 * 1024) return launch_fp4_tile<1>(jobs, njobs, max_rows, C, stream, live, n_live);
-    }
+    if (aligned && fp4_batch_supported(C)) return launch_fp4_batch(jobs, njobs, live, n_live, max_rows, max_tok, C, stream);
     dim3 grid((max_rows + 3) / 4, max_tok, njobs);
     if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
     nvfp4_generic_kernel<<<grid, 128, 0, stream>>>(jobs, live, n_live);

@@ -12,7 +12,7 @@
 // sequential loop per lane and the canonical fold is a chain through the sixteen lanes.  Each lane keeps
 // two weight rows (gate + up of the same output row, or two rows of one matrix).  Products are issued as
 // sm_100 packed pairs (add/mul/fma.rn.f32x2): each half of a pair is an independent IEEE
-// round-to-nearest operation.  Several tokens per weight row: q4_batch_kernels.cu.
+// round-to-nearest operation.  Several tokens per weight row: batch_kernels.cu.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -187,34 +187,6 @@ __device__ __forceinline__ void nibbles4(uint32_t h, const NibbleMagic& mg, f32x
     asm("lop3.b32 %0, %1, 0xf000, %2, 0xEA;" : "=r"(f3) : "r"(h), "r"(mg.m3));
     q01 = add2(pack2u(f0, f1), neg01);
     q23 = add2(pack2u(f2, f3), neg23);
-}
-
-// Canonical fold of one row whose 32 accumulators live 4 per lane in eight
-// adjacent lanes (octant u = lane & 7; lane holds acc[4u + j], j = 0..3).
-// Lane u of the octet gathers acc[4s + (u & 3)] from octant s = 0..7 in order and
-// runs the chain L_j = (((0 + acc[j]) + acc[4 + j]) + ...) for j = u & 3 (lanes
-// 4..7 repeat lanes 0..3); the four L values are then combined as
-// (L0 + L2) + (L1 + L3).  The result is valid in every lane of the octet.
-// mask: the lanes that take part (the whole warp, or the row's own eight lanes).
-__device__ __forceinline__ float fold_row_octants(const float (&a)[4], int u, uint32_t mask = 0xffffffffu) {
-    const int j = u & 3;
-    const int base = (threadIdx.x & 31) & ~7;
-    float L = 0.0f;
-#pragma unroll
-    for (int s = 0; s < 8; s++) {
-        // every lane offers all four of its accumulators; the reader picks column j of octant s
-        const float v0 = __shfl_sync(mask, a[0], base + s);
-        const float v1 = __shfl_sync(mask, a[1], base + s);
-        const float v2 = __shfl_sync(mask, a[2], base + s);
-        const float v3 = __shfl_sync(mask, a[3], base + s);
-        const float v = j == 0 ? v0 : (j == 1 ? v1 : (j == 2 ? v2 : v3));
-        L = __fadd_rn(L, v);
-    }
-    const float L0 = __shfl_sync(mask, L, base + 0);
-    const float L1 = __shfl_sync(mask, L, base + 1);
-    const float L2 = __shfl_sync(mask, L, base + 2);
-    const float L3 = __shfl_sync(mask, L, base + 3);
-    return __fadd_rn(__fadd_rn(L0, L2), __fadd_rn(L1, L3));
 }
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {

@@ -1,6 +1,6 @@
 // Grouped affine-Q4 projections: the choice of kernel, and the one that takes any C and any byte alignment with
 // absolute group indices (rows may straddle quantisation groups), one warp per (row, token).  It reproduces the
-// reference row DAG (src/kernels.c:220-250) bit for bit, like q4_batch_kernel for the aligned shapes.
+// reference row DAG (src/kernels.c:220-250) bit for bit, like batch_kernel for the aligned shapes.
 #include "internal.h"
 #include "pdl.cuh"
 #include "q4_core.cuh"

@@ -82,19 +82,41 @@ class SelectedProjectionJob(C.Structure):
                 ("batch", C.c_int), ("resource_slot", C.c_int), ("logical_resource_id", C.c_uint64)]
 
 
+_first_byte, _addressof = C.c_char.from_buffer, C.addressof
+
+
+def address(a):
+    """Host address of a numpy array (None: null).  The buffer protocol costs half of ``a.ctypes.data``, which is what a small call
+    spends most of its host time on; it refuses read-only, empty and strided arrays."""
+    try:
+        return _addressof(_first_byte(a))
+    except (TypeError, ValueError, BufferError):
+        return None if a is None else a.ctypes.data
+
+
 def ptr(a):
-    """Host address of a numpy array (or None)."""
-    return None if a is None else C.c_void_p(a.ctypes.data)
+    """Host address of a numpy array (or None) as a call argument."""
+    return None if a is None else C.c_void_p(address(a))
 
 
 def _ptr_array(arrs):
-    return (C.c_void_p * len(arrs))(*[a.ctypes.data if hasattr(a, "ctypes") else a for a in arrs])
+    return (C.c_void_p * len(arrs))(*[address(a) if hasattr(a, "ctypes") else a for a in arrs])
 
 
 class SaltGpu:
     def __init__(self):
         self.lib = load_library()
         self.lib.salt_b200_launch_count.restype = C.c_uint64
+        # the calls a decode loop makes: prototypes of their own, so that plain addresses can be passed
+        p, i = C.c_void_p, C.c_int
+        proto = C.CFUNCTYPE(i, p, p, p, i, i, p, p)
+        self._q4_matvec = proto(("salt_gpu_q4_matvec", self.lib))
+        self._q8_matvec = proto(("salt_gpu_q8_matvec", self.lib))
+        self._nvfp4_matvec = C.CFUNCTYPE(i, p, i, i, p, p)(("salt_gpu_nvfp4_matvec", self.lib))
+        self._nvfp4_matvec_batch = C.CFUNCTYPE(i, p, i, i, i, p, p)(("salt_gpu_nvfp4_matvec_batch", self.lib))
+        chain = C.CFUNCTYPE(i, p, i, i, i, p, p, p, p, C.c_size_t)
+        self._chain = chain(("salt_gpu_q4_moe_chain", self.lib)), chain(("salt_gpu_q4_moe_chain_selected", self.lib))
+        self._scratch = (C.c_float * 4)()       # the chain's scratch stays on the device; the host one only has to exist
 
     # lifecycle
     def init(self): return self.lib.salt_gpu_init()
@@ -171,7 +193,7 @@ class SaltGpu:
 
     # Q4 compute (host pointers)
     def q4_matvec(self, vals, scales, biases, R, Ccols, x, y):
-        return self.lib.salt_gpu_q4_matvec(ptr(vals), ptr(scales), ptr(biases), R, Ccols, ptr(x), ptr(y))
+        return self._q4_matvec(address(vals), address(scales), address(biases), R, Ccols, address(x), address(y))
 
     def q4_batch(self, vals, scales, biases, xs, ys, ids, Rj, Ccols):
         n = len(vals)
@@ -189,7 +211,7 @@ class SaltGpu:
         return self.lib.salt_gpu_bf16_matvec_batch(C.c_void_p(key), R, Ccols, B, ptr(xs), ptr(ys))
 
     def q8_matvec(self, vals, scales, biases, R, Ccols, x, y):
-        return self.lib.salt_gpu_q8_matvec(ptr(vals), ptr(scales), ptr(biases), R, Ccols, ptr(x), ptr(y))
+        return self._q8_matvec(address(vals), address(scales), address(biases), R, Ccols, address(x), address(y))
 
     def q8_batch(self, vals, scales, biases, xs, ys, ids, Rj, Ccols):
         n = len(vals)
@@ -213,10 +235,8 @@ class SaltGpu:
 
     def q4_moe_chain(self, experts, hidden, routed, inputs, outputs, selected=False):
         arr = (MoeExpert * len(experts))(*experts)
-        scratch = np.zeros(4, np.float32)
-        fn = self.lib.salt_gpu_q4_moe_chain_selected if selected else self.lib.salt_gpu_q4_moe_chain
-        return fn(arr, len(experts), hidden, routed, ptr(inputs), ptr(outputs), ptr(scratch), ptr(scratch),
-                  C.c_size_t(scratch.size))
+        return self._chain[bool(selected)](_addressof(arr), len(experts), hidden, routed, address(inputs),
+                                           address(outputs), _addressof(self._scratch), _addressof(self._scratch), 4)
 
     def q4_selected_shared(self, jobs, arena):
         arr = (SelectedProjectionJob * len(jobs))(*jobs)
@@ -228,10 +248,10 @@ class SaltGpu:
                                            ptr(scales), ptr(dequant))
 
     def nvfp4_matvec(self, key, R, Ccols, x, y):
-        return self.lib.salt_gpu_nvfp4_matvec(C.c_void_p(key), R, Ccols, ptr(x), ptr(y))
+        return self._nvfp4_matvec(key, R, Ccols, address(x), address(y))
 
     def nvfp4_matvec_batch(self, key, R, Ccols, xs, ys):
-        return self.lib.salt_gpu_nvfp4_matvec_batch(C.c_void_p(key), R, Ccols, xs.shape[0], ptr(xs), ptr(ys))
+        return self._nvfp4_matvec_batch(key, R, Ccols, xs.shape[0], address(xs), address(ys))
 
     # shared buffers / exact cells
     def shared_buffer_alloc(self, nbytes):

@@ -179,16 +179,42 @@ bool stage_reserve(size_t x_floats, size_t y_floats, size_t mid_floats, size_t j
            jobs <= B.job_cap;
 }
 
-// Run descriptor jobs (already in B.h_jobs[0..n)) and wait.
-static bool run_jobs(int njobs, int max_rows, int max_tok, int C, int nmat, bool aligned, int bits = 4) {
+bool stream_fence() {
     Backend& B = g_backend;
-    if (!cuda_ok(cudaMemcpyAsync(B.d_jobs, B.h_jobs, (size_t)njobs * sizeof(Q4Job), cudaMemcpyHostToDevice,
-                                 B.stream), "job upload"))
+    if (B.in_flight && !cuda_ok(cudaStreamSynchronize(B.stream), "fence")) return false;
+    B.in_flight = false;
+    return true;
+}
+
+bool stage_upload(size_t head, size_t bytes, const char* what) {
+    Backend& B = g_backend;
+    return cuda_ok(cudaMemcpyAsync((uint8_t*)B.d_x - head, (uint8_t*)B.h_x - head, head + bytes, cudaMemcpyHostToDevice,
+                                   B.stream), what);
+}
+
+float* stage_out(size_t bytes) { return bytes <= SB_DIRECT_OUT_BYTES ? g_backend.hd_y : g_backend.d_y; }
+
+bool stage_finish(size_t bytes, const char* what) {
+    Backend& B = g_backend;
+    B.in_flight = true;
+    if (bytes > SB_DIRECT_OUT_BYTES &&
+        !cuda_ok(cudaMemcpyAsync(B.h_y, B.d_y, bytes, cudaMemcpyDeviceToHost, B.stream), what))
         return false;
+    return stream_fence();
+}
+
+// Descriptors of a synchronous call of at most n jobs: they end where the activations begin.
+static Q4Job* staged_jobs(int n) { return (Q4Job*)g_backend.h_x - n; }
+
+// Upload the n descriptors at staged_jobs(n) and x_bytes of activations, and launch the first njobs of them.
+static bool run_jobs(int n, int njobs, size_t x_bytes, int max_rows, int max_tok, int C, int nmat, bool aligned, int bits = 4) {
+    Backend& B = g_backend;
+    const Q4Job* dj = (const Q4Job*)B.d_x - n;
+    B.in_flight = true;
+    if (!stage_upload((size_t)n * sizeof(Q4Job), x_bytes, "job and x upload")) return false;
     if (bits == 8) {
-        if (!cuda_ok(launch_q8_jobs(B.d_jobs, njobs, max_rows, max_tok, C, B.stream), "q8 launch")) return false;
-    } else if (!cuda_ok(launch_q4_jobs(B.d_jobs, njobs, nullptr, max_rows, max_tok, C, nmat, aligned, B.stream),
-                        "q4 launch"))
+        if (!cuda_ok(launch_q8_jobs(dj, njobs, max_rows, max_tok, C, B.stream), "q8 launch")) return false;
+    } else if (!cuda_ok(launch_q4_jobs(dj, njobs, nullptr, max_rows, max_tok, C, nmat, aligned, B.stream), "q4 launch"))
         return false;
     count_launches(1);
     return true;
@@ -239,18 +265,22 @@ int salt_gpu_init(void) {
     }
     const size_t stage = (size_t)SB_STAGE_FLOATS * sizeof(float);
     bool ok = cuda_ok(cudaStreamCreateWithFlags(&B.stream, cudaStreamNonBlocking), "stream") &&
-              cuda_ok(cudaMalloc((void**)&B.d_x, stage), "stage x") &&
+              cuda_ok(cudaMalloc((void**)&B.d_up, (size_t)SB_MAX_JOBS * sizeof(Q4Job) + stage), "stage x") &&
               cuda_ok(cudaMalloc((void**)&B.d_y, stage), "stage y") &&
               cuda_ok(cudaMalloc((void**)&B.d_mid, stage), "stage mid") &&
-              cuda_ok(cudaMalloc((void**)&B.d_jobs, (size_t)SB_MAX_JOBS * sizeof(Q4Job)), "jobs") &&
-              cuda_ok(cudaMalloc((void**)&B.d_status, sizeof(int)), "status") &&
-              cuda_ok(cudaMemset(B.d_status, 0, sizeof(int)), "status") &&
-              cuda_ok(cudaHostAlloc((void**)&B.h_x, stage, cudaHostAllocDefault), "pinned x") &&
-              cuda_ok(cudaHostAlloc((void**)&B.h_y, stage, cudaHostAllocDefault), "pinned y") &&
-              cuda_ok(cudaHostAlloc((void**)&B.h_jobs, (size_t)SB_MAX_JOBS * sizeof(Q4Job), cudaHostAllocDefault),
-                      "pinned jobs");
+              cuda_ok(cudaHostAlloc((void**)&B.h_status, sizeof(int), cudaHostAllocMapped), "status") &&
+              cuda_ok(cudaHostGetDevicePointer((void**)&B.d_status, B.h_status, 0), "status") &&
+              cuda_ok(cudaHostAlloc((void**)&B.h_up, (size_t)SB_MAX_JOBS * sizeof(Q4Job) + stage, cudaHostAllocDefault),
+                      "pinned x") &&
+              cuda_ok(cudaHostAlloc((void**)&B.h_y, stage, cudaHostAllocMapped), "pinned y") &&
+              cuda_ok(cudaHostGetDevicePointer((void**)&B.hd_y, B.h_y, 0), "pinned y");
     B.stage_floats = SB_STAGE_FLOATS;
     B.job_cap = SB_MAX_JOBS;
+    B.d_jobs = (Q4Job*)B.d_up;
+    B.h_jobs = (Q4Job*)B.h_up;
+    B.d_x = (float*)(B.d_jobs + SB_MAX_JOBS);
+    B.h_x = (float*)(B.h_jobs + SB_MAX_JOBS);
+    if (ok) *B.h_status = 0;
     if (!ok) {
         salt_gpu_free();
         return -1;
@@ -275,10 +305,10 @@ int salt_gpu_free(void) {
     residency_shutdown();
     B.selected.clear();
     B.logical_to_slot.clear();
-    cudaFree(B.d_x); cudaFree(B.d_y); cudaFree(B.d_mid); cudaFree(B.d_jobs); cudaFree(B.d_status);
-    if (B.h_x) cudaFreeHost(B.h_x);
+    cudaFree(B.d_up); cudaFree(B.d_y); cudaFree(B.d_mid);
+    if (B.h_up) cudaFreeHost(B.h_up);
     if (B.h_y) cudaFreeHost(B.h_y);
-    if (B.h_jobs) cudaFreeHost(B.h_jobs);
+    if (B.h_status) cudaFreeHost(B.h_status);
     if (B.stream) cudaStreamDestroy(B.stream);
     fp4_release();
     const SaltGpuBatchStatsV2 keep = B.stats;
@@ -301,15 +331,11 @@ int salt_gpu_defer(void) { return g_backend.defer; }
 int salt_gpu_sync(void) {
     Backend& B = g_backend;
     if (!B.ready) return 0;
-    if (!cuda_ok(cudaStreamSynchronize(B.stream), "sync")) return -1;
+    if (!stream_fence()) return -1;
     B.x_cursor = 0;
-    int status = 0;
-    if (!cuda_ok(cudaMemcpy(&status, B.d_status, sizeof status, cudaMemcpyDeviceToHost), "status")) return -1;
-    if (status) {
-        cudaMemset(B.d_status, 0, sizeof(int));
-        return -1;
-    }
-    return 0;
+    const int status = *(volatile int*)B.h_status;
+    *(volatile int*)B.h_status = 0;
+    return status ? -1 : 0;
 }
 
 void salt_gpu_set_mapped_only(int on) { g_backend.mapped_only = on ? 1 : 0; }
@@ -508,15 +534,17 @@ static int bf16_run(const void* key, int R, int C, int Bt, const float* in, floa
     }
     const size_t nin = (size_t)Bt * C, nout = (size_t)Bt * R;
     if (!in || !out || nin > B.stage_floats || nout > B.stage_floats) return -1;
-    if (!cuda_ok(cudaMemcpyAsync(B.d_x, in, nin * sizeof(float), cudaMemcpyHostToDevice, B.stream), "bf16 x upload"))
-        return -1;
-    const cudaError_t e = serial ? launch_bf16_batch(W, B.d_x, B.d_y, R, C, Bt, B.stream)
-                                 : launch_bf16_matvec(W, B.d_x, B.d_y, R, C, B.stream);
+    if (!stream_fence()) return -1;
+    memcpy(B.h_x, in, nin * sizeof(float));
+    float* const y_dev = stage_out(nout * sizeof(float));
+    B.in_flight = true;
+    if (!stage_upload(0, nin * sizeof(float), "bf16 x upload")) return -1;
+    const cudaError_t e = serial ? launch_bf16_batch(W, B.d_x, y_dev, R, C, Bt, B.stream)
+                                 : launch_bf16_matvec(W, B.d_x, y_dev, R, C, B.stream);
     if (!cuda_ok(e, "bf16 launch")) return -1;
     count_launches(1);
-    if (!cuda_ok(cudaMemcpyAsync(out, B.d_y, nout * sizeof(float), cudaMemcpyDeviceToHost, B.stream), "bf16 y download") ||
-        !cuda_ok(cudaStreamSynchronize(B.stream), "bf16 sync"))
-        return -1;
+    if (!stage_finish(nout * sizeof(float), "bf16 y download")) return -1;
+    memcpy(out, B.h_y, nout * sizeof(float));
     return 0;
 }
 
@@ -689,20 +717,15 @@ static int q4_same_weight(const void* key, const uint32_t* vals, const uint16_t*
         return -1;
     }
     if (!stage_reserve((size_t)Bt * C, (size_t)Bt * R, 0, 1)) return -1;
-    if (!cuda_ok(cudaStreamSynchronize(B.stream), "fence")) return -1;
+    if (!stream_fence()) return -1;
     for (int b = 0; b < Bt; b++) {
         if (!xs[b] || !ys[b]) return -1;
         memcpy(B.h_x + (size_t)b * C, xs[b], (size_t)C * sizeof(float));
     }
-    if (!cuda_ok(cudaMemcpyAsync(B.d_x, B.h_x, (size_t)Bt * C * sizeof(float), cudaMemcpyHostToDevice, B.stream),
-                 "x upload"))
-        return -1;
-    fill_job(B.h_jobs[0], *t, B.d_x, B.d_y, Bt, C, R);
+    const size_t y_bytes = (size_t)Bt * R * sizeof(float);
+    fill_job(*staged_jobs(1), *t, B.d_x, stage_out(y_bytes), Bt, C, R);
     const bool aligned = (C % 64) == 0;
-    if (!run_jobs(1, R, Bt, C, 1, aligned, bits) ||
-        !cuda_ok(cudaMemcpyAsync(B.h_y, B.d_y, (size_t)Bt * R * sizeof(float), cudaMemcpyDeviceToHost, B.stream),
-                 "y download") ||
-        !cuda_ok(cudaStreamSynchronize(B.stream), "sync"))
+    if (!run_jobs(1, 1, (size_t)Bt * C * sizeof(float), R, Bt, C, 1, aligned, bits) || !stage_finish(y_bytes, "y download"))
         return -1;
     for (int b = 0; b < Bt; b++) memcpy(ys[b], B.h_y + (size_t)b * R, (size_t)R * sizeof(float));
     count_kinds(kind == SALT_GPU_RESOURCE_TRUNK, kind == SALT_GPU_RESOURCE_EXPERT_LAYER,
@@ -732,7 +755,15 @@ static int q_batch(int bits, const uint32_t* const* vals, const uint16_t* const*
     if (!B.ready || !vals || !scales || !biases || !xs || !ys || !ids || !Rj || C < 1 || njobs < 1 ||
         (size_t)njobs > B.job_cap)
         return -1;
-    if (!cuda_ok(cudaStreamSynchronize(B.stream), "fence")) return -1;
+    if (!stream_fence()) return -1;
+    // the result buffer has to be known before the first descriptor: the kernel writes small results to the host
+    size_t y_total = 0;
+    for (int j = 0; j < njobs; j++) {
+        if (Rj[j] < 1) return -1;
+        y_total += (size_t)Rj[j];
+    }
+    float* const y_dev = stage_out(y_total * sizeof(float));
+    Q4Job* const staged = staged_jobs(njobs);
     size_t x_floats = 0, y_floats = 0;
     int max_rows = 0, ndesc = 0, max_tok = 1;
     bool trunk = false, expert = false, arena = false;
@@ -763,7 +794,7 @@ static int q_batch(int bits, const uint32_t* const* vals, const uint16_t* const*
             last_x = xs[j]; last_x_off = x_floats; last_run = run;
             x_floats += (size_t)run * C;
         }
-        fill_job(B.h_jobs[ndesc++], *t, B.d_x + xo, B.d_y + y_floats, run, C, Rj[j]);
+        fill_job(staged[ndesc++], *t, B.d_x + xo, y_dev + y_floats, run, C, Rj[j]);
         for (int i = 0; i < run; i++) yoff[(size_t)(j + i)] = y_floats + (size_t)i * Rj[j];
         y_floats += (size_t)run * Rj[j];
         max_rows = std::max(max_rows, Rj[j]);
@@ -773,12 +804,8 @@ static int q_batch(int bits, const uint32_t* const* vals, const uint16_t* const*
         arena |= kind == SALT_GPU_RESOURCE_ARENA;
         j += run;
     }
-    if (!cuda_ok(cudaMemcpyAsync(B.d_x, B.h_x, x_floats * sizeof(float), cudaMemcpyHostToDevice, B.stream),
-                 "x upload") ||
-        !run_jobs(ndesc, max_rows, max_tok, C, 1, (C % 64) == 0, bits) ||
-        !cuda_ok(cudaMemcpyAsync(B.h_y, B.d_y, y_floats * sizeof(float), cudaMemcpyDeviceToHost, B.stream),
-                 "y download") ||
-        !cuda_ok(cudaStreamSynchronize(B.stream), "sync"))
+    if (!run_jobs(njobs, ndesc, x_floats * sizeof(float), max_rows, max_tok, C, 1, (C % 64) == 0, bits) ||
+        !stage_finish(y_total * sizeof(float), "y download"))
         return -1;
     for (int j = 0; j < njobs; j++) memcpy(ys[j], B.h_y + yoff[(size_t)j], (size_t)Rj[j] * sizeof(float));
     count_kinds(trunk, expert, arena);
@@ -838,6 +865,7 @@ int salt_gpu_proj_batch_indexed(const uint32_t* vals, const uint16_t* scales, co
     }
     float* dx = B.d_x + B.x_cursor;
     B.x_cursor += need;
+    B.in_flight = true;
     if (!cuda_ok(cudaMemcpyAsync(dx, xs + (size_t)first_job * C, need * sizeof(float), cudaMemcpyHostToDevice,
                                  B.stream), "x upload"))
         return -1;
@@ -849,6 +877,7 @@ int salt_gpu_proj_batch_indexed(const uint32_t* vals, const uint16_t* scales, co
     Q4Job* hj = B.h_jobs + B.job_cursor;
     Q4Job* dj = B.d_jobs + B.job_cursor;
     B.job_cursor++;
+    B.in_flight = true;
     fill_job(*hj, *t, dx, (float*)output->backend + y_float_offset + (size_t)first_job * R, job_count, C, R);
     if (!cuda_ok(cudaMemcpyAsync(dj, hj, sizeof(Q4Job), cudaMemcpyHostToDevice, B.stream), "job upload") ||
         !cuda_ok(launch_q4_jobs(dj, 1, nullptr, R, job_count, C, 1, (C % 64) == 0, B.stream), "launch"))
@@ -924,7 +953,10 @@ static int moe_chain(const SaltGpuMoeExpert* experts, int count, int hidden, int
         max_group = std::max(max_group, experts[i].group);
     }
     if (total_rows * (uint64_t)hidden > B.stage_floats || total_rows * (uint64_t)routed > B.stage_floats) return -1;
-    if (!cuda_ok(cudaStreamSynchronize(B.stream), "fence")) return -1;
+    if (!stream_fence()) return -1;
+    const size_t in_bytes = (size_t)total_rows * hidden * sizeof(float);
+    float* const y_dev = stage_out(in_bytes);
+    Q4Job* const staged = staged_jobs(2 * count);
     bool aligned = (hidden % 64) == 0 && (routed % 64) == 0;
     size_t row = 0;
     for (int i = 0; i < count; i++) {
@@ -939,24 +971,22 @@ static int moe_chain(const SaltGpuMoeExpert* experts, int count, int hidden, int
                           e.logical_resource_id, require_selected, &d, &kind))
             return -1;
         aligned = aligned && ptr_aligned16(g) && ptr_aligned16(u) && ptr_aligned16(d);
-        Q4Job& gu = B.h_jobs[i];
+        Q4Job& gu = staged[i];
         fill_job(gu, g, B.d_x + row * hidden, B.d_mid + row * routed, e.group, hidden, routed);
         gu.vals2 = u.dv; gu.scales2 = u.ds; gu.biases2 = u.db;
-        Q4Job& dn = B.h_jobs[count + i];
-        fill_job(dn, d, B.d_mid + row * routed, B.d_y + row * hidden, e.group, routed, hidden);
+        Q4Job& dn = staged[count + i];
+        fill_job(dn, d, B.d_mid + row * routed, y_dev + row * hidden, e.group, routed, hidden);
         row += (size_t)e.group;
     }
-    const size_t in_bytes = (size_t)total_rows * hidden * sizeof(float);
-    if (!cuda_ok(cudaMemcpyAsync(B.d_x, inputs, in_bytes, cudaMemcpyHostToDevice, B.stream), "x upload") ||
-        !cuda_ok(cudaMemcpyAsync(B.d_jobs, B.h_jobs, (size_t)(2 * count) * sizeof(Q4Job), cudaMemcpyHostToDevice,
-                                 B.stream), "job upload") ||
-        !cuda_ok(launch_q4_jobs(B.d_jobs, count, nullptr, routed, max_group, hidden, 2, aligned, B.stream),
-                 "gate/up launch") ||
-        !cuda_ok(launch_q4_jobs(B.d_jobs + count, count, nullptr, hidden, max_group, routed, 1, aligned, B.stream),
-                 "down launch") ||
-        !cuda_ok(cudaMemcpyAsync(outputs, B.d_y, in_bytes, cudaMemcpyDeviceToHost, B.stream), "y download") ||
-        !cuda_ok(cudaStreamSynchronize(B.stream), "sync"))
+    memcpy(B.h_x, inputs, in_bytes);
+    const Q4Job* const dj = (const Q4Job*)B.d_x - 2 * count;
+    B.in_flight = true;
+    if (!stage_upload((size_t)(2 * count) * sizeof(Q4Job), in_bytes, "job and x upload") ||
+        !cuda_ok(launch_q4_jobs(dj, count, nullptr, routed, max_group, hidden, 2, aligned, B.stream, 0), "gate/up launch") ||
+        !cuda_ok(launch_q4_jobs(dj + count, count, nullptr, hidden, max_group, routed, 1, aligned, B.stream, 1), "down launch") ||
+        !stage_finish(in_bytes, "y download"))
         return -1;
+    memcpy(outputs, B.h_y, in_bytes);
     count_launches(2);
     B.stats.expert_layer_batches++;
     B.stats.direct_output_batches++;
@@ -984,7 +1014,9 @@ int salt_gpu_q4_selected_shared(const SaltGpuSelectedProjectionJob* jobs, int jo
         !arena->backend || arena->nbytes < sizeof(float))
         return -1;
     const uintptr_t a0 = (uintptr_t)arena->contents, a1 = a0 + arena->nbytes;
-    if (!cuda_ok(cudaStreamSynchronize(B.stream), "fence")) return -1;
+    if (!stream_fence()) return -1;
+    Q4Job* const staged = staged_jobs(job_count);
+    const Q4Job* const dj = (const Q4Job*)B.d_x - job_count;
     std::vector<int> order((size_t)job_count);
     for (int i = 0; i < job_count; i++) order[(size_t)i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return jobs[a].cols < jobs[b].cols; });
@@ -1003,13 +1035,12 @@ int salt_gpu_q4_selected_shared(const SaltGpuSelectedProjectionJob* jobs, int jo
         if (in0 < a0 || in0 > a1 || in_bytes > a1 - in0 || out0 < a0 || out0 > a1 || out_bytes > a1 - out0 ||
             (in0 < out0 + out_bytes && out0 < in0 + in_bytes))
             return -1;
-        fill_job(B.h_jobs[n], t, (const float*)((uint8_t*)arena->backend + (in0 - a0)),
+        fill_job(staged[n], t, (const float*)((uint8_t*)arena->backend + (in0 - a0)),
                  (float*)((uint8_t*)arena->backend + (out0 - a0)), j.batch, j.cols, j.rows);
         aligned_by_desc[(size_t)n] = ptr_aligned16(t) && (j.cols % 64) == 0 && ((in0 - a0) % 16) == 0;
     }
-    if (!cuda_ok(cudaMemcpyAsync(B.d_jobs, B.h_jobs, (size_t)job_count * sizeof(Q4Job), cudaMemcpyHostToDevice,
-                                 B.stream), "job upload"))
-        return -1;
+    B.in_flight = true;
+    if (!stage_upload((size_t)job_count * sizeof(Q4Job), 0, "job upload")) return -1;
     for (int n0 = 0; n0 < job_count;) {
         int n1 = n0, max_rows = 0, max_tok = 1;
         bool aligned = true;
@@ -1020,13 +1051,13 @@ int salt_gpu_q4_selected_shared(const SaltGpuSelectedProjectionJob* jobs, int jo
             aligned = aligned && aligned_by_desc[(size_t)n1];
             n1++;
         }
-        if (!cuda_ok(launch_q4_jobs(B.d_jobs + n0, n1 - n0, nullptr, max_rows, max_tok, C, 1, aligned, B.stream),
+        if (!cuda_ok(launch_q4_jobs(dj + n0, n1 - n0, nullptr, max_rows, max_tok, C, 1, aligned, B.stream),
                      "selected launch"))
             return -1;
         count_launches(1);
         n0 = n1;
     }
-    if (!cuda_ok(cudaStreamSynchronize(B.stream), "sync")) return -1;
+    if (!stream_fence()) return -1;
     B.stats.expert_layer_batches++;
     B.stats.direct_output_batches++;
     B.stats.direct_output_jobs += (uint64_t)job_count;
@@ -1073,9 +1104,9 @@ static bool cell_view(const SaltGpuSharedBuffer* b, size_t offset, size_t elemen
 int salt_gpu_exact_cells(const SaltGpuExactCell* cells, int count) {
     Backend& B = g_backend;
     if (!B.ready || !cells || count < 1) return -1;
-    if (!cuda_ok(cudaStreamSynchronize(B.stream), "fence") ||
-        !cuda_ok(cudaMemsetAsync(B.d_status, 0, sizeof(int), B.stream), "status"))
-        return -1;
+    if (!stream_fence()) return -1;
+    *(volatile int*)B.h_status = 0;
+    B.in_flight = true;
     for (int i = 0; i < count; i++) {
         const SaltGpuExactCell& c = cells[i];
         void* v[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};

@@ -23,7 +23,6 @@ constexpr int FMT_NVFP4 = 104;
 struct Fp4Scratch {
     uint8_t *d_packed = nullptr, *d_scales = nullptr;
     float *d_ig = nullptr, *h_ig = nullptr;
-    Fp4Job *d_jobs = nullptr, *h_jobs = nullptr;
     bool ready = false;
 };
 static Fp4Scratch g_fp4;
@@ -37,18 +36,14 @@ static bool fp4_ready() {
     bool ok = cuda_ok(cudaMalloc((void**)&g_fp4.d_packed, B.stage_floats / 2), "fp4 packed") &&
               cuda_ok(cudaMalloc((void**)&g_fp4.d_scales, B.stage_floats / 16), "fp4 scales") &&
               cuda_ok(cudaMalloc((void**)&g_fp4.d_ig, rows_cap * sizeof(float)), "fp4 ig") &&
-              cuda_ok(cudaHostAlloc((void**)&g_fp4.h_ig, rows_cap * sizeof(float), cudaHostAllocDefault), "fp4 ig") &&
-              cuda_ok(cudaMalloc((void**)&g_fp4.d_jobs, SB_MAX_JOBS * sizeof(Fp4Job)), "fp4 jobs") &&
-              cuda_ok(cudaHostAlloc((void**)&g_fp4.h_jobs, SB_MAX_JOBS * sizeof(Fp4Job), cudaHostAllocDefault),
-                      "fp4 jobs");
+              cuda_ok(cudaHostAlloc((void**)&g_fp4.h_ig, rows_cap * sizeof(float), cudaHostAllocDefault), "fp4 ig");
     g_fp4.ready = ok;
     return ok;
 }
 
 void fp4_release() {
-    cudaFree(g_fp4.d_packed); cudaFree(g_fp4.d_scales); cudaFree(g_fp4.d_ig); cudaFree(g_fp4.d_jobs);
+    cudaFree(g_fp4.d_packed); cudaFree(g_fp4.d_scales); cudaFree(g_fp4.d_ig);
     if (g_fp4.h_ig) cudaFreeHost(g_fp4.h_ig);
-    if (g_fp4.h_jobs) cudaFreeHost(g_fp4.h_jobs);
     g_fp4 = Fp4Scratch();
 }
 
@@ -99,7 +94,16 @@ static int fp4_run(const std::vector<Tensor*>& tensors, const float* const* inpu
     if (total_rows > SB_MAX_JOBS || total_rows * (size_t)C > B.stage_floats || out_floats > B.stage_floats ||
         (size_t)njobs > SB_MAX_JOBS)
         return -1;
-    if (!cuda_ok(cudaStreamSynchronize(B.stream), "fence")) return -1;
+    if (!stream_fence()) return -1;
+    // descriptors | input global scales, right before the activations: one copy takes all three
+    static_assert(sizeof(Fp4Job) + sizeof(float) <= sizeof(Q4Job), "the upload block has room for every job and row");
+    const size_t ig_bytes = (total_rows * sizeof(float) + 15) & ~(size_t)15, head = ig_bytes + (size_t)njobs * sizeof(Fp4Job);
+    if (head > (size_t)SB_MAX_JOBS * sizeof(Q4Job)) return -1;
+    float* const h_ig = (float*)((uint8_t*)B.h_x - ig_bytes);
+    Fp4Job* const h_jobs = (Fp4Job*)h_ig - njobs;
+    const float* const d_ig = (const float*)((const uint8_t*)B.d_x - ig_bytes);
+    const Fp4Job* const d_jobs = (const Fp4Job*)d_ig - njobs;
+    float* const y_dev = stage_out(out_floats * sizeof(float));
     size_t row = 0, yoff = 0;
     int max_rows = 0, max_tok = 1;
     bool aligned = true;
@@ -107,10 +111,10 @@ static int fp4_run(const std::vector<Tensor*>& tensors, const float* const* inpu
     for (int j = 0; j < njobs; j++) {
         const Tensor& t = *tensors[(size_t)j];
         memcpy(B.h_x + row * C, inputs[j], (size_t)batches[j] * C * sizeof(float));
-        for (int b = 0; b < batches[j]; b++) g_fp4.h_ig[row + b] = t.input_global;
-        Fp4Job& fj = g_fp4.h_jobs[j];
+        for (int b = 0; b < batches[j]; b++) h_ig[row + b] = t.input_global;
+        Fp4Job& fj = h_jobs[j];
         fj.codes = t.dv; fj.scales = t.ds; fj.wg = 1.0f / t.weight_divisor;
-        fj.x = B.d_mid + row * C; fj.y = B.d_y + yoff;
+        fj.x = B.d_mid + row * C; fj.y = y_dev + yoff;
         fj.R = t.R; fj.C = C; fj.ntok = batches[j]; fj.x_stride = C; fj.y_stride = t.R;
         aligned = aligned && ((((uintptr_t)t.dv | (uintptr_t)t.ds) & 15) == 0);
         max_rows = std::max(max_rows, t.R);
@@ -120,16 +124,12 @@ static int fp4_run(const std::vector<Tensor*>& tensors, const float* const* inpu
         yoff += (size_t)batches[j] * t.R;
     }
     const size_t in_bytes = total_rows * C * sizeof(float);
-    if (!cuda_ok(cudaMemcpyAsync(B.d_x, B.h_x, in_bytes, cudaMemcpyHostToDevice, B.stream), "fp4 x") ||
-        !cuda_ok(cudaMemcpyAsync(g_fp4.d_ig, g_fp4.h_ig, total_rows * sizeof(float), cudaMemcpyHostToDevice,
-                                 B.stream), "fp4 ig") ||
-        !cuda_ok(cudaMemcpyAsync(g_fp4.d_jobs, g_fp4.h_jobs, (size_t)njobs * sizeof(Fp4Job), cudaMemcpyHostToDevice,
-                                 B.stream), "fp4 jobs") ||
-        !cuda_ok(launch_nvfp4_qdq(B.d_x, (int)total_rows, C, g_fp4.d_ig, g_fp4.d_packed, g_fp4.d_scales, B.d_mid,
+    B.in_flight = true;
+    if (!stage_upload(head, in_bytes, "fp4 upload") ||
+        !cuda_ok(launch_nvfp4_qdq(B.d_x, (int)total_rows, C, d_ig, g_fp4.d_packed, g_fp4.d_scales, B.d_mid,
                                   B.d_status, B.stream), "fp4 qdq") ||
-        !cuda_ok(launch_nvfp4_jobs(g_fp4.d_jobs, njobs, max_rows, max_tok, C, aligned, B.stream), "fp4 proj") ||
-        !cuda_ok(cudaMemcpyAsync(B.h_y, B.d_y, out_floats * sizeof(float), cudaMemcpyDeviceToHost, B.stream),
-                 "fp4 y"))
+        !cuda_ok(launch_nvfp4_jobs(d_jobs, njobs, max_rows, max_tok, C, aligned, B.stream), "fp4 proj") ||
+        !stage_finish(out_floats * sizeof(float), "fp4 y"))
         return -1;
     count_launches(2);
     if (salt_gpu_sync() != 0) return -1;   // also reports non-finite activations
@@ -205,8 +205,9 @@ int salt_gpu_nvfp4_qdq(const float* input, int C, float input_global_scale, uint
     if (!fp4_ready() || !input || !packed || !scales || !dequant || C < 16 || (C & 15) ||
         !isfinite(input_global_scale) || !(input_global_scale > 0.0f) || (size_t)C > B.stage_floats)
         return -1;
-    if (!cuda_ok(cudaStreamSynchronize(B.stream), "fence")) return -1;
+    if (!stream_fence()) return -1;
     g_fp4.h_ig[0] = input_global_scale;
+    B.in_flight = true;
     uint8_t* hp = (uint8_t*)B.h_y;                      // pinned scratch for the byte outputs
     if (!cuda_ok(cudaMemcpyAsync(B.d_x, input, (size_t)C * sizeof(float), cudaMemcpyHostToDevice, B.stream), "x") ||
         !cuda_ok(cudaMemcpyAsync(g_fp4.d_ig, g_fp4.h_ig, sizeof(float), cudaMemcpyHostToDevice, B.stream), "ig") ||

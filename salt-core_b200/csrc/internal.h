@@ -247,9 +247,10 @@ struct GlueArgs {
     int* status;
 };
 cudaError_t launch_glue(const GlueArgs& a, int rows, cudaStream_t stream);
-// logits[t][e] = serial dot of W[e][:] with x[t][:]  (+ bias[e])
-cudaError_t launch_router_logits(const float* W, const float* bias, const float* x, float* logits, int rows, int E,
-                                 int H, cudaStream_t stream);
+// ---- router_logits.cu: logits[t][e] = serial dot of W[e][:] with x[t][:] -------
+// W [E][H], H a multiple of 64
+cudaError_t launch_router_logits(const float* W, const float* x, float* logits, int rows, int E, int H, int* status,
+                                 cudaStream_t stream);
 // softmax top-k with renormalised weights, selections sorted by expert id
 cudaError_t launch_router_topk(const float* logits, const float* per_expert_scale, int32_t* selected, float* weights,
                                int rows, int E, int topk, int sort_by_expert, int* status, cudaStream_t stream);

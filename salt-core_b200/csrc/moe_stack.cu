@@ -300,7 +300,7 @@ int salt_b200_stack_add_nvfp4_layer(void* stack, const SaltB200Nvfp4LayerSpec* s
     l.nvfp4 = true;
     const size_t local = (size_t)(s->expert_end - s->expert_begin);
     const uint8_t* src = (const uint8_t*)spec->pool + (size_t)s->expert_begin * spec->expert_stride;
-    bool ok = upload(&l.router_w, spec->router_w, (size_t)E * s->hidden) &&
+    bool ok = upload(&l.router_w, spec->router_w, (size_t)s->n_experts * s->hidden) &&
               upload(&l.router_scale, spec->router_scale, (size_t)s->hidden) &&
               upload(&l.per_expert_scale, spec->per_expert_scale, (size_t)E) &&
               upload(&l.pool, src, local * spec->expert_stride) &&
@@ -409,7 +409,7 @@ static int layer_router(Stack* s, const Layer& l, const float* d_router_src, int
     }
     {
         Timed t(s, KC_LOGITS, st);
-        if (!cuda_ok(launch_router_logits(l.router_w, nullptr, s->rin, s->logits, B, E, H, st), "logits")) return -1;
+        if (!cuda_ok(launch_router_logits(l.router_w, s->rin, s->logits, B, E, H, s->status, st), "logits")) return -1;
     }
     if (!fused_topk) {
         Timed t(s, KC_TOPK, st);

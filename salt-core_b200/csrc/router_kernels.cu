@@ -507,338 +507,13 @@ cudaError_t launch_router_input(const float* x, const float* scale, float* out, 
     return cudaGetLastError();
 }
 
-// Small batches: one block per (expert, block of up to LOGIT_TB rows).  All
-// threads form the products fl(W[e][c]*x[r][c]) (coalesced loads) into shared
-// memory; then one thread per row runs the reference chain
-// acc = fl(acc + p[c]) over them (src/kernels.c:98-106).
-constexpr int LOGIT_TB = 8;
-
-__global__ void __launch_bounds__(256)
-router_logits_block_kernel(const float* __restrict__ W, const float* __restrict__ bias,
-                           const float* __restrict__ x, float* __restrict__ logits, int rows, int E, int H) {
-    extern __shared__ __align__(16) float sprod[];       // [nr][pitch]
-    const int e = blockIdx.x;
-    const int r0 = blockIdx.y * LOGIT_TB;
-    const int nr = min(LOGIT_TB, rows - r0);
-    const int pitch = ((H + 3) & ~3) + 4;                // +4 floats: rows start in different banks
-    const float* w = W + (size_t)e * H;
-    if ((H & 3) == 0) {
-        // 16-byte loads; the (up to 4) W quads of a thread are all in flight before the first product
-        const int nq = H >> 2;
-        float4 wq[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int q = threadIdx.x + i * 256;
-            wq[i] = q < nq ? __ldg((const float4*)w + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        for (int q0 = 0; q0 < nq; q0 += 1024) {
-            if (q0 > 0) {
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int q = q0 + threadIdx.x + i * 256;
-                    wq[i] = q < nq ? __ldg((const float4*)w + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            }
-            for (int r = 0; r < nr; r++) {
-                const float4* xr = (const float4*)(x + (size_t)(r0 + r) * H);
-                float4 xq[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int q = q0 + threadIdx.x + i * 256;
-                    xq[i] = q < nq ? __ldg(xr + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int q = q0 + threadIdx.x + i * 256;
-                    if (q < nq)
-                        *(float4*)(sprod + r * pitch + 4 * q) =
-                            make_float4(__fmul_rn(wq[i].x, xq[i].x), __fmul_rn(wq[i].y, xq[i].y),
-                                        __fmul_rn(wq[i].z, xq[i].z), __fmul_rn(wq[i].w, xq[i].w));
-                }
-            }
-        }
-    } else {
-        for (int c = threadIdx.x; c < H; c += blockDim.x) {
-            const float wv = __ldg(w + c);
-            for (int r = 0; r < nr; r++) sprod[r * pitch + c] = __fmul_rn(wv, __ldg(x + (size_t)(r0 + r) * H + c));
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < nr) {
-        const float acc = serial_sum(sprod + threadIdx.x * pitch, H);
-        logits[(size_t)(r0 + threadIdx.x) * E + e] = __fadd_rn(acc, bias ? bias[e] : 0.0f);
-    }
-}
-
-// Decode batches of a few rows: one WARP per (expert, row).  Lane l forms the products of
-// columns [l*CH, (l+1)*CH) in registers (H == 32*CH), then the reference chain
-// acc = fl(acc + p[c]), c ascending (src/kernels.c:98-106), runs lane after lane: lane l
-// takes the running value from lane l-1 and adds its CH products from registers, so each
-// step costs one dependent-add latency and nothing else.
-template <int CH>
-__global__ void __launch_bounds__(32)
-router_logits_warp_kernel(const float* __restrict__ W, const float* __restrict__ bias, const float* __restrict__ x,
-                          float* __restrict__ logits, int E, int H) {
-    const int e = blockIdx.x, r = blockIdx.y, lane = threadIdx.x;
-    const float4* w4 = (const float4*)(W + (size_t)e * H + lane * CH);
-    const float4* x4 = (const float4*)(x + (size_t)r * H + lane * CH);
-    float p[CH];
-#pragma unroll
-    for (int i = 0; i < CH / 4; i++) {       // the router weights do not depend on the previous kernel
-        const float4 wv = __ldg(w4 + i);
-        p[4 * i + 0] = wv.x; p[4 * i + 1] = wv.y; p[4 * i + 2] = wv.z; p[4 * i + 3] = wv.w;
-    }
-    pdl_wait();
-    pdl_launch_dependents();
-#pragma unroll
-    for (int i = 0; i < CH / 4; i++) {
-        const float4 xv = x4[i];
-        p[4 * i + 0] = __fmul_rn(p[4 * i + 0], xv.x);
-        p[4 * i + 1] = __fmul_rn(p[4 * i + 1], xv.y);
-        p[4 * i + 2] = __fmul_rn(p[4 * i + 2], xv.z);
-        p[4 * i + 3] = __fmul_rn(p[4 * i + 3], xv.w);
-    }
-    float acc = 0.0f;
-#pragma unroll 1
-    for (int l = 0; l < 32; l++) {
-        float a = __shfl_sync(0xffffffffu, acc, (l + 31) & 31);
-        if (l == 0) a = 0.0f;
-        if (lane == l) {
-#pragma unroll
-            for (int i = 0; i < CH; i++) a = __fadd_rn(a, p[i]);
-            acc = a;
-        }
-    }
-    if (lane == 31) logits[(size_t)r * E + e] = __fadd_rn(acc, bias ? bias[e] : 0.0f);
-}
-
-// Thread per (row, expert) for large batches: 8 experts x 8 rows per block of 64 threads
-// (many small blocks: 64 rows x 128 experts already fill the GPU).  W and x stream through
-// shared memory in 256-column slabs, four slabs deep with 16-byte cp.async copies, so the
-// only thing a thread ever waits for is its own dependent-add chain.
-constexpr int LT_SLAB = 256, LT_PITCH = LT_SLAB + 4, LT_STAGES = 4;
-
-__global__ void __launch_bounds__(64)
-router_logits_tile_kernel(const float* __restrict__ W, const float* __restrict__ bias, const float* __restrict__ x,
-                          float* __restrict__ logits, int rows, int E, int H) {
-    extern __shared__ __align__(16) float lt_sm[];      // [LT_STAGES][16][LT_PITCH]: 8 W rows, then 8 x rows
-    const int tid = threadIdx.x;
-    const int el = tid & 7, rl = tid >> 3;
-    const int e0 = blockIdx.x * 8, row0 = blockIdx.y * 8;
-    const int nslab = (H + LT_SLAB - 1) / LT_SLAB;
-    auto issue = [&](int sl) {
-        float* st = lt_sm + (size_t)(sl % LT_STAGES) * 16 * LT_PITCH;
-        const int c0 = sl * LT_SLAB;
-        const int pieces = (min(LT_SLAB, H - c0) + 3) >> 2;          // 16-byte pieces per row (H % 4 == 0)
-        for (int p = tid; p < 16 * pieces; p += 64) {
-            const int r = p / pieces, pc = p - r * pieces;
-            const float* src;
-            if (r < 8) src = W + (size_t)min(e0 + r, E - 1) * H + c0 + pc * 4;
-            else src = x + (size_t)min(row0 + r - 8, rows - 1) * H + c0 + pc * 4;
-            cp_async16(st + r * LT_PITCH + pc * 4, src);
-        }
-    };
-    for (int sl = 0; sl < LT_STAGES - 1; sl++) {
-        if (sl < nslab) issue(sl);
-        cp_async_commit();
-    }
-    float acc = 0.0f;
-    for (int sl = 0; sl < nslab; sl++) {
-        cp_async_wait_dyn(LT_STAGES - 2);      // slab sl has landed (one group per slab, empty ones included)
-        __syncthreads();                       // ... for every thread, and slab sl - 1 is no longer read
-        if (sl + LT_STAGES - 1 < nslab) issue(sl + LT_STAGES - 1);
-        cp_async_commit();
-        const float* st = lt_sm + (size_t)(sl % LT_STAGES) * 16 * LT_PITCH;
-        const float4* w4 = (const float4*)(st + el * LT_PITCH);
-        const float4* x4 = (const float4*)(st + (8 + rl) * LT_PITCH);
-        const int kc = min(LT_SLAB, H - sl * LT_SLAB);
-        int c = 0;
-#pragma unroll 4
-        for (; c + 4 <= kc; c += 4) {
-            const float4 wv = w4[c >> 2], xv = x4[c >> 2];
-            acc = __fadd_rn(acc, __fmul_rn(wv.x, xv.x));
-            acc = __fadd_rn(acc, __fmul_rn(wv.y, xv.y));
-            acc = __fadd_rn(acc, __fmul_rn(wv.z, xv.z));
-            acc = __fadd_rn(acc, __fmul_rn(wv.w, xv.w));
-        }
-    }
-    const int e = e0 + el, row = row0 + rl;
-    if (e < E && row < rows) logits[(size_t)row * E + e] = __fadd_rn(acc, bias ? bias[e] : 0.0f);
-}
-
-// Prefill-sized batches: 16 * RL threads as 16 experts x RL rows, each thread EPT x RPT outputs
-// (independent dependent-add chains, so a warp always has an add to issue), tiles of
-// 16*EPT experts x RL*RPT rows.  The 8 x 8 tiles above re-read W and x from L2 sixteen times
-// more often per output than a 32 x 32 tile; past a few hundred rows that traffic, not the
-// chains, set their time.
-template <int EPT, int RPT, int RL>
-struct LogitsBig {
-    static constexpr int THREADS = 16 * RL;                  // 16 expert lanes x RL row lanes
-    static constexpr int TE = 16 * EPT, TR = RL * RPT, ROWS = TE + TR;
-    // the smallest tiles (one chain per lane, chosen when the grid would not fill the SMs otherwise) run one block
-    // per SM: their copy ring is deep enough to cover the L2 latency of a slab that takes a third of a
-    // microsecond to consume; the larger tiles keep three stages so that several blocks share an SM
-    static constexpr int SLAB = 128, PITCH = SLAB + 4, STAGES = (RL == 8 && EPT == 1) ? 6 : 3;
-    static constexpr size_t SMEM = (size_t)STAGES * ROWS * PITCH * sizeof(float);
-};
-
-// RL = 16 (256 threads, two blocks per SM) for a thousand rows and more; RL = 8 (128 threads: one warp per
-// scheduler, so a warp's dependent-add chains never wait for an issue slot) for a few hundred rows, where
-// the number of chains - rows x experts - is what limits the machine and the work should reach many SMs.
-template <int EPT, int RPT, int RL>
-__global__ void __launch_bounds__(16 * RL, RL == 16 ? 2 : 1)
-router_logits_big_kernel(const float* __restrict__ W, const float* __restrict__ bias, const float* __restrict__ x,
-                         float* __restrict__ logits, int rows, int E, int H) {
-    using G = LogitsBig<EPT, RPT, RL>;
-    extern __shared__ __align__(16) float lt_sm[];      // [STAGES][TE W rows, then TR x rows][PITCH]
-    const int tid = threadIdx.x;
-    const int el = tid & 15, rl = tid >> 4;
-    const int e0 = blockIdx.x * G::TE, row0 = blockIdx.y * G::TR;
-    const int nslab = (H + G::SLAB - 1) / G::SLAB;
-    // a slab row is 32 pieces of 16 bytes: thread tid copies piece tid & 31 of rows tid >> 5, + THREADS / 32, ...
-    const int pc = tid & 31;
-    auto issue = [&](int sl) {
-        float* st = lt_sm + (size_t)(sl % G::STAGES) * G::ROWS * G::PITCH;
-        const int c = sl * G::SLAB + pc * 4;
-        if (c >= H) return;
-#pragma unroll
-        for (int r = tid >> 5; r < G::ROWS; r += G::THREADS / 32) {
-            const float* src = r < G::TE ? W + (size_t)min(e0 + r, E - 1) * H + c
-                                         : x + (size_t)min(row0 + r - G::TE, rows - 1) * H + c;
-            cp_async16(st + r * G::PITCH + pc * 4, src);
-        }
-    };
-    for (int sl = 0; sl < G::STAGES - 1; sl++) {
-        if (sl < nslab) issue(sl);
-        cp_async_commit();
-    }
-    float acc[EPT][RPT];
-#pragma unroll
-    for (int i = 0; i < EPT; i++)
-#pragma unroll
-        for (int j = 0; j < RPT; j++) acc[i][j] = 0.0f;
-    for (int sl = 0; sl < nslab; sl++) {
-        cp_async_wait_dyn(G::STAGES - 2);
-        __syncthreads();
-        if (sl + G::STAGES - 1 < nslab) issue(sl + G::STAGES - 1);
-        cp_async_commit();
-        const float* st = lt_sm + (size_t)(sl % G::STAGES) * G::ROWS * G::PITCH;
-        const int kc = min(G::SLAB, H - sl * G::SLAB);
-#pragma unroll 2
-        for (int c = 0; c + 4 <= kc; c += 4) {
-            float4 wv[EPT], xv[RPT];
-#pragma unroll
-            for (int i = 0; i < EPT; i++) wv[i] = *(const float4*)(st + (el + 16 * i) * G::PITCH + c);
-#pragma unroll
-            for (int j = 0; j < RPT; j++) xv[j] = *(const float4*)(st + (G::TE + rl + RL * j) * G::PITCH + c);
-#pragma unroll
-            for (int i = 0; i < EPT; i++)
-#pragma unroll
-                for (int j = 0; j < RPT; j++) {
-                    float a = acc[i][j];
-                    a = __fadd_rn(a, __fmul_rn(wv[i].x, xv[j].x));
-                    a = __fadd_rn(a, __fmul_rn(wv[i].y, xv[j].y));
-                    a = __fadd_rn(a, __fmul_rn(wv[i].z, xv[j].z));
-                    a = __fadd_rn(a, __fmul_rn(wv[i].w, xv[j].w));
-                    acc[i][j] = a;
-                }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < EPT; i++)
-#pragma unroll
-        for (int j = 0; j < RPT; j++) {
-            const int e = e0 + el + 16 * i, row = row0 + rl + RL * j;
-            if (e < E && row < rows) logits[(size_t)row * E + e] = __fadd_rn(acc[i][j], bias ? bias[e] : 0.0f);
-        }
-}
-
-template <int EPT, int RPT, int RL>
-static cudaError_t launch_logits_big(const float* W, const float* bias, const float* x, float* logits, int rows, int E,
-                                     int H, cudaStream_t stream) {
-    using G = LogitsBig<EPT, RPT, RL>;
-    cudaError_t e = ensure_dynamic_smem((const void*)router_logits_big_kernel<EPT, RPT, RL>, G::SMEM);
-    if (e != cudaSuccess) return e;
-    dim3 grid((E + G::TE - 1) / G::TE, (rows + G::TR - 1) / G::TR);
-    router_logits_big_kernel<EPT, RPT, RL><<<grid, G::THREADS, G::SMEM, stream>>>(W, bias, x, logits, rows, E, H);
-    return cudaGetLastError();
-}
-
-// The same without alignment requirements (H not a multiple of 4, or unaligned operands):
-// plain loads, 32 experts x 8 rows per block, 64-column slabs.
-__global__ void __launch_bounds__(256)
-router_logits_tile_plain_kernel(const float* __restrict__ W, const float* __restrict__ bias,
-                                const float* __restrict__ x, float* __restrict__ logits, int rows, int E, int H) {
-    __shared__ float sW[32][65];
-    __shared__ float sX[8][64];
-    const int el = threadIdx.x & 31, rl = threadIdx.x >> 5;
-    const int e = blockIdx.x * 32 + el, row = blockIdx.y * 8 + rl;
-    float acc = 0.0f;
-    for (int c0 = 0; c0 < H; c0 += 64) {
-        const int kc = min(64, H - c0);
-        for (int i = threadIdx.x; i < 32 * 64; i += 256) {
-            const int ee = i >> 6, cc = i & 63;
-            const int ge = blockIdx.x * 32 + ee;
-            sW[ee][cc] = (ge < E && cc < kc) ? W[(size_t)ge * H + c0 + cc] : 0.0f;
-        }
-        for (int i = threadIdx.x; i < 8 * 64; i += 256) {
-            const int rr = i >> 6, cc = i & 63;
-            const int gr = blockIdx.y * 8 + rr;
-            sX[rr][cc] = (gr < rows && cc < kc) ? x[(size_t)gr * H + c0 + cc] : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int c = 0; c < kc; c++) acc = __fadd_rn(acc, __fmul_rn(sW[el][c], sX[rl][c]));
-        __syncthreads();
-    }
-    if (e < E && row < rows) logits[(size_t)row * E + e] = __fadd_rn(acc, bias ? bias[e] : 0.0f);
-}
-
-cudaError_t launch_router_logits(const float* W, const float* bias, const float* x, float* logits, int rows, int E,
-                                 int H, cudaStream_t stream) {
-    if (rows < 1) return cudaSuccess;
-    const bool aligned16 = ((((uintptr_t)W) | ((uintptr_t)x)) & 15) == 0;
-    if (rows <= 4 && aligned16 && (H == 32 * 88 || H == 32 * 160)) {
-        dim3 grid(E, rows);
-        if (H == 32 * 88) return launch_pdl(router_logits_warp_kernel<88>, grid, dim3(32), 0, stream, W, bias, x, logits, E, H);
-        return launch_pdl(router_logits_warp_kernel<160>, grid, dim3(32), 0, stream, W, bias, x, logits, E, H);
-    }
-    if (rows <= 32) {
-        const int nr = rows < LOGIT_TB ? rows : LOGIT_TB;
-        const size_t smem = (size_t)nr * (((H + 3) & ~3) + 4) * sizeof(float);
-        if (smem > 48 * 1024) {
-            cudaError_t e = ensure_dynamic_smem((const void*)router_logits_block_kernel, (size_t)(200 * 1024));
-            if (e != cudaSuccess) return e;
-        }
-        if (smem > 200 * 1024) return cudaErrorInvalidValue;
-        dim3 grid(E, (rows + LOGIT_TB - 1) / LOGIT_TB);
-        router_logits_block_kernel<<<grid, 256, smem, stream>>>(W, bias, x, logits, rows, E, H);
-    } else if (aligned16 && (H & 3) == 0 && rows >= 1024) {
-        return launch_logits_big<2, 2, 16>(W, bias, x, logits, rows, E, H, stream);
-    } else if (aligned16 && (H & 3) == 0 && rows >= 256) {
-        // two chains per lane while that still gives every SM a block, else one chain per lane and twice the blocks
-        if (((E + 31) / 32) * ((rows + 7) / 8) >= 148) return launch_logits_big<2, 1, 8>(W, bias, x, logits, rows, E, H, stream);
-        return launch_logits_big<1, 1, 8>(W, bias, x, logits, rows, E, H, stream);
-    } else if (aligned16 && (H & 3) == 0) {
-        const size_t smem = (size_t)LT_STAGES * 16 * LT_PITCH * sizeof(float);
-        {
-            cudaError_t e = ensure_dynamic_smem((const void*)router_logits_tile_kernel, (size_t)((int)smem));
-            if (e != cudaSuccess) return e;
-        }
-        dim3 grid((E + 7) / 8, (rows + 7) / 8);
-        router_logits_tile_kernel<<<grid, 64, smem, stream>>>(W, bias, x, logits, rows, E, H);
-    } else {
-        dim3 grid((E + 31) / 32, (rows + 7) / 8);
-        router_logits_tile_plain_kernel<<<grid, 256, 0, stream>>>(W, bias, x, logits, rows, E, H);
-    }
-    return cudaGetLastError();
-}
-
 __global__ void __launch_bounds__(128)
 router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ per_expert_scale,
                    int32_t* __restrict__ selected, float* __restrict__ weights, int E, int topk, int sort_by_expert,
                    int* status) {
     extern __shared__ __align__(16) float tk_sm[];
+    pdl_wait();                    // the logits come from the previous kernel
+    pdl_launch_dependents();
     float* sc = tk_sm + topk_scratch_floats(E, topk) - 4;
     topk_group(true, logits + (size_t)blockIdx.x * E, per_expert_scale, selected + (size_t)blockIdx.x * topk,
                weights + (size_t)blockIdx.x * topk, E, topk, sort_by_expert, status, tk_sm, sc, threadIdx.x,
@@ -849,9 +524,8 @@ cudaError_t launch_router_topk(const float* logits, const float* per_expert_scal
                                int rows, int E, int topk, int sort_by_expert, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
     size_t smem = (size_t)topk_scratch_floats(E, topk) * sizeof(float);
-    router_topk_kernel<<<rows, 128, smem, stream>>>(logits, per_expert_scale, selected, weights, E, topk,
-                                                    sort_by_expert, status);
-    return cudaGetLastError();
+    return launch_pdl(router_topk_kernel, dim3(rows), dim3(128), smem, stream, logits, per_expert_scale, selected, weights, E,
+                      topk, sort_by_expert, status);
 }
 
 // The two projection jobs of grouped rows [g0, g0 + cnt) of expert e.
@@ -887,6 +561,8 @@ static __device__ __forceinline__ void write_expert_jobs(const MoePlanArgs& a, i
 __global__ void __launch_bounds__(1024) moe_plan_kernel(MoePlanArgs a) {
     extern __shared__ __align__(16) int sp[];
     const int E = a.n_experts;
+    pdl_wait();                    // the logits or the selections come from the previous kernel
+    pdl_launch_dependents();
     if (a.logits != nullptr) {
         // fused router top-k for small batches: 128 threads per row, up to 8 rows
         float* tk = (float*)(sp + (34 * E + 4));
@@ -1141,8 +817,7 @@ cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream) {
         if (e != cudaSuccess) return e;
     }
     if (smem > 160 * 1024) return cudaErrorInvalidValue;
-    moe_plan_kernel<<<1, 1024, smem, stream>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(moe_plan_kernel, dim3(1), dim3(1024), smem, stream, a);
 }
 
 }  // namespace sb

@@ -103,8 +103,8 @@ int q4_layer_decode_jobs_per_round(int H, int M, int E, int topk, int n_jobs_max
 cudaError_t launch_q8_jobs(const Q4Job* jobs, int njobs, int max_rows, int max_tok, int C, cudaStream_t stream);
 
 // ---- q4_gemm_tc.cu (tcgen05 / TMEM, tolerance path) --------------------------
-cudaError_t launch_gather_convert(const float* x, const int32_t* g2c, void* xh, void* xl, int jobs, int topk,
-                                  int hidden, cudaStream_t stream);
+cudaError_t launch_gather_convert(const float* x, const int32_t* g2c, void* xh, void* xl, void* sums_h, void* sums_l, int jobs,
+                                  int topk, int hidden, cudaStream_t stream);
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda)
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                       const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -117,25 +117,25 @@ struct TcMaps {
     CUtensorMap lo[4];
 };
 cudaError_t make_tc_maps(TcMaps* out, const void* hi, const void* lo, int rows, int cols);
-// fused: gate/up + GeGLU -> out_h (+ out_l) [grouped rows][R] fp16; plain: -> out_f [grouped rows][R] fp32.
-// split: operands carried as hi + lo fp16 halves.  bmaps describes the activations (grouped order).
-// Tiled maps over a layer's expert pool (packed nibbles) and its (scale << 16) | bias tables, one per tensor
-// of an expert slot (gate, up, down); tab_tma[k]: tensor k's table rows are a multiple of 16 bytes and come
-// by tiled copies (otherwise a row tile's table is copied whole).
+// Columns of the group means of a row of `cols` columns, in the layout of the correction chunks (32 groups per 64 columns).
+inline int tc_sums_cols(int cols) { return (cols / 64 + 31) / 32 * 64; }
+// Tiled maps over a layer's expert pool (packed nibbles; gate, up: boxes of 128 rows, down: 256), and its derived tables:
+// (scale << 16) | bias words, and per weight row a power of two that brings the row into fp16, with its inverse
+// ([experts][2 inter + hidden]; hi + lo precision).
 struct TcWeightMaps {
-    CUtensorMap w[3];
-    CUtensorMap t[3];
-    CUtensorMap w256[3];      // the same with boxes of 256 rows (wide single-precision kernel)
-    CUtensorMap t256[3];
+    CUtensorMap w[2];
+    CUtensorMap w256;
     const uint8_t* pool;
     size_t expert_stride;
     const uint32_t* tables;
-    int tab_tma[3];
+    const float *row_scale, *row_unscale;
 };
+cudaError_t launch_q4_row_scales(const uint32_t* tables, int hidden, int inter, int experts, float* scale, float* unscale,
+                                 cudaStream_t stream);
 cudaError_t make_q4_tc_weight_maps(TcWeightMaps* out, const uint8_t* pool, size_t expert_stride, const uint32_t* tables,
-                                   int hidden, int inter, int experts);
+                                   const float* row_scale, const float* row_unscale, int hidden, int inter, int experts);
 // Can the tensor-core kernels take this geometry?  Sizes must be multiples of 64; a size that is no multiple of
-// 256 keeps a tile's scale table in shared memory and must not exceed 3520 (single) / 960 (hi + lo halves).
+// 256 must not exceed 3520 (single) / 960 (hi + lo halves).
 bool q4_tc_supported(int hidden, int inter, bool split);
 // Work lists of a layer's two tensor-core launches (written on the device from the grouped jobs): items_* hold
 // q4_tc_work_items_max() entries of 16 bytes each, work eight ints: {items, next, largest pass, -} of the fused
@@ -145,9 +145,12 @@ cudaError_t launch_q4_tc_work_list(const Q4Job* gateup_jobs, const int* njobs_de
                                    int y_cols, const TcWeightMaps& wm, int hidden, int inter, void* items_fused,
                                    void* items_plain, int* work, cudaStream_t stream);
 // items / work: this launch's list and its {items, next, largest pass} triple.  R, C: rows and columns of the weight matrices.
-cudaError_t launch_q4_gemm_tc(bool fused, bool split, const void* items, int* work, const TcMaps& bmaps,
-                              const TcWeightMaps& wm, void* out_h, void* out_l, float* out_f, int R, int C, int* status,
-                              cudaStream_t stream);
+// fused: gate/up + GeGLU -> out_h [grouped rows][R] fp16 (split: out_l and the group means sums_h, sums_l too); plain: -> out_f
+// [grouped rows][R] fp32.  split: activations carried as hi + lo fp16 halves, weights exactly.  x, sums: the activations
+// (grouped order) and their group means.
+cudaError_t launch_q4_gemm_tc(bool fused, bool split, const void* items, int* work, const TcMaps& x, const TcMaps& sums,
+                              const TcWeightMaps& wm, void* out_h, void* out_l, void* sums_h, void* sums_l, float* out_f, int R,
+                              int C, int* status, cudaStream_t stream);
 
 // ---- bf16_kernels.cu ---------------------------------------------------------
 // y[r] = W[r][:] . x in the reference's eight-accumulator order; ys[t][r] in the serial column order

@@ -31,6 +31,7 @@ struct Layer {
     float* norm_weight = nullptr;
     uint8_t* pool = nullptr;   // local experts only; slot of expert e at pool + (e - expert_begin) * stride
     uint8_t* sb_tables = nullptr;   // derived copy for the fused decode kernels: (scale << 16) | bias words, [local][3][groups]
+    float *row_scale = nullptr, *row_unscale = nullptr;   // tensor-core path: power of two per weight row, and its inverse
     int* lit_flags = nullptr;       // [local] bit k: tensor k of the expert has a scale that needs the two-rounding form
     size_t expert_stride = 0;
     float eps = 0.0f;
@@ -89,6 +90,8 @@ struct Stack {
     bool tc_ready = false;                     // tensor maps built and the geometry fits the single-precision tensor-core kernel
     bool tc_split_ready = false;               // ... and the hi + lo form
     TcMaps x_maps, chain_maps;                 // TMA descriptors of (xh, xl) and (chain_h, chain_l)
+    void *xs_h = nullptr, *xs_l = nullptr, *cs_h = nullptr, *cs_l = nullptr;     // their group means (hi + lo precision)
+    TcMaps xs_maps, cs_maps;
     void *tc_items_fused = nullptr, *tc_items_plain = nullptr;   // work lists of the tensor-core launches (device-written)
     int* tc_work = nullptr;                    // {items, next, largest pass, -} of the fused launch, then of the plain one
     // workspace of the whole feed-forward block (allocated by the first attach)
@@ -133,6 +136,7 @@ static void free_stack(Stack* s) {
     for (auto& l : s->layers) {
         cudaFree(l.router_w); cudaFree(l.router_scale); cudaFree(l.per_expert_scale);
         cudaFree(l.norm_weight); cudaFree(l.pool); cudaFree(l.sb_tables); cudaFree(l.lit_flags); cudaFree(l.fp4_experts);
+        cudaFree(l.row_scale); cudaFree(l.row_unscale);
         cudaFree(l.pre_ffn_norm); cudaFree(l.pre_ffn_norm_2); cudaFree(l.post_ffn_norm_1);
         cudaFree(l.post_ffn_norm_2); cudaFree(l.post_ffn_norm); cudaFree(l.dense); cudaFree(l.dense_jobs);
     }
@@ -148,6 +152,7 @@ static void free_stack(Stack* s) {
     cudaFree(s->fp4_dq_gu); cudaFree(s->fp4_dq_dn); cudaFree(s->fp4_gate); cudaFree(s->fp4_up); cudaFree(s->fp4_ig_gu);
     cudaFree(s->fp4_ig_dn); cudaFree(s->fp4_packed); cudaFree(s->fp4_scales); cudaFree(s->fp4_gu_jobs); cudaFree(s->fp4_dn_jobs);
     cudaFree(s->fp4_tc_gu); cudaFree(s->fp4_tc_dn); cudaFree(s->fp4_live);
+    cudaFree(s->xs_h); cudaFree(s->xs_l); cudaFree(s->cs_h); cudaFree(s->cs_l);
     cudaFree(s->xh); cudaFree(s->xl); cudaFree(s->chain_h); cudaFree(s->chain_l);
     cudaFree(s->tc_items_fused); cudaFree(s->tc_items_plain); cudaFree(s->tc_work);
     if (s->h_in) cudaFreeHost(s->h_in);
@@ -224,7 +229,19 @@ int salt_b200_stack_create(int max_tokens, int hidden, int inter, int n_experts,
     }
     s->tc_ready = q4_tc_supported(hidden, inter, false) && make_tc_maps(&s->x_maps, s->xh, s->xl, (int)J, hidden) == cudaSuccess &&
                   make_tc_maps(&s->chain_maps, s->chain_h, s->chain_l, (int)J, inter) == cudaSuccess;
-    s->tc_split_ready = s->tc_ready && q4_tc_supported(hidden, inter, true);
+    if (s->tc_ready && q4_tc_supported(hidden, inter, true)) {
+        // columns past the last group stay zero, as do the weights they meet
+        const size_t xs = J * (size_t)tc_sums_cols(hidden), cs = J * (size_t)tc_sums_cols(inter);
+        if (!dev_alloc((uint16_t**)&s->xs_h, xs) || !dev_alloc((uint16_t**)&s->xs_l, xs) || !dev_alloc((uint16_t**)&s->cs_h, cs) ||
+            !dev_alloc((uint16_t**)&s->cs_l, cs) || !cuda_ok(cudaMemset(s->xs_h, 0, xs * 2), "sums") ||
+            !cuda_ok(cudaMemset(s->xs_l, 0, xs * 2), "sums") || !cuda_ok(cudaMemset(s->cs_h, 0, cs * 2), "sums") ||
+            !cuda_ok(cudaMemset(s->cs_l, 0, cs * 2), "sums")) {
+            free_stack(s);
+            return -1;
+        }
+        s->tc_split_ready = make_tc_maps(&s->xs_maps, s->xs_h, s->xs_l, (int)J, tc_sums_cols(hidden)) == cudaSuccess &&
+                            make_tc_maps(&s->cs_maps, s->cs_h, s->cs_l, (int)J, tc_sums_cols(inter)) == cudaSuccess;
+    }
     *stack_out = s;
     return 0;
 }
@@ -257,15 +274,21 @@ int salt_b200_stack_add_q4_layer(void* stack, const SaltB200Q4LayerSpec* spec) {
     const size_t groups = elems / 64;
     ok = ok && dev_alloc(&l.sb_tables, local * 3 * groups * 4) && dev_alloc(&l.lit_flags, local) &&
          cuda_ok(launch_q4_interleave_tables(l.pool, l.expert_stride, tensor_bytes, elems / 2, groups, (int)local,
-                                             (uint32_t*)l.sb_tables, l.lit_flags, 0), "scale tables") &&
-         cuda_ok(cudaDeviceSynchronize(), "scale tables");
+                                             (uint32_t*)l.sb_tables, l.lit_flags, 0), "scale tables");
+    if (ok && s->tc_split_ready) {
+        const size_t rows = local * (size_t)(2 * s->inter + s->hidden);
+        ok = dev_alloc(&l.row_scale, rows) && dev_alloc(&l.row_unscale, rows) &&
+             cuda_ok(launch_q4_row_scales((const uint32_t*)l.sb_tables, s->hidden, s->inter, (int)local, l.row_scale,
+                                          l.row_unscale, 0), "row scales");
+    }
+    ok = ok && cuda_ok(cudaDeviceSynchronize(), "scale tables");
     if (!ok) {
         cudaFree(l.router_w); cudaFree(l.router_scale); cudaFree(l.per_expert_scale); cudaFree(l.pool);
-        cudaFree(l.norm_weight); cudaFree(l.sb_tables); cudaFree(l.lit_flags);
+        cudaFree(l.norm_weight); cudaFree(l.sb_tables); cudaFree(l.lit_flags); cudaFree(l.row_scale); cudaFree(l.row_unscale);
         return -1;
     }
     l.q4_tc_ok = s->tc_ready && make_q4_tc_weight_maps(&l.q4_tc, l.pool, l.expert_stride, (const uint32_t*)l.sb_tables,
-                                                        s->hidden, s->inter, (int)local) == cudaSuccess;
+                                                        l.row_scale, l.row_unscale, s->hidden, s->inter, (int)local) == cudaSuccess;
     s->layers.push_back(l);
     return (int)s->layers.size() - 1;
 }
@@ -554,21 +577,21 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
         // tolerance path: fp16 operands on tcgen05, fp32 accumulation in TMEM
         {
             Timed t(s, KC_ROUTER_INPUT, st);
-            if (!cuda_ok(launch_gather_convert(d_x, s->g2c, s->xh, split ? s->xl : nullptr, jobs, K, H, st), "gather/convert")) return -1;
+            if (!cuda_ok(launch_gather_convert(d_x, s->g2c, s->xh, split ? s->xl : nullptr, s->xs_h, s->xs_l, jobs, K, H, st), "gather/convert")) return -1;
             if (!cuda_ok(launch_q4_tc_work_list(s->gateup_jobs, s->counters, njobs_max, s->chain, M, l.q4_tc, H, M,
                                                 s->tc_items_fused, s->tc_items_plain, s->tc_work, st), "tc work list"))
                 return -1;
         }
         {
             Timed t(s, KC_GATE_UP, st);
-            if (!cuda_ok(launch_q4_gemm_tc(true, split, s->tc_items_fused, s->tc_work, s->x_maps, l.q4_tc, s->chain_h,
-                                           s->chain_l, nullptr, M, H, s->status, st), "tc gate/up"))
+            if (!cuda_ok(launch_q4_gemm_tc(true, split, s->tc_items_fused, s->tc_work, s->x_maps, split ? s->xs_maps : s->x_maps,
+                                           l.q4_tc, s->chain_h, s->chain_l, s->cs_h, s->cs_l, nullptr, M, H, s->status, st), "tc gate/up"))
                 return -1;
         }
         {
             Timed t(s, KC_DOWN, st);
-            if (!cuda_ok(launch_q4_gemm_tc(false, split, s->tc_items_plain, s->tc_work + 4, s->chain_maps, l.q4_tc, nullptr,
-                                           nullptr, s->grouped_out, H, M, s->status, st), "tc down"))
+            if (!cuda_ok(launch_q4_gemm_tc(false, split, s->tc_items_plain, s->tc_work + 4, s->chain_maps, split ? s->cs_maps : s->chain_maps,
+                                           l.q4_tc, nullptr, nullptr, nullptr, nullptr, s->grouped_out, H, M, s->status, st), "tc down"))
                 return -1;
         }
         count_launches(6);

@@ -65,17 +65,16 @@ namespace sb {
 
 constexpr int TC_GROUP = 256;                // converter threads of one chunk (two groups take alternate chunks)
 constexpr int TC_CONVERTERS = 2 * TC_GROUP;
-constexpr int TC_THREADS = TC_CONVERTERS + 64;   // + issuer warp + producer warp
-constexpr int TC_ISSUER_WARP = TC_CONVERTERS / 32, TC_PRODUCER_WARP = TC_ISSUER_WARP + 1;
+constexpr int TC_THREADS = TC_CONVERTERS + 96;   // + issuer, weight and token warps
+constexpr int TC_ISSUER_WARP = TC_CONVERTERS / 32, TC_WEIGHT_WARP = TC_ISSUER_WARP + 1, TC_TOKEN_WARP = TC_ISSUER_WARP + 2;
 constexpr int TC_KC = 64;                    // K columns per chunk
 constexpr uint32_t TC_TMEM_COLS = 512;
 constexpr int TC_PK_BYTES = 128 * TC_KC / 2; // packed chunk of 128 rows (one matrix' share of a fused stage)
-constexpr int TC_TAB_BYTES = 128 * 16;       // scale | bias words of 128 rows x 4 chunks
 constexpr int TC_MAX_NT = 128;
 constexpr int TC_MAX_SLOTS = 8;
-// Entries of the ring through which the producing thread passes work items to the other roles.  The producer is
-// at most TC_MAX_SLOTS chunks, i.e. at most TC_MAX_SLOTS units, ahead of the last completed MMA, and no role is more
-// than two units behind that, so 16 entries are never overrun and need no "free" barrier.
+// Entries of the ring through which the thread that draws the units passes them to the other roles.  It is at most
+// TC_MAX_SLOTS chunks, i.e. units, ahead of the converters, and no role is more than three chunks and a unit behind
+// those, so 16 entries are never overrun and need no "free" barrier.
 constexpr int TC_ITEM_RING = 16;
 constexpr int TC_SMEM_BYTES = 225 * 1024;    // dynamic shared memory of every launch (one block per SM)
 
@@ -160,10 +159,9 @@ __device__ __forceinline__ void dequant_half_chunk_f16(const uint4& p, uint32_t 
     }
 }
 
-// The same 32 elements through fp32 (any scale), optionally with the fp16 residuals lo = fp16(v - hi).
-template <bool SPLIT>
+// The same 32 elements through fp32 (any scale).
 __device__ __forceinline__ void dequant_half_chunk_f32(const NibbleMagic& mg, const uint4& p, uint32_t s_bits,
-                                                       uint32_t b_bits, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
+                                                       uint32_t b_bits, uint32_t (&o)[16]) {
     const float s = bf16_bits_to_f32(s_bits), b = bf16_bits_to_f32(b_bits);
     const uint32_t w[4] = {p.x, p.y, p.z, p.w};
     const f32x2 ss = pack2(s, s), bb = pack2(b, b);
@@ -176,12 +174,53 @@ __device__ __forceinline__ void dequant_half_chunk_f32(const NibbleMagic& mg, co
 #pragma unroll
         for (int k = 0; k < 4; k++) unpack2(fma2(q[k], ss, bb), v[2 * k], v[2 * k + 1]);
 #pragma unroll
-        for (int k = 0; k < 4; k++) {   // half2 k holds columns (k, k + 4)
-            const uint32_t h = f16x2_from(v[k], v[k + 4]);
-            hi[4 * i + k] = h;
-            if (SPLIT) lo[4 * i + k] = f16x2_from(v[k] - f16_lo_to_f32(h), v[k + 4] - f16_hi_to_f32(h));
-        }
+        for (int k = 0; k < 4; k++) o[4 * i + k] = f16x2_from(v[k], v[k + 4]);   // half2 k holds columns (k, k + 4)
     }
+}
+
+__device__ __forceinline__ uint32_t hmul2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+// Hi + lo precision: (q - 8) * s of 32 elements.  q - 8 has three bits and s eight, so the fp16 product is exact: no lo
+// half of the weights is needed; what is left of w = (q - 8) s + c, c = b + 8 s, is constant in a group and goes through
+// the correction chunks.
+__device__ __forceinline__ void dequant_exact(const uint4& p, uint32_t s2, uint32_t s2_16, uint32_t (&o)[16]) {
+    const uint32_t w[4] = {p.x, p.y, p.z, p.w};
+    const uint32_t k1024 = 0x64006400u, k1032 = 0x64086408u, k1152 = 0x64806480u;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t w0 = w[i], w1 = w[i] >> 8;
+        uint32_t a0, a1, a2, a3;
+        asm("lop3.b32 %0, %1, 0x000f000f, %2, 0xEA;" : "=r"(a0) : "r"(w0), "r"(k1024));   // cols (0,4)
+        asm("lop3.b32 %0, %1, 0x00f000f0, %2, 0xEA;" : "=r"(a1) : "r"(w0), "r"(k1024));   // cols (1,5) * 16
+        asm("lop3.b32 %0, %1, 0x000f000f, %2, 0xEA;" : "=r"(a2) : "r"(w1), "r"(k1024));   // cols (2,6)
+        asm("lop3.b32 %0, %1, 0x00f000f0, %2, 0xEA;" : "=r"(a3) : "r"(w1), "r"(k1024));   // cols (3,7) * 16
+        o[4 * i + 0] = hmul2(hsub2(a0, k1032), s2);
+        o[4 * i + 1] = hmul2(hsub2(a1, k1152), s2_16);
+        o[4 * i + 2] = hmul2(hsub2(a2, k1032), s2);
+        o[4 * i + 3] = hmul2(hsub2(a3, k1152), s2_16);
+    }
+}
+
+// 32 columns of this lane -> 16: the sums with lane ^ 16, of columns 0..15 in the lower half of the warp, 16..31 in the upper.
+__device__ __forceinline__ void sum_halves(uint32_t (&v)[32], int upper) {
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const float mine = __uint_as_float(upper ? v[16 + i] : v[i]), other = __uint_as_float(upper ? v[i] : v[16 + i]);
+        v[i] = __float_as_uint(mine + __shfl_xor_sync(0xffffffffu, other, 16));
+    }
+}
+
+// Mean of quantisation group g of a row as the correction chunks read it: chunk g / 32, K step (g % 32) / 8, columns
+// g % 8 and 8 + g % 8 (against the hi and lo halves of the group's constant).
+__device__ __forceinline__ void store_group_mean(__half* hi, __half* lo, size_t row, int g, float mean) {
+    const __half h = __float2half_rn(mean), l = __float2half_rn(mean - __half2float(h));
+    const size_t at = row + (size_t)(g >> 5) * TC_KC + ((g & 31) >> 3) * 16 + (g & 7);
+    hi[at] = h; hi[at + 8] = h;
+    lo[at] = l; lo[at + 8] = l;
 }
 
 // One unit of work: one token pass (up to 128 tokens) of one row tile of one expert group.
@@ -196,18 +235,22 @@ struct TcArgs {
     const TcItem* items;       // the launch's work list (written on the device)
     int* work;                 // [0] number of items, [1] next item to hand out, [2] most tokens of any item
     int R, C;                  // rows and columns of the weight matrices of this launch
+    int extra;                 // split: correction chunks after a unit's C / 64 chunks
     __half* out_h;             // fused: GeGLU output [grouped rows][R] fp16, columns in operand K order
     __half* out_l;             // its fp16 residual (split precision) or null
+    __half *sums_h, *sums_l;   // fused, split: group means of the GeGLU output in the correction chunks' K order
+    int sums_stride;
     float* out_f;              // plain: projection output [grouped rows][R] fp32
     int* status;
     const uint32_t* tables;    // (scale << 16) | bias words, [local expert][3 tensors][R * C/64]
+    const float* row_scale;    // split: power of two per weight row, [local expert][2 inter + hidden], gate | up | down ...
+    const float* row_unscale;  // ... and its inverse
+    int scale_stride;          // 2 inter + hidden
     int tensor0;               // first tensor of the slot this launch reads (0: gate, then up; 2: down)
-    int tab_tma;               // table rows are a multiple of 16 bytes: blocks of 4 groups come by tiled TMA
-    int tab_bufs;              // untiled form: buffers for a tile's whole table (2, or 1 where shared memory is short)
+    int scale_off;             // offset of that tensor's rows in row_scale (0, or 2 inter)
 };
 
-// Bounded wait for two barriers at once: both polls are in flight together, so the pair costs one
-// barrier round trip instead of two.
+// A wait for two barriers at once: both polls are in flight together, so the pair costs one barrier round trip.
 __device__ __forceinline__ bool mbar_wait2(uint64_t* bar_a, uint32_t par_a, uint64_t* bar_b, uint32_t par_b,
                                            volatile int* fail) {
     const uint32_t aa = smem_u32(bar_a), ab = smem_u32(bar_b);
@@ -239,83 +282,92 @@ __device__ __forceinline__ bool mbar_wait2(uint64_t* bar_a, uint32_t par_a, uint
     return false;
 }
 
+// One look at a barrier; asked for ahead of time, because the answer takes some 150 cycles.
+__device__ __forceinline__ uint32_t mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(r)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return r;
+}
+
 __device__ __forceinline__ uint4 lds_v4(const uint8_t* p) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_u32(p)));
     return v;
 }
 
+// gelu_tanh(g) * u.  0.5 (1 + tanh i) = 1 / (1 + exp(-2 i)): a tenth of tanhf's instructions, and no cancellation for
+// large negative g (relative error a few 2^-23; the epilogue of a unit of 44 chunks took 10000 cycles with tanhf).
+__device__ __forceinline__ float geglu_fast(float g, float u) {
+    const float inner = 0.7978845608028654f * (g + 0.044715f * g * g * g);
+    return __fdividef(g * u, 1.0f + __expf(-2.0f * inner));
+}
+
 constexpr int TW_ROWS = 256;                        // rows of a converted stage
 constexpr int TW_PK_BYTES = TW_ROWS * TC_KC / 2;    // packed chunk
-constexpr int TW_TAB_BYTES = TW_ROWS * 16;          // table block (4 chunks)
 constexpr int TW_B_BYTES = TW_ROWS * TC_KC * 2;     // converted chunk
-constexpr int TW_TOK_BYTES = TC_MAX_NT * TC_KC * 2; // token tile
-constexpr int TW_STAGES = 3;
+constexpr int TW_TOK_BYTES = TC_MAX_NT * TC_KC * 2; // token tile of 128 rows
+constexpr int TW_STAGES = 3;                        // converted stages, and token tiles
+constexpr int TW_PACK_MAX = 64;                     // split: passes of up to this many tokens carry hi and lo in ONE tile
 
 template <bool FUSED, bool SPLIT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __grid_constant__ TcWeightMaps wm) {
+q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __grid_constant__ TcMaps sums,
+                  const __grid_constant__ TcWeightMaps wm) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bar_in[TC_MAX_SLOTS];    // input slot landed (TMA transaction bytes)
-    __shared__ __align__(8) uint64_t bar_done[TC_MAX_SLOTS];  // the chunk's MMAs are complete (tcgen05.commit)
+    __shared__ __align__(8) uint64_t bar_w[TC_MAX_SLOTS];     // packed chunk landed (TMA transaction bytes)
+    __shared__ __align__(8) uint64_t bar_wfree[TC_MAX_SLOTS]; // ... and is in its converters' registers (8 warp arrivals)
+    __shared__ __align__(8) uint64_t bar_tok[TW_STAGES];      // token tile landed
     __shared__ __align__(8) uint64_t bar_full[TW_STAGES];     // stage converted (8 warp arrivals)
+    __shared__ __align__(8) uint64_t bar_done[TW_STAGES];     // the MMAs that read stage and token tile are complete
     // A unit = one token pass of one row tile.  Accumulators are double-buffered by unit parity (256 columns each).
     __shared__ __align__(8) uint64_t bar_acc[2];              // a unit's accumulators are final
     __shared__ __align__(8) uint64_t bar_epi[2];              // ... and have been read (16 warp arrivals)
-    __shared__ __align__(8) uint64_t bar_tab[2];              // a tile's whole scale table landed (untiled form)
-    __shared__ __align__(8) uint64_t bar_tabfree[2];          // ... and its last conversion is over (16 warp arrivals)
     // The block draws units from the launch's work list (one atomic per unit, by the producing thread, which
     // passes the item to the other roles through a small ring).
     __shared__ __align__(16) TcItem s_items[TC_ITEM_RING];
     __shared__ __align__(8) uint64_t bar_item[TC_ITEM_RING];  // ring entry published
+    __shared__ float s_half[2][TC_MAX_NT];                    // half sums of two 64-column groups (fused, split)
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
 
     constexpr int NMAT = FUSED ? 2 : 1;
     constexpr int RT = TW_ROWS / NMAT;                        // weight rows of a tile, per matrix
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int C = a.C, nchunks = C / TC_KC;
-    constexpr int NPART = SPLIT ? 2 : 1;                     // hi (+ lo) copies of every operand tile
-    constexpr int STAGES = SPLIT ? 2 : TW_STAGES;
-    constexpr int STAGE_BYTES = NPART * TW_B_BYTES;          // [hi][lo] converted chunks
-    const bool tab_tma = a.tab_tma != 0;
-    // carve-up: converted stages | whole-tile table (untiled form) | input slots, each
-    // [packed weights, 8 KB][table block, 4 KB (tiled form)][token tile(s): hi, lo]
+    const int nchunks = a.C / TC_KC, total = nchunks + (SPLIT ? a.extra : 0);
+    // carve-up: converted stages | token tiles (room for the launch's largest pass) | packed chunks.  The MMA always
+    // reads 128 token rows: those above the copied boxes are stale bytes and only reach accumulator lanes nobody reads.
     uint8_t* stage_base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    // untiled tables: two buffers, so the next unit's table lands while this one is in use - or one where two do
-    // not fit (the host decides): the producer then waits for the unit's last conversion
-    const uint32_t TABBUF = (uint32_t)a.tab_bufs;
-    const uint32_t tabw_bytes = tab_tma ? 0u : (((uint32_t)(TW_ROWS * nchunks * 4) + 1023u) & ~1023u);
-    uint8_t* tabw = stage_base + STAGES * STAGE_BYTES;
-    uint8_t* in_base = tabw + TABBUF * tabw_bytes;
-    const uint32_t tok_off = TW_PK_BYTES + (tab_tma ? TW_TAB_BYTES : 0);
-    // The MMA always reads 128 token rows: rows above the copied box (16, 32, 64 or 128 rows, by the pass' size)
-    // are stale bytes of the slot's other part, of the next slot or of the pad behind the last one, and only reach
-    // accumulator lanes nobody reads.
-    // room of a token tile: the TMA box (16, 32, 64 or 128 rows) that holds the launch's largest pass
+    uint8_t* tok_base = stage_base + TW_STAGES * TW_B_BYTES;
     const int nt_max = *(volatile const int*)&a.work[2];
-    const uint32_t tok_room = nt_max <= 16 ? 2048u : nt_max <= 32 ? 4096u : nt_max <= 64 ? 8192u : (uint32_t)TW_TOK_BYTES;
-    const uint32_t slot_bytes = tok_off + NPART * tok_room;
-    const int avail = TC_SMEM_BYTES - 1024 - STAGES * STAGE_BYTES - (int)(TABBUF * tabw_bytes) - (TW_TOK_BYTES - (int)tok_room);
-    const uint32_t NQ = (uint32_t)min(TC_MAX_SLOTS, avail / (int)slot_bytes);
-    if ((int)NQ < STAGES) {                                   // the host checks the geometry; never expected
-        if (tid == 0 && a.status) atomicOr(a.status, SB_ERR_INDEX);
-        return;
-    }
+    const uint32_t tok_room = SPLIT ? (nt_max <= TW_PACK_MAX ? (uint32_t)TW_TOK_BYTES : 2u * TW_TOK_BYTES)
+                                    : (nt_max <= 16 ? 2048u : nt_max <= 32 ? 4096u : nt_max <= 64 ? 8192u : (uint32_t)TW_TOK_BYTES);
+    uint8_t* pk_base = tok_base + TW_STAGES * tok_room;
+    const uint32_t pk_avail = (uint32_t)TC_SMEM_BYTES - 1024u - TW_STAGES * ((uint32_t)TW_B_BYTES + tok_room);
+    const uint32_t NW = pk_avail >= 8u * TW_PK_BYTES ? 8u : 4u;          // 128-token split passes: exactly four
+    static_assert(TC_SMEM_BYTES - 1024 - TW_STAGES * (TW_B_BYTES + 2 * TW_TOK_BYTES) >= 4 * TW_PK_BYTES, "packed ring");
+    const uint32_t nw_shift = NW == 8u ? 3u : 2u;
     volatile int* fail = &s_fail;
 
     if (tid == 0) {
         for (int s = 0; s < TC_MAX_SLOTS; s++) {
-            mbar_init(&bar_in[s], 1);
+            mbar_init(&bar_w[s], 1);
+            mbar_init(&bar_wfree[s], TC_GROUP / 32);
+        }
+        for (int s = 0; s < TW_STAGES; s++) {
+            mbar_init(&bar_tok[s], 1);
+            mbar_init(&bar_full[s], TC_GROUP / 32);
             mbar_init(&bar_done[s], 1);
         }
-        for (int s = 0; s < TW_STAGES; s++) mbar_init(&bar_full[s], TC_GROUP / 32);
         for (int s = 0; s < TC_ITEM_RING; s++) mbar_init(&bar_item[s], 1);
         for (int s = 0; s < 2; s++) {
             mbar_init(&bar_acc[s], 1);
             mbar_init(&bar_epi[s], TC_CONVERTERS / 32);
-            mbar_init(&bar_tab[s], 1);
-            mbar_init(&bar_tabfree[s], TC_CONVERTERS / 32);
         }
         s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -330,20 +382,16 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
-
-    uint32_t it = 0;          // running chunk counter across token passes (every role counts the same chunks)
-    uint32_t p_issued = 0;    // producer: chunks requested
-    uint32_t i_committed = 0; // issuer: chunks committed
-    uint32_t p_tabs = 0;      // producer: whole-tile table copies requested
+    uint32_t requested = 0;       // copies requested by this thread / chunks committed (issuer)
 
     if (warp < TC_ISSUER_WARP) {
-        // ================= converters, then the epilogue of every pass =================
+        // ================= converters, then the epilogue of every unit =================
         const uint32_t grp = (uint32_t)warp >> 3;
         const int crow = (warp & 7) * 32 + lane;                 // stage row
-        const uint32_t b_off = (uint32_t)crow * 128;             // the row's 128-byte line in the 256 x 64 fp16 tile
-        const uint32_t b_sw = (uint32_t)crow & 7;
+        uint8_t* const line = stage_base + (uint32_t)crow * 128; // the row's 128-byte line in the 256 x 64 fp16 tile
+        const uint32_t b_sw = ((uint32_t)crow & 7) << 4;
         const NibbleMagic mg = load_nibble_magic();
-        uint32_t cs = 0, cq = 0, cq_ph = 0, dq = 0, dq_ph = 0;
+        uint32_t it0 = 0, w0 = 0;                                // chunks, packed chunks before this unit
         bool alive = true;
         for (uint32_t unit = 0; alive && !*fail; unit++) {
             alive = __all_sync(0xffffffffu, mbar_wait(&bar_item[unit % TC_ITEM_RING], (unit / TC_ITEM_RING) & 1u, fail));
@@ -351,249 +399,276 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
             const TcItem item = s_items[unit % TC_ITEM_RING];
             if (item.nt < 1) break;                                      // end of the work
             const int r0 = item.r0, rows_here = min(RT, a.R - r0);      // rows_here: a multiple of 64
-            const int nt_real = item.nt;
-            const uint32_t tbuf = unit % TABBUF;
-            const uint8_t* tabt = tabw + tbuf * tabw_bytes;
-            if (!tab_tma) alive = __all_sync(0xffffffffu, mbar_wait(&bar_tab[tbuf], (unit / TABBUF) & 1u, fail));
-            if (!alive) break;
-            for (int kc0 = 0; kc0 < nchunks; kc0 += 4) {
-                uint32_t tw[4];             // table words of this thread's row for four chunks
-#pragma unroll
-                for (int d = 0; d < 4; d++) {
-                    const int kc = kc0 + d;
-                    if (kc >= nchunks) break;
-                    uint8_t* st = stage_base + cs * STAGE_BYTES + b_off;
-                    const uint8_t* slot = in_base + cq * slot_bytes;
-                    const bool mine = (it & 1u) == grp;
-                    if (!tab_tma && d == 0) {
-#pragma unroll
-                        for (int dd = 0; dd < 4; dd++)
-                            tw[dd] = kc0 + dd < nchunks ? *(const uint32_t*)(tabt + (size_t)(crow * nchunks + kc0 + dd) * 4) : 0u;
+            const int mat = FUSED ? crow / RT : 0, row = min(r0 + crow % RT, a.R - 1);
+            const uint32_t* tab = a.tables + ((size_t)(item.expert * 3 + a.tensor0 + mat) * a.R + row) * nchunks;
+            float rs = 1.0f;
+            if (SPLIT) rs = __ldg(a.row_scale + (size_t)item.expert * a.scale_stride + a.scale_off + mat * a.R + row);
+            // this group's chunks of the unit: every other one of the block's running count
+            const int first = (int)((it0 ^ grp) & 1u);
+            uint32_t word_next = first < nchunks ? __ldg(tab + first) : 0u;
+            for (int kc = first; kc < total; kc += 2) {
+                const uint32_t it = it0 + (uint32_t)kc, s = it % TW_STAGES, round = it / TW_STAGES;
+                uint8_t* const st = line + s * TW_B_BYTES;
+                if (!SPLIT || kc < nchunks) {
+                    const uint32_t slot = (w0 + kc) & (NW - 1), wph = ((w0 + kc) >> nw_shift) & 1u;
+                    const uint32_t word = word_next;
+                    word_next = kc + 2 < nchunks ? __ldg(tab + kc + 2) : 0u;     // a chunk pair ahead: its latency is covered
+                    if (!__all_sync(0xffffffffu, mbar_wait(&bar_w[slot], wph, fail))) { alive = false; break; }
+                    const uint8_t* pk = pk_base + slot * TW_PK_BYTES + crow * 32;
+                    const uint4 p[2] = {lds_v4(pk), lds_v4(pk + 16)};
+                    // the MMAs that last read this stage: asked now, needed after the conversion
+                    uint32_t stage_free = round == 0 ? 1u : mbar_test(&bar_done[s], (round - 1) & 1u);
+                    uint32_t o[2][16];
+                    const uint32_t s_bits = word >> 16, b_bits = word & 0xffffu;
+                    if (SPLIT) {
+                        const float sc = bf16_bits_to_f32(s_bits) * rs;
+                        const uint32_t s2 = f16x2_from(sc, sc), s2_16 = f16x2_from(sc * 0.0625f, sc * 0.0625f);
+                        dequant_exact(p[0], s2, s2_16, o[0]);
+                        dequant_exact(p[1], s2, s2_16, o[1]);
+                    } else if (fp16_path_ok(s_bits, b_bits)) {
+                        dequant_half_chunk_f16(p[0], s_bits, b_bits, o[0]);
+                        dequant_half_chunk_f16(p[1], s_bits, b_bits, o[1]);
+                    } else {
+                        dequant_half_chunk_f32(mg, p[0], s_bits, b_bits, o[0]);
+                        dequant_half_chunk_f32(mg, p[1], s_bits, b_bits, o[1]);
                     }
-                    if (mine) {
-                        // the chunk's packed weights have landed, and the MMAs that last read this stage are complete
-                        bool ok = it < (uint32_t)STAGES ? mbar_wait(&bar_in[cq], cq_ph, fail)
-                                                        : mbar_wait2(&bar_in[cq], cq_ph, &bar_done[dq], dq_ph, fail);
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (!ok) { alive = false; kc0 = nchunks; break; }
-                        // tiled form: the table block of these four chunks rides in the slots of the block's first two
-                        // chunks, one copy for each group (chunk and column parities agree: C is a multiple of 256)
-                        if (tab_tma && d < 2) {
-                            const uint4 t = lds_v4(slot + TW_PK_BYTES + crow * 16);
-                            tw[0] = t.x; tw[1] = t.y; tw[2] = t.z; tw[3] = t.w;
-                        }
-                        const uint32_t s_bits = tw[d] >> 16, b_bits = tw[d] & 0xffffu;
-                        const bool half_math = !SPLIT && fp16_path_ok(s_bits, b_bits);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bar_wfree[slot]);        // the packed bytes have been used
+                    if (!__all_sync(0xffffffffu, stage_free) &&
+                        !__all_sync(0xffffffffu, mbar_wait(&bar_done[s], (round - 1) & 1u, fail))) { alive = false; break; }
 #pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            const uint4 pk = lds_v4(slot + crow * 32 + h * 16);
-                            uint32_t o[16], lo[16];
-                            if (half_math) dequant_half_chunk_f16(pk, s_bits, b_bits, o);
-                            else dequant_half_chunk_f32<SPLIT>(mg, pk, s_bits, b_bits, o, lo);
+                    for (int i = 0; i < 8; i++)
+                        *(uint4*)(st + (((uint32_t)i << 4) ^ b_sw)) =
+                            make_uint4(o[i >> 2][4 * (i & 3)], o[i >> 2][4 * (i & 3) + 1], o[i >> 2][4 * (i & 3) + 2],
+                                       o[i >> 2][4 * (i & 3) + 3]);
+                } else {
+                    // correction chunk: 32 groups, eight per K step of 16 columns: 64 c as hi, then as lo halves
+                    if (round > 0 && !__all_sync(0xffffffffu, mbar_wait(&bar_done[s], (round - 1) & 1u, fail))) { alive = false; break; }
+                    const int g0 = (kc - nchunks) * 32;
+#pragma unroll 1
+                    for (int ks = 0; ks < 4; ks++) {
+                        uint32_t hi[4], lo[4];
 #pragma unroll
-                            for (int i = 0; i < 4; i++) {
-                                const uint32_t off = (((uint32_t)(h * 4 + i)) ^ b_sw) << 4;
-                                *(uint4*)(st + off) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
-                                if (SPLIT)
-                                    *(uint4*)(st + TW_B_BYTES + off) = make_uint4(lo[4 * i], lo[4 * i + 1], lo[4 * i + 2], lo[4 * i + 3]);
+                        for (int j = 0; j < 4; j++) {
+                            float c[2];
+#pragma unroll
+                            for (int k = 0; k < 2; k++) {
+                                const int g = g0 + ks * 8 + 2 * j + k;
+                                const uint32_t w = g < nchunks ? __ldg(tab + g) : 0u;
+                                c[k] = (bf16_bits_to_f32(w & 0xffffu) + 8.0f * bf16_bits_to_f32(w >> 16)) * (64.0f * rs);
                             }
+                            hi[j] = f16x2_from(c[0], c[1]);
+                            lo[j] = f16x2_from(c[0] - f16_lo_to_f32(hi[j]), c[1] - f16_hi_to_f32(hi[j]));
                         }
-                        // generic-proxy writes -> visible to the tensor core (async proxy), then one arrival per warp
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&bar_full[cs]);
+                        *(uint4*)(st + (((uint32_t)(2 * ks) << 4) ^ b_sw)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                        *(uint4*)(st + (((uint32_t)(2 * ks + 1) << 4) ^ b_sw)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
                     }
-                    if (it >= (uint32_t)STAGES && ++dq == NQ) { dq = 0; dq_ph ^= 1u; }
-                    if (++cs == (uint32_t)STAGES) cs = 0;
-                    if (++cq == NQ) { cq = 0; cq_ph ^= 1u; }
-                    it++;
                 }
-            }
-            // ---- epilogue of this pass: warp w reads lane quarter w % 4 (tokens) and a quarter of the columns
-            if (!tab_tma && alive) {                                  // this unit's table is no longer read
+                // generic-proxy writes -> visible to the tensor core (async proxy), then one arrival per warp
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&bar_tabfree[tbuf]);
+                if (lane == 0) mbar_arrive(&bar_full[s]);
             }
-            if (alive && __all_sync(0xffffffffu, mbar_wait(&bar_acc[unit & 1u], (unit >> 1) & 1u, fail))) {
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int q = warp & 3;
-                const int n = q * 32 + lane;                        // token of the pass
-                const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (unit & 1u) * TW_ROWS;
-                if (q * 32 < nt_real) {                             // warp-uniform: the quarter holds tokens
-                    if (FUSED) {
-                        const int col = (warp >> 2) * 32;           // output columns col ... col + 31 of the tile
-                        if (col < rows_here) {
-                            uint32_t g[32], u[32];
-                            tmem_ld32(trow + col, g);
-                            tmem_ld32(trow + RT + col, u);
-                            if (n < nt_real) {
-                                const size_t o_off = (size_t)(item.grow + n) * a.R + r0 + col;
-                                __half* dst = a.out_h + o_off;
+            it0 += (uint32_t)total;
+            w0 += (uint32_t)nchunks;
+            // ---- epilogue: warp w reads lane quarter w % 4 (tokens) and a quarter of the columns
+            if (!alive || !__all_sync(0xffffffffu, mbar_wait(&bar_acc[unit & 1u], (unit >> 1) & 1u, fail))) { alive = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int q = warp & 3, cq = warp >> 2;
+            const bool packed = SPLIT && item.nt <= TW_PACK_MAX;
+            // packed: lanes 0..15 of a quarter hold sixteen tokens' hi products, lanes 16..31 the lo products of the same
+            // tokens; after their sum the two halves of the warp share the columns
+            const int n = packed ? q * 16 + (lane & 15) : q * 32 + lane;         // token of the pass
+            const int half0 = packed ? lane >> 4 : 0, halves = packed ? 1 : 2;
+            const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (unit & 1u) * TW_ROWS;
+            const float* un = SPLIT ? a.row_unscale + (size_t)item.expert * a.scale_stride + a.scale_off + r0 : nullptr;
+            if ((packed ? q * 16 : q * 32) < item.nt) {                          // warp-uniform: the quarter holds tokens
+                if (FUSED) {
+                    const int col = cq * 32;                                     // output columns col ... col + 31 of the tile
+                    if (col < rows_here) {
+                        uint32_t g[32], u[32];
+                        tmem_ld32(trow + col, g);
+                        tmem_ld32(trow + RT + col, u);
+                        if (packed) {
+                            sum_halves(g, half0);
+                            sum_halves(u, half0);
+                        }
+                        float sum = 0.0f;
+                        for (int h = 0; h < halves; h++) {
+                            const int c0 = col + (packed ? half0 : h) * 16;
+                            const size_t o_off = (size_t)(item.grow + n) * a.R + r0 + c0;
+                            float o[16];
 #pragma unroll
-                                for (int i8 = 0; i8 < 32; i8 += 8) {
-                                    float o[8];
+                            for (int i = 0; i < 16; i++) {
+                                float gv = __uint_as_float(h == 0 ? g[i] : g[16 + i]), uv = __uint_as_float(h == 0 ? u[i] : u[16 + i]);
+                                if (SPLIT) {
+                                    gv *= __ldg(un + c0 + i);
+                                    uv *= __ldg(un + a.R + c0 + i);
+                                }
+                                o[i] = geglu_fast(gv, uv);
+                                sum += o[i];
+                            }
+                            if (n < item.nt) {
 #pragma unroll
-                                    for (int i = 0; i < 8; i++) {
-                                        const float gv = __uint_as_float(g[i8 + i]), uv = __uint_as_float(u[i8 + i]);
-                                        const float inner = 0.7978845608028654f * (gv + 0.044715f * gv * gv * gv);
-                                        o[i] = 0.5f * gv * (1.0f + tanhf(inner)) * uv;
-                                    }
+                                for (int i8 = 0; i8 < 16; i8 += 8) {
                                     // the next GEMM's K order inside a group of 8: [0,4,1,5,2,6,3,7]
-                                    const uint4 hv = make_uint4(f16x2_from(o[0], o[4]), f16x2_from(o[1], o[5]),
-                                                                f16x2_from(o[2], o[6]), f16x2_from(o[3], o[7]));
-                                    *(uint4*)(dst + i8) = hv;
-                                    if (SPLIT) {
-                                        const uint32_t hw[4] = {hv.x, hv.y, hv.z, hv.w};
-                                        uint32_t lw[4];
+                                    uint32_t hw[4], lw[4];
 #pragma unroll
-                                        for (int kk = 0; kk < 4; kk++)
-                                            lw[kk] = f16x2_from(o[kk] - f16_lo_to_f32(hw[kk]), o[kk + 4] - f16_hi_to_f32(hw[kk]));
-                                        *(uint4*)(a.out_l + o_off + i8) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+                                    for (int kk = 0; kk < 4; kk++) {
+                                        hw[kk] = f16x2_from(o[i8 + kk], o[i8 + kk + 4]);
+                                        if (SPLIT)
+                                            lw[kk] = f16x2_from(o[i8 + kk] - f16_lo_to_f32(hw[kk]), o[i8 + kk + 4] - f16_hi_to_f32(hw[kk]));
                                     }
+                                    *(uint4*)(a.out_h + o_off + i8) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+                                    if (SPLIT) *(uint4*)(a.out_l + o_off + i8) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
                                 }
                             }
                         }
-                    } else {
+                        if (SPLIT) {
+                            // mean of a 64-column group: 32 columns here, 32 in the warp four further on
+                            if (packed) sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+                            if (cq & 1) s_half[cq >> 1][n] = sum;
+                            asm volatile("bar.sync %0, 64;" ::"r"(1 + q * 2 + (cq >> 1)) : "memory");
+                            if (!(cq & 1) && n < item.nt && (!packed || lane < 16))
+                                store_group_mean(a.sums_h, a.sums_l, (size_t)(item.grow + n) * a.sums_stride, (r0 + col) / TC_KC,
+                                                 (sum + s_half[cq >> 1][n]) * (1.0f / TC_KC));
+                        }
+                    }
+                } else {
+#pragma unroll 1
+                    for (int c1 = 0; c1 < 64; c1 += 32) {
+                        const int col = cq * 64 + c1;
+                        if (col >= rows_here) break;
+                        uint32_t g[32];
+                        tmem_ld32(trow + col, g);
+                        if (packed) sum_halves(g, half0);
+                        if (n < item.nt) {
+                            for (int h = 0; h < halves; h++) {
+                                const int c0 = col + (packed ? half0 : h) * 16;
+                                float* dst = a.out_f + (size_t)(item.grow + n) * a.R + r0 + c0;
 #pragma unroll
-                        for (int c0 = 0; c0 < 64; c0 += 32) {
-                            const int col = (warp >> 2) * 64 + c0;
-                            if (col >= rows_here) break;
-                            uint32_t g[32];
-                            tmem_ld32(trow + col, g);
-                            if (n < nt_real) {
-                                float* dst = a.out_f + (size_t)(item.grow + n) * a.R + r0 + col;
-#pragma unroll
-                                for (int i = 0; i < 32; i += 4)
-                                    *(float4*)(dst + i) = make_float4(__uint_as_float(g[i]), __uint_as_float(g[i + 1]),
-                                                                      __uint_as_float(g[i + 2]), __uint_as_float(g[i + 3]));
+                                for (int i = 0; i < 16; i += 4) {
+                                    float4 v;
+                                    v.x = __uint_as_float(h == 0 ? g[i] : g[16 + i]);
+                                    v.y = __uint_as_float(h == 0 ? g[i + 1] : g[17 + i]);
+                                    v.z = __uint_as_float(h == 0 ? g[i + 2] : g[18 + i]);
+                                    v.w = __uint_as_float(h == 0 ? g[i + 3] : g[19 + i]);
+                                    if (SPLIT) {
+                                        const float4 k = __ldg((const float4*)(un + c0 + i));
+                                        v.x *= k.x; v.y *= k.y; v.z *= k.z; v.w *= k.w;
+                                    }
+                                    *(float4*)(dst + i) = v;
+                                }
                             }
                         }
                     }
                 }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bar_epi[unit & 1u]);
             }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_epi[unit & 1u]);
         }
     } else if (warp == TC_ISSUER_WARP) {
         // ================= issuer (one thread) =================
         if (lane == 0) {
             const uint32_t w_lo0 = DESC_B_LO | ((smem_u32(stage_base) & 0x3ffffu) >> 4);
-            const uint32_t t_lo0 = DESC_B_LO | ((smem_u32(in_base + tok_off) & 0x3ffffu) >> 4);
-            uint32_t is = 0, is_ph = 0, iq = 0, iq_ph = 0;
-            uint32_t ready = 0;
+            const uint32_t t_lo0 = DESC_B_LO | ((smem_u32(tok_base) & 0x3ffffu) >> 4);
+            uint32_t s = 0, ph = 0, ready = 0;
             bool ok = true;
             for (uint32_t unit = 0; ok && !*fail; unit++) {
                 if (!mbar_wait(&bar_item[unit % TC_ITEM_RING], (unit / TC_ITEM_RING) & 1u, fail)) break;
                 const TcItem item = s_items[unit % TC_ITEM_RING];
                 if (item.nt < 1) break;                                  // end of the work
+                const bool packed = item.nt <= TW_PACK_MAX;
                 const uint32_t idesc = umma_idesc_f16(128, FUSED ? TW_ROWS : min(RT, a.R - item.r0));
                 // this unit's accumulator buffer was last used two units ago: those accumulators have been read
                 if (unit >= 2 && !mbar_wait(&bar_epi[unit & 1u], ((unit >> 1) - 1) & 1u, fail)) { ok = false; break; }
                 const uint32_t acc_base = tmem + (unit & 1u) * TW_ROWS;
-                for (int kc = 0; kc < nchunks; kc++) {
+                for (int kc = 0; kc < total; kc++) {
                     // the converted weights of the stage, and the chunk's token tile: the tensor core reads it
                     // through the async proxy, so the issuing thread observes that barrier itself
-                    if (!ready) ok = mbar_wait2(&bar_full[is], is_ph, &bar_in[iq], iq_ph, fail);
+                    if (!ready) ok = mbar_wait2(&bar_full[s], ph, &bar_tok[s], ph, fail);
                     if (!ok) break;
                     // poll the next chunk's barriers now; the answer arrives behind this chunk's MMAs
-                    uint32_t ns = is + 1, ns_ph = is_ph, nq = iq + 1, nq_ph = iq_ph;
-                    if (ns == (uint32_t)STAGES) { ns = 0; ns_ph ^= 1u; }
-                    if (nq == NQ) { nq = 0; nq_ph ^= 1u; }
-                    uint32_t r_full, r_in;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                        "selp.u32 %0, 1, 0, p;\n\t}\n"
-                        : "=r"(r_full)
-                        : "r"(smem_u32(&bar_full[ns])), "r"(ns_ph)
-                        : "memory");
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                        "selp.u32 %0, 1, 0, p;\n\t}\n"
-                        : "=r"(r_in)
-                        : "r"(smem_u32(&bar_in[nq])), "r"(nq_ph)
-                        : "memory");
+                    const uint32_t ns = s + 1 == TW_STAGES ? 0 : s + 1, nph = s + 1 == TW_STAGES ? ph ^ 1u : ph;
+                    const uint32_t r_full = mbar_test(&bar_full[ns], nph), r_tok = mbar_test(&bar_tok[ns], nph);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t wlo = w_lo0 + is * (STAGE_BYTES >> 4);
-                    const uint32_t tlo = t_lo0 + iq * (slot_bytes >> 4);
+                    const uint32_t wlo = w_lo0 + s * (TW_B_BYTES >> 4), tlo = t_lo0 + s * (tok_room >> 4);
 #pragma unroll
                     for (int j = 0; j < TC_KC / 16; j++) {
-                        const uint64_t th = make_desc(tlo + j * 2, DESC_B_HI), wh = make_desc(wlo + j * 2, DESC_B_HI);
-                        umma_f16(acc_base, th, wh, idesc, (kc > 0 || j > 0) ? 1u : 0u);
-                        if (SPLIT) {
-                            // x_hi * w_lo, then x_lo * w_hi
-                            umma_f16(acc_base, th, make_desc(wlo + (TW_B_BYTES >> 4) + j * 2, DESC_B_HI), idesc, 1u);
-                            umma_f16(acc_base, make_desc(tlo + (tok_room >> 4) + j * 2, DESC_B_HI), wh, idesc, 1u);
-                        }
+                        const uint64_t w = make_desc(wlo + j * 2, DESC_B_HI);
+                        umma_f16(acc_base, make_desc(tlo + j * 2, DESC_B_HI), w, idesc, (kc > 0 || j > 0) ? 1u : 0u);
+                        if (SPLIT && !packed) umma_f16(acc_base, make_desc(tlo + (TW_TOK_BYTES >> 4) + j * 2, DESC_B_HI), w, idesc, 1u);
                     }
-                    umma_commit(&bar_done[iq]);
-                    if (kc == nchunks - 1) umma_commit(&bar_acc[unit & 1u]);
-                    i_committed++;
-                    ready = r_full & r_in;
-                    is = ns; is_ph = ns_ph; iq = nq; iq_ph = nq_ph;
+                    umma_commit(&bar_done[s]);
+                    if (kc == total - 1) umma_commit(&bar_acc[unit & 1u]);
+                    requested++;
+                    ready = r_full & r_tok;
+                    s = ns; ph = nph;
+                }
+            }
+        }
+    } else if (warp == TC_WEIGHT_WARP) {
+        // ================= units and packed weights (one thread) =================
+        if (lane == 0) {
+            bool pok = true;
+            const int n_items = *(volatile const int*)&a.work[0];
+            for (uint32_t unit = 0; pok && !*fail; unit++) {
+                const int idx = atomicAdd(&a.work[1], 1);
+                TcItem item = {0, 0, 0, 0};
+                if (idx < n_items) {
+                    const int4 v = *(const int4*)&a.items[idx];
+                    item.expert = v.x; item.r0 = v.y; item.grow = v.z; item.nt = v.w;
+                }
+                s_items[unit % TC_ITEM_RING] = item;
+                mbar_arrive(&bar_item[unit % TC_ITEM_RING]);       // release: the entry is visible to who sees the phase
+                if (item.nt < 1) break;
+                for (int kc = 0; kc < nchunks; kc++) {
+                    const uint32_t slot = requested & (NW - 1), round = requested >> nw_shift;
+                    if (round > 0 && !mbar_wait(&bar_wfree[slot], (round - 1) & 1u, fail)) { pok = false; break; }
+                    const uint32_t dst = smem_u32(pk_base + slot * TW_PK_BYTES);
+                    mbar_expect_tx(&bar_w[slot], TW_PK_BYTES);
+                    if (FUSED) {
+                        // 128 rows of gate, then the same 128 rows of up
+#pragma unroll
+                        for (int m = 0; m < 2; m++)
+                            tma_load_3d(dst + m * TC_PK_BYTES, &wm.w[m], kc * 32, item.r0, item.expert, &bar_w[slot]);
+                    } else {
+                        tma_load_3d(dst, &wm.w256, kc * 32, item.r0, item.expert, &bar_w[slot]);
+                    }
+                    requested++;
                 }
             }
         }
     } else if (lane == 0) {
-        // ================= producer (one thread) =================
-        uint32_t pq = 0, pq_ph = 0;
+        // ================= token tiles (one thread) =================
         bool pok = true;
-        const int n_items = *(volatile const int*)&a.work[0];
         for (uint32_t unit = 0; pok && !*fail; unit++) {
-            const int idx = atomicAdd(&a.work[1], 1);
-            TcItem item;
-            if (idx < n_items) {
-                const int4 v = *(const int4*)&a.items[idx];
-                item.expert = v.x; item.r0 = v.y; item.grow = v.z; item.nt = v.w;
-            } else {
-                item.expert = 0; item.r0 = 0; item.grow = 0; item.nt = 0;
-            }
-            s_items[unit % TC_ITEM_RING] = item;
-            mbar_arrive(&bar_item[unit % TC_ITEM_RING]);       // release: the entry is visible to who sees the phase
+            if (!mbar_wait(&bar_item[unit % TC_ITEM_RING], (unit / TC_ITEM_RING) & 1u, fail)) break;
+            const TcItem item = s_items[unit % TC_ITEM_RING];
             if (item.nt < 1) break;
-            const int r0 = item.r0, expert = item.expert;
+            const bool packed = SPLIT && item.nt <= TW_PACK_MAX;
+            const int boxes = (item.nt + 15) / 16;
             const int variant = item.nt <= 16 ? 0 : item.nt <= 32 ? 1 : item.nt <= 64 ? 2 : 3;
-            const uint32_t tok_bytes = (16u << variant) * 128u;
-            if (!tab_tma) {
-                // the tile's whole table, into the buffer whose previous unit has been converted to the end
-                const uint32_t tbuf = unit % TABBUF, round = unit / TABBUF;
-                if (round > 0 && !mbar_wait(&bar_tabfree[tbuf], (round - 1) & 1u, fail)) break;
-                const uint32_t bytes = (uint32_t)(min(RT, a.R - r0) * nchunks * 4);
-                mbar_expect_tx(&bar_tab[tbuf], NMAT * bytes);
-                p_tabs++;
-#pragma unroll
-                for (int m = 0; m < NMAT; m++) {
-                    const uint32_t* src = a.tables + ((size_t)(expert * 3 + a.tensor0 + m) * a.R + r0) * nchunks;
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                     smem_u32(tabw + tbuf * tabw_bytes + (size_t)m * RT * nchunks * 4)),
-                                 "l"(src), "r"(bytes), "r"(smem_u32(&bar_tab[tbuf]))
-                                 : "memory");
-                }
-            }
-            for (int kc = 0; kc < nchunks; kc++) {
-                // the slot's previous chunk has been consumed: its MMAs (which followed its conversion) are complete
-                if (p_issued >= NQ && !mbar_wait(&bar_done[pq], pq_ph ^ 1u, fail)) { pok = false; break; }
-                const uint32_t dst = smem_u32(in_base + pq * slot_bytes);
-                const bool with_tab = tab_tma && (kc & 3) < 2;     // one copy for each converter group
-                mbar_expect_tx(&bar_in[pq], TW_PK_BYTES + (with_tab ? TW_TAB_BYTES : 0) + NPART * tok_bytes);
-                if (FUSED) {
-                    // 128 rows of gate, then the same 128 rows of up
-#pragma unroll
-                    for (int m = 0; m < 2; m++) {
-                        tma_load_3d(dst + m * TC_PK_BYTES, &wm.w[m], kc * 32, r0, expert, &bar_in[pq]);
-                        if (with_tab)
-                            tma_load_3d(dst + TW_PK_BYTES + m * TC_TAB_BYTES, &wm.t[m], (kc & ~3) * 4, r0, expert, &bar_in[pq]);
+            const uint32_t bytes = packed ? (uint32_t)boxes * 2u * 2048u : (SPLIT ? 2u : 1u) * ((16u << variant) * 128u);
+            for (int kc = 0; kc < total; kc++) {
+                const uint32_t s = requested % TW_STAGES, round = requested / TW_STAGES;
+                if (round > 0 && !mbar_wait(&bar_done[s], (round - 1) & 1u, fail)) { pok = false; break; }
+                const uint32_t dst = smem_u32(tok_base + s * tok_room);
+                const TcMaps& m = kc < nchunks ? maps : sums;
+                const int x = (kc < nchunks ? kc : kc - nchunks) * TC_KC;
+                mbar_expect_tx(&bar_tok[s], bytes);
+                if (packed) {
+                    // sixteen tokens' hi rows, then their lo rows, in every quarter of the tile
+                    for (int b = 0; b < boxes; b++) {
+                        tma_load_2d(dst + b * 4096, &m.hi[0], x, item.grow + 16 * b, &bar_tok[s]);
+                        tma_load_2d(dst + b * 4096 + 2048, &m.lo[0], x, item.grow + 16 * b, &bar_tok[s]);
                     }
                 } else {
-                    tma_load_3d(dst, &wm.w256[2], kc * 32, r0, expert, &bar_in[pq]);
-                    if (with_tab) tma_load_3d(dst + TW_PK_BYTES, &wm.t256[2], (kc & ~3) * 4, r0, expert, &bar_in[pq]);
+                    tma_load_2d(dst, &m.hi[variant], x, item.grow, &bar_tok[s]);
+                    if (SPLIT) tma_load_2d(dst + TW_TOK_BYTES, &m.lo[variant], x, item.grow, &bar_tok[s]);
                 }
-                tma_load_2d(dst + tok_off, &maps.hi[variant], kc * TC_KC, item.grow, &bar_in[pq]);
-                if (SPLIT) tma_load_2d(dst + tok_off + tok_room, &maps.lo[variant], kc * TC_KC, item.grow, &bar_in[pq]);
-                p_issued++;
-                if (++pq == NQ) { pq = 0; pq_ph ^= 1u; }
+                requested++;
             }
         }
     }
@@ -601,16 +676,14 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
         // wait (bounded, no early exit) for the copies and MMAs still in flight before shared memory and
         // TMEM are released
         int none = 0;
-        if (warp == TC_PRODUCER_WARP && lane == 0) {
-            if (p_tabs > 0) {       // the last table copy requested
-                const uint32_t t = p_tabs - 1;
-                (void)mbar_wait(&bar_tab[t % TABBUF], (t / TABBUF) & 1u, &none);
-            }
-            for (uint32_t t = (p_issued > NQ ? p_issued - NQ : 0); t < p_issued; t++)
-                (void)mbar_wait(&bar_in[t % NQ], (t / NQ) & 1, &none);
-        }
-        if (warp == TC_ISSUER_WARP && lane == 0 && i_committed > 0)
-            (void)mbar_wait(&bar_done[(i_committed - 1) % NQ], ((i_committed - 1) / NQ) & 1, &none);
+        if (lane == 0 && warp == TC_WEIGHT_WARP)
+            for (uint32_t t = (requested > NW ? requested - NW : 0); t < requested; t++)
+                (void)mbar_wait(&bar_w[t & (NW - 1)], (t >> nw_shift) & 1u, &none);
+        if (lane == 0 && warp == TC_TOKEN_WARP)
+            for (uint32_t t = (requested > TW_STAGES ? requested - TW_STAGES : 0); t < requested; t++)
+                (void)mbar_wait(&bar_tok[t % TW_STAGES], (t / TW_STAGES) & 1u, &none);
+        if (lane == 0 && warp == TC_ISSUER_WARP && requested > 0)
+            (void)mbar_wait(&bar_done[(requested - 1) % TW_STAGES], ((requested - 1) / TW_STAGES) & 1u, &none);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -620,15 +693,16 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
     }
 }
 
-// x (fp32, token rows) -> fp16 rows in grouped order: xh[g] = fp16(x[g2c[g] / topk]),
-// and (when xl != null) the residuals xl[g] = fp16(x - xh).  Columns inside every group
-// of 8 are written in the operands' K order.
+// x (fp32, token rows) -> fp16 rows in grouped order: xh[g] = fp16(x[g2c[g] / topk]), and (when xl != null) the
+// residuals xl[g] = fp16(x - xh) and the means of the 64-column groups.  Columns inside every group of 8 are written in
+// the operands' K order.
 __global__ void __launch_bounds__(256)
 gather_convert_kernel(const float* __restrict__ x, const int32_t* __restrict__ g2c, __half* __restrict__ xh,
-                      __half* __restrict__ xl, int topk, int hidden) {
+                      __half* __restrict__ xl, __half* __restrict__ sums_h, __half* __restrict__ sums_l, int sums_stride,
+                      int topk, int hidden) {
     const int g = blockIdx.y;
     const int d = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
-    if (d >= hidden) return;
+    if (d >= hidden) return;                      // hidden is a multiple of 64: the eight lanes of a group stay together
     const float* src = x + (size_t)(g2c[g] / topk) * hidden + d;
     const float4 v0 = *(const float4*)src, v1 = *(const float4*)(src + 4);
     const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
@@ -639,15 +713,53 @@ gather_convert_kernel(const float* __restrict__ x, const int32_t* __restrict__ g
         lo[k] = f16x2_from(v[k] - f16_lo_to_f32(hi[k]), v[k + 4] - f16_hi_to_f32(hi[k]));
     }
     *(uint4*)(xh + (size_t)g * hidden + d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    if (xl) *(uint4*)(xl + (size_t)g * hidden + d) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    if (xl) {
+        *(uint4*)(xl + (size_t)g * hidden + d) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        const uint32_t octet = 0xffu << (threadIdx.x & 24);
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(octet, sum, o);
+        if ((threadIdx.x & 7) == 0) store_group_mean(sums_h, sums_l, (size_t)g * sums_stride, d / TC_KC, sum * (1.0f / TC_KC));
+    }
 }
 
-cudaError_t launch_gather_convert(const float* x, const int32_t* g2c, void* xh, void* xl, int jobs, int topk,
-                                  int hidden, cudaStream_t stream) {
+cudaError_t launch_gather_convert(const float* x, const int32_t* g2c, void* xh, void* xl, void* sums_h, void* sums_l, int jobs,
+                                  int topk, int hidden, cudaStream_t stream) {
     if (jobs < 1) return cudaSuccess;
-    if (hidden % 8) return cudaErrorInvalidValue;
+    if (hidden % 64) return cudaErrorInvalidValue;
     dim3 grid((hidden / 8 + 255) / 256, jobs);
-    gather_convert_kernel<<<grid, 256, 0, stream>>>(x, g2c, (__half*)xh, (__half*)xl, topk, hidden);
+    gather_convert_kernel<<<grid, 256, 0, stream>>>(x, g2c, (__half*)xh, (__half*)xl, (__half*)sums_h, (__half*)sums_l,
+                                                    tc_sums_cols(hidden), topk, hidden);
+    return cudaGetLastError();
+}
+
+// Powers of two that bring every weight row of an expert pool into fp16: the largest of 8 |s| and 64 |c| of a row becomes
+// 2^9 .. 2^10.  Small scales of the row lose bits only below 2^-27 of its largest weight.
+__global__ void __launch_bounds__(256)
+q4_row_scale_kernel(const uint32_t* __restrict__ tables, int hidden, int inter, int experts, float* __restrict__ scale,
+                    float* __restrict__ unscale) {
+    const int per = 2 * inter + hidden, n = experts * per;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int e = i / per, r = i % per, k = r < inter ? 0 : (r < 2 * inter ? 1 : 2), row = r - k * inter;
+        const int groups = (k < 2 ? hidden : inter) / TC_KC;
+        const uint32_t* t = tables + ((size_t)(e * 3 + k) * ((size_t)hidden * inter / TC_KC)) + (size_t)row * groups;
+        float top = 0.0f;
+        for (int g = 0; g < groups; g++) {
+            const float s = bf16_bits_to_f32(t[g] >> 16), b = bf16_bits_to_f32(t[g] & 0xffffu);
+            top = fmaxf(top, fmaxf(8.0f * fabsf(s), 64.0f * fabsf(b + 8.0f * s)));
+        }
+        int ex = 0;
+        if (top > 0.0f && top < 3.0e38f) frexpf(top, &ex);       // top = m 2^ex, 1/2 <= m < 1
+        ex = min(max(10 - ex, -100), 100);
+        scale[i] = ldexpf(1.0f, ex);
+        unscale[i] = ldexpf(1.0f, -ex);
+    }
+}
+
+cudaError_t launch_q4_row_scales(const uint32_t* tables, int hidden, int inter, int experts, float* scale, float* unscale,
+                                 cudaStream_t stream) {
+    if (experts < 1) return cudaSuccess;
+    q4_row_scale_kernel<<<592, 256, 0, stream>>>(tables, hidden, inter, experts, scale, unscale);
     return cudaGetLastError();
 }
 
@@ -691,12 +803,10 @@ cudaError_t make_tc_maps(TcMaps* out, const void* hi, const void* lo, int rows, 
     return cudaSuccess;
 }
 
-// Tiled maps over a layer's expert pool, one per tensor of a slot (gate, up, down): packed nibbles as
-// [C/2 bytes][R rows][experts] in boxes of one chunk (32 bytes) x 128 rows, and - where a table row is a multiple
-// of 16 bytes (C a multiple of 256) - the (scale << 16) | bias words as [C/16 bytes][R rows][experts] in boxes of
-// four chunks (16 bytes) x 128 rows.  Rows past R read as zero.
+// Tiled maps over a layer's expert pool: packed nibbles as [C/2 bytes][R rows][experts] in boxes of one chunk (32 bytes) x
+// 128 rows of gate and of up, 256 rows of down.  Rows past R read as zero.
 cudaError_t make_q4_tc_weight_maps(TcWeightMaps* out, const uint8_t* pool, size_t expert_stride, const uint32_t* tables,
-                                   int hidden, int inter, int experts) {
+                                   const float* row_scale, const float* row_unscale, int hidden, int inter, int experts) {
     TensorMapEncodeFn encode = nullptr;
     {
         cudaError_t e = tensor_map_encoder(&encode);
@@ -710,85 +820,39 @@ cudaError_t make_q4_tc_weight_maps(TcWeightMaps* out, const uint8_t* pool, size_
     if ((tensor_bytes % 16) != 0) return cudaErrorInvalidValue;
     for (int k = 0; k < 3; k++) {
         const int R = k < 2 ? inter : hidden, C = k < 2 ? hidden : inter;
-        {
-            cuuint64_t dims[3] = {(cuuint64_t)(C / 2), (cuuint64_t)R, (cuuint64_t)experts};
-            cuuint64_t strides[2] = {(cuuint64_t)(C / 2), (cuuint64_t)expert_stride};
-            cuuint32_t box[3] = {(cuuint32_t)(TC_KC / 2), 128u, 1u};
-            cuuint32_t estr[3] = {1, 1, 1};
-            if ((C / 2) % 16) return cudaErrorInvalidValue;
-            CUresult r = encode(&out->w[k], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,
-                                const_cast<uint8_t*>(pool + (size_t)k * tensor_bytes), dims, strides, box, estr,
-                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-        }
-        {
-            cuuint64_t dims[3] = {(cuuint64_t)(C / 2), (cuuint64_t)R, (cuuint64_t)experts};
-            cuuint64_t strides[2] = {(cuuint64_t)(C / 2), (cuuint64_t)expert_stride};
-            cuuint32_t box[3] = {(cuuint32_t)(TC_KC / 2), (cuuint32_t)TW_ROWS, 1u};
-            cuuint32_t estr[3] = {1, 1, 1};
-            CUresult r = encode(&out->w256[k], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,
-                                const_cast<uint8_t*>(pool + (size_t)k * tensor_bytes), dims, strides, box, estr,
-                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-        }
-        out->tab_tma[k] = (C % 256) == 0 ? 1 : 0;
-        if (out->tab_tma[k]) {
-            cuuint64_t dims[3] = {(cuuint64_t)(C / 16), (cuuint64_t)R, (cuuint64_t)experts};
-            cuuint64_t strides[2] = {(cuuint64_t)(C / 16), (cuuint64_t)(3 * (elems / 64) * 4)};
-            cuuint32_t box[3] = {16u, 128u, 1u};
-            cuuint32_t estr[3] = {1, 1, 1};
-            CUresult r = encode(&out->t[k], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,
-                                const_cast<uint32_t*>(tables + (size_t)k * (elems / 64)), dims, strides, box, estr,
-                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-            box[1] = (cuuint32_t)TW_ROWS;
-            r = encode(&out->t256[k], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,
-                       const_cast<uint32_t*>(tables + (size_t)k * (elems / 64)), dims, strides, box, estr,
-                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-        } else {
-            out->t[k] = out->w[k];   // never read
-            out->t256[k] = out->w256[k];
-        }
+        cuuint64_t dims[3] = {(cuuint64_t)(C / 2), (cuuint64_t)R, (cuuint64_t)experts};
+        cuuint64_t strides[2] = {(cuuint64_t)(C / 2), (cuuint64_t)expert_stride};
+        cuuint32_t box[3] = {(cuuint32_t)(TC_KC / 2), k < 2 ? 128u : (cuuint32_t)TW_ROWS, 1u};
+        cuuint32_t estr[3] = {1, 1, 1};
+        CUresult r = encode(k < 2 ? &out->w[k] : &out->w256, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3,
+                            const_cast<uint8_t*>(pool + (size_t)k * tensor_bytes), dims, strides, box, estr,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
     }
     out->pool = pool;
     out->expert_stride = expert_stride;
     out->tables = tables;
+    out->row_scale = row_scale;
+    out->row_unscale = row_unscale;
     return cudaSuccess;
 }
 
-// Does the kernel's shared-memory carve-up hold at least as many input slots as stages for a tensor with C
-// columns, in the widest token tile?  (The untiled table form keeps 256 rows x C/64 words resident.)
-static bool tc_geometry_ok(int C, bool split, int tab_bufs) {
-    const int npart = split ? 2 : 1, stages = split ? 2 : TW_STAGES;
-    const bool tab_tma = (C % 256) == 0;
-    const int tabw = tab_tma ? 0 : tab_bufs * ((TW_ROWS * (C / TC_KC) * 4 + 1023) & ~1023);
-    const int slot = TW_PK_BYTES + (tab_tma ? TW_TAB_BYTES : 0) + npart * TW_TOK_BYTES;
-    const int avail = TC_SMEM_BYTES - 1024 - stages * npart * TW_B_BYTES - tabw;
-    return avail / slot >= stages;
-}
-// Buffers for the untiled tables of a tensor with C columns: 2 where they fit, else 1, 0 if the plan does not hold at all.
-static int tc_table_buffers(int C, bool split) {
-    return tc_geometry_ok(C, split, 2) ? 2 : (tc_geometry_ok(C, split, 1) ? 1 : 0);
-}
-
+// The documented limits of the two precisions (a size that is no multiple of 256 is bounded).
 bool q4_tc_supported(int hidden, int inter, bool split) {
     if (hidden < TC_KC || inter < TC_KC || (hidden % TC_KC) || (inter % TC_KC)) return false;
-    return tc_table_buffers(hidden, split) > 0 && tc_table_buffers(inter, split) > 0;
+    const int limit = split ? 960 : 3520;
+    return ((hidden % 256) == 0 || hidden <= limit) && ((inter % 256) == 0 || inter <= limit);
 }
 
 template <bool FUSED, bool SPLIT>
-static cudaError_t launch_tc(const TcArgs& a, const TcMaps& maps, const TcWeightMaps& wm, dim3 grid,
-                                  cudaStream_t stream) {
+static cudaError_t launch_tc(const TcArgs& a, const TcMaps& maps, const TcMaps& sums, const TcWeightMaps& wm, dim3 grid,
+                             cudaStream_t stream) {
     {
         cudaError_t e = ensure_dynamic_smem((const void*)q4_gemm_tc_kernel<FUSED, SPLIT>, (size_t)TC_SMEM_BYTES);
         if (e != cudaSuccess) return e;
     }
-    q4_gemm_tc_kernel<FUSED, SPLIT><<<grid, TC_THREADS, TC_SMEM_BYTES, stream>>>(a, maps, wm);
+    q4_gemm_tc_kernel<FUSED, SPLIT><<<grid, TC_THREADS, TC_SMEM_BYTES, stream>>>(a, maps, sums, wm);
     return cudaGetLastError();
 }
 
@@ -862,18 +926,21 @@ cudaError_t launch_q4_tc_work_list(const Q4Job* gateup_jobs, const int* njobs_de
     return cudaGetLastError();
 }
 
-cudaError_t launch_q4_gemm_tc(bool fused, bool split, const void* items, int* work, const TcMaps& bmaps,
-                              const TcWeightMaps& wm, void* out_h, void* out_l, float* out_f, int R, int C, int* status,
-                              cudaStream_t stream) {
+cudaError_t launch_q4_gemm_tc(bool fused, bool split, const void* items, int* work, const TcMaps& x, const TcMaps& sums,
+                              const TcWeightMaps& wm, void* out_h, void* out_l, void* sums_h, void* sums_l, float* out_f, int R,
+                              int C, int* status, cudaStream_t stream) {
     TcArgs a;
     a.items = (const TcItem*)items; a.work = work;
     a.R = R; a.C = C;
+    a.extra = tc_sums_cols(C) / TC_KC;
     a.out_h = (__half*)out_h; a.out_l = (__half*)out_l; a.out_f = out_f; a.status = status;
+    a.sums_h = (__half*)sums_h; a.sums_l = (__half*)sums_l; a.sums_stride = tc_sums_cols(R);
     a.tables = wm.tables;
     a.tensor0 = fused ? 0 : 2;
-    a.tab_tma = wm.tab_tma[fused ? 0 : 2];
-    a.tab_bufs = tc_table_buffers(C, split);
-    if (a.tab_bufs < 1) return cudaErrorInvalidValue;
+    a.row_scale = wm.row_scale; a.row_unscale = wm.row_unscale;
+    const int inter = fused ? R : C, hidden = fused ? C : R;
+    a.scale_stride = 2 * inter + hidden;
+    a.scale_off = fused ? 0 : 2 * inter;
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -881,8 +948,8 @@ cudaError_t launch_q4_gemm_tc(bool fused, bool split, const void* items, int* wo
     // one resident block per SM; each draws units (one token pass of one row tile) from the work list until it is empty
     dim3 grid((unsigned)sms, 1, 1);
     if (fused)
-        return split ? launch_tc<true, true>(a, bmaps, wm, grid, stream) : launch_tc<true, false>(a, bmaps, wm, grid, stream);
-    return split ? launch_tc<false, true>(a, bmaps, wm, grid, stream) : launch_tc<false, false>(a, bmaps, wm, grid, stream);
+        return split ? launch_tc<true, true>(a, x, sums, wm, grid, stream) : launch_tc<true, false>(a, x, sums, wm, grid, stream);
+    return split ? launch_tc<false, true>(a, x, sums, wm, grid, stream) : launch_tc<false, false>(a, x, sums, wm, grid, stream);
 }
 
 }  // namespace sb

@@ -1,57 +1,56 @@
-// Grouped affine-Q4 expert GEMMs on the 5th-generation tensor cores (tcgen05 +
-// TMEM) for prefill-sized token groups.  TOLERANCE path: operands are fp16
-// (weights dequantised as q*s+b and rounded to fp16; activations rounded to
-// fp16), accumulation is fp32 in TMEM.  The bit-exact kernels in q4_kernels.cu
+// Grouped affine-Q4 expert GEMMs on the 5th-generation tensor cores (tcgen05 + TMEM) for prefill-sized token groups.
+// TOLERANCE path: fp16 operands, fp32 accumulation in TMEM.  The bit-exact kernels in batch_kernels.cu and q4_kernels.cu
 // remain the reference-conformant path.
 //
 // Two precisions (template SPLIT):
-//   single  one MMA per k-step, operands rounded to fp16 once: measured
-//           max |err| / max(|ref|, row rms) about 2e-3 (5e-4 of the row maximum)
-//   split   every operand is carried as hi + lo fp16 halves (lo = fp16(v - hi)) and
-//           each k-step issues Xh*Wh + Xh*Wl + Xl*Wh: operand error ~2^-22, three
-//           times the tensor work
+//   single  weights dequantised as q*s+b and rounded to fp16, activations rounded to fp16: max |err| about 5e-4 to
+//           7e-4 of the row maximum
+//   split   x * (q s + b) = x * (q - 8) s + x * (b + 8 s).  (q - 8) s has at most 4 + 8 significant bits, so it is EXACT
+//           in fp16 once the row is scaled by a power of two (q4_row_scale_kernel) that keeps it in range; b + 8 s is
+//           constant over a quantisation group, so its part of the sum is a second, 64 times shorter contraction of the
+//           groups' means of x with c = b + 8 s (hi + lo halves): one or a few "correction" chunks after the ordinary
+//           ones.  Activations are hi + lo halves (lo = fp16(x - hi)).  So a K step takes two products, Xh W and Xl W,
+//           instead of three with split weights, and a stage holds one weight tile, not two: max |err| 1.6e-5 of the row
+//           maximum, from the halves of x.  Passes of up to 64 tokens put the hi and the lo rows into ONE 128-row tile
+//           (sixteen hi rows, then their lo rows, in every quarter) and take a single MMA; the epilogue adds the two.
 //
-// A unit of work = one 128-token pass of one tile of weight rows of one expert group.  A small kernel writes
-// the layer's units into a work list from the grouped jobs (pass and tile counts are only known on the device);
-// one resident block per SM draws units from it with an atomic counter until it is empty, its pipeline (input
-// ring, converted stages, double-buffered accumulators) running on from one unit into the next.  Grids of one
-// block per tile paid for every block's launch with 225 KB of shared memory, for the empty blocks of experts
+// A unit of work = one 128-token pass of one tile of weight rows of one expert group.  A small kernel writes the layer's
+// units into a work list from the grouped jobs (pass and tile counts are only known on the device); one resident block per
+// SM draws units from it with an atomic counter until it is empty, its pipeline running on from one unit into the next.
+// Grids of one block per tile paid for every block's launch with 225 KB of shared memory, for the empty blocks of experts
 // with fewer passes than the grid allowed, and for experts with several hundred tokens finishing last.
-// The tokens of a pass (up to 128, stale rows above them) are the MMA's M side, read from shared
-// memory as they arrive by TMA; 256 weight rows are the N side, dequantised into a K-major
-// 128-byte-swizzled shared-memory stage.  The 256 rows are one tile of the down matrix, or - fused -
-// 128 rows of gate followed by the same 128 rows of up: gate and up of a chunk are ONE instruction
-// (M128 x N256 x K16), and the GeGLU pairs accumulator column c with 128 + c.  Accumulators: lane =
-// token, column = weight row.  K advances in 64-column chunks = one quantisation group per row.
-//   producer thread   draws the unit and passes it to the other roles through a shared-memory ring; packed
-//                     nibbles (tiled TMA over the expert pool: bytes x rows x experts),
-//                     the (scale << 16) | bias words of the rows (tiled TMA in blocks of four
-//                     chunks where a table row is a multiple of 16 bytes, otherwise one bulk copy
-//                     of the tile's whole table) and the tokens' fp16 activations (128-byte swizzle)
-//                     into a ring of input slots, several chunks ahead
-//   converter warps   two groups of eight warps on alternate chunks (thread = stage row): shared
-//                     memory -> registers -> Q4 -> fp16 -> the stage; one mbarrier arrival per warp
-//   issuer thread     tcgen05.mma.kind::f16 of every converted chunk, tcgen05.commit on the
-//                     chunk's "done" barrier (frees the input slot and, some chunks later, the stage);
-//                     polls the next chunk's barriers before issuing, so the answer arrives behind
-//                     the MMAs
-//   epilogue          all converter warps tcgen05.ld the accumulators after a unit (warp w: lane
-//                     quarter w % 4, a quarter of the columns): GeGLU (fused gate/up) or plain store (down);
-//                     the issuer is already filling the other accumulator buffer
-// What was measured on the way here (B200, 1965 MHz): a register ring of global loads does not prefetch -
-// waiting for the oldest load also waits for the younger ones that share its scoreboard, so every chunk paid
-// a full memory latency (hence TMA); one mbarrier operation costs the issuing thread 100-190 cycles, so the
-// one-thread issuer carries as few of them as possible; a tcgen05.mma costs the issuing thread about 100
-// cycles for any N <= 128 (weights on M, in shared memory or dequantised straight into tensor memory with
-// tcgen05.st, 128 rows per instruction: both forms ran 8 such instructions per fused chunk), so the weights sit
-// on N, 256 rows per instruction.  What bounds this form is shared-memory traffic: about 110 KB per fused chunk
-// (stage written once and read once, token tile read by every instruction) against 128 bytes per cycle.
-// Column order inside every group of 8 K columns is permuted to [0,4,1,5,2,6,3,7] in
-// BOTH operands (a contraction does not care): it is the order in which two masks
-// and one shift peel half2 pairs out of a packed 32-bit word.
-// Every mbarrier wait is bounded: on expiry the block raises a shared flag, records
-// an error in the status word, every role leaves its loop, outstanding copies and
-// MMAs are waited for (bounded), TMEM is freed and the block returns.
+// The tokens of a pass (stale rows above them) are the MMA's M side, read from shared memory as they arrive by TMA; 256
+// weight rows are the N side, dequantised into a K-major 128-byte-swizzled stage.  The 256 rows are one tile of the down
+// matrix, or - fused - 128 rows of gate followed by the same 128 rows of up: one instruction is M128 x N256 x K16, and the
+// GeGLU pairs accumulator column c with 128 + c.  Accumulators: lane = token, column = weight row, double-buffered by unit.
+// K advances in 64-column chunks = one quantisation group per row.
+//   weight thread     draws the unit and passes it to the other roles through a shared-memory ring; loads packed nibbles
+//                     (tiled TMA over the expert pool: bytes x rows x experts) into a ring of four 8 KB slots
+//   token thread      loads the tokens' fp16 rows (128-byte swizzle) into a ring of three or four tiles.  A ring of its
+//                     own: a packed slot is free as soon as its bytes are in registers, a token tile only after its MMAs
+//   converter warps   two groups of eight warps on alternate chunks (thread = stage row): packed bytes -> registers ->
+//                     fp16 -> the stage; the row's (scale << 16) | bias word comes straight from global memory a chunk
+//                     pair ahead; one mbarrier arrival per warp
+//   issuer thread     tcgen05.mma.kind::f16 of every converted chunk, tcgen05.commit on the chunk's "done" barrier; polls
+//                     the next chunk's barriers before issuing, so the answer arrives behind the MMAs
+//   epilogue          all converter warps tcgen05.ld the accumulators of a unit (warp w: lane quarter w % 4, a quarter of
+//                     the columns), sixteen columns at a time to stay inside 96 registers: GeGLU (fused gate/up) or plain
+//                     store (down).  It runs after the group's second chunk of the NEXT unit, so that the tensor core
+//                     does not drain at a unit's end
+// Measured (B200, 1965 MHz, a whole expert layer: hidden 2816, inter 704, 128 experts,
+// top-8): 512 tokens in split precision 800 us with three MMAs per K step on split weights -> 515 with exact weights and
+// separate rings -> 473 with the delayed epilogue, four stages and the correction chunk's table words loaded at once (they
+// came in four serial batches, 9000 cycles a chunk).  1999 tokens in single precision 780 -> 707 -> 694.  In the same
+// state the tensor pipe is busy 35 to 40 % of the time and the schedulers issue in 45 % of the cycles.
+// What was measured on the way here: a register ring of global loads for the packed bytes does not prefetch - waiting for
+// the oldest load also waits for the younger ones that share its scoreboard (hence TMA); one mbarrier wait costs 150 to 250
+// cycles even when its phase is complete, so the phases needed next are tested ahead; a tcgen05.mma costs the issuing
+// thread about 100 cycles for any N <= 128 (weights on M, from shared memory or from tensor memory: both forms ran 8 such
+// instructions per fused chunk), so the weights sit on N, 256 rows per instruction.
+// Column order inside every group of 8 K columns is permuted to [0,4,1,5,2,6,3,7] in BOTH operands (a contraction does not
+// care): it is the order in which two masks and one shift peel half2 pairs out of a packed 32-bit word.
+// Every mbarrier wait is bounded: on expiry the block raises a shared flag, records an error in the status word, every role
+// leaves its loop, outstanding copies and MMAs are waited for (bounded), TMEM is freed and the block returns.
 #include <cuda_fp16.h>
 
 #include <stdlib.h>
@@ -71,7 +70,7 @@ constexpr int TC_KC = 64;                    // K columns per chunk
 constexpr uint32_t TC_TMEM_COLS = 512;
 constexpr int TC_PK_BYTES = 128 * TC_KC / 2; // packed chunk of 128 rows (one matrix' share of a fused stage)
 constexpr int TC_MAX_NT = 128;
-constexpr int TC_MAX_SLOTS = 8;
+constexpr int TC_MAX_SLOTS = 4;              // packed chunks in flight
 // Entries of the ring through which the thread that draws the units passes them to the other roles.  It is at most
 // TC_MAX_SLOTS chunks, i.e. units, ahead of the converters, and no role is more than three chunks and a unit behind
 // those, so 16 entries are never overrun and need no "free" barrier.
@@ -206,12 +205,22 @@ __device__ __forceinline__ void dequant_exact(const uint4& p, uint32_t s2, uint3
 }
 
 // 32 columns of this lane -> 16: the sums with lane ^ 16, of columns 0..15 in the lower half of the warp, 16..31 in the upper.
-__device__ __forceinline__ void sum_halves(uint32_t (&v)[32], int upper) {
+__device__ __forceinline__ void sum_halves(const uint32_t (&v)[32], int upper, uint32_t (&o)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; i++) {
         const float mine = __uint_as_float(upper ? v[16 + i] : v[i]), other = __uint_as_float(upper ? v[i] : v[16 + i]);
-        v[i] = __float_as_uint(mine + __shfl_xor_sync(0xffffffffu, other, 16));
+        o[i] = __float_as_uint(mine + __shfl_xor_sync(0xffffffffu, other, 16));
     }
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
 // Mean of quantisation group g of a row as the correction chunks read it: chunk g / 32, K step (g % 32) / 8, columns
@@ -312,7 +321,7 @@ constexpr int TW_ROWS = 256;                        // rows of a converted stage
 constexpr int TW_PK_BYTES = TW_ROWS * TC_KC / 2;    // packed chunk
 constexpr int TW_B_BYTES = TW_ROWS * TC_KC * 2;     // converted chunk
 constexpr int TW_TOK_BYTES = TC_MAX_NT * TC_KC * 2; // token tile of 128 rows
-constexpr int TW_STAGES = 3;                        // converted stages, and token tiles
+constexpr int TW_STAGES = 4;                        // most converted stages, and token tiles
 constexpr int TW_PACK_MAX = 64;                     // split: passes of up to this many tokens carry hi and lo in ONE tile
 
 template <bool FUSED, bool SPLIT>
@@ -333,6 +342,7 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
     __shared__ __align__(16) TcItem s_items[TC_ITEM_RING];
     __shared__ __align__(8) uint64_t bar_item[TC_ITEM_RING];  // ring entry published
     __shared__ float s_half[2][TC_MAX_NT];                    // half sums of two 64-column groups (fused, split)
+    __shared__ __align__(8) uint64_t bar_half[2][8];          // ... written by one warp of a pair, read by the other
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
 
@@ -343,15 +353,17 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
     // carve-up: converted stages | token tiles (room for the launch's largest pass) | packed chunks.  The MMA always
     // reads 128 token rows: those above the copied boxes are stale bytes and only reach accumulator lanes nobody reads.
     uint8_t* stage_base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    uint8_t* tok_base = stage_base + TW_STAGES * TW_B_BYTES;
     const int nt_max = *(volatile const int*)&a.work[2];
     const uint32_t tok_room = SPLIT ? (nt_max <= TW_PACK_MAX ? (uint32_t)TW_TOK_BYTES : 2u * TW_TOK_BYTES)
                                     : (nt_max <= 16 ? 2048u : nt_max <= 32 ? 4096u : nt_max <= 64 ? 8192u : (uint32_t)TW_TOK_BYTES);
-    uint8_t* pk_base = tok_base + TW_STAGES * tok_room;
-    const uint32_t pk_avail = (uint32_t)TC_SMEM_BYTES - 1024u - TW_STAGES * ((uint32_t)TW_B_BYTES + tok_room);
-    const uint32_t NW = pk_avail >= 8u * TW_PK_BYTES ? 8u : 4u;          // 128-token split passes: exactly four
-    static_assert(TC_SMEM_BYTES - 1024 - TW_STAGES * (TW_B_BYTES + 2 * TW_TOK_BYTES) >= 4 * TW_PK_BYTES, "packed ring");
-    const uint32_t nw_shift = NW == 8u ? 3u : 2u;
+    // stages, token tiles and packed chunks in flight: four of each (two stages per converter group), or three stages
+    // where a token tile holds 128 rows of hi and of lo; the rest is packed chunks
+    const uint32_t ND = tok_room <= (uint32_t)TW_TOK_BYTES ? 4u : 3u;
+    uint8_t* tok_base = stage_base + ND * TW_B_BYTES;
+    uint8_t* pk_base = tok_base + ND * tok_room;
+    constexpr uint32_t NW = 4, nw_shift = 2;
+    static_assert(TC_SMEM_BYTES - 1024 - 3 * (TW_B_BYTES + 2 * TW_TOK_BYTES) >= (int)NW * TW_PK_BYTES, "packed ring");
+    static_assert(TC_SMEM_BYTES - 1024 - 4 * (TW_B_BYTES + TW_TOK_BYTES) >= (int)NW * TW_PK_BYTES, "packed ring");
     volatile int* fail = &s_fail;
 
     if (tid == 0) {
@@ -368,6 +380,7 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
         for (int s = 0; s < 2; s++) {
             mbar_init(&bar_acc[s], 1);
             mbar_init(&bar_epi[s], TC_CONVERTERS / 32);
+            for (int i = 0; i < 8; i++) mbar_init(&bar_half[s][i], 1);
         }
         s_fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -392,118 +405,55 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
         const uint32_t b_sw = ((uint32_t)crow & 7) << 4;
         const NibbleMagic mg = load_nibble_magic();
         uint32_t it0 = 0, w0 = 0;                                // chunks, packed chunks before this unit
-        bool alive = true;
-        for (uint32_t unit = 0; alive && !*fail; unit++) {
-            alive = __all_sync(0xffffffffu, mbar_wait(&bar_item[unit % TC_ITEM_RING], (unit / TC_ITEM_RING) & 1u, fail));
-            if (!alive) break;
-            const TcItem item = s_items[unit % TC_ITEM_RING];
-            if (item.nt < 1) break;                                      // end of the work
-            const int r0 = item.r0, rows_here = min(RT, a.R - r0);      // rows_here: a multiple of 64
-            const int mat = FUSED ? crow / RT : 0, row = min(r0 + crow % RT, a.R - 1);
-            const uint32_t* tab = a.tables + ((size_t)(item.expert * 3 + a.tensor0 + mat) * a.R + row) * nchunks;
-            float rs = 1.0f;
-            if (SPLIT) rs = __ldg(a.row_scale + (size_t)item.expert * a.scale_stride + a.scale_off + mat * a.R + row);
-            // this group's chunks of the unit: every other one of the block's running count
-            const int first = (int)((it0 ^ grp) & 1u);
-            uint32_t word_next = first < nchunks ? __ldg(tab + first) : 0u;
-            for (int kc = first; kc < total; kc += 2) {
-                const uint32_t it = it0 + (uint32_t)kc, s = it % TW_STAGES, round = it / TW_STAGES;
-                uint8_t* const st = line + s * TW_B_BYTES;
-                if (!SPLIT || kc < nchunks) {
-                    const uint32_t slot = (w0 + kc) & (NW - 1), wph = ((w0 + kc) >> nw_shift) & 1u;
-                    const uint32_t word = word_next;
-                    word_next = kc + 2 < nchunks ? __ldg(tab + kc + 2) : 0u;     // a chunk pair ahead: its latency is covered
-                    if (!__all_sync(0xffffffffu, mbar_wait(&bar_w[slot], wph, fail))) { alive = false; break; }
-                    const uint8_t* pk = pk_base + slot * TW_PK_BYTES + crow * 32;
-                    const uint4 p[2] = {lds_v4(pk), lds_v4(pk + 16)};
-                    // the MMAs that last read this stage: asked now, needed after the conversion
-                    uint32_t stage_free = round == 0 ? 1u : mbar_test(&bar_done[s], (round - 1) & 1u);
-                    uint32_t o[2][16];
-                    const uint32_t s_bits = word >> 16, b_bits = word & 0xffffu;
-                    if (SPLIT) {
-                        const float sc = bf16_bits_to_f32(s_bits) * rs;
-                        const uint32_t s2 = f16x2_from(sc, sc), s2_16 = f16x2_from(sc * 0.0625f, sc * 0.0625f);
-                        dequant_exact(p[0], s2, s2_16, o[0]);
-                        dequant_exact(p[1], s2, s2_16, o[1]);
-                    } else if (fp16_path_ok(s_bits, b_bits)) {
-                        dequant_half_chunk_f16(p[0], s_bits, b_bits, o[0]);
-                        dequant_half_chunk_f16(p[1], s_bits, b_bits, o[1]);
-                    } else {
-                        dequant_half_chunk_f32(mg, p[0], s_bits, b_bits, o[0]);
-                        dequant_half_chunk_f32(mg, p[1], s_bits, b_bits, o[1]);
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bar_wfree[slot]);        // the packed bytes have been used
-                    if (!__all_sync(0xffffffffu, stage_free) &&
-                        !__all_sync(0xffffffffu, mbar_wait(&bar_done[s], (round - 1) & 1u, fail))) { alive = false; break; }
-#pragma unroll
-                    for (int i = 0; i < 8; i++)
-                        *(uint4*)(st + (((uint32_t)i << 4) ^ b_sw)) =
-                            make_uint4(o[i >> 2][4 * (i & 3)], o[i >> 2][4 * (i & 3) + 1], o[i >> 2][4 * (i & 3) + 2],
-                                       o[i >> 2][4 * (i & 3) + 3]);
-                } else {
-                    // correction chunk: 32 groups, eight per K step of 16 columns: 64 c as hi, then as lo halves
-                    if (round > 0 && !__all_sync(0xffffffffu, mbar_wait(&bar_done[s], (round - 1) & 1u, fail))) { alive = false; break; }
-                    const int g0 = (kc - nchunks) * 32;
-#pragma unroll 1
-                    for (int ks = 0; ks < 4; ks++) {
-                        uint32_t hi[4], lo[4];
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            float c[2];
-#pragma unroll
-                            for (int k = 0; k < 2; k++) {
-                                const int g = g0 + ks * 8 + 2 * j + k;
-                                const uint32_t w = g < nchunks ? __ldg(tab + g) : 0u;
-                                c[k] = (bf16_bits_to_f32(w & 0xffffu) + 8.0f * bf16_bits_to_f32(w >> 16)) * (64.0f * rs);
-                            }
-                            hi[j] = f16x2_from(c[0], c[1]);
-                            lo[j] = f16x2_from(c[0] - f16_lo_to_f32(hi[j]), c[1] - f16_hi_to_f32(hi[j]));
-                        }
-                        *(uint4*)(st + (((uint32_t)(2 * ks) << 4) ^ b_sw)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                        *(uint4*)(st + (((uint32_t)(2 * ks + 1) << 4) ^ b_sw)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-                    }
-                }
-                // generic-proxy writes -> visible to the tensor core (async proxy), then one arrival per warp
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bar_full[s]);
+        uint32_t half_phase = 0;                                 // phase of this warp's half sums
+        // Epilogue of a unit: warp w reads lane quarter w % 4 (tokens) and a quarter of the columns.
+        auto epilogue = [&](const TcItem& item, uint32_t unit) -> bool {
+            // the unit's row factors, a column per lane, on their way before the accumulators are final
+            const int q = warp & 3, cq = warp >> 2, rows_here = min(RT, a.R - item.r0), r0 = item.r0;
+            float un_a = 1.0f, un_b = 1.0f;                              // fused: gate, up; plain: columns 0..31, 32..63
+            if (SPLIT) {
+                const float* un = a.row_unscale + (size_t)item.expert * a.scale_stride + a.scale_off + r0;
+                const int c = FUSED ? cq * 32 : cq * 64;
+                if (c < rows_here) un_a = __ldg(un + c + lane);
+                if (FUSED ? c < rows_here : c + 32 < rows_here) un_b = __ldg(un + (FUSED ? a.R + c : c + 32) + lane);
             }
-            it0 += (uint32_t)total;
-            w0 += (uint32_t)nchunks;
-            // ---- epilogue: warp w reads lane quarter w % 4 (tokens) and a quarter of the columns
-            if (!alive || !__all_sync(0xffffffffu, mbar_wait(&bar_acc[unit & 1u], (unit >> 1) & 1u, fail))) { alive = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(&bar_acc[unit & 1u], (unit >> 1) & 1u, fail))) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int q = warp & 3, cq = warp >> 2;
             const bool packed = SPLIT && item.nt <= TW_PACK_MAX;
             // packed: lanes 0..15 of a quarter hold sixteen tokens' hi products, lanes 16..31 the lo products of the same
             // tokens; after their sum the two halves of the warp share the columns
             const int n = packed ? q * 16 + (lane & 15) : q * 32 + lane;         // token of the pass
             const int half0 = packed ? lane >> 4 : 0, halves = packed ? 1 : 2;
             const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (unit & 1u) * TW_ROWS;
-            const float* un = SPLIT ? a.row_unscale + (size_t)item.expert * a.scale_stride + a.scale_off + r0 : nullptr;
+            // sixteen columns of this lane: the sums of the two halves, or columns c ... c + 15
+            auto sixteen = [&](uint32_t c, int h, uint32_t (&v)[16]) {
+                if (packed) {
+                    uint32_t t[32];
+                    tmem_ld32(trow + c, t);
+                    sum_halves(t, half0, v);
+                } else {
+                    tmem_ld16(trow + c + h * 16, v);
+                }
+            };
             if ((packed ? q * 16 : q * 32) < item.nt) {                          // warp-uniform: the quarter holds tokens
                 if (FUSED) {
                     const int col = cq * 32;                                     // output columns col ... col + 31 of the tile
                     if (col < rows_here) {
-                        uint32_t g[32], u[32];
-                        tmem_ld32(trow + col, g);
-                        tmem_ld32(trow + RT + col, u);
-                        if (packed) {
-                            sum_halves(g, half0);
-                            sum_halves(u, half0);
-                        }
                         float sum = 0.0f;
+#pragma unroll 1
                         for (int h = 0; h < halves; h++) {
-                            const int c0 = col + (packed ? half0 : h) * 16;
+                            const int cc = (packed ? half0 : h) * 16, c0 = col + cc;
                             const size_t o_off = (size_t)(item.grow + n) * a.R + r0 + c0;
+                            uint32_t g[16], u[16];
+                            sixteen(col, h, g);
+                            sixteen(RT + col, h, u);
                             float o[16];
 #pragma unroll
                             for (int i = 0; i < 16; i++) {
-                                float gv = __uint_as_float(h == 0 ? g[i] : g[16 + i]), uv = __uint_as_float(h == 0 ? u[i] : u[16 + i]);
+                                float gv = __uint_as_float(g[i]), uv = __uint_as_float(u[i]);
                                 if (SPLIT) {
-                                    gv *= __ldg(un + c0 + i);
-                                    uv *= __ldg(un + a.R + c0 + i);
+                                    gv *= __shfl_sync(0xffffffffu, un_a, cc + i);
+                                    uv *= __shfl_sync(0xffffffffu, un_b, cc + i);
                                 }
                                 o[i] = geglu_fast(gv, uv);
                                 sum += o[i];
@@ -527,11 +477,21 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
                         if (SPLIT) {
                             // mean of a 64-column group: 32 columns here, 32 in the warp four further on
                             if (packed) sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-                            if (cq & 1) s_half[cq >> 1][n] = sum;
-                            asm volatile("bar.sync %0, 64;" ::"r"(1 + q * 2 + (cq >> 1)) : "memory");
-                            if (!(cq & 1) && n < item.nt && (!packed || lane < 16))
-                                store_group_mean(a.sums_h, a.sums_l, (size_t)(item.grow + n) * a.sums_stride, (r0 + col) / TC_KC,
-                                                 (sum + s_half[cq >> 1][n]) * (1.0f / TC_KC));
+                            float* half = s_half[cq >> 1];
+                            const int pair = q * 2 + (cq >> 1);
+                            // the writer waits until the sums before have been read (at its first time: passes at once)
+                            const uint32_t parity = half_phase ^ (uint32_t)(cq & 1);
+                            half_phase ^= 1u;
+                            if (!__all_sync(0xffffffffu, mbar_wait(&bar_half[cq & 1][pair], parity, fail))) return false;
+                            if (cq & 1) {
+                                half[n] = sum;
+                            } else {
+                                if (n < item.nt && (!packed || lane < 16))
+                                    store_group_mean(a.sums_h, a.sums_l, (size_t)(item.grow + n) * a.sums_stride, (r0 + col) / TC_KC,
+                                                     (sum + half[n]) * (1.0f / TC_KC));
+                            }
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&bar_half[(cq & 1) ^ 1][pair]);
                         }
                     }
                 } else {
@@ -539,26 +499,22 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
                     for (int c1 = 0; c1 < 64; c1 += 32) {
                         const int col = cq * 64 + c1;
                         if (col >= rows_here) break;
-                        uint32_t g[32];
-                        tmem_ld32(trow + col, g);
-                        if (packed) sum_halves(g, half0);
-                        if (n < item.nt) {
-                            for (int h = 0; h < halves; h++) {
-                                const int c0 = col + (packed ? half0 : h) * 16;
-                                float* dst = a.out_f + (size_t)(item.grow + n) * a.R + r0 + c0;
+                        const float f = c1 ? un_b : un_a;
+#pragma unroll 1
+                        for (int h = 0; h < halves; h++) {
+                            const int cc = (packed ? half0 : h) * 16;
+                            uint32_t g[16];
+                            sixteen(col, h, g);
+                            float* dst = a.out_f + (size_t)(item.grow + n) * a.R + r0 + col + cc;
+                            float o[16];
 #pragma unroll
-                                for (int i = 0; i < 16; i += 4) {
-                                    float4 v;
-                                    v.x = __uint_as_float(h == 0 ? g[i] : g[16 + i]);
-                                    v.y = __uint_as_float(h == 0 ? g[i + 1] : g[17 + i]);
-                                    v.z = __uint_as_float(h == 0 ? g[i + 2] : g[18 + i]);
-                                    v.w = __uint_as_float(h == 0 ? g[i + 3] : g[19 + i]);
-                                    if (SPLIT) {
-                                        const float4 k = __ldg((const float4*)(un + c0 + i));
-                                        v.x *= k.x; v.y *= k.y; v.z *= k.z; v.w *= k.w;
-                                    }
-                                    *(float4*)(dst + i) = v;
-                                }
+                            for (int i = 0; i < 16; i++) {
+                                o[i] = __uint_as_float(g[i]);
+                                if (SPLIT) o[i] *= __shfl_sync(0xffffffffu, f, cc + i);
+                            }
+                            if (n < item.nt) {
+#pragma unroll
+                                for (int i = 0; i < 16; i += 4) *(float4*)(dst + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
                             }
                         }
                     }
@@ -567,6 +523,114 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar_epi[unit & 1u]);
+            return true;
+        };
+        bool alive = true, pending = false;
+        TcItem prev = {0, 0, 0, 0};
+        for (uint32_t unit = 0; alive && !*fail; unit++) {
+            alive = __all_sync(0xffffffffu, mbar_wait(&bar_item[unit % TC_ITEM_RING], (unit / TC_ITEM_RING) & 1u, fail));
+            if (!alive) break;
+            const TcItem item = s_items[unit % TC_ITEM_RING];
+            const int mine = item.nt < 1 ? 0 : total;                    // nt < 1: end of the work
+            const int mat = FUSED ? crow / RT : 0, row = min(item.r0 + crow % RT, a.R - 1);
+            const uint32_t* tab = a.tables + ((size_t)(item.expert * 3 + a.tensor0 + mat) * a.R + row) * nchunks;
+            float rs = 1.0f;
+            if (SPLIT) rs = __ldg(a.row_scale + (size_t)item.expert * a.scale_stride + a.scale_off + mat * a.R + row);
+            // this group's chunks of the unit: every other one of the block's running count
+            const int first = (int)((it0 ^ grp) & 1u);
+            uint32_t word_next = mine > 0 && first < nchunks ? __ldg(tab + first) : 0u;
+            // The unit before is finished after this group's second chunk: the tensor core has work while its accumulators
+            // are read, and no converter waits for its last MMA.
+            uint32_t w_here = 0u;
+            for (int kc = first, n = 0;; kc += 2, n++) {
+                if (pending && (n == 2 || kc >= mine)) {
+                    pending = false;
+                    if (!epilogue(prev, unit - 1)) { alive = false; break; }
+                }
+                if (kc >= mine) break;
+                const uint32_t it = it0 + (uint32_t)kc, round = ND == 4u ? it >> 2 : it / 3u, s = it - round * ND;
+                uint8_t* const st = line + s * TW_B_BYTES;
+                if (!SPLIT || kc < nchunks) {
+                    const uint32_t slot = (w0 + kc) & (NW - 1), wph = ((w0 + kc) >> nw_shift) & 1u;
+                    const uint32_t word = word_next;
+                    word_next = kc + 2 < nchunks ? __ldg(tab + kc + 2) : 0u;     // a chunk pair ahead: its latency is covered
+                    if (!__all_sync(0xffffffffu, w_here) && !__all_sync(0xffffffffu, mbar_wait(&bar_w[slot], wph, fail))) { alive = false; break; }
+                    const uint8_t* pk = pk_base + slot * TW_PK_BYTES + crow * 32;
+                    const uint4 p[2] = {lds_v4(pk), lds_v4(pk + 16)};
+                    // the MMAs that last read this stage: asked now, needed after the conversion
+                    uint32_t stage_free = round == 0 ? 1u : mbar_test(&bar_done[s], (round - 1) & 1u);
+                    uint32_t o[2][16];
+                    const uint32_t s_bits = word >> 16, b_bits = word & 0xffffu;
+                    if (SPLIT) {
+                        const float sc = bf16_bits_to_f32(s_bits) * rs;
+                        const uint32_t s2 = f16x2_from(sc, sc), s2_16 = f16x2_from(sc * 0.0625f, sc * 0.0625f);
+                        dequant_exact(p[0], s2, s2_16, o[0]);
+                        dequant_exact(p[1], s2, s2_16, o[1]);
+                    } else if (fp16_path_ok(s_bits, b_bits)) {
+                        dequant_half_chunk_f16(p[0], s_bits, b_bits, o[0]);
+                        dequant_half_chunk_f16(p[1], s_bits, b_bits, o[1]);
+                    } else {
+                        dequant_half_chunk_f32(mg, p[0], s_bits, b_bits, o[0]);
+                        dequant_half_chunk_f32(mg, p[1], s_bits, b_bits, o[1]);
+                    }
+                    // this group's next packed chunk: asked now, needed in the next round (not across units: the slot's
+                    // chunk before has to be one that this group has used, or the parity could be that of an older phase)
+                    w_here = 0u;
+                    if (kc + 2 < nchunks && kc + 2 >= (int)NW)
+                        w_here = mbar_test(&bar_w[(w0 + kc + 2) & (NW - 1)], ((w0 + kc + 2) >> nw_shift) & 1u);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bar_wfree[slot]);        // the packed bytes have been used
+                    if (!__all_sync(0xffffffffu, stage_free) &&
+                        !__all_sync(0xffffffffu, mbar_wait(&bar_done[s], (round - 1) & 1u, fail))) { alive = false; break; }
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        *(uint4*)(st + (((uint32_t)i << 4) ^ b_sw)) =
+                            make_uint4(o[i >> 2][4 * (i & 3)], o[i >> 2][4 * (i & 3) + 1], o[i >> 2][4 * (i & 3) + 2],
+                                       o[i >> 2][4 * (i & 3) + 3]);
+                } else {
+                    // correction chunk: 32 groups, eight per K step of 16 columns: 64 c as hi, then as lo halves
+                    if (round > 0 && !__all_sync(0xffffffffu, mbar_wait(&bar_done[s], (round - 1) & 1u, fail))) { alive = false; break; }
+                    const int g0 = (kc - nchunks) * 32;
+                    uint32_t w[32];                                      // all words of the row at once: one latency
+                    if ((nchunks & 3) == 0) {
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                            if (g0 + 4 * j < nchunks) v = __ldg((const uint4*)(tab + g0) + j);
+                            w[4 * j] = v.x; w[4 * j + 1] = v.y; w[4 * j + 2] = v.z; w[4 * j + 3] = v.w;
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) w[j] = g0 + j < nchunks ? __ldg(tab + g0 + j) : 0u;
+                    }
+#pragma unroll
+                    for (int ks = 0; ks < 4; ks++) {
+                        uint32_t hi[4], lo[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            float c[2];
+#pragma unroll
+                            for (int k = 0; k < 2; k++) {
+                                const uint32_t v = w[ks * 8 + 2 * j + k];
+                                c[k] = (bf16_bits_to_f32(v & 0xffffu) + 8.0f * bf16_bits_to_f32(v >> 16)) * (64.0f * rs);
+                            }
+                            hi[j] = f16x2_from(c[0], c[1]);
+                            lo[j] = f16x2_from(c[0] - f16_lo_to_f32(hi[j]), c[1] - f16_hi_to_f32(hi[j]));
+                        }
+                        *(uint4*)(st + (((uint32_t)(2 * ks) << 4) ^ b_sw)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                        *(uint4*)(st + (((uint32_t)(2 * ks + 1) << 4) ^ b_sw)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    }
+                }
+                // generic-proxy writes -> visible to the tensor core (async proxy), then one arrival per warp
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_full[s]);
+            }
+            if (mine == 0) break;
+            it0 += (uint32_t)total;
+            w0 += (uint32_t)nchunks;
+            prev = item;
+            pending = true;
         }
     } else if (warp == TC_ISSUER_WARP) {
         // ================= issuer (one thread) =================
@@ -590,7 +654,7 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
                     if (!ready) ok = mbar_wait2(&bar_full[s], ph, &bar_tok[s], ph, fail);
                     if (!ok) break;
                     // poll the next chunk's barriers now; the answer arrives behind this chunk's MMAs
-                    const uint32_t ns = s + 1 == TW_STAGES ? 0 : s + 1, nph = s + 1 == TW_STAGES ? ph ^ 1u : ph;
+                    const uint32_t ns = s + 1 == ND ? 0 : s + 1, nph = s + 1 == ND ? ph ^ 1u : ph;
                     const uint32_t r_full = mbar_test(&bar_full[ns], nph), r_tok = mbar_test(&bar_tok[ns], nph);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t wlo = w_lo0 + s * (TW_B_BYTES >> 4), tlo = t_lo0 + s * (tok_room >> 4);
@@ -652,7 +716,7 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
             const int variant = item.nt <= 16 ? 0 : item.nt <= 32 ? 1 : item.nt <= 64 ? 2 : 3;
             const uint32_t bytes = packed ? (uint32_t)boxes * 2u * 2048u : (SPLIT ? 2u : 1u) * ((16u << variant) * 128u);
             for (int kc = 0; kc < total; kc++) {
-                const uint32_t s = requested % TW_STAGES, round = requested / TW_STAGES;
+                const uint32_t round = ND == 4u ? requested >> 2 : requested / 3u, s = requested - round * ND;
                 if (round > 0 && !mbar_wait(&bar_done[s], (round - 1) & 1u, fail)) { pok = false; break; }
                 const uint32_t dst = smem_u32(tok_base + s * tok_room);
                 const TcMaps& m = kc < nchunks ? maps : sums;
@@ -680,10 +744,10 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
             for (uint32_t t = (requested > NW ? requested - NW : 0); t < requested; t++)
                 (void)mbar_wait(&bar_w[t & (NW - 1)], (t >> nw_shift) & 1u, &none);
         if (lane == 0 && warp == TC_TOKEN_WARP)
-            for (uint32_t t = (requested > TW_STAGES ? requested - TW_STAGES : 0); t < requested; t++)
-                (void)mbar_wait(&bar_tok[t % TW_STAGES], (t / TW_STAGES) & 1u, &none);
+            for (uint32_t t = (requested > ND ? requested - ND : 0); t < requested; t++)
+                (void)mbar_wait(&bar_tok[t % ND], (t / ND) & 1u, &none);
         if (lane == 0 && warp == TC_ISSUER_WARP && requested > 0)
-            (void)mbar_wait(&bar_done[(requested - 1) % TW_STAGES], ((requested - 1) / TW_STAGES) & 1u, &none);
+            (void)mbar_wait(&bar_done[(requested - 1) % ND], ((requested - 1) / ND) & 1u, &none);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

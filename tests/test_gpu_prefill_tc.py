@@ -84,3 +84,35 @@ def test_tensor_core_prefill_one_table_buffer_and_refusal(orc, synth):
     assert err1 <= TOL, err1
     assert st.status() == 0
     st.close()
+
+
+# Passes at the edges of the packed hi/lo tile (64 tokens) and of a pass (128); hidden = 36 groups: two correction chunks
+# for gate and up.  Rows whose scales span ten decades (fp16 holds them only after the rows' power-of-two factors) and
+# biases that are no multiple of the scale; every output column is held against its own scale.
+@pytest.mark.parametrize("B", [1, 16, 17, 64, 65, 129])
+def test_split_precision_row_scales_and_pass_edges(orc, synth, B):
+    H, M, E, K = 2304, 256, 2, 2                        # top-2 of 2: every expert gets all B tokens
+    layer = synth.make_q4_moe_layer(300 + B, hidden=H, inter=M, n_experts=E, topk=K)
+    rng = np.random.default_rng(301)
+    tb = layer.expert_stride // 3
+    for e in range(E):
+        for which, (lo, hi) in enumerate(((-3.0, 0.0), (-3.0, 0.0), (-6.0, 4.0))):
+            R, C = (H, M) if which == 2 else (M, H)
+            vb, gb = synth.q4_tensor_bytes(R, C)
+            blob = layer.pool[e * layer.expert_stride + which * tb:][:tb]
+            # both experts' rows alike, so that a column of the sum is as small as its parts
+            row = 10.0 ** np.random.default_rng(302 + which).uniform(lo, hi, (R, 1))
+            s = synth.bf16_round((row * rng.uniform(0.005, 0.02, (R, C // 64))).astype(np.float32))
+            b = synth.bf16_round((synth.bf16_to_f32(s) * rng.uniform(-16.0, 2.0, s.shape)).astype(np.float32))
+            blob[vb:vb + gb] = s.reshape(-1).view(np.uint8)
+            blob[vb + gb:] = b.reshape(-1).view(np.uint8)
+    x = synth.make_tokens(303 + B, B, H)
+    st = stack_mod().MoeStack(B, H, M, E, K)
+    st.add_layer(layer)
+    y = _run_tc_layer(st, x, B, H, "split")
+    want = orc.moe_layer_q4(layer, x, threads=16)[0]
+    row = row.reshape(1, H)                             # the down rows' factors: the columns of y on one scale
+    err = float(np.abs((y.astype(np.float64) - want) / row).max() / np.sqrt(((want / row) ** 2).mean()))
+    print(f"split precision, scales over ten decades, {B} tokens: {err:.3e} of the scaled columns' rms")
+    assert err <= TOL, err
+    st.close()

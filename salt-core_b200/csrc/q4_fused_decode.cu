@@ -454,13 +454,13 @@ constexpr int LAYER_NV = 5;                 // columns per thread of the row-wis
 constexpr int LAYER_SLOTS = 40;
 
 struct LayerScratch {                        // offsets in floats from the start of shared memory
-    int sq, rin, wrow, logits, pes, lit, topk, scan, end;
+    int sq, prod, wrow, pes, lit, topk, scan, end;
 };
 static __host__ __device__ __forceinline__ LayerScratch layer_scratch(int H, int E, int topk) {
     LayerScratch L;
-    const int h4 = (H + 3) & ~3;
-    L.sq = 0; L.rin = h4; L.wrow = 2 * h4; L.logits = 3 * h4;
-    L.pes = L.logits + ((E + 3) & ~3);           // the layer's per-expert scales ...
+    const int h64 = (H + 63) & ~63;
+    L.sq = 0; L.prod = h64; L.wrow = 2 * h64;
+    L.pes = 3 * h64;                             // the layer's per-expert scales ...
     L.lit = L.pes + ((E + 3) & ~3);              // ... and literal-dequantisation flags, fetched before the grid dependency
     L.topk = L.lit + ((E + 3) & ~3);
     L.scan = L.topk + topk_scratch_floats(E, topk);
@@ -487,9 +487,8 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
     const LayerScratch L = layer_scratch(H, E, K);
     float* const fsm = (float*)smem;
     float* const sq = fsm + L.sq;                 // squares / products for the in-order chains
-    float* const rin = fsm + L.rin;               // router input
+    float* const prod = fsm + L.prod;             // router input times the expert's weights
     float* const wrow = fsm + L.wrow;             // router weights of this block's expert
-    float* const s_logits = fsm + L.logits;
     float* const s_pes = fsm + L.pes;
     int* const s_lit = (int*)(fsm + L.lit);
     float* const tk = fsm + L.topk;
@@ -502,6 +501,7 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
     bool bad = false, timeout = false;
 
     // ---- before the dependency: barriers, this block's router row, the norm weights ----
+    if (tid == 32) s_root = __fdiv_rn(1.0f, sqrtf_exact((float)H));      // beside the copies: not in the chain below
     if (tid == 0) {
         if (STACKED && li > 0) S.inval_barriers();    // every wait of the previous layer is over (block barrier at its end)
         S.init_barriers();
@@ -614,78 +614,49 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
         const float ss = layer_ordered_sum(sq, H, bad, scan);
         if (tid == 0) {
             s_inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)H), a.eps_router));
-            s_root = __fdiv_rn(1.0f, sqrtf_exact((float)H));
             if (!finite_f(s_inv) || !finite_f(s_root)) flag(a.f.status, SB_ERR_NONFINITE);
         }
+        if (cta < E && !fused_mbar_wait(S.bar_x, 0)) timeout = true;     // the router row, long here
         __syncthreads();
         const float inv = s_inv, root = s_root;
 #pragma unroll
         for (int j = 0; j < NV; j++) {
-            const int d = tid + j * NT;
-            if (d < H) {
-                const float t = __fmul_rn(__fmul_rn(__fmul_rn(v[j], inv), rs[j]), root);
-                bad |= !finite_f(t);
-                rin[d] = t;
-            }
+            const float t = __fmul_rn(__fmul_rn(__fmul_rn(v[j], inv), rs[j]), root);
+            if (tid + j * NT < H) bad |= !finite_f(t);
+            v[j] = t;
         }
     }
     if (bad) flag(a.f.status, SB_ERR_NONFINITE);
-    __syncthreads();                // the router input is complete
-    // ---- router logits: expert e = cta, cta + grid, ... ----
+    // ---- router logits: expert e = cta, cta + grid, ...: acc = fl(acc + fl(W[c] * rin[c])), c ascending (reference
+    // src/kernels.c:98-106).  Every thread leaves the products of its columns, one warp adds them (a product of +0 past
+    // the last column changes nothing: a sum that starts at +0 is never -0).  The products in one warp's registers, the
+    // sum handed from lane to lane, took 16800 cycles where this takes about 12000 ----
     uint32_t ph_w = 0;
+    const int H64 = (H + 63) & ~63;
     for (int e = cta; e < E; e += ncta) {
-        if (e != cta && tid == 0) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_expect_tx(S.bar_x, (uint32_t)(H * 4));
-            bulk_g2s(wrow, a.router_w + (size_t)e * H, (uint32_t)(H * 4), S.bar_x);
-        }
-        if (warp == 0) {
-            if (!fused_mbar_wait(S.bar_x, ph_w & 1)) timeout = true;
-            // acc = fl(acc + fl(W[c] * rin[c])), c ascending (reference src/kernels.c:98-106), handed from
-            // lane to lane.  The row is cut into passes of 32 * CHP columns; in a pass lane l holds the
-            // products of columns [l*CHP, (l+1)*CHP) in registers, so a step of the chain costs one
-            // dependent-add latency and nothing else.  Every lane runs the adds of every turn on its own
-            // products (no divergence); only the lane whose turn it is keeps the result.
-            constexpr int CHP = 44;
-            float acc = 0.0f;
-            float cur[CHP];
-            const int npass = (H + 32 * CHP - 1) / (32 * CHP);
-#pragma unroll 1
-            for (int ps = 0; ps < npass; ps++) {
-                const int c0 = ps * 32 * CHP + lane * CHP;
-#pragma unroll
-                for (int i = 0; i < CHP; i += 4) {
-                    // columns past H read scratch that is never added
-                    const float4 wv = *(const float4*)(wrow + c0 + i), xv = *(const float4*)(rin + c0 + i);
-                    cur[i] = __fmul_rn(wv.x, xv.x); cur[i + 1] = __fmul_rn(wv.y, xv.y);
-                    cur[i + 2] = __fmul_rn(wv.z, xv.z); cur[i + 3] = __fmul_rn(wv.w, xv.w);
-                }
-                const bool full = (ps + 1) * 32 * CHP <= H;                 // every lane has CHP valid columns
-                const int mine = min(CHP, max(0, H - c0));
-#pragma unroll 1
-                for (int l = 0; l < 32; l++) {
-                    float s = __shfl_sync(0xffffffffu, acc, (l + 31) & 31);
-                    if (l == 0 && ps == 0) s = 0.0f;
-                    if (full) {
-#pragma unroll
-                        for (int i = 0; i < CHP; i++) s = __fadd_rn(s, cur[i]);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < CHP; i++) {
-                            const float t = __fadd_rn(s, cur[i]);
-                            s = i < mine ? t : s;
-                        }
-                    }
-                    acc = lane == l ? s : acc;
-                }
+        if (e != cta) {
+            __syncthreads();               // the row and the products of the expert before are no longer read
+            if (tid == 0) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                mbar_expect_tx(S.bar_x, (uint32_t)(H * 4));
+                bulk_g2s(wrow, a.router_w + (size_t)e * H, (uint32_t)(H * 4), S.bar_x);
             }
-            if (lane == 31) {
+            if (!fused_mbar_wait(S.bar_x, ph_w & 1)) timeout = true;
+        }
+        ph_w++;
+#pragma unroll
+        for (int j = 0; j < NV; j++) {
+            const int d = tid + j * NT;
+            if (d < H64) prod[d] = d < H ? __fmul_rn(wrow[d], v[j]) : 0.0f;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const float acc = chain_sum(prod, H64);
+            if (lane == 0) {
                 a.logits[e] = acc;
                 asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(a.logits_count) : "memory");
             }
         }
-        ph_w++;
-        if (e + ncta < E) __syncthreads();     // the router row is free for the next expert's copy
     }
     // ---- all logits, then top-k and the job list, by every block for itself ----
     if (tid == 0) {
@@ -694,10 +665,8 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
         if (i >= FUSED_SPIN_LIMIT) timeout = true;
     }
     __syncthreads();
-    for (int e = tid; e < E; e += NT) s_logits[e] = __ldcg(a.logits + e);
-    __syncthreads();
-    topk_group(tid < 128, s_logits, s_pes, s_sel, s_wts, E, K, 1, cta == 0 ? a.f.status : nullptr, tk,
-               tk + topk_scratch_floats(E, K) - 4, tid & 127, 128);
+    topk_group(tid < 160, a.logits, s_pes, s_sel, s_wts, E, K, 1, cta == 0 ? a.f.status : nullptr, tk,
+               tk + topk_scratch_floats(E, K) - 4, tid, 160);
     __syncthreads();
     // job list: thread j takes selection j (its slot = the local selections before it; the list keeps rank order)
     if (tid < K) {

@@ -10,6 +10,39 @@ static __device__ __forceinline__ void flag(int* status, int bit) {
     if (status) atomicOr(status, bit);
 }
 
+// Operations that stay where they are written: the compiler moved loads down to their uses and products to their adds,
+// which a lone warp pays for with their whole latency.
+static __device__ __forceinline__ float4 load_now(const float* p) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+    return v;
+}
+static __device__ __forceinline__ void add_now(float& a, float p) { asm volatile("add.rn.f32 %0, %0, %1;" : "+f"(a) : "f"(p)); }
+
+// 0 + p[0] + p[1] + ... + p[n - 1], in order, by one warp on a scheduler of its own (all lanes alike).  p in shared memory,
+// 16-byte aligned; n a positive multiple of 64.  32 terms are loaded between the adds of the 32 before them.
+static __device__ __forceinline__ float chain_sum(const float* p, int n) {
+    float4 a[8], b[8];
+    float acc = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) a[i] = load_now(p + 4 * i);
+#pragma unroll 1
+    for (int c = 0; c < n; c += 64) {
+        const float* next = p + (c + 64 < n ? c + 64 : c);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            b[i] = load_now(p + c + 32 + 4 * i);
+            add_now(acc, a[i].x); add_now(acc, a[i].y); add_now(acc, a[i].z); add_now(acc, a[i].w);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            a[i] = load_now(next + 4 * i);
+            add_now(acc, b[i].x); add_now(acc, b[i].y); add_now(acc, b[i].z); add_now(acc, b[i].w);
+        }
+    }
+    return acc;
+}
+
 // Serial sum of squares of one row, in element order, as the reference does
 // (gemma4.c:46-62, src/text_verify_cpu.c:642-655).  The squares are formed in
 // parallel beforehand; one thread then runs the add chain over them, reading
@@ -203,30 +236,44 @@ static __device__ float block_sum_nonneg(const float* sq, int n, uint32_t* scrat
                 const uint32_t my_e = mine < ns ? sp_e[mine] : 0u;
                 const float my_v = mine < ns ? sq[my_idx] : 0.0f;
                 const int cnt = (int)min(32u, ns + 1u - base0);
+                // Every lane prepares its point: the run before it as ONE integer to add to the bits of the running sum
+                // (adding units of the last place is adding to the bits while the binade lasts), with the binade it needs.
+                // The chain is then one integer and one floating-point addition per point, and the binades are checked
+                // beside it; a batch with a wrong prediction is walked again, run by run.
+                int p_idx = __shfl_up_sync(0xffffffffu, my_idx, 1);
+                unsigned long long p_i = __shfl_up_sync(0xffffffffu, my_i, 1);
+                uint32_t p_e = __shfl_up_sync(0xffffffffu, my_e, 1);
+                if (lane == 0) { p_idx = prev; p_i = iprev; p_e = E; }
+                const bool run = lane < cnt && my_idx - 1 > p_idx;
+                const unsigned long long my_tot = my_i - p_i;
+                const uint32_t my_add = run ? (uint32_t)(my_tot < 0xffffffull ? my_tot : 0xffffffull) : 0u;
+                const uint32_t my_bin = run ? p_e << 23 : 0xffffffffu;
+                float F = S;
+                uint32_t off = 0;                        // bits that differ from the predicted binade, of all runs
+#pragma unroll 8
                 for (int j = 0; j < cnt; j++) {
-                    const uint32_t jx = base0 + (uint32_t)j;
-                    const int idx = __shfl_sync(0xffffffffu, my_idx, j);
-                    const unsigned long long inow = __shfl_sync(0xffffffffu, my_i, j);
-                    const uint32_t e_after = __shfl_sync(0xffffffffu, my_e, j);
+                    const uint32_t add = __shfl_sync(0xffffffffu, my_add, j), bin = __shfl_sync(0xffffffffu, my_bin, j);
                     const float term = __shfl_sync(0xffffffffu, my_v, j);
-                    if (idx - 1 > prev) {
-                        const unsigned long long tot = inow - iprev;
-                        const uint32_t sb = __float_as_uint(S);
-                        const uint32_t M = (sb & 0x7fffffu) | 0x800000u;
-                        if ((sb >> 23) == E && tot < (unsigned long long)(ONE24 - M)) {
-                            const uint32_t M2 = M + (uint32_t)tot;
-                            S = __uint_as_float((E << 23) | (M2 & 0x7fffffu));
-                        } else {
-                            for (int i = prev + 1; i < idx; i++) S = __fadd_rn(S, sq[i]);   // prediction missed
-                        }
-                    }
-                    if (jx < ns) {
+                    const uint32_t b0 = __float_as_uint(F), b1 = b0 + add;
+                    if (bin != 0xffffffffu) off |= (b0 ^ bin) | (b1 ^ bin);
+                    F = __fadd_rn(__uint_as_float(b1), term);            // past the last point: + 0
+                }
+                if (off < 0x800000u) {
+                    S = F;
+                } else {
+                    for (int j = 0; j < cnt; j++) {
+                        const int idx = __shfl_sync(0xffffffffu, my_idx, j), from = __shfl_sync(0xffffffffu, p_idx, j) + 1;
+                        const uint32_t add = __shfl_sync(0xffffffffu, my_add, j), bin = __shfl_sync(0xffffffffu, my_bin, j);
+                        const float term = __shfl_sync(0xffffffffu, my_v, j);
+                        const uint32_t b0 = __float_as_uint(S), b1 = b0 + add;
+                        if (((b0 ^ bin) | (b1 ^ bin)) < 0x800000u) S = __uint_as_float(b1);
+                        else for (int i = from; i < idx; i++) S = __fadd_rn(S, sq[i]);   // prediction missed
                         S = __fadd_rn(S, term);
-                        prev = idx;
-                        iprev = inow;
-                        E = e_after;
                     }
                 }
+                prev = __shfl_sync(0xffffffffu, my_idx, 31);
+                iprev = __shfl_sync(0xffffffffu, my_i, 31);
+                E = __shfl_sync(0xffffffffu, my_e, 31);
             }
         }
         if (lane == 0) scratch[0] = __float_as_uint(S);
@@ -254,39 +301,64 @@ static __device__ __forceinline__ float ordered_sum_of_squares(const float* sq, 
 // ranking by (logit descending, expert ascending); the softmax denominator and
 // the renormalisation sum are serial chains in expert / rank order.
 //
-// Executed by a group of `gsize` consecutive threads (ltid = index in group) on
-// one row; every thread of the block must call it (block-wide barriers inside),
-// groups without a row pass active = false.  sm = this group's scratch of
-// 2E + 2*topk floats (16-byte aligned), sc = 4 floats of per-group scalars.
+// Executed by a group of `gsize` >= 64 consecutive threads (ltid = index in group, whole warps) on one row; every thread of
+// the block must call it (block-wide barriers inside), groups without a row pass active = false.  lr: the row's logits in
+// global memory.  sm = this group's scratch of 2E + 2*topk floats (16-byte aligned), sc = 4 floats of per-group scalars.
+//
+// Nothing but latencies: up to 128 experts the group's first warp picks the selections, the largest of four keys per lane
+// at a time, while the other warps evaluate the exponentials; it then does all the rest without another barrier (the
+// divisions side by side, the two serial sums by all lanes alike).  Ranking every expert against all others, and one
+// thread dividing by the sum rank after rank, took 6800 cycles of a decode layer; this takes about half.
 static __device__ __forceinline__ void topk_group(bool active, const float* lr, const float* per_expert_scale,
                                                   int32_t* sel_out, float* w_out, int E, int topk,
                                                   int sort_by_expert, int* status, float* sm, float* sc,
                                                   int ltid, int gsize) {
-    float* sl = sm;                  // [E] logits
+    constexpr int KEYS = 4;          // experts per lane of the first warp
+    float* sl = sm;                  // [E] logits (more than 32 * KEYS experts)
     float* se = sm + E;              // [E] exp(l - max)
     int* ssel = (int*)(sm + 2 * E);  // [topk]
     float* sw = sm + 2 * E + topk;   // [topk]
     int* s_bad = (int*)(sc + 3);
-    if (ltid == 0) *s_bad = 0;
-    __syncthreads();
-    if (active)
-        for (int e = ltid; e < E; e += gsize) {
-            const float v = lr[e];
-            sl[e] = v;
-            if (!finite_f(v) || (per_expert_scale && !finite_f(per_expert_scale[e]))) *s_bad = 1;
+    const bool few = E <= 32 * KEYS;
+    float own = 0.0f;                // the first expert whose exponential this thread evaluates
+    if (active && few && ltid >= 32 && ltid - 32 < E) own = __ldcg(lr + ltid - 32);
+    uint32_t key[KEYS];
+    if (active && ltid < 32) {
+        float m = __int_as_float(0xff800000);
+        bool bad = false;
+        if (few) {
+#pragma unroll
+            for (int i = 0; i < KEYS; i++) {
+                const int e = ltid + 32 * i;
+                key[i] = 0u;                                     // below every finite logit's key
+                if (e < E) {
+                    const float v = __ldcg(lr + e);
+                    bad |= !finite_f(v) || (per_expert_scale && !finite_f(per_expert_scale[e]));
+                    m = fmaxf(m, v);
+                    const uint32_t b = __float_as_uint(__fadd_rn(v, 0.0f));      // -0 ranks like +0
+                    key[i] = (b & 0x80000000u) ? ~b : b | 0x80000000u;
+                }
+            }
+        } else {
+            for (int e = ltid; e < E; e += 32) {
+                const float v = __ldcg(lr + e);
+                bad |= !finite_f(v) || (per_expert_scale && !finite_f(per_expert_scale[e]));
+                m = fmaxf(m, v);
+                sl[e] = v;
+            }
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        bad = __any_sync(0xffffffffu, bad);
+        if (ltid == 0) {
+            sc[0] = m;
+            *s_bad = bad ? 1 : 0;
+        }
+    }
     __syncthreads();
     // the reference rejects non-finite logits before ranking (gemma4.c:149-152)
     const bool go = active && !*s_bad;
-    if (go && ltid < 32) {
-        float m = __int_as_float(0xff800000);
-        for (int e = ltid; e < E; e += 32) m = fmaxf(m, sl[e]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (ltid == 0) sc[0] = m;
-    }
-    __syncthreads();
-    if (go) {
+    if (go && !few) {
         const float mx = sc[0];
         for (int e = ltid; e < E; e += gsize) {
             const float v = sl[e];
@@ -298,26 +370,39 @@ static __device__ __forceinline__ void topk_group(bool active, const float* lr, 
             }
             if (rank < topk) ssel[rank] = e;
         }
-    }
-    __syncthreads();
-    if (go && ltid == 0) {
-        const float all = serial_sum(se, E);
-        int bad = (!(all > 0.0f) || !finite_f(all)) ? 1 : 0;
-        float selsum = 0.0f;
+    } else if (go && ltid >= 32) {
+        const float mx = sc[0];
+        for (int e = ltid - 32; e < E; e += gsize - 32)
+            se[e] = expf_exact(__fsub_rn(e == ltid - 32 ? own : __ldcg(lr + e), mx));
+    } else if (go) {
         for (int j = 0; j < topk; j++) {
-            const float w = __fdiv_rn(se[ssel[j]], all);
-            sw[j] = w;
-            selsum = __fadd_rn(selsum, w);
+            uint32_t best = key[0];
+#pragma unroll
+            for (int i = 1; i < KEYS; i++) best = max(best, key[i]);
+            best = __reduce_max_sync(0xffffffffu, best);
+            uint32_t e = 0xffffffffu;                            // the lowest expert of those that tie
+#pragma unroll
+            for (int i = KEYS - 1; i >= 0; i--)
+                if (key[i] == best) e = (uint32_t)(ltid + 32 * i);
+            e = __reduce_min_sync(0xffffffffu, e);
+#pragma unroll
+            for (int i = 0; i < KEYS; i++)
+                if (e == (uint32_t)(ltid + 32 * i)) key[i] = 0u;
+            if (ltid == 0) ssel[j] = (int)e;
         }
-        sc[1] = selsum;
-        if (!(selsum > 0.0f) || !finite_f(selsum)) bad = 1;
-        if (bad) *s_bad = 1;
     }
     __syncthreads();
-    if (go)
-        for (int j = ltid; j < topk; j += gsize) {
+    if (go && ltid < 32) {
+        const float all = serial_sum(se, E);
+        bool bad = !(all > 0.0f) || !finite_f(all);
+        for (int j = ltid; j < topk; j += 32) sw[j] = __fdiv_rn(se[ssel[j]], all);
+        __syncwarp();
+        float selsum = 0.0f;
+        for (int j = 0; j < topk; j++) selsum = __fadd_rn(selsum, sw[j]);
+        if (!(selsum > 0.0f) || !finite_f(selsum)) bad = true;
+        for (int j = ltid; j < topk; j += 32) {
             const int e = ssel[j];
-            const float nrm = __fdiv_rn(sw[j], sc[1]);
+            const float nrm = __fdiv_rn(sw[j], selsum);
             const float w = __fmul_rn(nrm, per_expert_scale ? per_expert_scale[e] : 1.0f);
             int pos = j;
             if (sort_by_expert) {
@@ -327,6 +412,8 @@ static __device__ __forceinline__ void topk_group(bool active, const float* lr, 
             sel_out[pos] = e;
             w_out[pos] = w;
         }
+        if (ltid == 0 && bad) *s_bad = 1;
+    }
     if (active && ltid == 0 && *s_bad) flag(status, SB_ERR_NONFINITE);
 }
 

@@ -253,6 +253,7 @@ __global__ void __launch_bounds__(GLUE_NV == 4 ? 1024 : 512) glue_rows_kernel(Gl
         rs[j] = (a.router_scale != nullptr && d < n) ? __ldg(a.router_scale + d) : 1.0f;
         v[j] = 0.0f;
     }
+    if (tid == 32) s_root = __fdiv_rn(1.0f, sqrtf_exact((float)n));     // beside the loads, not in the chain below
     // the rank table was written by the plan kernel, at least two launches back (unless tables_late)
     int early_g = -1;
     float early_w = 0.0f;
@@ -347,7 +348,6 @@ __global__ void __launch_bounds__(GLUE_NV == 4 ? 1024 : 512) glue_rows_kernel(Gl
         const float ss = ordered_sum_of_squares<GLUE_NV>(sq, n, bad, s_scan);
         if (tid == 0) {
             s_inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)n), a.eps_router));
-            s_root = __fdiv_rn(1.0f, sqrtf_exact((float)n));
             if (!finite_f(s_inv) || !finite_f(s_root)) flag(a.status, SB_ERR_NONFINITE);
         }
         __syncthreads();
@@ -500,6 +500,9 @@ cudaError_t launch_rmsnorm(const float* x, const float* weight, float* y, int ro
     return cudaGetLastError();
 }
 
+// Threads of a row's top-k: one warp selects, four evaluate the exponentials of up to 128 experts.
+constexpr int TOPK_THREADS = 160;
+
 cudaError_t launch_router_input(const float* x, const float* scale, float* out, int rows, int n, float eps,
                                 float root, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
@@ -507,7 +510,7 @@ cudaError_t launch_router_input(const float* x, const float* scale, float* out, 
     return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(TOPK_THREADS)
 router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ per_expert_scale,
                    int32_t* __restrict__ selected, float* __restrict__ weights, int E, int topk, int sort_by_expert,
                    int* status) {
@@ -524,7 +527,7 @@ cudaError_t launch_router_topk(const float* logits, const float* per_expert_scal
                                int rows, int E, int topk, int sort_by_expert, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
     size_t smem = (size_t)topk_scratch_floats(E, topk) * sizeof(float);
-    return launch_pdl(router_topk_kernel, dim3(rows), dim3(128), smem, stream, logits, per_expert_scale, selected, weights, E,
+    return launch_pdl(router_topk_kernel, dim3(rows), dim3(TOPK_THREADS), smem, stream, logits, per_expert_scale, selected, weights, E,
                       topk, sort_by_expert, status);
 }
 
@@ -718,12 +721,12 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(MoePlanArgs a) {
 }
 
 // The same plan for at most 32 selections (decode batches of a few tokens), with the
-// router top-k always fused: 128 threads per row run the top-k, then ONE warp places the
+// router top-k always fused: TOPK_THREADS threads per row run the top-k, then ONE warp places the
 // selections (slot = selections with a smaller expert + earlier selections of the same
 // expert, which is the stable counting sort) and every thread derives its experts' group
 // starts and descriptors by counting over the <= 32 selections.  No histogram, no block
 // scans: a handful of barriers instead of a dozen.
-__global__ void __launch_bounds__(512) moe_plan_small_kernel(MoePlanArgs a) {
+__global__ void __launch_bounds__(4 * TOPK_THREADS) moe_plan_small_kernel(MoePlanArgs a) {
     extern __shared__ __align__(16) int sp[];
     const int E = a.n_experts;
     pdl_wait();                    // the logits come from the previous kernel
@@ -732,13 +735,13 @@ __global__ void __launch_bounds__(512) moe_plan_small_kernel(MoePlanArgs a) {
     if (a.fused_done != nullptr && threadIdx.x < FUSED_MAX_JOBS) a.fused_done[threadIdx.x] = 0;
     {
         float* tk = (float*)sp;
-        const int grp = threadIdx.x >> 7, ltid = threadIdx.x & 127;
+        const int grp = threadIdx.x / TOPK_THREADS, ltid = threadIdx.x % TOPK_THREADS;
         const int per = topk_scratch_floats(E, a.topk);
         float* mine = tk + grp * per;
         const bool active = grp < a.rows;
         const int row = active ? grp : 0;
         topk_group(active, a.logits + (size_t)row * E, a.per_expert_scale, a.selected_out + (size_t)row * a.topk,
-                   a.weights_out + (size_t)row * a.topk, E, a.topk, 1, a.status, mine, mine + per - 4, ltid, 128);
+                   a.weights_out + (size_t)row * a.topk, E, a.topk, 1, a.status, mine, mine + per - 4, ltid, TOPK_THREADS);
         __syncthreads();   // selections written by this block are read back below
     }
     const int jobs = a.rows * a.topk;
@@ -804,7 +807,7 @@ cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream) {
     if (a.logits != nullptr && a.rows >= 1 && a.rows <= 4 && a.rows * a.topk <= 32) {
         const size_t small = (size_t)a.rows * topk_scratch_floats(a.n_experts, a.topk) * sizeof(float);
         if (small <= 40 * 1024) {
-            return launch_pdl(moe_plan_small_kernel, dim3(1), dim3(128 * a.rows), small, stream, a);
+            return launch_pdl(moe_plan_small_kernel, dim3(1), dim3(TOPK_THREADS * a.rows), small, stream, a);
         }
     }
     size_t smem = (size_t)(34 * a.n_experts + 4) * sizeof(int);

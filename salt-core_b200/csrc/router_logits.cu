@@ -5,7 +5,7 @@
 // experts chains are all the parallelism there is.  A warp alone on its scheduler issues in order and every shared load
 // holds it for about four cycles (measured: 4.5 cycles per column for add + multiply from registers, 8.8 with a 4-byte
 // load per column), so a lane owns whole chains and reads 16 bytes at a time:
-//   * up to four rows of the usual hidden sizes (router_logits_warp_kernel): a warp per chain, products in registers.
+//   * up to four rows (router_logits_chain_kernel): a block per chain, products in shared memory, one warp adds.
 //   * few rows (router_logits_few_kernel): eight experts x eight rows per block.  Helper warps form the products of a slab
 //     of 128 columns and leave them in shared memory, a chain per row; a lane of an adding warp reads four products and
 //     does four adds, nothing else.  Few experts per block because a block's weights all come through one SM.
@@ -63,15 +63,7 @@ __device__ __forceinline__ void arrive_when_copied(uint64_t* bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Operations that stay where they are written: the compiler moved loads down to their uses and products to their adds,
-// which a lone warp pays for with their whole latency.
-__device__ __forceinline__ float4 load_now(const float* p) {
-    float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(smem_u32(p)));
-    return v;
-}
 __device__ __forceinline__ void mul_now(float& p, float a, float b) { asm volatile("mul.rn.f32 %0, %1, %2;" : "=f"(p) : "f"(a), "f"(b)); }
-__device__ __forceinline__ void add_now(float& a, float p) { asm volatile("add.rn.f32 %0, %0, %1;" : "+f"(a) : "f"(p)); }
 
 // A fetching warp: slab after slab of `n` rows of src (from row r0, the last one being `last`) into rows `at`, at + 1, ... of
 // a ring of `stages` stages of stage_bytes, one row (512 bytes, a 16-byte cp.async per lane) per instruction.  (Bulk
@@ -334,45 +326,42 @@ cudaError_t launch_many(const float* W, const float* x, float* logits, int rows,
     return launch_pdl(router_logits_many_kernel<NSL, R>, grid, dim3(192), (size_t)G::SMEM, stream, W, x, logits, rows, E, H, status);
 }
 
-// ---- up to four rows: one WARP per (expert, row).  Lane l forms the products of
-// columns [l*CH, (l+1)*CH) in registers (H == 32*CH), then the reference chain
-// acc = fl(acc + p[c]), c ascending (src/kernels.c:98-106), runs lane after lane: lane l
-// takes the running value from lane l-1 and adds its CH products from registers, so each
-// step costs one dependent-add latency and nothing else.
-template <int CH>
-__global__ void __launch_bounds__(32)
-router_logits_warp_kernel(const float* __restrict__ W, const float* __restrict__ x, float* __restrict__ logits, int E, int H) {
-    const int e = blockIdx.x, r = blockIdx.y, lane = threadIdx.x;
-    const float4* w4 = (const float4*)(W + (size_t)e * H + lane * CH);
-    const float4* x4 = (const float4*)(x + (size_t)r * H + lane * CH);
-    float p[CH];
+// ---- up to four rows: a block per (expert, row).  All its threads form the products, coalesced, in shared memory; one
+// warp adds them.  (A warp per chain with the products in its lanes' registers, handed from lane to lane, paid for
+// strided loads of the weights and for a shuffle and a branch in every turn.)
+constexpr int CHAIN_THREADS = 128;
+template <int N4>                             // 16-byte pieces per thread
+__global__ void __launch_bounds__(CHAIN_THREADS)
+router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict__ x, float* __restrict__ logits, int E, int H) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int e = blockIdx.x, r = blockIdx.y, n4 = H >> 2;
+    const float4* w4 = (const float4*)(W + (size_t)e * H);
+    const float4* x4 = (const float4*)(x + (size_t)r * H);
+    float4 w[N4], v[N4];
 #pragma unroll
-    for (int i = 0; i < CH / 4; i++) {       // the router weights do not depend on the previous kernel
-        const float4 wv = __ldg(w4 + i);
-        p[4 * i + 0] = wv.x; p[4 * i + 1] = wv.y; p[4 * i + 2] = wv.z; p[4 * i + 3] = wv.w;
+    for (int i = 0; i < N4; i++) {            // the router weights do not depend on the previous kernel
+        const int k = threadIdx.x + i * CHAIN_THREADS;
+        if (k < n4) w[i] = __ldg(w4 + k);
     }
     pdl_wait();
     pdl_launch_dependents();
 #pragma unroll
-    for (int i = 0; i < CH / 4; i++) {
-        const float4 xv = x4[i];
-        p[4 * i + 0] = __fmul_rn(p[4 * i + 0], xv.x);
-        p[4 * i + 1] = __fmul_rn(p[4 * i + 1], xv.y);
-        p[4 * i + 2] = __fmul_rn(p[4 * i + 2], xv.z);
-        p[4 * i + 3] = __fmul_rn(p[4 * i + 3], xv.w);
+    for (int i = 0; i < N4; i++) {
+        const int k = threadIdx.x + i * CHAIN_THREADS;
+        if (k < n4) v[i] = x4[k];
     }
-    float acc = 0.0f;
-#pragma unroll 1
-    for (int l = 0; l < 32; l++) {
-        float a = __shfl_sync(0xffffffffu, acc, (l + 31) & 31);
-        if (l == 0) a = 0.0f;
-        if (lane == l) {
 #pragma unroll
-            for (int i = 0; i < CH; i++) a = __fadd_rn(a, p[i]);
-            acc = a;
-        }
+    for (int i = 0; i < N4; i++) {
+        const int k = threadIdx.x + i * CHAIN_THREADS;
+        if (k < n4)
+            ((float4*)smem)[k] = make_float4(__fmul_rn(w[i].x, v[i].x), __fmul_rn(w[i].y, v[i].y), __fmul_rn(w[i].z, v[i].z),
+                                             __fmul_rn(w[i].w, v[i].w));
     }
-    if (lane == 31) logits[(size_t)r * E + e] = __fadd_rn(acc, 0.0f);
+    __syncthreads();
+    // blocks that share an SM add on different schedulers
+    if ((threadIdx.x >> 5) != (((blockIdx.y * gridDim.x + blockIdx.x) / 148) & 3)) return;
+    const float acc = chain_sum((const float*)smem, H);
+    if ((threadIdx.x & 31) == 0) logits[(size_t)r * E + e] = __fadd_rn(acc, 0.0f);
 }
 
 }  // namespace
@@ -381,10 +370,13 @@ cudaError_t launch_router_logits(const float* W, const float* x, float* logits, 
                                  cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
     if ((H % 64) != 0 || ((((uintptr_t)W) | ((uintptr_t)x)) & 15) != 0) return cudaErrorInvalidValue;
-    // a warp per chain while that is a few warps per SM (B = 2: 15 us between events against 17 with the next form)
-    if (rows <= 4 && (H == 32 * 88 || H == 32 * 160)) {
-        if (H == 32 * 88) return launch_pdl(router_logits_warp_kernel<88>, dim3(E, rows), dim3(32), 0, stream, W, x, logits, E, H);
-        return launch_pdl(router_logits_warp_kernel<160>, dim3(E, rows), dim3(32), 0, stream, W, x, logits, E, H);
+    // a block per chain while that is a few blocks per SM (more rows share the weights, below)
+    if (rows <= 4 && H <= 10 * 4 * CHAIN_THREADS) {
+        const dim3 grid(E, rows);
+        const size_t smem = (size_t)H * 4;
+        if (H <= 6 * 4 * CHAIN_THREADS)
+            return launch_pdl(router_logits_chain_kernel<6>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H);
+        return launch_pdl(router_logits_chain_kernel<10>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H);
     }
     // one chain per lane while one round of blocks holds them all, then as many per lane as keep it to one round
     const long few = (long)((E + FEW_E - 1) / FEW_E) * ((rows + FEW_ROWS - 1) / FEW_ROWS);

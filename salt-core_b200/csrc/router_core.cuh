@@ -92,7 +92,7 @@ static __device__ __forceinline__ float serial_sum(const float* sq, int n) {
 // Needs blockDim.x * V >= n (V = elements per thread) and blockDim.x a multiple of 32.  scratch: POSSUM_SCRATCH words
 // of shared memory.  Every thread of the block must call; all return the sum.
 constexpr int POSSUM_V = 4, POSSUM_HEAD = 64, POSSUM_NS = 192;
-constexpr int POSSUM_SCRATCH = 8 + 32 + 32 + 64 + 32 + POSSUM_NS * 4;
+constexpr int POSSUM_SCRATCH = 8 + 32 + 32 + 64 + 32 + POSSUM_NS * 4 + 96;
 
 template <int V = POSSUM_V>
 static __device__ float block_sum_nonneg(const float* sq, int n, uint32_t* scratch) {
@@ -105,6 +105,8 @@ static __device__ float block_sum_nonneg(const float* sq, int n, uint32_t* scrat
     uint32_t* sp_k = scratch + 168;                    // [NS] index of serial point
     uint32_t* sp_e = sp_k + POSSUM_NS;                 // [NS] predicted exponent field after it
     unsigned long long* sp_i = (unsigned long long*)(sp_e + POSSUM_NS);   // [NS] integer prefix at it
+    uint2* pt_run = (uint2*)(sp_i + POSSUM_NS);         // [32] runs of the batch being walked: bits to add, binade
+    float* pt_term = (float*)(pt_run + 32);            // [32] ... and the terms after them
     const int base = tid * V;
 
     // ---- 1. approximate inclusive prefix sums
@@ -216,64 +218,56 @@ static __device__ float block_sum_nonneg(const float* sq, int n, uint32_t* scrat
         }
     __syncthreads();
 
-    // ---- 4. the exact walk, by warp 0: lane j fetches serial point j of a chunk of 32 (its index, integer
-    // prefix, predicted exponent and the term itself), so that the chain below only waits for shuffles and
-    // its own arithmetic; every lane runs the same chain on the same values
+    // ---- 4. the exact walk, by warp 0.  Lane j of a batch of 32 points prepares point j: the run of certain elements before
+    // it as ONE integer to add to the bits of the running sum (adding units of the last place is adding to the bits while
+    // the binade lasts), with the binade it needs, and the point's own term.  The chain, which all lanes run alike, is then
+    // one integer and one floating-point addition per point; the binades are checked beside it, and a batch with a wrong
+    // prediction is walked again, run by run.  (The points go through shared memory: a shuffle in a loop whose length the
+    // compiler does not know to be the same for all lanes took up to 240 cycles, three of them per point.)
     if (warp == 0) {
         float S;
         if (ns > (uint32_t)POSSUM_NS || n <= POSSUM_HEAD) {
-            S = lane == 0 ? serial_sum(sq, n) : 0.0f;
+            S = serial_sum(sq, n);
         } else {
-            S = lane == 0 ? serial_sum(sq, POSSUM_HEAD) : 0.0f;
-            S = __shfl_sync(0xffffffffu, S, 0);
-            int prev = POSSUM_HEAD - 1;
-            unsigned long long iprev = 0;
-            uint32_t E = scratch[2];
+            S = (((uintptr_t)sq) & 15) == 0 ? chain_sum(sq, POSSUM_HEAD) : serial_sum(sq, POSSUM_HEAD);
+            const uint32_t E0 = scratch[2];
             for (uint32_t base0 = 0; base0 <= ns; base0 += 32) {
                 const uint32_t mine = base0 + (uint32_t)lane;
-                const int my_idx = mine < ns ? (int)sp_k[mine] : n;
-                const unsigned long long my_i = mine < ns ? sp_i[mine] : itotal;
-                const uint32_t my_e = mine < ns ? sp_e[mine] : 0u;
-                const float my_v = mine < ns ? sq[my_idx] : 0.0f;
+                if (mine <= ns) {
+                    const int idx = mine < ns ? (int)sp_k[mine] : n, from = mine ? (int)sp_k[mine - 1] + 1 : POSSUM_HEAD;
+                    const unsigned long long tot = (mine < ns ? sp_i[mine] : itotal) - (mine ? sp_i[mine - 1] : 0ull);
+                    const uint32_t bin = (mine ? sp_e[mine - 1] : E0) << 23;
+                    const bool some = idx > from;
+                    pt_run[lane] = make_uint2(some ? (uint32_t)(tot < 0xffffffull ? tot : 0xffffffull) : 0u, some ? bin : 0xffffffffu);
+                    pt_term[lane] = mine < ns ? sq[idx] : 0.0f;              // past the last point: + 0
+                }
+                __syncwarp();
                 const int cnt = (int)min(32u, ns + 1u - base0);
-                // Every lane prepares its point: the run before it as ONE integer to add to the bits of the running sum
-                // (adding units of the last place is adding to the bits while the binade lasts), with the binade it needs.
-                // The chain is then one integer and one floating-point addition per point, and the binades are checked
-                // beside it; a batch with a wrong prediction is walked again, run by run.
-                int p_idx = __shfl_up_sync(0xffffffffu, my_idx, 1);
-                unsigned long long p_i = __shfl_up_sync(0xffffffffu, my_i, 1);
-                uint32_t p_e = __shfl_up_sync(0xffffffffu, my_e, 1);
-                if (lane == 0) { p_idx = prev; p_i = iprev; p_e = E; }
-                const bool run = lane < cnt && my_idx - 1 > p_idx;
-                const unsigned long long my_tot = my_i - p_i;
-                const uint32_t my_add = run ? (uint32_t)(my_tot < 0xffffffull ? my_tot : 0xffffffull) : 0u;
-                const uint32_t my_bin = run ? p_e << 23 : 0xffffffffu;
                 float F = S;
-                uint32_t off = 0;                        // bits that differ from the predicted binade, of all runs
-#pragma unroll 8
+                uint32_t off = 0;                        // bits in which a run's ends differ from its predicted binade
+#pragma unroll 4
                 for (int j = 0; j < cnt; j++) {
-                    const uint32_t add = __shfl_sync(0xffffffffu, my_add, j), bin = __shfl_sync(0xffffffffu, my_bin, j);
-                    const float term = __shfl_sync(0xffffffffu, my_v, j);
-                    const uint32_t b0 = __float_as_uint(F), b1 = b0 + add;
-                    if (bin != 0xffffffffu) off |= (b0 ^ bin) | (b1 ^ bin);
-                    F = __fadd_rn(__uint_as_float(b1), term);            // past the last point: + 0
+                    const uint2 r = pt_run[j];
+                    const uint32_t b0 = __float_as_uint(F), b1 = b0 + r.x;
+                    off |= r.y != 0xffffffffu ? (b0 ^ r.y) | (b1 ^ r.y) : 0u;
+                    F = __fadd_rn(__uint_as_float(b1), pt_term[j]);
                 }
                 if (off < 0x800000u) {
                     S = F;
                 } else {
                     for (int j = 0; j < cnt; j++) {
-                        const int idx = __shfl_sync(0xffffffffu, my_idx, j), from = __shfl_sync(0xffffffffu, p_idx, j) + 1;
-                        const uint32_t add = __shfl_sync(0xffffffffu, my_add, j), bin = __shfl_sync(0xffffffffu, my_bin, j);
-                        const float term = __shfl_sync(0xffffffffu, my_v, j);
-                        const uint32_t b0 = __float_as_uint(S), b1 = b0 + add;
-                        if (((b0 ^ bin) | (b1 ^ bin)) < 0x800000u) S = __uint_as_float(b1);
-                        else for (int i = from; i < idx; i++) S = __fadd_rn(S, sq[i]);   // prediction missed
-                        S = __fadd_rn(S, term);
+                        const uint2 r = pt_run[j];
+                        const uint32_t b0 = __float_as_uint(S), b1 = b0 + r.x, jx = base0 + (uint32_t)j;
+                        if (((b0 ^ r.y) | (b1 ^ r.y)) < 0x800000u) {
+                            S = __uint_as_float(b1);
+                        } else {                                             // no run, or the prediction missed
+                            const int idx = jx < ns ? (int)sp_k[jx] : n;
+                            for (int i = jx ? (int)sp_k[jx - 1] + 1 : POSSUM_HEAD; i < idx; i++) S = __fadd_rn(S, sq[i]);
+                        }
+                        S = __fadd_rn(S, pt_term[j]);
                     }
                 }
-                prev = __shfl_sync(0xffffffffu, my_idx, 31);
-                iprev = __shfl_sync(0xffffffffu, my_i, 31);
-                E = __shfl_sync(0xffffffffu, my_e, 31);
+                __syncwarp();
             }
         }
         if (lane == 0) scratch[0] = __float_as_uint(S);

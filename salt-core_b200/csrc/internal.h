@@ -90,6 +90,7 @@ struct alignas(16) LayerDecodeArgs {
     const uint8_t* tables;         // derived scale | bias tables of the local experts
     const int* lit_flags;          // [local experts]
     size_t expert_stride, tensor_bytes, value_bytes, group_bytes;
+    int last;                      // the next kernel is another one
 };
 bool q4_layer_decode_plan(int H, int M, int E, int topk, int n_jobs_max, FusedLaunch* out);
 cudaError_t launch_q4_layer_decode(const LayerDecodeArgs& args, int n_jobs_max, cudaStream_t stream);

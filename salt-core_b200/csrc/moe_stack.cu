@@ -1064,6 +1064,7 @@ static int forward_decode_layers(Stack* s, int first, int count, const float* d_
         a.E = s->n_experts; a.topk = K; a.expert_begin = s->expert_begin; a.expert_end = s->expert_end;
         a.selected = s->selected; a.weights_out = wbuf[i & 1]; a.c2g = s->c2g; a.g2c = s->g2c;
         a.group_offsets = s->group_offsets;
+        a.last = i == count - 1;
         a.pool = l.pool; a.tables = l.sb_tables; a.lit_flags = l.lit_flags; a.expert_stride = l.expert_stride;
         a.value_bytes = elems / 2; a.group_bytes = elems / 64 * 2; a.tensor_bytes = a.value_bytes + 2 * a.group_bytes;
         if (stacked) {

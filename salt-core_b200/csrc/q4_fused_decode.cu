@@ -525,7 +525,7 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
     }
     if (!STACKED) {
         pdl_wait();                // the previous layer's outputs
-        pdl_launch_dependents();
+        if (!a.last) pdl_launch_dependents();
     } else if (li > 0) {
         // the previous layer's outputs: every block of the grid has finished it
         if (tid == 0) {
@@ -721,6 +721,7 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
 __global__ void __launch_bounds__(16 * LAYER_SLOTS, 1) q4_layer_decode_kernel(LayerDecodeArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     layer_decode_body<false>(a, smem, 0, nullptr, nullptr);
+    if (a.last) pdl_launch_dependents();
 }
 
 // All layers of a decode step in ONE launch: the blocks (one per SM) stay resident, so the code of a layer is

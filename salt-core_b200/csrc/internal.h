@@ -104,8 +104,6 @@ int q4_layer_decode_jobs_per_round(int H, int M, int E, int topk, int n_jobs_max
 cudaError_t launch_q8_jobs(const Q4Job* jobs, int njobs, int max_rows, int max_tok, int C, cudaStream_t stream);
 
 // ---- q4_gemm_tc.cu (tcgen05 / TMEM, tolerance path) --------------------------
-cudaError_t launch_gather_convert(const float* x, const int32_t* g2c, void* xh, void* xl, void* sums_h, void* sums_l, int jobs,
-                                  int topk, int hidden, cudaStream_t stream);
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda)
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                       const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -138,13 +136,15 @@ cudaError_t make_q4_tc_weight_maps(TcWeightMaps* out, const uint8_t* pool, size_
 // Can the tensor-core kernels take this geometry?  Sizes must be multiples of 64; a size that is no multiple of
 // 256 must not exceed 3520 (single) / 960 (hi + lo halves).
 bool q4_tc_supported(int hidden, int inter, bool split);
-// Work lists of a layer's two tensor-core launches (written on the device from the grouped jobs): items_* hold
+// What the tensor-core launches of a layer read: the tokens' rows in grouped order (fp16; split: residuals and group means
+// too) and the two launches' work lists (written on the device from the grouped jobs): items_* hold
 // q4_tc_work_items_max() entries of 16 bytes each, work eight ints: {items, next, largest pass, -} of the fused
 // launch, then of the plain one.
 size_t q4_tc_work_items_max(int n_experts, int rows_total, int hidden, int inter);
-cudaError_t launch_q4_tc_work_list(const Q4Job* gateup_jobs, const int* njobs_dev, int njobs_max, const float* y_base,
-                                   int y_cols, const TcWeightMaps& wm, int hidden, int inter, void* items_fused,
-                                   void* items_plain, int* work, cudaStream_t stream);
+cudaError_t launch_tc_prepare(const float* x, const int32_t* c2g, void* xh, void* xl, void* sums_h, void* sums_l, int rows,
+                              int topk, int hidden, int inter, const Q4Job* gateup_jobs, const int* njobs_dev, int njobs_max,
+                              const float* y_base, int y_cols, const TcWeightMaps& wm, void* items_fused, void* items_plain,
+                              int* work, cudaStream_t stream);
 // items / work: this launch's list and its {items, next, largest pass} triple.  R, C: rows and columns of the weight matrices.
 // fused: gate/up + GeGLU -> out_h [grouped rows][R] fp16 (split: out_l and the group means sums_h, sums_l too); plain: -> out_f
 // [grouped rows][R] fp32.  split: activations carried as hi + lo fp16 halves, weights exactly.  x, sums: the activations

@@ -533,7 +533,7 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
                                       s->status, st, nullptr, 1, 1, s->fp4_up), "nvfp4 geglu + qdq") ||
             !cuda_ok(launch_nvfp4_gemm_tc(s->fp4_tc_dn, E, H, M, md, s->status, st), "nvfp4 tc down"))
             return -1;
-        count_launches(6);
+        count_launches(5);
         return 0;
     }
     if (l.nvfp4) {
@@ -577,9 +577,9 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
         // tolerance path: fp16 operands on tcgen05, fp32 accumulation in TMEM
         {
             Timed t(s, KC_ROUTER_INPUT, st);
-            if (!cuda_ok(launch_gather_convert(d_x, s->g2c, s->xh, split ? s->xl : nullptr, s->xs_h, s->xs_l, jobs, K, H, st), "gather/convert")) return -1;
-            if (!cuda_ok(launch_q4_tc_work_list(s->gateup_jobs, s->counters, njobs_max, s->chain, M, l.q4_tc, H, M,
-                                                s->tc_items_fused, s->tc_items_plain, s->tc_work, st), "tc work list"))
+            if (!cuda_ok(launch_tc_prepare(d_x, s->c2g, s->xh, split ? s->xl : nullptr, s->xs_h, s->xs_l, B, K, H, M, s->gateup_jobs,
+                                           s->counters, njobs_max, s->chain, M, l.q4_tc, s->tc_items_fused, s->tc_items_plain,
+                                           s->tc_work, st), "tc rows and work lists"))
                 return -1;
         }
         {

@@ -757,17 +757,97 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
     }
 }
 
-// x (fp32, token rows) -> fp16 rows in grouped order: xh[g] = fp16(x[g2c[g] / topk]), and (when xl != null) the
-// residuals xl[g] = fp16(x - xh) and the means of the 64-column groups.  Columns inside every group of 8 are written in
-// the operands' K order.
-__global__ void __launch_bounds__(256)
-gather_convert_kernel(const float* __restrict__ x, const int32_t* __restrict__ g2c, __half* __restrict__ xh,
-                      __half* __restrict__ xl, __half* __restrict__ sums_h, __half* __restrict__ sums_l, int sums_stride,
-                      int topk, int hidden) {
-    const int g = blockIdx.y;
-    const int d = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+// Work lists of a layer's two launches: for every expert group with tokens, every 128-token pass, every row
+// tile one item (tiles of a pass adjacent, so neighbouring blocks share the pass' token rows in L2).  One block; a warp
+// per group (all threads on one group after the other took 10 us for 128 groups).
+struct WorkListArgs {
+    const Q4Job* jobs;
+    const int* njobs_dev;
+    int njobs_max;
+    const float* y_base;
+    int y_cols;
+    const uint8_t* pool;
+    size_t expert_stride;
+    int nx_fused, nx_plain;
+    TcItem *items_fused, *items_plain;
+    int* work;
+};
+__device__ __forceinline__ void write_work_lists(const WorkListArgs& a, int* s_list) {
+    // s_list: [njobs_max + 1] first pass of every job, then expert, first row, tokens
+    int* s_base = s_list;
+    int* s_expert = s_list + a.njobs_max + 1;
+    int* s_g0 = s_expert + a.njobs_max;
+    int* s_ntok = s_g0 + a.njobs_max;
+    const int njobs = a.njobs_dev ? min(*a.njobs_dev, a.njobs_max) : a.njobs_max;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int j = threadIdx.x; j < njobs; j += blockDim.x) {
+        const Q4Job& jb = a.jobs[j];
+        s_expert[j] = (int)((size_t)(jb.vals - a.pool) / a.expert_stride);
+        s_g0[j] = (int)((jb.y - a.y_base) / a.y_cols);
+        s_ntok[j] = max(jb.ntok, 0);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int run = 0, nt_max = 0;
+        for (int j0 = 0; j0 < njobs; j0 += 32) {
+            const int j = j0 + lane, ntok = j < njobs ? s_ntok[j] : 0, np = (ntok + TC_MAX_NT - 1) / TC_MAX_NT;
+            int inc = np;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += t;
+            }
+            if (j < njobs) s_base[j] = run + inc - np;
+            run += __shfl_sync(0xffffffffu, inc, 31);
+            nt_max = max(nt_max, min(ntok, TC_MAX_NT));
+        }
+        nt_max = __reduce_max_sync(0xffffffffu, nt_max);
+        if (lane == 0) {
+            s_base[njobs] = run;
+            a.work[0] = run * a.nx_fused; a.work[1] = 0; a.work[2] = nt_max;
+            a.work[4] = run * a.nx_plain; a.work[5] = 0; a.work[6] = nt_max;
+        }
+    }
+    __syncthreads();
+    const int nxt = a.nx_fused + a.nx_plain;
+    for (int j = warp; j < njobs; j += blockDim.x >> 5) {
+        const int base = s_base[j], np = s_base[j + 1] - base;
+        for (int p = 0; p < np; p++) {
+            TcItem it;
+            it.expert = s_expert[j]; it.grow = s_g0[j] + p * TC_MAX_NT; it.nt = min(TC_MAX_NT, s_ntok[j] - p * TC_MAX_NT);
+            for (int x = lane; x < nxt; x += 32) {
+                if (x < a.nx_fused) {
+                    it.r0 = x * (TW_ROWS / 2);
+                    a.items_fused[(size_t)(base + p) * a.nx_fused + x] = it;
+                } else {
+                    it.r0 = (x - a.nx_fused) * TW_ROWS;
+                    a.items_plain[(size_t)(base + p) * a.nx_plain + (x - a.nx_fused)] = it;
+                }
+            }
+        }
+    }
+}
+
+// x (fp32, token rows) -> fp16 rows in grouped order: xh[c2g[t * topk + k]] = fp16(x[t]) for every selection k of token t,
+// and (when xl != null) the residuals xl = fp16(x - xh) and the means of the 64-column groups.  Columns inside every group
+// of 8 are written in the operands' K order.  A token's columns are loaded and converted once and stored topk times; with
+// a block per GROUPED row (eight times the blocks, loads and conversions) and the work lists in a launch of their own, 69 us
+// of a layer of 512 tokens and 99 of 1999 went into this and the first row-wise glue; now 37 and 46.
+// blockIdx.y = 0: the work lists (one block), beside the rows: both need nothing but the plan.
+constexpr int GATHER_THREADS = 128;
+__global__ void __launch_bounds__(GATHER_THREADS)
+scatter_convert_kernel(const float* __restrict__ x, const int32_t* __restrict__ c2g, __half* __restrict__ xh,
+                       __half* __restrict__ xl, __half* __restrict__ sums_h, __half* __restrict__ sums_l, int sums_stride,
+                       int jobs, int topk, int hidden, const WorkListArgs lists) {
+    if (blockIdx.y == 0) {
+        extern __shared__ int s_list[];
+        if (blockIdx.x == 0) write_work_lists(lists, s_list);
+        return;
+    }
+    const int token = blockIdx.y - 1;
+    const int d = (blockIdx.x * GATHER_THREADS + threadIdx.x) * 8;
     if (d >= hidden) return;                      // hidden is a multiple of 64: the eight lanes of a group stay together
-    const float* src = x + (size_t)(g2c[g] / topk) * hidden + d;
+    const float* src = x + (size_t)token * hidden + d;
     const float4 v0 = *(const float4*)src, v1 = *(const float4*)(src + 4);
     const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     uint32_t hi[4], lo[4];
@@ -776,25 +856,23 @@ gather_convert_kernel(const float* __restrict__ x, const int32_t* __restrict__ g
         hi[k] = f16x2_from(v[k], v[k + 4]);
         lo[k] = f16x2_from(v[k] - f16_lo_to_f32(hi[k]), v[k + 4] - f16_hi_to_f32(hi[k]));
     }
-    *(uint4*)(xh + (size_t)g * hidden + d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    float sum = 0.0f;
     if (xl) {
-        *(uint4*)(xl + (size_t)g * hidden + d) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-        float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
         const uint32_t octet = 0xffu << (threadIdx.x & 24);
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(octet, sum, o);
-        if ((threadIdx.x & 7) == 0) store_group_mean(sums_h, sums_l, (size_t)g * sums_stride, d / TC_KC, sum * (1.0f / TC_KC));
     }
-}
-
-cudaError_t launch_gather_convert(const float* x, const int32_t* g2c, void* xh, void* xl, void* sums_h, void* sums_l, int jobs,
-                                  int topk, int hidden, cudaStream_t stream) {
-    if (jobs < 1) return cudaSuccess;
-    if (hidden % 64) return cudaErrorInvalidValue;
-    dim3 grid((hidden / 8 + 255) / 256, jobs);
-    gather_convert_kernel<<<grid, 256, 0, stream>>>(x, g2c, (__half*)xh, (__half*)xl, (__half*)sums_h, (__half*)sums_l,
-                                                    tc_sums_cols(hidden), topk, hidden);
-    return cudaGetLastError();
+#pragma unroll 4
+    for (int k = 0; k < topk; k++) {
+        const int g = __ldg(c2g + (size_t)token * topk + k);
+        if (g < 0 || g >= jobs) continue;         // a selection without an expert (reported by the plan kernel)
+        *(uint4*)(xh + (size_t)g * hidden + d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        if (xl) {
+            *(uint4*)(xl + (size_t)g * hidden + d) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            if ((threadIdx.x & 7) == 0) store_group_mean(sums_h, sums_l, (size_t)g * sums_stride, d / TC_KC, sum * (1.0f / TC_KC));
+        }
+    }
 }
 
 // Powers of two that bring every weight row of an expert pool into fp16: the largest of 8 |s| and 64 |c| of a row becomes
@@ -920,73 +998,22 @@ static cudaError_t launch_tc(const TcArgs& a, const TcMaps& maps, const TcMaps& 
     return cudaGetLastError();
 }
 
-// Work lists of a layer's two launches: for every expert group with tokens, every 128-token pass, every row
-// tile one item (tiles of a pass adjacent, so neighbouring blocks share the pass' token rows in L2).  One block.
-__global__ void __launch_bounds__(256)
-q4_tc_work_list_kernel(const Q4Job* __restrict__ jobs, const int* __restrict__ njobs_dev, int njobs_max,
-                       const float* y_base, int y_cols, const uint8_t* pool, size_t expert_stride, int nx_fused,
-                       int nx_plain, TcItem* __restrict__ items_fused, TcItem* __restrict__ items_plain,
-                       int* __restrict__ work) {
-    extern __shared__ int s_list[];           // [njobs_max + 1] first pass of every job, then expert, first row, tokens
-    int* s_base = s_list;
-    int* s_expert = s_list + njobs_max + 1;
-    int* s_g0 = s_expert + njobs_max;
-    int* s_ntok = s_g0 + njobs_max;
-    __shared__ int s_nt_max;
-    const int njobs = njobs_dev ? min(*njobs_dev, njobs_max) : njobs_max;
-    if (threadIdx.x == 0) s_nt_max = 0;
-    __syncthreads();
-    for (int j = threadIdx.x; j < njobs_max; j += blockDim.x) {
-        int ntok = 0;
-        if (j < njobs) {
-            const Q4Job jb = jobs[j];
-            ntok = max(jb.ntok, 0);
-            s_expert[j] = (int)((size_t)(jb.vals - pool) / expert_stride);
-            s_g0[j] = (int)((jb.y - y_base) / y_cols);
-        }
-        s_ntok[j] = ntok;
-        s_base[j + 1] = (ntok + TC_MAX_NT - 1) / TC_MAX_NT;
-        if (ntok > 0) atomicMax(&s_nt_max, min(ntok, TC_MAX_NT));
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_base[0] = 0;
-        for (int j = 0; j < njobs_max; j++) s_base[j + 1] += s_base[j];
-        const int passes = s_base[njobs_max];
-        work[0] = passes * nx_fused; work[1] = 0; work[2] = s_nt_max;
-        work[4] = passes * nx_plain; work[5] = 0; work[6] = s_nt_max;
-    }
-    __syncthreads();
-    const int nxt = nx_fused + nx_plain;
-    for (int j = 0; j < njobs; j++) {
-        const int base = s_base[j], np = s_base[j + 1] - base;
-        for (int i = threadIdx.x; i < np * nxt; i += blockDim.x) {
-            const int p = i / nxt, x = i - p * nxt;
-            TcItem it;
-            it.expert = s_expert[j]; it.grow = s_g0[j] + p * TC_MAX_NT; it.nt = min(TC_MAX_NT, s_ntok[j] - p * TC_MAX_NT);
-            if (x < nx_fused) {
-                it.r0 = x * (TW_ROWS / 2);
-                items_fused[(size_t)(base + p) * nx_fused + x] = it;
-            } else {
-                it.r0 = (x - nx_fused) * TW_ROWS;
-                items_plain[(size_t)(base + p) * nx_plain + (x - nx_fused)] = it;
-            }
-        }
-    }
-}
-
 size_t q4_tc_work_items_max(int n_experts, int rows_total, int hidden, int inter) {
     const size_t passes = (size_t)n_experts + (size_t)rows_total / TC_MAX_NT + 1;
     return passes * (size_t)std::max((inter + 127) / 128, (hidden + TW_ROWS - 1) / TW_ROWS);
 }
 
-cudaError_t launch_q4_tc_work_list(const Q4Job* gateup_jobs, const int* njobs_dev, int njobs_max, const float* y_base,
-                                   int y_cols, const TcWeightMaps& wm, int hidden, int inter, void* items_fused,
-                                   void* items_plain, int* work, cudaStream_t stream) {
-    if (njobs_max < 1) return cudaSuccess;
-    q4_tc_work_list_kernel<<<1, 256, (size_t)(4 * njobs_max + 1) * sizeof(int), stream>>>(
-        gateup_jobs, njobs_dev, njobs_max, y_base, y_cols, wm.pool, wm.expert_stride, (inter + 127) / 128,
-        (hidden + TW_ROWS - 1) / TW_ROWS, (TcItem*)items_fused, (TcItem*)items_plain, work);
+cudaError_t launch_tc_prepare(const float* x, const int32_t* c2g, void* xh, void* xl, void* sums_h, void* sums_l, int rows,
+                              int topk, int hidden, int inter, const Q4Job* gateup_jobs, const int* njobs_dev, int njobs_max,
+                              const float* y_base, int y_cols, const TcWeightMaps& wm, void* items_fused, void* items_plain,
+                              int* work, cudaStream_t stream) {
+    if (rows < 1 || njobs_max < 1) return cudaSuccess;
+    if (hidden % 64 || rows >= 65535) return cudaErrorInvalidValue;
+    const WorkListArgs lists = {gateup_jobs, njobs_dev, njobs_max, y_base, y_cols, wm.pool, wm.expert_stride, (inter + 127) / 128,
+                                (hidden + TW_ROWS - 1) / TW_ROWS, (TcItem*)items_fused, (TcItem*)items_plain, work};
+    const dim3 grid((hidden / 8 + GATHER_THREADS - 1) / GATHER_THREADS, rows + 1);
+    scatter_convert_kernel<<<grid, GATHER_THREADS, (size_t)(4 * njobs_max + 1) * sizeof(int), stream>>>(
+        x, c2g, (__half*)xh, (__half*)xl, (__half*)sums_h, (__half*)sums_l, tc_sums_cols(hidden), rows * topk, topk, hidden, lists);
     return cudaGetLastError();
 }
 

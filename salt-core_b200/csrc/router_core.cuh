@@ -387,11 +387,12 @@ static __device__ __forceinline__ void topk_group(bool active, const float* lr, 
     }
     __syncthreads();
     if (go && ltid < 32) {
-        const float all = serial_sum(se, E);
+        const float all = (E & 63) == 0 && (((uintptr_t)se) & 15) == 0 ? chain_sum(se, E) : serial_sum(se, E);
         bool bad = !(all > 0.0f) || !finite_f(all);
         for (int j = ltid; j < topk; j += 32) sw[j] = __fdiv_rn(se[ssel[j]], all);
         __syncwarp();
         float selsum = 0.0f;
+#pragma unroll 8
         for (int j = 0; j < topk; j++) selsum = __fadd_rn(selsum, sw[j]);
         if (!(selsum > 0.0f) || !finite_f(selsum)) bad = true;
         for (int j = ltid; j < topk; j += 32) {
@@ -401,6 +402,7 @@ static __device__ __forceinline__ void topk_group(bool active, const float* lr, 
             int pos = j;
             if (sort_by_expert) {
                 pos = 0;
+#pragma unroll 8
                 for (int i = 0; i < topk; i++) pos += (ssel[i] < e) ? 1 : 0;
             }
             sel_out[pos] = e;

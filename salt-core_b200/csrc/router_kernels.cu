@@ -365,105 +365,105 @@ __global__ void __launch_bounds__(GLUE_NV == 4 ? 1024 : 512) glue_rows_kernel(Gl
     if (bad) flag(a.status, SB_ERR_NONFINITE);
 }
 
-// The same glue for batches of several hundred rows: one WARP per row, lane l holds the CH
-// consecutive columns [l*CH, (l+1)*CH) in registers, and each in-order sum is the plain
-// dependent-add chain handed from lane to lane (the reference's order: columns ascending from
-// +0).  A chain costs about 6.5 us, but thousands of rows run side by side (16 warps per SM),
-// where the block-per-row form above keeps a whole SM busy for 13 us per pair of rows.
+// The same glue for batches of several hundred rows: a warp per row, four rows per block.  Lane l holds 16-byte pieces l,
+// l + 32, ... of its row in registers.  The squares of the four rows go to shared memory and ONE warp runs the four
+// in-order sums side by side, a row per lane (the reference's order: columns ascending from +0).  A chain costs about
+// 6 us, but the rows of a few blocks per SM run side by side, where the block-per-row form above keeps a whole SM busy for
+// 13 us per pair of rows.  (Rows in lane-contiguous pieces, the sum handed from lane to lane, loaded 32 lines per
+// instruction: 1999 rows took 68 us for reduce and two sums, this takes 56; 256 rows of 5120 columns 38 us -> 29.)
+constexpr int GLUE_ROWS = 4;
+static __device__ __forceinline__ uint32_t glue_pitch(int n) { return (uint32_t)n + 4u; }    // the rows start four banks apart
+
+// Squares of the warps' rows in sq[GLUE_ROWS][pitch] -> s_inv[r] = pow(sum / n + eps, -0.5) for every row of the block.
 template <int CH>
-static __device__ __forceinline__ float warp_chain_sum_of_squares(const float (&v)[CH], int lane) {
-    float acc = 0.0f;
-#pragma unroll 1
-    for (int l = 0; l < 32; l++) {
-        float a = __shfl_sync(0xffffffffu, acc, (l + 31) & 31);
-        if (l == 0) a = 0.0f;
-        if (lane == l) {
+static __device__ __forceinline__ void glue_inv_rms(const float4 (&v)[CH / 4], float* sq, float* s_inv, float eps) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, n = 32 * CH;
+    float4* mine = (float4*)(sq + w * glue_pitch(n)) + lane;
 #pragma unroll
-            for (int i = 0; i < CH; i++) a = __fadd_rn(a, __fmul_rn(v[i], v[i]));
-            acc = a;
-        }
+    for (int i = 0; i < CH / 4; i++)
+        mine[32 * i] = make_float4(__fmul_rn(v[i].x, v[i].x), __fmul_rn(v[i].y, v[i].y), __fmul_rn(v[i].z, v[i].z), __fmul_rn(v[i].w, v[i].w));
+    __syncthreads();
+    if (w == ((blockIdx.x / 148) & 3)) {          // blocks that share an SM add on different schedulers
+        const float ss = chain_sum(sq + (lane & 3) * glue_pitch(n), n);
+        if (lane < GLUE_ROWS) s_inv[lane] = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)n), eps));
     }
-    return __shfl_sync(0xffffffffu, acc, 31);
+    __syncthreads();
 }
 
+static __device__ __forceinline__ bool all_finite(const float4& v) { return finite_f(v.x) && finite_f(v.y) && finite_f(v.z) && finite_f(v.w); }
+
 template <int CH>
-__global__ void __launch_bounds__(128, CH > 96 ? 2 : 4) glue_rows_warp_kernel(GlueArgs a, int rows) {
-    static_assert(CH % 4 == 0, "rows are moved in 16-byte pieces");
-    const int lane = threadIdx.x & 31;
-    const int row = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (row >= rows) return;
+__global__ void __launch_bounds__(32 * GLUE_ROWS, CH > 96 ? 2 : 4) glue_rows_warp_kernel(GlueArgs a, int rows) {
+    static_assert(CH % 4 == 0 && GLUE_ROWS == 4, "rows are moved in 16-byte pieces; four schedulers");
+    extern __shared__ __align__(16) float gsm[];
+    __shared__ float s_inv[GLUE_ROWS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const bool live = blockIdx.x * GLUE_ROWS + w < rows;            // rows past the end: the last one again, not stored
+    const int row = live ? blockIdx.x * GLUE_ROWS + w : rows - 1;
     const int n = a.n;                         // == 32 * CH
-    const int c0 = lane * CH;
     bool bad = false;
-    float v[CH];
+    float4 v[CH / 4];
 #pragma unroll
-    for (int i = 0; i < CH; i++) v[i] = 0.0f;
+    for (int i = 0; i < CH / 4; i++) v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (a.grouped != nullptr) {
         for (int r = 0; r < a.topk; r++) {
             const int g = a.c2g[row * a.topk + r];
-            const float w = a.weights[row * a.topk + r];
-            if (g < 0 || g >= a.jobs || !finite_f(w)) {
+            const float f = a.weights[row * a.topk + r];
+            if (g < 0 || g >= a.jobs || !finite_f(f)) {
                 if (lane == 0) flag(a.status, g < 0 || g >= a.jobs ? SB_ERR_INDEX : SB_ERR_NONFINITE);
                 continue;
             }
-            const float4* src = (const float4*)(a.grouped + (size_t)g * n + c0);
+            const float4* src = (const float4*)(a.grouped + (size_t)g * n) + lane;
 #pragma unroll
             for (int i = 0; i < CH / 4; i++) {
-                const float4 o = __ldg(src + i);
-                v[4 * i + 0] = __fadd_rn(v[4 * i + 0], __fmul_rn(w, o.x));
-                v[4 * i + 1] = __fadd_rn(v[4 * i + 1], __fmul_rn(w, o.y));
-                v[4 * i + 2] = __fadd_rn(v[4 * i + 2], __fmul_rn(w, o.z));
-                v[4 * i + 3] = __fadd_rn(v[4 * i + 3], __fmul_rn(w, o.w));
+                const float4 o = __ldg(src + 32 * i);
+                v[i].x = __fadd_rn(v[i].x, __fmul_rn(f, o.x));
+                v[i].y = __fadd_rn(v[i].y, __fmul_rn(f, o.y));
+                v[i].z = __fadd_rn(v[i].z, __fmul_rn(f, o.z));
+                v[i].w = __fadd_rn(v[i].w, __fmul_rn(f, o.w));
             }
         }
     } else {
-        const float4* src = (const float4*)(a.x_in + (size_t)row * n + c0);
+        const float4* src = (const float4*)(a.x_in + (size_t)row * n) + lane;
 #pragma unroll
-        for (int i = 0; i < CH / 4; i++) {
-            const float4 o = src[i];
-            v[4 * i + 0] = o.x; v[4 * i + 1] = o.y; v[4 * i + 2] = o.z; v[4 * i + 3] = o.w;
-        }
+        for (int i = 0; i < CH / 4; i++) v[i] = src[32 * i];
     }
     if (a.norm_w != nullptr) {
-        const float ss = warp_chain_sum_of_squares<CH>(v, lane);
-        const float inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)n), a.eps_norm));
+        glue_inv_rms<CH>(v, gsm, s_inv, a.eps_norm);
+        const float inv = s_inv[w];
         if (!finite_f(inv) && lane == 0) flag(a.status, SB_ERR_NONFINITE);
-        const float4* nw4 = (const float4*)(a.norm_w + c0);
+        const float4* nw4 = (const float4*)a.norm_w + lane;
 #pragma unroll
         for (int i = 0; i < CH / 4; i++) {
-            const float4 w = __ldg(nw4 + i);
-            bad |= !finite_f(v[4 * i]) || !finite_f(v[4 * i + 1]) || !finite_f(v[4 * i + 2]) || !finite_f(v[4 * i + 3]);
-            bad |= !finite_f(w.x) || !finite_f(w.y) || !finite_f(w.z) || !finite_f(w.w);
-            v[4 * i + 0] = __fmul_rn(__fmul_rn(v[4 * i + 0], inv), w.x);
-            v[4 * i + 1] = __fmul_rn(__fmul_rn(v[4 * i + 1], inv), w.y);
-            v[4 * i + 2] = __fmul_rn(__fmul_rn(v[4 * i + 2], inv), w.z);
-            v[4 * i + 3] = __fmul_rn(__fmul_rn(v[4 * i + 3], inv), w.w);
+            const float4 m = __ldg(nw4 + 32 * i);
+            bad |= !all_finite(v[i]) || !all_finite(m);
+            v[i].x = __fmul_rn(__fmul_rn(v[i].x, inv), m.x);
+            v[i].y = __fmul_rn(__fmul_rn(v[i].y, inv), m.y);
+            v[i].z = __fmul_rn(__fmul_rn(v[i].z, inv), m.z);
+            v[i].w = __fmul_rn(__fmul_rn(v[i].w, inv), m.w);
         }
     }
-    if (a.y_out != nullptr) {
-        float4* dst = (float4*)(a.y_out + (size_t)row * n + c0);
+    if (a.y_out != nullptr && live) {
+        float4* dst = (float4*)(a.y_out + (size_t)row * n) + lane;
 #pragma unroll
-        for (int i = 0; i < CH / 4; i++) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        for (int i = 0; i < CH / 4; i++) dst[32 * i] = v[i];
     }
     if (a.router_scale != nullptr) {
-        const float ss = warp_chain_sum_of_squares<CH>(v, lane);
-        const float inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)n), a.eps_router));
-        const float root = __fdiv_rn(1.0f, sqrtf_exact((float)n));
+        glue_inv_rms<CH>(v, gsm, s_inv, a.eps_router);
+        const float inv = s_inv[w], root = __fdiv_rn(1.0f, sqrtf_exact((float)n));
         if ((!finite_f(inv) || !finite_f(root)) && lane == 0) flag(a.status, SB_ERR_NONFINITE);
-        const float4* rs4 = (const float4*)(a.router_scale + c0);
-        float4* dst = (float4*)(a.rin + (size_t)row * n + c0);
+        const float4* rs4 = (const float4*)a.router_scale + lane;
+        float4* dst = (float4*)(a.rin + (size_t)row * n) + lane;
 #pragma unroll
         for (int i = 0; i < CH / 4; i++) {
-            const float4 w = __ldg(rs4 + i);
+            const float4 m = __ldg(rs4 + 32 * i);
             float4 t;
-            t.x = __fmul_rn(__fmul_rn(__fmul_rn(v[4 * i + 0], inv), w.x), root);
-            t.y = __fmul_rn(__fmul_rn(__fmul_rn(v[4 * i + 1], inv), w.y), root);
-            t.z = __fmul_rn(__fmul_rn(__fmul_rn(v[4 * i + 2], inv), w.z), root);
-            t.w = __fmul_rn(__fmul_rn(__fmul_rn(v[4 * i + 3], inv), w.w), root);
-            bad |= !finite_f(v[4 * i]) || !finite_f(v[4 * i + 1]) || !finite_f(v[4 * i + 2]) || !finite_f(v[4 * i + 3]);
-            bad |= !finite_f(w.x) || !finite_f(w.y) || !finite_f(w.z) || !finite_f(w.w);
-            bad |= !finite_f(t.x) || !finite_f(t.y) || !finite_f(t.z) || !finite_f(t.w);
-            dst[i] = t;
+            t.x = __fmul_rn(__fmul_rn(__fmul_rn(v[i].x, inv), m.x), root);
+            t.y = __fmul_rn(__fmul_rn(__fmul_rn(v[i].y, inv), m.y), root);
+            t.z = __fmul_rn(__fmul_rn(__fmul_rn(v[i].z, inv), m.z), root);
+            t.w = __fmul_rn(__fmul_rn(__fmul_rn(v[i].w, inv), m.w), root);
+            bad |= !all_finite(v[i]) || !all_finite(m) || !all_finite(t);
+            if (live) dst[32 * i] = t;
         }
     }
     if (bad) flag(a.status, SB_ERR_NONFINITE);
@@ -476,8 +476,13 @@ cudaError_t launch_glue(const GlueArgs& a, int rows, cudaStream_t stream) {
     const auto al16 = [](const void* p) { return (((uintptr_t)p) & 15) == 0; };
     if (rows >= 256 && (a.n == 32 * 88 || a.n == 32 * 160) && al16(a.grouped) && al16(a.x_in) && al16(a.y_out) &&
         al16(a.norm_w) && al16(a.router_scale) && al16(a.rin)) {
-        if (a.n == 32 * 88) glue_rows_warp_kernel<88><<<(rows + 3) / 4, 128, 0, stream>>>(a, rows);
-        else glue_rows_warp_kernel<160><<<(rows + 3) / 4, 128, 0, stream>>>(a, rows);
+        const size_t wsmem = (size_t)GLUE_ROWS * (a.n + 4) * sizeof(float);
+        const void* kernel = a.n == 32 * 88 ? (const void*)glue_rows_warp_kernel<88> : (const void*)glue_rows_warp_kernel<160>;
+        cudaError_t e = ensure_dynamic_smem(kernel, wsmem);
+        if (e != cudaSuccess) return e;
+        const int blocks = (rows + GLUE_ROWS - 1) / GLUE_ROWS;
+        if (a.n == 32 * 88) glue_rows_warp_kernel<88><<<blocks, 32 * GLUE_ROWS, wsmem, stream>>>(a, rows);
+        else glue_rows_warp_kernel<160><<<blocks, 32 * GLUE_ROWS, wsmem, stream>>>(a, rows);
         return cudaGetLastError();
     }
     if (a.n <= 4096) {

@@ -119,7 +119,7 @@ cudaError_t make_tc_maps(TcMaps* out, const void* hi, const void* lo, int rows, 
 // Columns of the group means of a row of `cols` columns, in the layout of the correction chunks (32 groups per 64 columns).
 inline int tc_sums_cols(int cols) { return (cols / 64 + 31) / 32 * 64; }
 // Tiled maps over a layer's expert pool (packed nibbles; gate, up: boxes of 128 rows, down: 256), and its derived tables:
-// (scale << 16) | bias words, and per weight row a power of two that brings the row into fp16, with its inverse
+// (scale << 16) | bias words by group, and per weight row a power of two that brings the row into fp16, with its inverse
 // ([experts][2 inter + hidden]; hi + lo precision).
 struct TcWeightMaps {
     CUtensorMap w[2];
@@ -129,8 +129,8 @@ struct TcWeightMaps {
     const uint32_t* tables;
     const float *row_scale, *row_unscale;
 };
-cudaError_t launch_q4_row_scales(const uint32_t* tables, int hidden, int inter, int experts, float* scale, float* unscale,
-                                 cudaStream_t stream);
+cudaError_t launch_q4_tc_tables(const uint32_t* tables, int hidden, int inter, int experts, uint32_t* by_group, float* scale,
+                                float* unscale, cudaStream_t stream);
 cudaError_t make_q4_tc_weight_maps(TcWeightMaps* out, const uint8_t* pool, size_t expert_stride, const uint32_t* tables,
                                    const float* row_scale, const float* row_unscale, int hidden, int inter, int experts);
 // Can the tensor-core kernels take this geometry?  Sizes must be multiples of 64; a size that is no multiple of

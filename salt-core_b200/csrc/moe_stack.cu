@@ -31,7 +31,8 @@ struct Layer {
     float* norm_weight = nullptr;
     uint8_t* pool = nullptr;   // local experts only; slot of expert e at pool + (e - expert_begin) * stride
     uint8_t* sb_tables = nullptr;   // derived copy for the fused decode kernels: (scale << 16) | bias words, [local][3][groups]
-    float *row_scale = nullptr, *row_unscale = nullptr;   // tensor-core path: power of two per weight row, and its inverse
+    uint32_t* tc_tables = nullptr;  // tensor-core path: the same words by group, [local][3][groups per row][rows] ...
+    float *row_scale = nullptr, *row_unscale = nullptr;   // ... a power of two per weight row, and its inverse
     int* lit_flags = nullptr;       // [local] bit k: tensor k of the expert has a scale that needs the two-rounding form
     size_t expert_stride = 0;
     float eps = 0.0f;
@@ -136,7 +137,7 @@ static void free_stack(Stack* s) {
     for (auto& l : s->layers) {
         cudaFree(l.router_w); cudaFree(l.router_scale); cudaFree(l.per_expert_scale);
         cudaFree(l.norm_weight); cudaFree(l.pool); cudaFree(l.sb_tables); cudaFree(l.lit_flags); cudaFree(l.fp4_experts);
-        cudaFree(l.row_scale); cudaFree(l.row_unscale);
+        cudaFree(l.tc_tables); cudaFree(l.row_scale); cudaFree(l.row_unscale);
         cudaFree(l.pre_ffn_norm); cudaFree(l.pre_ffn_norm_2); cudaFree(l.post_ffn_norm_1);
         cudaFree(l.post_ffn_norm_2); cudaFree(l.post_ffn_norm); cudaFree(l.dense); cudaFree(l.dense_jobs);
     }
@@ -275,19 +276,19 @@ int salt_b200_stack_add_q4_layer(void* stack, const SaltB200Q4LayerSpec* spec) {
     ok = ok && dev_alloc(&l.sb_tables, local * 3 * groups * 4) && dev_alloc(&l.lit_flags, local) &&
          cuda_ok(launch_q4_interleave_tables(l.pool, l.expert_stride, tensor_bytes, elems / 2, groups, (int)local,
                                              (uint32_t*)l.sb_tables, l.lit_flags, 0), "scale tables");
-    if (ok && s->tc_split_ready) {
+    if (ok && s->tc_ready) {
         const size_t rows = local * (size_t)(2 * s->inter + s->hidden);
-        ok = dev_alloc(&l.row_scale, rows) && dev_alloc(&l.row_unscale, rows) &&
-             cuda_ok(launch_q4_row_scales((const uint32_t*)l.sb_tables, s->hidden, s->inter, (int)local, l.row_scale,
-                                          l.row_unscale, 0), "row scales");
+        ok = dev_alloc(&l.tc_tables, local * 3 * groups) && dev_alloc(&l.row_scale, rows) && dev_alloc(&l.row_unscale, rows) &&
+             cuda_ok(launch_q4_tc_tables((const uint32_t*)l.sb_tables, s->hidden, s->inter, (int)local, l.tc_tables, l.row_scale,
+                                          l.row_unscale, 0), "tensor-core tables");
     }
     ok = ok && cuda_ok(cudaDeviceSynchronize(), "scale tables");
     if (!ok) {
         cudaFree(l.router_w); cudaFree(l.router_scale); cudaFree(l.per_expert_scale); cudaFree(l.pool);
-        cudaFree(l.norm_weight); cudaFree(l.sb_tables); cudaFree(l.lit_flags); cudaFree(l.row_scale); cudaFree(l.row_unscale);
+        cudaFree(l.norm_weight); cudaFree(l.sb_tables); cudaFree(l.lit_flags); cudaFree(l.tc_tables); cudaFree(l.row_scale); cudaFree(l.row_unscale);
         return -1;
     }
-    l.q4_tc_ok = s->tc_ready && make_q4_tc_weight_maps(&l.q4_tc, l.pool, l.expert_stride, (const uint32_t*)l.sb_tables,
+    l.q4_tc_ok = s->tc_ready && make_q4_tc_weight_maps(&l.q4_tc, l.pool, l.expert_stride, l.tc_tables,
                                                         l.row_scale, l.row_unscale, s->hidden, s->inter, (int)local) == cudaSuccess;
     s->layers.push_back(l);
     return (int)s->layers.size() - 1;

@@ -6,7 +6,7 @@
 //   single  weights dequantised as q*s+b and rounded to fp16, activations rounded to fp16: max |err| about 5e-4 to
 //           7e-4 of the row maximum
 //   split   x * (q s + b) = x * (q - 8) s + x * (b + 8 s).  (q - 8) s has at most 4 + 8 significant bits, so it is EXACT
-//           in fp16 once the row is scaled by a power of two (q4_row_scale_kernel) that keeps it in range; b + 8 s is
+//           in fp16 once the row is scaled by a power of two (q4_tc_tables_kernel) that keeps it in range; b + 8 s is
 //           constant over a quantisation group, so its part of the sum is a second, 64 times shorter contraction of the
 //           groups' means of x with c = b + 8 s (hi + lo halves): one or a few "correction" chunks after the ordinary
 //           ones.  Activations are hi + lo halves (lo = fp16(x - hi)).  So a K step takes two products, Xh W and Xl W,
@@ -40,7 +40,8 @@
 // Measured (B200, 1965 MHz, a whole expert layer: hidden 2816, inter 704, 128 experts,
 // top-8): 512 tokens in split precision 800 us with three MMAs per K step on split weights -> 515 with exact weights and
 // separate rings -> 473 with the delayed epilogue, four stages and the correction chunk's table words loaded at once (they
-// came in four serial batches, 9000 cycles a chunk).  1999 tokens in single precision 780 -> 707 -> 694.  In the same
+// came in four serial batches, 9000 cycles a chunk) -> 430 with cheaper kernels around the GEMMs and tables by group.
+// 1999 tokens in single precision 780 -> 707 -> 694 -> 607.  In that
 // state the tensor pipe is busy 35 to 40 % of the time and the schedulers issue in 45 % of the cycles.
 // What was measured on the way here: a register ring of global loads for the packed bytes does not prefetch - waiting for
 // the oldest load also waits for the younger ones that share its scoreboard (hence TMA); one mbarrier wait costs 150 to 250
@@ -251,7 +252,7 @@ struct TcArgs {
     int sums_stride;
     float* out_f;              // plain: projection output [grouped rows][R] fp32
     int* status;
-    const uint32_t* tables;    // (scale << 16) | bias words, [local expert][3 tensors][R * C/64]
+    const uint32_t* tables;    // (scale << 16) | bias words, [local expert][3 tensors][C/64][R]: a chunk's words of 32 rows are one line
     const float* row_scale;    // split: power of two per weight row, [local expert][2 inter + hidden], gate | up | down ...
     const float* row_unscale;  // ... and its inverse
     int scale_stride;          // 2 inter + hidden
@@ -302,6 +303,17 @@ __device__ __forceinline__ uint32_t mbar_test(uint64_t* bar, uint32_t parity) {
         : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
     return r;
+}
+
+__device__ __forceinline__ uint32_t take_now(uint32_t v) {
+    uint32_t r;
+    asm volatile("mov.b32 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+__device__ __forceinline__ uint32_t ldg_now(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
 }
 
 __device__ __forceinline__ uint4 lds_v4(const uint8_t* p) {
@@ -533,12 +545,12 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
             const TcItem item = s_items[unit % TC_ITEM_RING];
             const int mine = item.nt < 1 ? 0 : total;                    // nt < 1: end of the work
             const int mat = FUSED ? crow / RT : 0, row = min(item.r0 + crow % RT, a.R - 1);
-            const uint32_t* tab = a.tables + ((size_t)(item.expert * 3 + a.tensor0 + mat) * a.R + row) * nchunks;
+            const uint32_t* tab = a.tables + (size_t)(item.expert * 3 + a.tensor0 + mat) * a.R * nchunks + row;     // + group * R
             float rs = 1.0f;
             if (SPLIT) rs = __ldg(a.row_scale + (size_t)item.expert * a.scale_stride + a.scale_off + mat * a.R + row);
             // this group's chunks of the unit: every other one of the block's running count
             const int first = (int)((it0 ^ grp) & 1u);
-            uint32_t word_next = mine > 0 && first < nchunks ? __ldg(tab + first) : 0u;
+            uint32_t word_next = mine > 0 && first < nchunks ? __ldg(tab + (size_t)first * a.R) : 0u;
             // The unit before is finished after this group's second chunk: the tensor core has work while its accumulators
             // are read, and no converter waits for its last MMA.
             uint32_t w_here = 0u;
@@ -552,8 +564,10 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
                 uint8_t* const st = line + s * TW_B_BYTES;
                 if (!SPLIT || kc < nchunks) {
                     const uint32_t slot = (w0 + kc) & (NW - 1), wph = ((w0 + kc) >> nw_shift) & 1u;
-                    const uint32_t word = word_next;
-                    word_next = kc + 2 < nchunks ? __ldg(tab + kc + 2) : 0u;     // a chunk pair ahead: its latency is covered
+                    // the next word a chunk pair ahead; this one is taken over BEFORE that load is issued, or waiting for it
+                    // would also wait for the younger load on the same scoreboard (600 cycles a chunk)
+                    const uint32_t word = take_now(word_next);
+                    word_next = kc + 2 < nchunks ? ldg_now(tab + (size_t)(kc + 2) * a.R) : 0u;
                     if (!__all_sync(0xffffffffu, w_here) && !__all_sync(0xffffffffu, mbar_wait(&bar_w[slot], wph, fail))) { alive = false; break; }
                     const uint8_t* pk = pk_base + slot * TW_PK_BYTES + crow * 32;
                     const uint4 p[2] = {lds_v4(pk), lds_v4(pk + 16)};
@@ -589,20 +603,11 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
                                        o[i >> 2][4 * (i & 3) + 3]);
                 } else {
                     // correction chunk: 32 groups, eight per K step of 16 columns: 64 c as hi, then as lo halves
-                    if (round > 0 && !__all_sync(0xffffffffu, mbar_wait(&bar_done[s], (round - 1) & 1u, fail))) { alive = false; break; }
                     const int g0 = (kc - nchunks) * 32;
                     uint32_t w[32];                                      // all words of the row at once: one latency
-                    if ((nchunks & 3) == 0) {
 #pragma unroll
-                        for (int j = 0; j < 8; j++) {
-                            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                            if (g0 + 4 * j < nchunks) v = __ldg((const uint4*)(tab + g0) + j);
-                            w[4 * j] = v.x; w[4 * j + 1] = v.y; w[4 * j + 2] = v.z; w[4 * j + 3] = v.w;
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j++) w[j] = g0 + j < nchunks ? __ldg(tab + g0 + j) : 0u;
-                    }
+                    for (int j = 0; j < 32; j++) w[j] = g0 + j < nchunks ? ldg_now(tab + (size_t)(g0 + j) * a.R) : 0u;
+                    if (round > 0 && !__all_sync(0xffffffffu, mbar_wait(&bar_done[s], (round - 1) & 1u, fail))) { alive = false; break; }
 #pragma unroll
                     for (int ks = 0; ks < 4; ks++) {
                         uint32_t hi[4], lo[4];
@@ -875,20 +880,26 @@ scatter_convert_kernel(const float* __restrict__ x, const int32_t* __restrict__ 
     }
 }
 
-// Powers of two that bring every weight row of an expert pool into fp16: the largest of 8 |s| and 64 |c| of a row becomes
+// Derived tables of an expert pool: the (scale << 16) | bias words by group instead of by row (a converter warp's 32 rows
+// of a chunk lie in one line; by row its load touched 32 lines and took 300 to 500 cycles a chunk to issue), and
+// powers of two that bring every weight row into fp16: the largest of 8 |s| and 64 |c| of a row becomes
 // 2^9 .. 2^10.  Small scales of the row lose bits only below 2^-27 of its largest weight.
 __global__ void __launch_bounds__(256)
-q4_row_scale_kernel(const uint32_t* __restrict__ tables, int hidden, int inter, int experts, float* __restrict__ scale,
-                    float* __restrict__ unscale) {
+q4_tc_tables_kernel(const uint32_t* __restrict__ tables, int hidden, int inter, int experts, uint32_t* __restrict__ by_group,
+                    float* __restrict__ scale, float* __restrict__ unscale) {
     const int per = 2 * inter + hidden, n = experts * per;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int e = i / per, r = i % per, k = r < inter ? 0 : (r < 2 * inter ? 1 : 2), row = r - k * inter;
         const int groups = (k < 2 ? hidden : inter) / TC_KC;
-        const uint32_t* t = tables + ((size_t)(e * 3 + k) * ((size_t)hidden * inter / TC_KC)) + (size_t)row * groups;
+        const size_t tensor = (size_t)(e * 3 + k) * ((size_t)hidden * inter / TC_KC);
+        const uint32_t* t = tables + tensor + (size_t)row * groups;
+        uint32_t* o = by_group + tensor + row;
+        const int rows = k < 2 ? inter : hidden;
         float top = 0.0f;
         for (int g = 0; g < groups; g++) {
             const float s = bf16_bits_to_f32(t[g] >> 16), b = bf16_bits_to_f32(t[g] & 0xffffu);
             top = fmaxf(top, fmaxf(8.0f * fabsf(s), 64.0f * fabsf(b + 8.0f * s)));
+            o[(size_t)g * rows] = t[g];
         }
         int ex = 0;
         if (top > 0.0f && top < 3.0e38f) frexpf(top, &ex);       // top = m 2^ex, 1/2 <= m < 1
@@ -898,10 +909,10 @@ q4_row_scale_kernel(const uint32_t* __restrict__ tables, int hidden, int inter, 
     }
 }
 
-cudaError_t launch_q4_row_scales(const uint32_t* tables, int hidden, int inter, int experts, float* scale, float* unscale,
-                                 cudaStream_t stream) {
+cudaError_t launch_q4_tc_tables(const uint32_t* tables, int hidden, int inter, int experts, uint32_t* by_group, float* scale,
+                                float* unscale, cudaStream_t stream) {
     if (experts < 1) return cudaSuccess;
-    q4_row_scale_kernel<<<592, 256, 0, stream>>>(tables, hidden, inter, experts, scale, unscale);
+    q4_tc_tables_kernel<<<592, 256, 0, stream>>>(tables, hidden, inter, experts, by_group, scale, unscale);
     return cudaGetLastError();
 }
 
@@ -955,7 +966,7 @@ cudaError_t make_q4_tc_weight_maps(TcWeightMaps* out, const uint8_t* pool, size_
         if (e != cudaSuccess) return e;
     }
     if ((hidden % TC_KC) != 0 || (inter % TC_KC) != 0 || experts < 1 || (expert_stride % 16) != 0 ||
-        ((uintptr_t)pool % 16) != 0 || ((uintptr_t)tables % 16) != 0)
+        ((uintptr_t)pool % 16) != 0 || tables == nullptr || row_scale == nullptr || row_unscale == nullptr)
         return cudaErrorInvalidValue;
     const size_t elems = (size_t)hidden * inter;
     const size_t tensor_bytes = elems / 2 + 2 * (elems / 64 * 2);

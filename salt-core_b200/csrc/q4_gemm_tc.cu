@@ -316,6 +316,15 @@ __device__ __forceinline__ uint32_t ldg_now(const uint32_t* p) {
     return v;
 }
 
+// 32 bytes, 32-byte aligned, in one store.  The lanes of an epilogue warp write to 32 rows: every store instruction passes
+// the L1 as 32 lines whatever its width, so a 16-byte one takes twice as long for the same bytes and leaves half sectors
+// (a down unit of 128 tokens spent 4 to 8 us here with those).
+__device__ __forceinline__ void store_sector(void* p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+                 "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+
 __device__ __forceinline__ uint4 lds_v4(const uint8_t* p) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_u32(p)));
@@ -471,19 +480,16 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
                                 sum += o[i];
                             }
                             if (n < item.nt) {
+                                // the next GEMM's K order inside a group of 8: [0,4,1,5,2,6,3,7]
+                                uint32_t hw[8], lw[8];
 #pragma unroll
-                                for (int i8 = 0; i8 < 16; i8 += 8) {
-                                    // the next GEMM's K order inside a group of 8: [0,4,1,5,2,6,3,7]
-                                    uint32_t hw[4], lw[4];
-#pragma unroll
-                                    for (int kk = 0; kk < 4; kk++) {
-                                        hw[kk] = f16x2_from(o[i8 + kk], o[i8 + kk + 4]);
-                                        if (SPLIT)
-                                            lw[kk] = f16x2_from(o[i8 + kk] - f16_lo_to_f32(hw[kk]), o[i8 + kk + 4] - f16_hi_to_f32(hw[kk]));
-                                    }
-                                    *(uint4*)(a.out_h + o_off + i8) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-                                    if (SPLIT) *(uint4*)(a.out_l + o_off + i8) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+                                for (int kk = 0; kk < 8; kk++) {
+                                    const int i = (kk >> 2) * 8 + (kk & 3);
+                                    hw[kk] = f16x2_from(o[i], o[i + 4]);
+                                    if (SPLIT) lw[kk] = f16x2_from(o[i] - f16_lo_to_f32(hw[kk]), o[i + 4] - f16_hi_to_f32(hw[kk]));
                                 }
+                                store_sector(a.out_h + o_off, hw);
+                                if (SPLIT) store_sector(a.out_l + o_off, lw);
                             }
                         }
                         if (SPLIT) {
@@ -518,15 +524,13 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
                             uint32_t g[16];
                             sixteen(col, h, g);
                             float* dst = a.out_f + (size_t)(item.grow + n) * a.R + r0 + col + cc;
-                            float o[16];
+                            uint32_t o[2][8];
 #pragma unroll
-                            for (int i = 0; i < 16; i++) {
-                                o[i] = __uint_as_float(g[i]);
-                                if (SPLIT) o[i] *= __shfl_sync(0xffffffffu, f, cc + i);
-                            }
+                            for (int i = 0; i < 16; i++)
+                                o[i >> 3][i & 7] = SPLIT ? __float_as_uint(__uint_as_float(g[i]) * __shfl_sync(0xffffffffu, f, cc + i)) : g[i];
                             if (n < item.nt) {
-#pragma unroll
-                                for (int i = 0; i < 16; i += 4) *(float4*)(dst + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+                                store_sector(dst, o[0]);
+                                store_sector(dst + 8, o[1]);
                             }
                         }
                     }

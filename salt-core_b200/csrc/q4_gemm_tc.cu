@@ -467,7 +467,7 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
                             const size_t o_off = (size_t)(item.grow + n) * a.R + r0 + c0;
                             uint32_t g[16], u[16];
                             sixteen(col, h, g);
-                            sixteen(RT + col, h, u);
+                            sixteen((rows_here > RT / 2 ? RT : RT / 2) + col, h, u);
                             float o[16];
 #pragma unroll
                             for (int i = 0; i < 16; i++) {
@@ -548,7 +548,12 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
             if (!alive) break;
             const TcItem item = s_items[unit % TC_ITEM_RING];
             const int mine = item.nt < 1 ? 0 : total;                    // nt < 1: end of the work
-            const int mat = FUSED ? crow / RT : 0, row = min(item.r0 + crow % RT, a.R - 1);
+            // The last tile of gate and up may be 64 rows wide: the stage is then 64 rows of gate, 64 of up (one instruction of
+            // half the width) and the other warps only keep step.
+            const bool half = FUSED && a.R - item.r0 <= RT / 2;
+            const int mat = FUSED ? (half ? crow / (RT / 2) & 1 : crow / RT) : 0;
+            const int row = min(item.r0 + (half ? crow % (RT / 2) : crow % RT), a.R - 1);
+            const uint32_t pk_off = half ? (uint32_t)(mat * RT + crow % (RT / 2)) * 32u : (uint32_t)crow * 32u;
             const uint32_t* tab = a.tables + (size_t)(item.expert * 3 + a.tensor0 + mat) * a.R * nchunks + row;     // + group * R
             float rs = 1.0f;
             if (SPLIT) rs = __ldg(a.row_scale + (size_t)item.expert * a.scale_stride + a.scale_off + mat * a.R + row);
@@ -566,14 +571,21 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
                 if (kc >= mine) break;
                 const uint32_t it = it0 + (uint32_t)kc, round = ND == 4u ? it >> 2 : it / 3u, s = it - round * ND;
                 uint8_t* const st = line + s * TW_B_BYTES;
-                if (!SPLIT || kc < nchunks) {
+                if (FUSED && half && (warp & 4)) {
+                    if (!SPLIT || kc < nchunks) {
+                        const uint32_t slot = (w0 + kc) & (NW - 1), wph = ((w0 + kc) >> nw_shift) & 1u;
+                        if (!__all_sync(0xffffffffu, mbar_wait(&bar_w[slot], wph, fail))) { alive = false; break; }
+                        if (lane == 0) mbar_arrive(&bar_wfree[slot]);
+                    }
+                    if (round > 0 && !__all_sync(0xffffffffu, mbar_wait(&bar_done[s], (round - 1) & 1u, fail))) { alive = false; break; }
+                } else if (!SPLIT || kc < nchunks) {
                     const uint32_t slot = (w0 + kc) & (NW - 1), wph = ((w0 + kc) >> nw_shift) & 1u;
                     // the next word a chunk pair ahead; this one is taken over BEFORE that load is issued, or waiting for it
                     // would also wait for the younger load on the same scoreboard (600 cycles a chunk)
                     const uint32_t word = take_now(word_next);
                     word_next = kc + 2 < nchunks ? ldg_now(tab + (size_t)(kc + 2) * a.R) : 0u;
                     if (!__all_sync(0xffffffffu, w_here) && !__all_sync(0xffffffffu, mbar_wait(&bar_w[slot], wph, fail))) { alive = false; break; }
-                    const uint8_t* pk = pk_base + slot * TW_PK_BYTES + crow * 32;
+                    const uint8_t* pk = pk_base + slot * TW_PK_BYTES + pk_off;
                     const uint4 p[2] = {lds_v4(pk), lds_v4(pk + 16)};
                     // the MMAs that last read this stage: asked now, needed after the conversion
                     uint32_t stage_free = round == 0 ? 1u : mbar_test(&bar_done[s], (round - 1) & 1u);
@@ -653,7 +665,7 @@ q4_gemm_tc_kernel(const TcArgs a, const __grid_constant__ TcMaps maps, const __g
                 const TcItem item = s_items[unit % TC_ITEM_RING];
                 if (item.nt < 1) break;                                  // end of the work
                 const bool packed = item.nt <= TW_PACK_MAX;
-                const uint32_t idesc = umma_idesc_f16(128, FUSED ? TW_ROWS : min(RT, a.R - item.r0));
+                const uint32_t idesc = umma_idesc_f16(128, NMAT * min(RT, a.R - item.r0));
                 // this unit's accumulator buffer was last used two units ago: those accumulators have been read
                 if (unit >= 2 && !mbar_wait(&bar_epi[unit & 1u], ((unit >> 1) - 1) & 1u, fail)) { ok = false; break; }
                 const uint32_t acc_base = tmem + (unit & 1u) * TW_ROWS;

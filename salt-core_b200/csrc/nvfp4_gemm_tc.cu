@@ -168,24 +168,29 @@ nvfp4_gemm_tc_kernel(const Fp4TcArgs a, const __grid_constant__ Fp4TcMaps maps) 
         }
         __syncwarp();
     } else if (warp == 8) {
-        // ================= issuer =================
-        const uint32_t lo0 = DESC_B_LO | ((smem_u32(stage_base) & 0x3ffffu) >> 4);
-        uint32_t my = 0;
-        bool ok = true;
-        for (int i = 0; i < ntiles && ok; i++) {
-            const Fp4Tile& ti = s_tiles[i];
-            if (ti.ntok < 1) continue;
-            for (int tb = 0; tb < ti.ntok && ok; tb += FT_MAX_NT, issued_units++) {
-                const int NT = (min(FT_MAX_NT, ti.ntok - tb) + 15) & ~15;
-                const uint32_t idesc = umma_idesc_fp4(128, NT);
-                const uint32_t buf = issued_units & 1u;
-                // the epilogue has read this buffer's previous contents
-                if (issued_units >= 2u) ok = mbar_wait(&bar_accfree[buf], ((issued_units >> 1) - 1) & 1, fail);
-                for (int kc = 0; kc < nchunks && ok; kc++, my++) {
-                    const uint32_t s = my % FT_STAGES, ph = (my / FT_STAGES) & 1;
-                    ok = mbar_wait(&bar_full[s], ph, fail);
-                    if (ok) ok = mbar_wait(&bar_sf[s], ph, fail);
-                    if (ok && lane == 0) {
+        // ================= issuer (one thread) =================
+        // A barrier wait costs 150 to 250 cycles even when its phase is complete, and a stage needs two: they are polled
+        // together, and the next stage's before this stage's MMAs go out (a stage that this thread has used before is at
+        // most one phase behind, so the parity is not ambiguous).
+        if (lane == 0) {
+            const uint32_t lo0 = DESC_B_LO | ((smem_u32(stage_base) & 0x3ffffu) >> 4);
+            uint32_t my = 0, ready = 0;
+            bool ok = true;
+            for (int i = 0; i < ntiles && ok; i++) {
+                const Fp4Tile& ti = s_tiles[i];
+                const int ntok = ti.ntok;
+                for (int tb = 0; tb < ntok && ok; tb += FT_MAX_NT, issued_units++) {
+                    const int NT = (min(FT_MAX_NT, ntok - tb) + 15) & ~15;
+                    const uint32_t idesc = umma_idesc_fp4(128, NT);
+                    const uint32_t buf = issued_units & 1u;
+                    // the epilogue has read this buffer's previous contents
+                    if (issued_units >= 2u) ok = mbar_wait(&bar_accfree[buf], ((issued_units >> 1) - 1) & 1, fail);
+                    for (int kc = 0; kc < nchunks && ok; kc++, my++) {
+                        const uint32_t s = my % FT_STAGES, ph = (my / FT_STAGES) & 1;
+                        if (!ready) ok = mbar_wait2(&bar_full[s], ph, &bar_sf[s], ph, fail);
+                        if (!ok) break;
+                        const uint32_t ns = (my + 1) % FT_STAGES, nph = ((my + 1) / FT_STAGES) & 1;
+                        const uint32_t r_full = mbar_test(&bar_full[ns], nph), r_sf = mbar_test(&bar_sf[ns], nph);
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint32_t alo = lo0 + s * (FT_STAGE_BYTES >> 4);
                         const uint32_t blo = alo + (FT_A_BYTES >> 4);
@@ -197,11 +202,12 @@ nvfp4_gemm_tc_kernel(const Fp4TcArgs a, const __grid_constant__ Fp4TcMaps maps) 
                                      (kc > 0 || j > 0) ? 1u : 0u);
                         umma_commit(&bar_free[s]);
                         if (kc == nchunks - 1) umma_commit(&bar_done[buf]);
+                        ready = r_full & r_sf;
                     }
-                    __syncwarp();
                 }
             }
         }
+        __syncwarp();
     } else if (warp < 4) {
         // ================= scale warps =================
         // The producer's copies leave the chunk's 16 scale bytes of every row in the stage (weights: 128 rows,
@@ -209,18 +215,18 @@ nvfp4_gemm_tc_kernel(const Fp4TcArgs a, const __grid_constant__ Fp4TcMaps maps) 
         // l + 32, l + 64, l + 96 and stores them to its TMEM lane as 16 columns: column 4 j + c = K block j
         // (the MMA's K = 64) of row l + 32 c.
         const uint32_t tlane = tmem + ((uint32_t)(warp * 32) << 16);
-        uint32_t my = 0;
+        uint32_t my = 0, here = 0;
         bool ok = true;
         for (int i = 0; i < ntiles && ok; i++) {
-            const Fp4Tile& ti = s_tiles[i];
-            if (ti.ntok < 1) continue;
-            for (int tb = 0; tb < ti.ntok && ok; tb += FT_MAX_NT)
+            const int ntok = s_tiles[i].ntok;
+            for (int tb = 0; tb < ntok && ok; tb += FT_MAX_NT)
                 for (int kc = 0; kc < nchunks && ok; kc++, my++) {
                     const uint32_t s = my % FT_STAGES;
                     // landed copies also mean that the MMAs which last read this stage's scale columns are
                     // complete: the producer refilled the stage only after their commit
-                    ok = mbar_wait(&bar_full[s], (my / FT_STAGES) & 1, fail);
+                    if (!__all_sync(0xffffffffu, here)) ok = __all_sync(0xffffffffu, mbar_wait(&bar_full[s], (my / FT_STAGES) & 1, fail));
                     if (ok) {
+                        here = mbar_test(&bar_full[(my + 1) % FT_STAGES], ((my + 1) / FT_STAGES) & 1);    // asked ahead
                         const uint4* sfa = (const uint4*)(stage_base + s * FT_STAGE_BYTES + FT_A_BYTES + FT_B_BYTES);
                         const uint4* sfb = sfa + FT_SFA_BYTES / 16;
                         uint32_t wa[16], wb[16];

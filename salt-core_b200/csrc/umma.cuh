@@ -30,6 +30,51 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     return false;
 }
 
+// A wait for two barriers at once: both polls are in flight together, so the pair costs one barrier round trip.
+__device__ __forceinline__ bool mbar_wait2(uint64_t* bar_a, uint32_t par_a, uint64_t* bar_b, uint32_t par_b,
+                                           volatile int* fail) {
+    const uint32_t aa = smem_u32(bar_a), ab = smem_u32(bar_b);
+    uint32_t done_a = 0, done_b = 0;
+    for (uint32_t i = 0; i < TC_SPIN_LIMIT; i++) {
+        uint32_t ra = 1, rb = 1;
+        if (!done_a)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}\n"
+                : "=r"(ra)
+                : "r"(aa), "r"(par_a)
+                : "memory");
+        if (!done_b)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}\n"
+                : "=r"(rb)
+                : "r"(ab), "r"(par_b)
+                : "memory");
+        done_a |= ra;
+        done_b |= rb;
+        if (done_a && done_b) return true;
+        if ((i & 255u) == 255u && *fail) return false;
+    }
+    *fail = 1;
+    return false;
+}
+
+// One look at a barrier; asked for ahead of time, because the answer takes some 150 cycles.
+__device__ __forceinline__ uint32_t mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(r)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return r;
+}
+
 __device__ __forceinline__ uint64_t make_desc(uint32_t lo, uint32_t hi) {
     uint64_t d;
     asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));

@@ -536,7 +536,7 @@ int salt_b200_stack_profile(void *stack, int enable, int max_launches);
 int salt_b200_stack_profile_read(void *stack, float *ms_by_class, int *launches_by_class, int n_classes);
 /* Synchronise `stream`, read and clear the device error word.  0 = clean. */
 int salt_b200_stack_status(void *stack, void *stream);
-/* Number of kernel launches issued by this library since load. */
+/* Number of kernels this library has launched since load (a replayed graph adds nothing). */
 uint64_t salt_b200_launch_count(void);
 
 /* Debug tap: synchronise the device and copy nbytes of device memory to the host. */

@@ -10,6 +10,7 @@
 // CPU execution path in this file: a call that cannot run on the device
 // returns -1.
 #include <cuda_runtime.h>
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -31,8 +32,8 @@ namespace sb {
 
 void fp4_release();
 Backend g_backend;
-static uint64_t g_launches = 0;
-void count_launches(int n) { g_launches += (uint64_t)n; }
+static std::atomic<uint64_t> g_launches{0};      // stacks may be driven from several threads
+void count_launches(int n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
 
 cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes) {
     static std::mutex mu;
@@ -47,7 +48,7 @@ cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes) {
     if (e == cudaSuccess) have = bytes;
     return e;
 }
-uint64_t launch_count() { return g_launches; }
+uint64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 bool cuda_ok(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return true;
@@ -216,7 +217,6 @@ static bool run_jobs(int n, int njobs, size_t x_bytes, int max_rows, int max_tok
         if (!cuda_ok(launch_q8_jobs(dj, njobs, max_rows, max_tok, C, B.stream), "q8 launch")) return false;
     } else if (!cuda_ok(launch_q4_jobs(dj, njobs, nullptr, max_rows, max_tok, C, nmat, aligned, B.stream), "q4 launch"))
         return false;
-    count_launches(1);
     return true;
 }
 
@@ -542,7 +542,6 @@ static int bf16_run(const void* key, int R, int C, int Bt, const float* in, floa
     const cudaError_t e = serial ? launch_bf16_batch(W, B.d_x, y_dev, R, C, Bt, B.stream)
                                  : launch_bf16_matvec(W, B.d_x, y_dev, R, C, B.stream);
     if (!cuda_ok(e, "bf16 launch")) return -1;
-    count_launches(1);
     if (!stage_finish(nout * sizeof(float), "bf16 y download")) return -1;
     memcpy(out, B.h_y, nout * sizeof(float));
     return 0;
@@ -882,7 +881,6 @@ int salt_gpu_proj_batch_indexed(const uint32_t* vals, const uint16_t* scales, co
     if (!cuda_ok(cudaMemcpyAsync(dj, hj, sizeof(Q4Job), cudaMemcpyHostToDevice, B.stream), "job upload") ||
         !cuda_ok(launch_q4_jobs(dj, 1, nullptr, R, job_count, C, 1, (C % 64) == 0, B.stream), "launch"))
         return -1;
-    count_launches(1);
     count_kinds(kind == SALT_GPU_RESOURCE_TRUNK, kind == SALT_GPU_RESOURCE_EXPERT_LAYER,
                 kind == SALT_GPU_RESOURCE_ARENA);
     B.stats.direct_output_batches++;
@@ -987,7 +985,6 @@ static int moe_chain(const SaltGpuMoeExpert* experts, int count, int hidden, int
         !stage_finish(in_bytes, "y download"))
         return -1;
     memcpy(outputs, B.h_y, in_bytes);
-    count_launches(2);
     B.stats.expert_layer_batches++;
     B.stats.direct_output_batches++;
     B.stats.direct_output_jobs += (uint64_t)count;
@@ -1054,7 +1051,6 @@ int salt_gpu_q4_selected_shared(const SaltGpuSelectedProjectionJob* jobs, int jo
         if (!cuda_ok(launch_q4_jobs(dj + n0, n1 - n0, nullptr, max_rows, max_tok, C, 1, aligned, B.stream),
                      "selected launch"))
             return -1;
-        count_launches(1);
         n0 = n1;
     }
     if (!stream_fence()) return -1;
@@ -1171,7 +1167,6 @@ int salt_gpu_exact_cells(const SaltGpuExactCell* cells, int count) {
             default:
                 return -1;
         }
-        count_launches(1);
     }
     return salt_gpu_sync();
 }

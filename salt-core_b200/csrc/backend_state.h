@@ -89,7 +89,6 @@ bool stage_upload(size_t head, size_t bytes, const char* what);
 // Where a call's kernels put `bytes` of results, and the end of the call: results in h_y, stream idle.
 float* stage_out(size_t bytes);
 bool stage_finish(size_t bytes, const char* what);
-void count_launches(int n);
 uint64_t launch_count();
 uintptr_t residency_seat_address(int seat, size_t nbytes);
 void residency_shutdown();

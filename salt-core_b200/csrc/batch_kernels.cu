@@ -464,7 +464,7 @@ cudaError_t launch_batch(const void* jobs, int njobs_max, const int* live, const
     if (pdl >= 0)
         return launch_pdl(batch_kernel<FMT, NMAT, RL>, grid, dim3(NT), (size_t)G.smem, stream, jobs, live, njobs_dev, C, pdl);
     batch_kernel<FMT, NMAT, RL><<<grid, NT, G.smem, stream>>>(jobs, live, njobs_dev, C, 0);
-    return cudaGetLastError();
+    return launched();
 }
 
 // Rows per lane.  Four need a quarter of the shared loads per product; two make twice as many blocks, which start and

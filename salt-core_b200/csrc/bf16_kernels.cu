@@ -54,7 +54,7 @@ bf16_batch_serial_kernel(const uint16_t* __restrict__ W, const float* __restrict
 cudaError_t launch_bf16_matvec(const uint16_t* W, const float* x, float* y, int R, int C, cudaStream_t stream) {
     if (R < 1 || C < 1) return cudaErrorInvalidValue;
     bf16_matvec8_kernel<<<(R + 15) / 16, 128, 0, stream>>>(W, x, y, R, C);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t launch_bf16_batch(const uint16_t* W, const float* xs, float* ys, int R, int C, int B, cudaStream_t stream) {
@@ -66,7 +66,7 @@ cudaError_t launch_bf16_batch(const uint16_t* W, const float* xs, float* ys, int
         if (e != cudaSuccess) return e;
     }
     bf16_batch_serial_kernel<<<dim3((R + 127) / 128, B), 128, smem, stream>>>(W, xs, ys, R, C);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace sb

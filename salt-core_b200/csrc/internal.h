@@ -10,6 +10,14 @@ namespace sb {
 struct Q4Job;
 
 // ---- backend.cu ------------------------------------------------------------
+// Kernels launched since load, counted where they are launched: by launched() after an ordinary launch and by launch_pdl()
+// (pdl.cuh).  Totals kept by the callers went wrong when launches were merged.
+void count_launches(int n);
+inline cudaError_t launched() {
+    const cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) count_launches(1);
+    return e;
+}
 // Raises a kernel's dynamic shared memory limit to at least `bytes` on the CURRENT device (the limit
 // is a per-device attribute of the function; remembered per device and kernel, safe from any thread).
 cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes);

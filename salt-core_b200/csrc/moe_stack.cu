@@ -429,7 +429,6 @@ static int layer_router(Stack* s, const Layer& l, const float* d_router_src, int
         g.x_in = d_router_src; g.router_scale = l.router_scale; g.eps_router = l.eps; g.rin = s->rin; g.n = H;
         g.status = s->status;
         if (!cuda_ok(launch_glue(g, B, st), "router in")) return -1;
-        count_launches(1);
     }
     {
         Timed t(s, KC_LOGITS, st);
@@ -439,7 +438,6 @@ static int layer_router(Stack* s, const Layer& l, const float* d_router_src, int
         Timed t(s, KC_TOPK, st);
         if (!cuda_ok(launch_router_topk(s->logits, l.per_expert_scale, sel_out, w_out, B, E, K, 1, s->status, st), "topk"))
             return -1;
-        count_launches(1);
     }
     return 0;
 }
@@ -534,7 +532,6 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
                                       s->status, st, nullptr, 1, 1, s->fp4_up), "nvfp4 geglu + qdq") ||
             !cuda_ok(launch_nvfp4_gemm_tc(s->fp4_tc_dn, E, H, M, md, s->status, st), "nvfp4 tc down"))
             return -1;
-        count_launches(5);
         return 0;
     }
     if (l.nvfp4) {
@@ -553,7 +550,6 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
             !cuda_ok(launch_nvfp4_jobs(s->fp4_dn_jobs, live_max, H, B, M, true, st, s->fp4_live + 2 + 2 * E,
                                        s->fp4_live + 1), "nvfp4 down"))
             return -1;
-        count_launches(6);
         return 0;
     }
     if (fused) {
@@ -564,7 +560,6 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
         f.status = s->status;
         Timed t(s, KC_GATE_UP, st);
         if (!cuda_ok(launch_q4_fused(f, st), "fused experts")) return -1;
-        count_launches(3);
         return 0;
     }
     // tokens per job: at most B, or those of a pass
@@ -595,7 +590,6 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
                                            l.q4_tc, nullptr, nullptr, nullptr, nullptr, s->grouped_out, H, M, s->status, st), "tc down"))
                 return -1;
         }
-        count_launches(6);
         return 0;
     }
     {
@@ -608,7 +602,6 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
         if (!cuda_ok(launch_q4_jobs(s->down_jobs, njobs_max, s->counters, H, tok_hint, M, 1, true, st, 1), "down"))
             return -1;
     }
-    count_launches(4);
     return 0;
 }
 
@@ -691,7 +684,7 @@ int salt_b200_dispatch_plan(const int32_t* d_selected, int n, int n_experts, int
     if (n < 0 || n_experts < 1 || world < 1 || world > EP_MAX_WORLD || world > n_experts || !d_counts) return -1;
     if (n > 0 && (!d_selected || !d_order || !d_pos || !d_ids)) return -1;
     dispatch_plan_kernel<<<1, 1024, 0, (cudaStream_t)stream_>>>(d_selected, n, n_experts, world, d_order, d_pos, d_ids, d_counts);
-    return cuda_ok(cudaGetLastError(), "dispatch plan") ? 0 : -1;
+    return cuda_ok(launched(), "dispatch plan") ? 0 : -1;
 }
 
 // home rank: router of its own tokens -> caller-owned selected / weights
@@ -737,8 +730,7 @@ int salt_b200_layer_experts_routed(void* stack, int layer, const float* d_rows, 
     ungroup_rows_kernel<<<dim3(n_rows, (n4 + 255) / 256), 256, 0, st>>>((const float4*)s->grouped_out, s->c2g, d_experts,
                                                                       s->expert_begin, s->expert_end, n_rows,
                                                                       (float4*)d_out, n4, s->status);
-    count_launches(1);
-    return cuda_ok(cudaGetLastError(), "ungroup") ? 0 : -1;
+    return cuda_ok(launched(), "ungroup") ? 0 : -1;
 }
 
 // home rank: the returned rows in canonical order (token-major, rank order) -> ordered weighted reduce, norm,
@@ -771,7 +763,6 @@ int salt_b200_layer_combine_rows(void* stack, int layer, const float* d_rows, co
         Timed t(s, KC_REDUCE, st);
         if (!cuda_ok(launch_glue(g, B, st), "combine rows")) return -1;
     }
-    count_launches(1);
     return 0;
 }
 
@@ -798,7 +789,6 @@ int salt_b200_layer_combine(void* stack, int layer, int B, float* d_y, int flags
         Timed t(s, KC_REDUCE, st);
         if (!cuda_ok(launch_glue(g, B, st), "combine")) return -1;
     }
-    count_launches(1);
     return 0;
 }
 
@@ -896,7 +886,6 @@ int salt_b200_stack_ep_exchange(void* stack, int B, int phase, void* stream) {
     a.phase = phase; a.status = s->status; a.spin_limit = s->ep_spin_limit;
     Timed t(s, KC_NORM, (cudaStream_t)stream);
     if (!cuda_ok(launch_ep_exchange(a, B * s->topk, (cudaStream_t)stream), "ep exchange")) return -1;
-    count_launches(1);
     return 0;
 }
 
@@ -979,13 +968,12 @@ int salt_b200_ffn_block_forward(void* stack, int layer, const float* d_residual,
     };
     // dense branch: norm_a -> gate/up + GeGLU -> down
     patch_job_tokens_kernel<<<1, 32, 0, st>>>(l.dense_jobs, 2, B);
-    if (!norm(l.pre_ffn_norm, s->norm_a) ||
+    if (!cuda_ok(launched(), "dense tokens") || !norm(l.pre_ffn_norm, s->norm_a) ||
         !cuda_ok(launch_q4_jobs(l.dense_jobs, 1, nullptr, D, tok_hint, H, 2, true, st), "dense gate/up") ||
         !cuda_ok(launch_q4_jobs(l.dense_jobs + 1, 1, nullptr, H, tok_hint, D, 1, true, st), "dense down"))
         return -1;
     // routed branch: router on the residual, experts on norm_b
     if (!norm(l.pre_ffn_norm_2, s->norm_b)) return -1;
-    count_launches(5);
     if (layer_experts_impl(s, layer, d_residual, s->norm_b, B, 0, st) != 0) return -1;
     if (s->ep_world > 1 && salt_b200_stack_ep_exchange(stack, B, EP_PHASE_PUSH | EP_PHASE_PULL, stream_) != 0) return -1;
     {
@@ -1000,7 +988,6 @@ int salt_b200_ffn_block_forward(void* stack, int layer, const float* d_residual,
                                          s->combine_scratch + (size_t)s->max_tokens * H, d_out, B, H, l.eps,
                                          l.layer_scalar, s->status, st), "parallel combine"))
         return -1;
-    count_launches(2);
     return 0;
 }
 
@@ -1096,7 +1083,6 @@ static int forward_decode_layers(Stack* s, int first, int count, const float* d_
         Timed t(s, KC_REDUCE, st);
         if (!cuda_ok(launch_glue(g, 1, st), "last reduce")) return -1;
     }
-    count_launches(count + 1);
     return 0;
 }
 
@@ -1104,7 +1090,10 @@ int salt_b200_stack_forward_device(void* stack, int first, int count, const floa
                                    void* stream) {
     Stack* s = (Stack*)stack;
     if (!s || first < 0 || count < 1 || first + count > (int)s->layers.size() || !d_x || !d_y) return -1;
-    if (s->profile) profile_head_start_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(80000LL * count + 400000LL);
+    if (s->profile) {
+        profile_head_start_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(80000LL * count + 400000LL);
+        if (!cuda_ok(launched(), "head start")) return -1;
+    }
     if (decode_layers_apply(s, B)) return forward_decode_layers(s, first, count, d_x, d_y, (cudaStream_t)stream);
     const float* in = d_x;
     for (int i = 0; i < count; i++) {
@@ -1242,7 +1231,6 @@ int salt_b200_q4_matvec_device(const void* d_vals, const void* d_scales, const v
     if (!cuda_ok(cudaMemcpyAsync(d_job, &j, sizeof j, cudaMemcpyHostToDevice, (cudaStream_t)stream), "job upload") ||
         !cuda_ok(launch_q4_jobs(d_job, 1, nullptr, R, B, C, 1, aligned, (cudaStream_t)stream), "launch"))
         return -1;
-    count_launches(1);
     return 0;
 }
 
@@ -1275,7 +1263,6 @@ int salt_b200_route_group_device(const int32_t* d_selected, int rows, int topk, 
     if (!cuda_ok(cudaMemsetAsync(scratch, 0, 4 * sizeof(int32_t), (cudaStream_t)stream), "scratch") ||
         !cuda_ok(launch_moe_plan(a, (cudaStream_t)stream), "plan"))
         return -1;
-    count_launches(1);
     int32_t status = 0;
     if (!cuda_ok(cudaStreamSynchronize((cudaStream_t)stream), "sync") ||
         !cuda_ok(cudaMemcpy(&status, scratch + 2, sizeof status, cudaMemcpyDeviceToHost), "status"))

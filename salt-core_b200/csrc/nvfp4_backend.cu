@@ -131,7 +131,6 @@ static int fp4_run(const std::vector<Tensor*>& tensors, const float* const* inpu
         !cuda_ok(launch_nvfp4_jobs(d_jobs, njobs, max_rows, max_tok, C, aligned, B.stream), "fp4 proj") ||
         !stage_finish(out_floats * sizeof(float), "fp4 y"))
         return -1;
-    count_launches(2);
     if (salt_gpu_sync() != 0) return -1;   // also reports non-finite activations
     yoff = 0;
     for (int j = 0; j < njobs; j++) {
@@ -217,7 +216,6 @@ int salt_gpu_nvfp4_qdq(const float* input, int C, float input_global_scale, uint
         !cuda_ok(cudaMemcpyAsync(hp + C, g_fp4.d_scales, (size_t)C / 16, cudaMemcpyDeviceToHost, B.stream), "sc") ||
         !cuda_ok(cudaMemcpyAsync(B.h_x, B.d_mid, (size_t)C * sizeof(float), cudaMemcpyDeviceToHost, B.stream), "dq"))
         return -1;
-    count_launches(1);
     if (salt_gpu_sync() != 0) return -1;
     memcpy(packed, hp, (size_t)C / 2);
     memcpy(scales, hp + C, (size_t)C / 16);

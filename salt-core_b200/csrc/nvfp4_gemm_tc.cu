@@ -400,7 +400,7 @@ cudaError_t launch_nvfp4_gemm_tc(const Fp4TcJob* jobs, int njobs, int R, int C, 
     const int total = njobs * a.tiles_per_job;
     const int grid = std::max(std::min(sms, total), (total + FT_MAX_TILES - 1) / FT_MAX_TILES);
     nvfp4_gemm_tc_kernel<<<grid, FT_THREADS, FT_SMEM_BYTES, stream>>>(a, maps);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace sb

@@ -273,7 +273,7 @@ cudaError_t launch_nvfp4_jobs(const Fp4Job* jobs, int njobs, int max_rows, int m
     dim3 grid((max_rows + 3) / 4, max_tok, njobs);
     if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
     nvfp4_generic_kernel<<<grid, 128, 0, stream>>>(jobs, live, n_live);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace sb

@@ -770,7 +770,7 @@ cudaError_t launch_q4_interleave_tables(const uint8_t* pool, size_t expert_strid
     if (e != cudaSuccess) return e;
     q4_interleave_tables_kernel<<<dim3(32, n_experts, 3), 256, 0, stream>>>(pool, expert_stride, tensor_bytes, value_bytes, groups,
                                                                           words, flags);
-    return cudaGetLastError();
+    return launched();
 }
 
 // ---- host side ---------------------------------------------------------------------------

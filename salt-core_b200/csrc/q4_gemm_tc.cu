@@ -884,7 +884,7 @@ cudaError_t launch_q4_tc_tables(const uint32_t* tables, int hidden, int inter, i
                                 float* unscale, cudaStream_t stream) {
     if (experts < 1) return cudaSuccess;
     q4_tc_tables_kernel<<<592, 256, 0, stream>>>(tables, hidden, inter, experts, by_group, scale, unscale);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t tensor_map_encoder(TensorMapEncodeFn* out) {
@@ -977,7 +977,7 @@ static cudaError_t launch_tc(const TcArgs& a, const TcMaps& maps, const TcMaps& 
         if (e != cudaSuccess) return e;
     }
     q4_gemm_tc_kernel<FUSED, SPLIT><<<grid, TC_THREADS, TC_SMEM_BYTES, stream>>>(a, maps, sums, wm);
-    return cudaGetLastError();
+    return launched();
 }
 
 size_t q4_tc_work_items_max(int n_experts, int rows_total, int hidden, int inter) {
@@ -996,7 +996,7 @@ cudaError_t launch_tc_prepare(const float* x, const int32_t* c2g, void* xh, void
     const dim3 grid((hidden / 8 + GATHER_THREADS - 1) / GATHER_THREADS, rows + 1);
     scatter_convert_kernel<<<grid, GATHER_THREADS, (size_t)(4 * njobs_max + 1) * sizeof(int), stream>>>(
         x, c2g, (__half*)xh, (__half*)xl, (__half*)sums_h, (__half*)sums_l, tc_sums_cols(hidden), rows * topk, topk, hidden, lists);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t launch_q4_gemm_tc(bool fused, bool split, const void* items, int* work, const TcMaps& x, const TcMaps& sums,

@@ -62,7 +62,7 @@ cudaError_t launch_q4_jobs(const Q4Job* jobs, int njobs_max, const int* njobs_de
     if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
     if (nmat == 2) q4_generic_kernel<2><<<grid, 128, 0, stream>>>(jobs, njobs_dev);
     else q4_generic_kernel<1><<<grid, 128, 0, stream>>>(jobs, njobs_dev);
-    return cudaGetLastError();
+    return launched();
 }
 
 }  // namespace sb

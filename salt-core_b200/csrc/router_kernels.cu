@@ -102,7 +102,7 @@ cudaError_t launch_q8_jobs(const Q4Job* jobs, int njobs, int max_rows, int max_t
         if (e != cudaSuccess) return e;
     }
     q8_rows_kernel<<<dim3(max_rows, max_tok, njobs), 128, smem, stream>>>(jobs);
-    return cudaGetLastError();
+    return launched();
 }
 
 // ---- consumers of the routed-expert output (exact cells) -------------------------------------
@@ -205,7 +205,7 @@ cudaError_t launch_residual_postnorm(const float* residual, const float* branch,
         if (e != cudaSuccess) return e;
     }
     residual_postnorm_rows_kernel<<<rows, 1024, smem, stream>>>(residual, branch, weight, out, n, eps, status);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t launch_parallel_combine(const float* residual, const float* dense, const float* routed, const float* wd,
@@ -220,13 +220,13 @@ cudaError_t launch_parallel_combine(const float* residual, const float* dense, c
     }
     parallel_combine_rows_kernel<<<rows, 1024, smem, stream>>>(residual, dense, routed, wd, wr, wf, scratch_a, scratch_b,
                                                                out, n, eps, scalar, status);
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t launch_softcap(float* logits, int n, float cap, int* status, cudaStream_t stream) {
     if (n < 1) return cudaSuccess;
     softcap_kernel<<<(n + 255) / 256, 256, 0, stream>>>(logits, n, cap, status);
-    return cudaGetLastError();
+    return launched();
 }
 
 // Each thread owns the columns d = threadIdx.x + j * blockDim.x (j < GLUE_NV, compile
@@ -483,7 +483,7 @@ cudaError_t launch_glue(const GlueArgs& a, int rows, cudaStream_t stream) {
         const int blocks = (rows + GLUE_ROWS - 1) / GLUE_ROWS;
         if (a.n == 32 * 88) glue_rows_warp_kernel<88><<<blocks, 32 * GLUE_ROWS, wsmem, stream>>>(a, rows);
         else glue_rows_warp_kernel<160><<<blocks, 32 * GLUE_ROWS, wsmem, stream>>>(a, rows);
-        return cudaGetLastError();
+        return launched();
     }
     if (a.n <= 4096) {
         // every thread owns 4 columns: wide rows and small batches get the largest block
@@ -494,7 +494,7 @@ cudaError_t launch_glue(const GlueArgs& a, int rows, cudaStream_t stream) {
     } else {
         return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
+    return launched();
 }
 
 cudaError_t launch_rmsnorm(const float* x, const float* weight, float* y, int rows, int n, float eps, int with_scale,
@@ -502,7 +502,7 @@ cudaError_t launch_rmsnorm(const float* x, const float* weight, float* y, int ro
     if (rows < 1) return cudaSuccess;
     norm_rows_kernel<0><<<rows, 256, (size_t)(2 * n + 8) * sizeof(float), stream>>>(x, weight, y, n, eps, with_scale, 0.0f,
                                                                            status);
-    return cudaGetLastError();
+    return launched();
 }
 
 // Threads of a row's top-k: one warp selects, four evaluate the exponentials of up to 128 experts.
@@ -512,7 +512,7 @@ cudaError_t launch_router_input(const float* x, const float* scale, float* out, 
                                 float root, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
     norm_rows_kernel<1><<<rows, 256, (size_t)(2 * n + 8) * sizeof(float), stream>>>(x, scale, out, n, eps, 1, root, status);
-    return cudaGetLastError();
+    return launched();
 }
 
 __global__ void __launch_bounds__(TOPK_THREADS)

@@ -117,10 +117,9 @@ extern "C" int salt_b200_q4_expert_chain_static(const void* d_gate_vals, const v
     // Nothing in the scratch has to start at zero: both descriptors and every
     // chain row that the down projection reads are written earlier in this call.
     static_write_jobs<<<1, 32, 0, st>>>(gu, dn);
-    if (!cuda_ok(cudaGetLastError(), "static descriptors") ||
+    if (!cuda_ok(launched(), "static descriptors") ||
         !cuda_ok(launch_q4_jobs(jobs, 1, nullptr, inter, ntok, hidden, 2, true, st), "static gate/up") ||
         !cuda_ok(launch_q4_jobs(jobs + 1, 1, nullptr, hidden, ntok, inter, 1, true, st), "static down"))
         return -1;
-    count_launches(3);
     return 0;
 }

@@ -193,12 +193,14 @@ bool stage_upload(size_t head, size_t bytes, const char* what) {
                                    B.stream), what);
 }
 
-float* stage_out(size_t bytes) { return bytes <= SB_DIRECT_OUT_BYTES ? g_backend.hd_y : g_backend.d_y; }
+float* stage_out(size_t bytes, bool whole_lines) {
+    return bytes <= (whole_lines ? SB_DIRECT_LINES : SB_DIRECT_FLOATS) ? g_backend.hd_y : g_backend.d_y;
+}
 
-bool stage_finish(size_t bytes, const char* what) {
+bool stage_finish(const float* y_dev, size_t bytes, const char* what) {
     Backend& B = g_backend;
     B.in_flight = true;
-    if (bytes > SB_DIRECT_OUT_BYTES &&
+    if (y_dev == B.d_y &&
         !cuda_ok(cudaMemcpyAsync(B.h_y, B.d_y, bytes, cudaMemcpyDeviceToHost, B.stream), what))
         return false;
     return stream_fence();
@@ -536,13 +538,13 @@ static int bf16_run(const void* key, int R, int C, int Bt, const float* in, floa
     if (!in || !out || nin > B.stage_floats || nout > B.stage_floats) return -1;
     if (!stream_fence()) return -1;
     memcpy(B.h_x, in, nin * sizeof(float));
-    float* const y_dev = stage_out(nout * sizeof(float));
+    float* const y_dev = stage_out(nout * sizeof(float), serial);
     B.in_flight = true;
     if (!stage_upload(0, nin * sizeof(float), "bf16 x upload")) return -1;
     const cudaError_t e = serial ? launch_bf16_batch(W, B.d_x, y_dev, R, C, Bt, B.stream)
                                  : launch_bf16_matvec(W, B.d_x, y_dev, R, C, B.stream);
     if (!cuda_ok(e, "bf16 launch")) return -1;
-    if (!stage_finish(nout * sizeof(float), "bf16 y download")) return -1;
+    if (!stage_finish(y_dev, nout * sizeof(float), "bf16 y download")) return -1;
     memcpy(out, B.h_y, nout * sizeof(float));
     return 0;
 }
@@ -722,9 +724,11 @@ static int q4_same_weight(const void* key, const uint32_t* vals, const uint16_t*
         memcpy(B.h_x + (size_t)b * C, xs[b], (size_t)C * sizeof(float));
     }
     const size_t y_bytes = (size_t)Bt * R * sizeof(float);
-    fill_job(*staged_jobs(1), *t, B.d_x, stage_out(y_bytes), Bt, C, R);
     const bool aligned = (C % 64) == 0;
-    if (!run_jobs(1, 1, (size_t)Bt * C * sizeof(float), R, Bt, C, 1, aligned, bits) || !stage_finish(y_bytes, "y download"))
+    float* const y_dev = stage_out(y_bytes, bits == 4 && q4_stores_lines(C, 1, aligned));
+    fill_job(*staged_jobs(1), *t, B.d_x, y_dev, Bt, C, R);
+    if (!run_jobs(1, 1, (size_t)Bt * C * sizeof(float), R, Bt, C, 1, aligned, bits) ||
+        !stage_finish(y_dev, y_bytes, "y download"))
         return -1;
     for (int b = 0; b < Bt; b++) memcpy(ys[b], B.h_y + (size_t)b * R, (size_t)R * sizeof(float));
     count_kinds(kind == SALT_GPU_RESOURCE_TRUNK, kind == SALT_GPU_RESOURCE_EXPERT_LAYER,
@@ -761,7 +765,8 @@ static int q_batch(int bits, const uint32_t* const* vals, const uint16_t* const*
         if (Rj[j] < 1) return -1;
         y_total += (size_t)Rj[j];
     }
-    float* const y_dev = stage_out(y_total * sizeof(float));
+    const bool aligned = (C % 64) == 0;
+    float* const y_dev = stage_out(y_total * sizeof(float), bits == 4 && q4_stores_lines(C, 1, aligned));
     Q4Job* const staged = staged_jobs(njobs);
     size_t x_floats = 0, y_floats = 0;
     int max_rows = 0, ndesc = 0, max_tok = 1;
@@ -803,8 +808,8 @@ static int q_batch(int bits, const uint32_t* const* vals, const uint16_t* const*
         arena |= kind == SALT_GPU_RESOURCE_ARENA;
         j += run;
     }
-    if (!run_jobs(njobs, ndesc, x_floats * sizeof(float), max_rows, max_tok, C, 1, (C % 64) == 0, bits) ||
-        !stage_finish(y_total * sizeof(float), "y download"))
+    if (!run_jobs(njobs, ndesc, x_floats * sizeof(float), max_rows, max_tok, C, 1, aligned, bits) ||
+        !stage_finish(y_dev, y_total * sizeof(float), "y download"))
         return -1;
     for (int j = 0; j < njobs; j++) memcpy(ys[j], B.h_y + yoff[(size_t)j], (size_t)Rj[j] * sizeof(float));
     count_kinds(trunk, expert, arena);
@@ -953,7 +958,6 @@ static int moe_chain(const SaltGpuMoeExpert* experts, int count, int hidden, int
     if (total_rows * (uint64_t)hidden > B.stage_floats || total_rows * (uint64_t)routed > B.stage_floats) return -1;
     if (!stream_fence()) return -1;
     const size_t in_bytes = (size_t)total_rows * hidden * sizeof(float);
-    float* const y_dev = stage_out(in_bytes);
     Q4Job* const staged = staged_jobs(2 * count);
     bool aligned = (hidden % 64) == 0 && (routed % 64) == 0;
     size_t row = 0;
@@ -973,8 +977,14 @@ static int moe_chain(const SaltGpuMoeExpert* experts, int count, int hidden, int
         fill_job(gu, g, B.d_x + row * hidden, B.d_mid + row * routed, e.group, hidden, routed);
         gu.vals2 = u.dv; gu.scales2 = u.ds; gu.biases2 = u.db;
         Q4Job& dn = staged[count + i];
-        fill_job(dn, d, B.d_mid + row * routed, y_dev + row * hidden, e.group, routed, hidden);
+        fill_job(dn, d, B.d_mid + row * routed, nullptr, e.group, routed, hidden);
         row += (size_t)e.group;
+    }
+    float* const y_dev = stage_out(in_bytes, q4_stores_lines(routed, 1, aligned));
+    row = 0;
+    for (int i = 0; i < count; i++) {
+        staged[count + i].y = y_dev + row * hidden;
+        row += (size_t)experts[i].group;
     }
     memcpy(B.h_x, inputs, in_bytes);
     const Q4Job* const dj = (const Q4Job*)B.d_x - 2 * count;
@@ -982,7 +992,7 @@ static int moe_chain(const SaltGpuMoeExpert* experts, int count, int hidden, int
     if (!stage_upload((size_t)(2 * count) * sizeof(Q4Job), in_bytes, "job and x upload") ||
         !cuda_ok(launch_q4_jobs(dj, count, nullptr, routed, max_group, hidden, 2, aligned, B.stream, 0), "gate/up launch") ||
         !cuda_ok(launch_q4_jobs(dj + count, count, nullptr, hidden, max_group, routed, 1, aligned, B.stream, 1), "down launch") ||
-        !stage_finish(in_bytes, "y download"))
+        !stage_finish(y_dev, in_bytes, "y download"))
         return -1;
     memcpy(outputs, B.h_y, in_bytes);
     B.stats.expert_layer_batches++;

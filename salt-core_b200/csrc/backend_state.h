@@ -77,18 +77,23 @@ struct Backend {
     bool in_flight = false;            // asynchronous calls since the last synchronisation
 };
 
-// Results up to this size are written straight into pinned host memory by the kernel; a copy afterwards costs about
-// 3 us more than the writes take (16 KB: 14.4 against 16.6 us for upload + kernel + result, 512 KB: 35 against 39).
-constexpr size_t SB_DIRECT_OUT_BYTES = (size_t)512 * 1024;
+// Results up to these sizes are written straight into pinned host memory by the kernel, larger ones are copied afterwards.
+// A kernel whose stores leave as whole lines (batch_kernels.cu, bf16 batches) gains 2 us at 16 KB and 10 at 128 KB (32768
+// rows of 256 columns: 37 -> 27 us; 1000 rows x 100 tokens, 390 KB, is the first shape where it loses, 68 against 71).  One
+// float per block or warp (q8, any-shape Q4 and NVFP4) or four (bf16 matvec) are as many separate writes over the bus: direct
+// is 1 to 7 us faster at 16 KB, between 2 us slower and 4 us faster at 32 to 64 KB from host to host, and far slower above
+// (any-shape Q4, 131072 rows of 72: 179 to 207 us against 89).
+constexpr size_t SB_DIRECT_LINES = (size_t)512 * 1024, SB_DIRECT_FLOATS = (size_t)32 * 1024;
 
 extern Backend g_backend;
 bool cuda_ok(cudaError_t e, const char* what);
 bool stream_fence();                   // waits for asynchronous calls, if there were any
 // Uploads `head` bytes of descriptors (already at (uint8_t*)h_x - head) and `bytes` of activations in one copy.
 bool stage_upload(size_t head, size_t bytes, const char* what);
-// Where a call's kernels put `bytes` of results, and the end of the call: results in h_y, stream idle.
-float* stage_out(size_t bytes);
-bool stage_finish(size_t bytes, const char* what);
+// Where a call's kernels put `bytes` of results (whole_lines: how they store them), and the end of the call: the results that
+// were put at y_dev are in h_y, the stream is idle.
+float* stage_out(size_t bytes, bool whole_lines);
+bool stage_finish(const float* y_dev, size_t bytes, const char* what);
 uint64_t launch_count();
 uintptr_t residency_seat_address(int seat, size_t nbytes);
 void residency_shutdown();

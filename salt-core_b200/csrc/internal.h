@@ -31,6 +31,8 @@ cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes);
 // the weights are prefetched while the previous kernel is still running.
 cudaError_t launch_q4_jobs(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
                            int nmat, bool aligned, cudaStream_t stream, int pdl = -1);
+// Do these jobs run on a kernel whose results leave the chip as whole lines?
+bool q4_stores_lines(int C, int nmat, bool aligned);
 
 // ---- batch_kernels.cu --------------------------------------------------------
 // The same jobs for aligned tensors with C a multiple of 64, and NVFP4 jobs with C a multiple of 256.

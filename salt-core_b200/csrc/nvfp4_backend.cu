@@ -103,10 +103,11 @@ static int fp4_run(const std::vector<Tensor*>& tensors, const float* const* inpu
     Fp4Job* const h_jobs = (Fp4Job*)h_ig - njobs;
     const float* const d_ig = (const float*)((const uint8_t*)B.d_x - ig_bytes);
     const Fp4Job* const d_jobs = (const Fp4Job*)d_ig - njobs;
-    float* const y_dev = stage_out(out_floats * sizeof(float));
+    bool aligned = true;
+    for (int j = 0; j < njobs; j++) aligned = aligned && ((((uintptr_t)tensors[(size_t)j]->dv | (uintptr_t)tensors[(size_t)j]->ds) & 15) == 0);
+    float* const y_dev = stage_out(out_floats * sizeof(float), aligned && fp4_batch_supported(C));
     size_t row = 0, yoff = 0;
     int max_rows = 0, max_tok = 1;
-    bool aligned = true;
     uint64_t wbytes = 0, sbytes = 0;
     for (int j = 0; j < njobs; j++) {
         const Tensor& t = *tensors[(size_t)j];
@@ -116,7 +117,6 @@ static int fp4_run(const std::vector<Tensor*>& tensors, const float* const* inpu
         fj.codes = t.dv; fj.scales = t.ds; fj.wg = 1.0f / t.weight_divisor;
         fj.x = B.d_mid + row * C; fj.y = y_dev + yoff;
         fj.R = t.R; fj.C = C; fj.ntok = batches[j]; fj.x_stride = C; fj.y_stride = t.R;
-        aligned = aligned && ((((uintptr_t)t.dv | (uintptr_t)t.ds) & 15) == 0);
         max_rows = std::max(max_rows, t.R);
         max_tok = std::max(max_tok, batches[j]);
         wbytes += t.vbytes; sbytes += t.gbytes;
@@ -129,7 +129,7 @@ static int fp4_run(const std::vector<Tensor*>& tensors, const float* const* inpu
         !cuda_ok(launch_nvfp4_qdq(B.d_x, (int)total_rows, C, d_ig, g_fp4.d_packed, g_fp4.d_scales, B.d_mid,
                                   B.d_status, B.stream), "fp4 qdq") ||
         !cuda_ok(launch_nvfp4_jobs(d_jobs, njobs, max_rows, max_tok, C, aligned, B.stream), "fp4 proj") ||
-        !stage_finish(out_floats * sizeof(float), "fp4 y"))
+        !stage_finish(y_dev, out_floats * sizeof(float), "fp4 y"))
         return -1;
     if (salt_gpu_sync() != 0) return -1;   // also reports non-finite activations
     yoff = 0;

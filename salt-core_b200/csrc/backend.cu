@@ -35,6 +35,19 @@ Backend g_backend;
 static std::atomic<uint64_t> g_launches{0};      // stacks may be driven from several threads
 void count_launches(int n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
 
+int device_sms() {
+    constexpr int MAXDEV = 64;
+    static std::atomic<int> known[MAXDEV];
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAXDEV) return 148;
+    sms = known[dev].load(std::memory_order_relaxed);
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 148;
+        known[dev].store(sms, std::memory_order_relaxed);
+    }
+    return sms;
+}
+
 cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes) {
     static std::mutex mu;
     static std::map<std::pair<int, const void*>, size_t> done;

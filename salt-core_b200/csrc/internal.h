@@ -18,6 +18,8 @@ inline cudaError_t launched() {
     if (e == cudaSuccess) count_launches(1);
     return e;
 }
+// SMs of the current device (of a B200 if it cannot be asked).
+int device_sms();
 // Raises a kernel's dynamic shared memory limit to at least `bytes` on the CURRENT device (the limit
 // is a per-device attribute of the function; remembered per device and kernel, safe from any thread).
 cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes);

@@ -367,23 +367,34 @@ __global__ void __launch_bounds__(GLUE_NV == 4 ? 1024 : 512) glue_rows_kernel(Gl
 
 // The same glue for batches of several hundred rows: a warp per row, four rows per block.  Lane l holds 16-byte pieces l,
 // l + 32, ... of its row in registers.  The squares of the four rows go to shared memory and ONE warp runs the four
-// in-order sums side by side, a row per lane (the reference's order: columns ascending from +0).  A chain costs about
+// in-order sums side by side, a row per lane (the reference's order: columns ascending from +0).  A chain of 2816 costs about
 // 6 us, but the rows of a few blocks per SM run side by side, where the block-per-row form above keeps a whole SM busy for
-// 13 us per pair of rows.  (Rows in lane-contiguous pieces, the sum handed from lane to lane, loaded 32 lines per
-// instruction: 1999 rows took 68 us for reduce and two sums, this takes 56; 256 rows of 5120 columns 38 us -> 29.)
+// 12 us per row with two sums.  (Rows in lane-contiguous pieces, the sum handed from lane to lane, loaded 32 lines per
+// instruction: 1999 rows took 68 us for reduce and two sums, this takes 56.)
+// P: pieces per lane, an even number, for rows of more than 128 (P - 2) and at most 128 P columns; FULL: exactly 128 P.  The
+// row takes 4 P registers of a lane and what is left of its share holds the loads in flight, and pieces that may lie outside
+// the row cost a test each: with P in steps of eight, 320 to 592 rows of 2816 columns took 35 us against 30, 256 rows of 5120
+// 43 us, with tests of the last two pieces 41, without 39.  Blocks per SM (of registers): four up to 22 pieces, two above 24,
+// where three left so few loads in flight that 512 rows of 4096 columns took 46 us against 36.
 constexpr int GLUE_ROWS = 4;
+constexpr int GLUE_PIECES = 48;            // most: 192 registers, two blocks per SM
 static __device__ __forceinline__ uint32_t glue_pitch(int n) { return (uint32_t)n + 4u; }    // the rows start four banks apart
 
+// Does the lane's piece i lie inside the row?  FULL: the row has exactly 128 P columns.
+template <int P, bool FULL>
+static __device__ __forceinline__ bool glue_in_row(int i, int lane, int n) { return FULL || i < P - 2 || 4 * (lane + 32 * i) < n; }
+
 // Squares of the warps' rows in sq[GLUE_ROWS][pitch] -> s_inv[r] = pow(sum / n + eps, -0.5) for every row of the block.
-template <int CH>
-static __device__ __forceinline__ void glue_inv_rms(const float4 (&v)[CH / 4], float* sq, float* s_inv, float eps) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, n = 32 * CH;
+template <int P, bool FULL>
+static __device__ __forceinline__ void glue_inv_rms(const float4 (&v)[P], float* sq, float* s_inv, int n, float eps, int sms) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float4* mine = (float4*)(sq + w * glue_pitch(n)) + lane;
 #pragma unroll
-    for (int i = 0; i < CH / 4; i++)
-        mine[32 * i] = make_float4(__fmul_rn(v[i].x, v[i].x), __fmul_rn(v[i].y, v[i].y), __fmul_rn(v[i].z, v[i].z), __fmul_rn(v[i].w, v[i].w));
+    for (int i = 0; i < P; i++)
+        if (glue_in_row<P, FULL>(i, lane, n))
+            mine[32 * i] = make_float4(__fmul_rn(v[i].x, v[i].x), __fmul_rn(v[i].y, v[i].y), __fmul_rn(v[i].z, v[i].z), __fmul_rn(v[i].w, v[i].w));
     __syncthreads();
-    if (w == ((blockIdx.x / 148) & 3)) {          // blocks that share an SM add on different schedulers
+    if (w == ((blockIdx.x / sms) & 3)) {          // blocks that share an SM add on different schedulers
         const float ss = chain_sum(sq + (lane & 3) * glue_pitch(n), n);
         if (lane < GLUE_ROWS) s_inv[lane] = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)n), eps));
     }
@@ -392,19 +403,19 @@ static __device__ __forceinline__ void glue_inv_rms(const float4 (&v)[CH / 4], f
 
 static __device__ __forceinline__ bool all_finite(const float4& v) { return finite_f(v.x) && finite_f(v.y) && finite_f(v.z) && finite_f(v.w); }
 
-template <int CH>
-__global__ void __launch_bounds__(32 * GLUE_ROWS, CH > 96 ? 2 : 4) glue_rows_warp_kernel(GlueArgs a, int rows) {
-    static_assert(CH % 4 == 0 && GLUE_ROWS == 4, "rows are moved in 16-byte pieces; four schedulers");
+template <int P, bool FULL>
+__global__ void __launch_bounds__(32 * GLUE_ROWS, P <= 22 ? 4 : (P <= 24 ? 3 : 2)) glue_rows_warp_kernel(GlueArgs a, int rows, int sms) {
+    static_assert(GLUE_ROWS == 4, "four schedulers");
     extern __shared__ __align__(16) float gsm[];
     __shared__ float s_inv[GLUE_ROWS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const bool live = blockIdx.x * GLUE_ROWS + w < rows;            // rows past the end: the last one again, not stored
     const int row = live ? blockIdx.x * GLUE_ROWS + w : rows - 1;
-    const int n = a.n;                         // == 32 * CH
+    const int n = FULL ? 128 * P : a.n;
     bool bad = false;
-    float4 v[CH / 4];
+    float4 v[P];
 #pragma unroll
-    for (int i = 0; i < CH / 4; i++) v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int i = 0; i < P; i++) v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (a.grouped != nullptr) {
         for (int r = 0; r < a.topk; r++) {
             const int g = a.c2g[row * a.topk + r];
@@ -415,58 +426,89 @@ __global__ void __launch_bounds__(32 * GLUE_ROWS, CH > 96 ? 2 : 4) glue_rows_war
             }
             const float4* src = (const float4*)(a.grouped + (size_t)g * n) + lane;
 #pragma unroll
-            for (int i = 0; i < CH / 4; i++) {
-                const float4 o = __ldg(src + 32 * i);
-                v[i].x = __fadd_rn(v[i].x, __fmul_rn(f, o.x));
-                v[i].y = __fadd_rn(v[i].y, __fmul_rn(f, o.y));
-                v[i].z = __fadd_rn(v[i].z, __fmul_rn(f, o.z));
-                v[i].w = __fadd_rn(v[i].w, __fmul_rn(f, o.w));
-            }
+            for (int i = 0; i < P; i++)
+                if (glue_in_row<P, FULL>(i, lane, n)) {
+                    const float4 o = __ldg(src + 32 * i);
+                    v[i].x = __fadd_rn(v[i].x, __fmul_rn(f, o.x));
+                    v[i].y = __fadd_rn(v[i].y, __fmul_rn(f, o.y));
+                    v[i].z = __fadd_rn(v[i].z, __fmul_rn(f, o.z));
+                    v[i].w = __fadd_rn(v[i].w, __fmul_rn(f, o.w));
+                }
         }
     } else {
         const float4* src = (const float4*)(a.x_in + (size_t)row * n) + lane;
 #pragma unroll
-        for (int i = 0; i < CH / 4; i++) v[i] = src[32 * i];
+        for (int i = 0; i < P; i++)
+            if (glue_in_row<P, FULL>(i, lane, n)) v[i] = src[32 * i];
     }
     if (a.norm_w != nullptr) {
-        glue_inv_rms<CH>(v, gsm, s_inv, a.eps_norm);
+        glue_inv_rms<P, FULL>(v, gsm, s_inv, n, a.eps_norm, sms);
         const float inv = s_inv[w];
         if (!finite_f(inv) && lane == 0) flag(a.status, SB_ERR_NONFINITE);
         const float4* nw4 = (const float4*)a.norm_w + lane;
 #pragma unroll
-        for (int i = 0; i < CH / 4; i++) {
-            const float4 m = __ldg(nw4 + 32 * i);
-            bad |= !all_finite(v[i]) || !all_finite(m);
-            v[i].x = __fmul_rn(__fmul_rn(v[i].x, inv), m.x);
-            v[i].y = __fmul_rn(__fmul_rn(v[i].y, inv), m.y);
-            v[i].z = __fmul_rn(__fmul_rn(v[i].z, inv), m.z);
-            v[i].w = __fmul_rn(__fmul_rn(v[i].w, inv), m.w);
-        }
+        for (int i = 0; i < P; i++)
+            if (glue_in_row<P, FULL>(i, lane, n)) {
+                const float4 m = __ldg(nw4 + 32 * i);
+                bad |= !all_finite(v[i]) || !all_finite(m);
+                v[i].x = __fmul_rn(__fmul_rn(v[i].x, inv), m.x);
+                v[i].y = __fmul_rn(__fmul_rn(v[i].y, inv), m.y);
+                v[i].z = __fmul_rn(__fmul_rn(v[i].z, inv), m.z);
+                v[i].w = __fmul_rn(__fmul_rn(v[i].w, inv), m.w);
+            }
     }
     if (a.y_out != nullptr && live) {
         float4* dst = (float4*)(a.y_out + (size_t)row * n) + lane;
 #pragma unroll
-        for (int i = 0; i < CH / 4; i++) dst[32 * i] = v[i];
+        for (int i = 0; i < P; i++)
+            if (glue_in_row<P, FULL>(i, lane, n)) dst[32 * i] = v[i];
     }
     if (a.router_scale != nullptr) {
-        glue_inv_rms<CH>(v, gsm, s_inv, a.eps_router);
+        glue_inv_rms<P, FULL>(v, gsm, s_inv, n, a.eps_router, sms);
         const float inv = s_inv[w], root = __fdiv_rn(1.0f, sqrtf_exact((float)n));
         if ((!finite_f(inv) || !finite_f(root)) && lane == 0) flag(a.status, SB_ERR_NONFINITE);
         const float4* rs4 = (const float4*)a.router_scale + lane;
         float4* dst = (float4*)(a.rin + (size_t)row * n) + lane;
 #pragma unroll
-        for (int i = 0; i < CH / 4; i++) {
-            const float4 m = __ldg(rs4 + 32 * i);
-            float4 t;
-            t.x = __fmul_rn(__fmul_rn(__fmul_rn(v[i].x, inv), m.x), root);
-            t.y = __fmul_rn(__fmul_rn(__fmul_rn(v[i].y, inv), m.y), root);
-            t.z = __fmul_rn(__fmul_rn(__fmul_rn(v[i].z, inv), m.z), root);
-            t.w = __fmul_rn(__fmul_rn(__fmul_rn(v[i].w, inv), m.w), root);
-            bad |= !all_finite(v[i]) || !all_finite(m) || !all_finite(t);
-            if (live) dst[32 * i] = t;
-        }
+        for (int i = 0; i < P; i++)
+            if (glue_in_row<P, FULL>(i, lane, n)) {
+                const float4 m = __ldg(rs4 + 32 * i);
+                float4 t;
+                t.x = __fmul_rn(__fmul_rn(__fmul_rn(v[i].x, inv), m.x), root);
+                t.y = __fmul_rn(__fmul_rn(__fmul_rn(v[i].y, inv), m.y), root);
+                t.z = __fmul_rn(__fmul_rn(__fmul_rn(v[i].z, inv), m.z), root);
+                t.w = __fmul_rn(__fmul_rn(__fmul_rn(v[i].w, inv), m.w), root);
+                bad |= !all_finite(v[i]) || !all_finite(m) || !all_finite(t);
+                if (live) dst[32 * i] = t;
+            }
     }
     if (bad) flag(a.status, SB_ERR_NONFINITE);
+}
+
+template <int P>
+static cudaError_t launch_glue_warps(const GlueArgs& a, int rows, int sms, cudaStream_t stream) {
+    if constexpr (P < GLUE_PIECES)
+        if (a.n > 128 * P) return launch_glue_warps<P + 2>(a, rows, sms, stream);
+    const size_t smem = (size_t)GLUE_ROWS * (a.n + 4) * sizeof(float);
+    const auto kernel = a.n == 128 * P ? glue_rows_warp_kernel<P, true> : glue_rows_warp_kernel<P, false>;
+    cudaError_t e = ensure_dynamic_smem((const void*)kernel, smem);
+    if (e != cudaSuccess) return e;
+    kernel<<<(rows + GLUE_ROWS - 1) / GLUE_ROWS, 32 * GLUE_ROWS, smem, stream>>>(a, rows, sms);
+    return launched();
+}
+
+// Most rows for which the block-per-row form is the faster one.  It takes a full round of the chip for every `at_once` rows
+// (one block per SM; four of 256 threads for narrow rows), the warp form about as long for one row as for several hundred.
+// Measured with 148 SMs, two sums (one launch, us, block / warp form): 1024 columns 592 rows 13.2 / 12.5, 768 rows 19 / 14;
+// 2048 columns 148 rows 12 / 21, 296 rows 23.5 / 20.7, 320 rows 34 / 21, 2048 rows 167 / 45; 4096 columns 296 rows 26 / 33, 320
+// rows 38 / 33; 5120 columns 148 rows 24 / 39, 192 rows 45 / 39; 6144 columns 192 rows 48 / 51, 320 rows 72 / 53.  One sum lies
+// alike.  Without a sum the block form's rounds are three times shorter: 2816 columns 320 rows 10.4 / 12.4, 512 rows 13.8 /
+// 12.4; 5120 columns 192 rows 12.4 / 10.4.
+static int glue_block_rows(const GlueArgs& a, int sms) {
+    const int at_once = a.n <= 1024 ? 4 * sms : sms;
+    int rounds = a.n <= 1024 || (a.n > 4096 && a.n <= 5120) ? 1 : 2;
+    if (a.norm_w == nullptr && a.router_scale == nullptr && a.n <= 4096) rounds++;
+    return rounds * at_once;
 }
 
 cudaError_t launch_glue(const GlueArgs& a, int rows, cudaStream_t stream) {
@@ -474,27 +516,17 @@ cudaError_t launch_glue(const GlueArgs& a, int rows, cudaStream_t stream) {
     if (a.topk > 64) return cudaErrorInvalidValue;
     const size_t smem = (size_t)(a.n + 8) * sizeof(float);
     const auto al16 = [](const void* p) { return (((uintptr_t)p) & 15) == 0; };
-    if (rows >= 256 && (a.n == 32 * 88 || a.n == 32 * 160) && al16(a.grouped) && al16(a.x_in) && al16(a.y_out) &&
-        al16(a.norm_w) && al16(a.router_scale) && al16(a.rin)) {
-        const size_t wsmem = (size_t)GLUE_ROWS * (a.n + 4) * sizeof(float);
-        const void* kernel = a.n == 32 * 88 ? (const void*)glue_rows_warp_kernel<88> : (const void*)glue_rows_warp_kernel<160>;
-        cudaError_t e = ensure_dynamic_smem(kernel, wsmem);
-        if (e != cudaSuccess) return e;
-        const int blocks = (rows + GLUE_ROWS - 1) / GLUE_ROWS;
-        if (a.n == 32 * 88) glue_rows_warp_kernel<88><<<blocks, 32 * GLUE_ROWS, wsmem, stream>>>(a, rows);
-        else glue_rows_warp_kernel<160><<<blocks, 32 * GLUE_ROWS, wsmem, stream>>>(a, rows);
-        return launched();
-    }
+    const int sms = device_sms();
+    if (rows > glue_block_rows(a, sms) && a.n % 64 == 0 && a.n <= 128 * GLUE_PIECES && al16(a.grouped) && al16(a.x_in) && al16(a.y_out) &&
+        al16(a.norm_w) && al16(a.router_scale) && al16(a.rin))
+        return launch_glue_warps<2>(a, rows, sms, stream);
     if (a.n <= 4096) {
         // every thread owns 4 columns: wide rows and small batches get the largest block
         const int threads = (rows <= 16 || a.n > 1024) ? 1024 : 256;
         return launch_pdl(glue_rows_kernel<4, 8>, dim3(rows), dim3(threads), smem, stream, a);
-    } else if (a.n <= 8192) {
-        return launch_pdl(glue_rows_kernel<16, 2>, dim3(rows), dim3(512), smem, stream, a);
-    } else {
-        return cudaErrorInvalidValue;
     }
-    return launched();
+    if (a.n <= 8192) return launch_pdl(glue_rows_kernel<16, 2>, dim3(rows), dim3(512), smem, stream, a);
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_rmsnorm(const float* x, const float* weight, float* y, int rows, int n, float eps, int with_scale,

@@ -493,7 +493,7 @@ cudaError_t launch_batch(const void* jobs, int njobs_max, const int* live, const
 // Rows per lane.  Four need a quarter of the shared loads per product; two make twice as many blocks, which start and
 // end more evenly: better below about thirteen blocks per SM (2 tokens of the layer above 76 -> 72 us; one 4096 x 4096
 // row product from the host 62 -> 51).  One row per lane was slower still.  `blocks`: of four rows per lane.
-bool two_rows_per_lane(long blocks) { return blocks < 13 * 148; }
+bool two_rows_per_lane(long blocks) { return blocks < 13L * device_sms(); }
 
 }  // namespace
 

@@ -24,6 +24,8 @@
 // Every wait is bounded (spin_limit polls of about half a microsecond): when a slot does not arrive
 // the block gives up, the kernel sets SB_ERR_TIMEOUT in the status word and still advances the epoch.
 // After a timeout the ranks' epochs may differ; ep_region_reset on every rank (all idle) starts over.
+#include <algorithm>
+
 #include "internal.h"
 #include "pdl.cuh"
 
@@ -129,7 +131,7 @@ cudaError_t launch_ep_exchange(const EpExchangeArgs& a, int rows, cudaStream_t s
     // two slots per thread when the whole batch fits one wave, never more than one block per SM
     const long long work = (long long)rows * (a.width >> 1);
     long long blocks = (work + 2 * EP_THREADS - 1) / (2 * EP_THREADS);
-    blocks = blocks < 8 ? 8 : (blocks > 148 ? 148 : blocks);
+    blocks = std::max(8LL, std::min(blocks, (long long)device_sms()));
     return launch_pdl(ep_exchange_kernel, dim3((unsigned)blocks), dim3(EP_THREADS), 0, stream, a);
 }
 

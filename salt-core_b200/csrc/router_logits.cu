@@ -332,7 +332,7 @@ cudaError_t launch_many(const float* W, const float* x, float* logits, int rows,
 constexpr int CHAIN_THREADS = 128;
 template <int N4>                             // 16-byte pieces per thread
 __global__ void __launch_bounds__(CHAIN_THREADS)
-router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict__ x, float* __restrict__ logits, int E, int H) {
+router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict__ x, float* __restrict__ logits, int E, int H, int sms) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int e = blockIdx.x, r = blockIdx.y, n4 = H >> 2;
     const float4* w4 = (const float4*)(W + (size_t)e * H);
@@ -359,7 +359,7 @@ router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict_
     }
     __syncthreads();
     // blocks that share an SM add on different schedulers
-    if ((threadIdx.x >> 5) != (((blockIdx.y * gridDim.x + blockIdx.x) / 148) & 3)) return;
+    if ((threadIdx.x >> 5) != (((blockIdx.y * gridDim.x + blockIdx.x) / sms) & 3)) return;
     const float acc = chain_sum((const float*)smem, H);
     if ((threadIdx.x & 31) == 0) logits[(size_t)r * E + e] = __fadd_rn(acc, 0.0f);
 }
@@ -370,27 +370,28 @@ cudaError_t launch_router_logits(const float* W, const float* x, float* logits, 
                                  cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
     if ((H % 64) != 0 || ((((uintptr_t)W) | ((uintptr_t)x)) & 15) != 0) return cudaErrorInvalidValue;
+    const int sms = device_sms();
     // a block per chain while that is a few blocks per SM (more rows share the weights, below)
     if (rows <= 4 && H <= 10 * 4 * CHAIN_THREADS) {
         const dim3 grid(E, rows);
         const size_t smem = (size_t)H * 4;
         if (H <= 6 * 4 * CHAIN_THREADS)
-            return launch_pdl(router_logits_chain_kernel<6>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H);
-        return launch_pdl(router_logits_chain_kernel<10>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H);
+            return launch_pdl(router_logits_chain_kernel<6>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H, sms);
+        return launch_pdl(router_logits_chain_kernel<10>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H, sms);
     }
     // one chain per lane while one round of blocks holds them all, then as many per lane as keep it to one round
     const long few = (long)((E + FEW_E - 1) / FEW_E) * ((rows + FEW_ROWS - 1) / FEW_ROWS);
-    if (few <= 148) {
+    if (few <= sms) {
         cudaError_t e = ensure_dynamic_smem((const void*)router_logits_few_kernel, FEW_SMEM);
         if (e != cudaSuccess) return e;
         return launch_pdl(router_logits_few_kernel, dim3((E + FEW_E - 1) / FEW_E, (rows + FEW_ROWS - 1) / FEW_ROWS), dim3(FEW_THREADS),
                           (size_t)FEW_SMEM, stream, W, x, logits, rows, E, H, status);
     }
     const long lanes = (long)((E + 31) / 32) * ((rows + 3) / 4);                 // blocks of one chain per lane
-    if (lanes <= 148) return launch_many<1, 1>(W, x, logits, rows, E, H, status, stream);
-    if (lanes <= 2 * 148) return launch_many<1, 2>(W, x, logits, rows, E, H, status, stream);
-    if (lanes <= 4 * 148) return launch_many<2, 2>(W, x, logits, rows, E, H, status, stream);
-    if (lanes <= 8 * 148) return launch_many<2, 4>(W, x, logits, rows, E, H, status, stream);
+    if (lanes <= sms) return launch_many<1, 1>(W, x, logits, rows, E, H, status, stream);
+    if (lanes <= 2 * sms) return launch_many<1, 2>(W, x, logits, rows, E, H, status, stream);
+    if (lanes <= 4 * sms) return launch_many<2, 2>(W, x, logits, rows, E, H, status, stream);
+    if (lanes <= 8 * sms) return launch_many<2, 4>(W, x, logits, rows, E, H, status, stream);
     return launch_many<2, 8>(W, x, logits, rows, E, H, status, stream);
 }
 

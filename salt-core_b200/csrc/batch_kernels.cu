@@ -27,7 +27,8 @@
 // 32-column step a token takes 16 of them, the dequantisation 20.  Measured (hidden 2816, inter 704, 128 experts,
 // top-8; gate/up + down of a layer): 64 tokens 698 -> 438 us, 16 tokens 274 -> 175 us, 6 tokens 140 -> 98 us against
 // two rows per lane and whole groups as blocks; 2 tokens 46 us, where one persistent launch for both phases took 51.
-// NVFP4 (hidden 5120, inter 1536, 64 experts, top-4; expert phase of a layer): 1 token 71 -> 51 us, 16 tokens 640 -> 291.
+// NVFP4 (hidden 5120, inter 1536, 64 experts, top-4; expert phase of a layer): 1 token 71 -> 51 us, 16 tokens 640 -> 291; whole layers
+// with jobs of passes instead of empty blocks: 16 tokens 338 -> 308 us, 64 tokens 875 -> 769, 256 tokens 3030 -> 2570.
 #include "fp4_core.cuh"
 #include "internal.h"
 #include "pdl.cuh"
@@ -363,10 +364,10 @@ __device__ __forceinline__ void run_tokens(const Q4Job& jb, Loader<NMAT, RL>& ld
     else run_pass<NMAT, RL, 1, STEP>(jb, ld, G, smem, r0, nvalid, tb);
 }
 
-// blockIdx: row tile, job (entry of the live list if there is one), pass of the job's tokens
+// blockIdx: row tile, job, pass of the job's tokens
 template <int FMT, int NMAT, int RL>
 __global__ void __launch_bounds__(NT, RL == 4 ? 4 : 6)
-batch_kernel(const void* __restrict__ jobs, const int* __restrict__ live, const int* __restrict__ njobs_dev, int C, int jobs_early) {
+batch_kernel(const void* __restrict__ jobs, const int* __restrict__ njobs_dev, int C, int jobs_early) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int ROWS = 4 * RL * WARPS, ROWS_A = ROWS / NMAT;
     // jobs_early: the job table was written at least two launches back, so everything except the activation rows
@@ -380,7 +381,7 @@ batch_kernel(const void* __restrict__ jobs, const int* __restrict__ live, const 
     __shared__ __align__(16) Q4Job jb;
     float wg = 0.0f;
     if (FMT == FMT_FP4) {                                   // the same descriptor in the shared form
-        const Fp4Job& f = ((const Fp4Job*)jobs)[live != nullptr ? live[blockIdx.y] : (int)blockIdx.y];
+        const Fp4Job& f = ((const Fp4Job*)jobs)[blockIdx.y];
         wg = f.wg;
         if (threadIdx.x == 0) {
             jb.vals = f.codes; jb.scales = f.scales; jb.x = f.x; jb.y = f.y; jb.x_rows = nullptr;
@@ -476,8 +477,8 @@ batch_kernel(const void* __restrict__ jobs, const int* __restrict__ live, const 
 }
 
 template <int FMT, int NMAT, int RL>
-cudaError_t launch_batch(const void* jobs, int njobs_max, const int* live, const int* njobs_dev, int max_rows, int max_tok,
-                         int C, cudaStream_t stream, int pdl) {
+cudaError_t launch_batch(const void* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
+                         cudaStream_t stream, int pdl) {
     const BatchGeom G = batch_geom(FMT, C, NMAT, RL);
     cudaError_t e = ensure_dynamic_smem((const void*)batch_kernel<FMT, NMAT, RL>, G.smem);
     if (e != cudaSuccess) return e;
@@ -485,15 +486,18 @@ cudaError_t launch_batch(const void* jobs, int njobs_max, const int* live, const
     const dim3 grid((max_rows + ROWS_A - 1) / ROWS_A, njobs_max, (max_tok + MAX_T - 1) / MAX_T);
     if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
     if (pdl >= 0)
-        return launch_pdl(batch_kernel<FMT, NMAT, RL>, grid, dim3(NT), (size_t)G.smem, stream, jobs, live, njobs_dev, C, pdl);
-    batch_kernel<FMT, NMAT, RL><<<grid, NT, G.smem, stream>>>(jobs, live, njobs_dev, C, 0);
+        return launch_pdl(batch_kernel<FMT, NMAT, RL>, grid, dim3(NT), (size_t)G.smem, stream, jobs, njobs_dev, C, pdl);
+    batch_kernel<FMT, NMAT, RL><<<grid, NT, G.smem, stream>>>(jobs, njobs_dev, C, 0);
     return launched();
 }
 
 // Rows per lane.  Four need a quarter of the shared loads per product; two make twice as many blocks, which start and
-// end more evenly: better below about thirteen blocks per SM (2 tokens of the layer above 76 -> 72 us; one 4096 x 4096
-// row product from the host 62 -> 51).  One row per lane was slower still.  `blocks`: of four rows per lane.
-bool two_rows_per_lane(long blocks) { return blocks < 13L * device_sms(); }
+// end more evenly.  `blocks`: of four rows per lane in the grid (the most that the jobs of the batch can make).  Q4: two are
+// better below about thirteen blocks per SM (2 tokens of the layer above 76 -> 72 us; one 4096 x 4096 row product from the host
+// 62 -> 51).  NVFP4: below about six: 1536 rows x 5120 x 7 tokens from the host
+// 61 -> 49 us, 6144 x 5120 x 32 (5.2 blocks per SM) 254 -> 247; layers (5120 x 1536, top-4) 1 token 88 -> 82 us, 3 tokens (6.5)
+// 138 with four against 140, 8 tokens 218 / 226.  One row per lane was slower still.
+bool two_rows_per_lane(int fmt, long blocks) { return blocks < (fmt == FMT_Q4 ? 13L : 6L) * device_sms(); }
 
 }  // namespace
 
@@ -502,8 +506,8 @@ bool q4_batch_supported(int C, int nmat) { return C >= 64 && (C % 64) == 0 && ba
 cudaError_t launch_q4_batch(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
                             int nmat, cudaStream_t stream, int pdl) {
     const long blocks = (long)((max_rows + 64 / nmat - 1) / (64 / nmat)) * njobs_max * ((max_tok + MAX_T - 1) / MAX_T);
-    const bool two = two_rows_per_lane(blocks);
-#define SB_BATCH(NM, RL) launch_batch<FMT_Q4, NM, RL>(jobs, njobs_max, nullptr, njobs_dev, max_rows, max_tok, C, stream, pdl)
+    const bool two = two_rows_per_lane(FMT_Q4, blocks);
+#define SB_BATCH(NM, RL) launch_batch<FMT_Q4, NM, RL>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, pdl)
     if (nmat == 2) return two ? SB_BATCH(2, 2) : SB_BATCH(2, 4);
     return two ? SB_BATCH(1, 2) : SB_BATCH(1, 4);
 #undef SB_BATCH
@@ -511,12 +515,12 @@ cudaError_t launch_q4_batch(const Q4Job* jobs, int njobs_max, const int* njobs_d
 
 bool fp4_batch_supported(int C) { return C >= 256 && (C % 256) == 0; }
 
-cudaError_t launch_fp4_batch(const Fp4Job* jobs, int njobs_max, const int* live, const int* n_live, int max_rows, int max_tok,
-                             int C, cudaStream_t stream) {
+cudaError_t launch_fp4_batch(const Fp4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
+                             cudaStream_t stream) {
     const long blocks = (long)((max_rows + 63) / 64) * njobs_max * ((max_tok + MAX_T - 1) / MAX_T);
-    return two_rows_per_lane(blocks)
-               ? launch_batch<FMT_FP4, 1, 2>(jobs, njobs_max, live, n_live, max_rows, max_tok, C, stream, 0)
-               : launch_batch<FMT_FP4, 1, 4>(jobs, njobs_max, live, n_live, max_rows, max_tok, C, stream, 0);
+    return two_rows_per_lane(FMT_FP4, blocks)
+               ? launch_batch<FMT_FP4, 1, 2>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, 0)
+               : launch_batch<FMT_FP4, 1, 4>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, 0);
 }
 
 }  // namespace sb

@@ -44,8 +44,8 @@ bool q4_batch_supported(int C, int nmat);
 cudaError_t launch_q4_batch(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
                             int nmat, cudaStream_t stream, int pdl);
 bool fp4_batch_supported(int C);
-cudaError_t launch_fp4_batch(const Fp4Job* jobs, int njobs_max, const int* live, const int* n_live, int max_rows, int max_tok,
-                             int C, cudaStream_t stream);
+cudaError_t launch_fp4_batch(const Fp4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
+                             cudaStream_t stream);
 
 // ---- q4_fused_decode.cu ------------------------------------------------------
 // Decode-sized expert execution in one launch (gate | up -> GeGLU -> down).
@@ -192,13 +192,24 @@ struct Fp4ExpertDesc {
     const uint8_t* scales[3];
     float wg[3], ig[3];
 };
-// Jobs of a grouped NVFP4 MoE layer (gu_jobs: [2E] gate then up; dn_jobs: [E]; groups of remote experts get
-// ntok = 0) and the per-row input global scales (ig_gu: [2J], ig_dn: [J]).
-cudaError_t launch_nvfp4_moe_plan(const int* group_offsets, int E, int expert_begin, int expert_end, int J,
-                                  const Fp4ExpertDesc* experts, int H, int M, const float* dq_gu, float* gate_out,
-                                  float* up_out, const float* dq_dn, float* grouped_out, Fp4Job* gu_jobs, Fp4Job* dn_jobs,
-                                  float* ig_gu, float* ig_dn, cudaStream_t stream, struct Fp4TcJob* tc_gu = nullptr,
-                                  struct Fp4TcJob* tc_dn = nullptr, int* live = nullptr);
+// Jobs of a grouped NVFP4 MoE layer and the input global scales of its rows.
+struct Fp4PlanArgs {
+    const int* group_offsets;    // [E + 1]
+    int n_experts, expert_begin, expert_end;   // experts owned by this device (others are skipped)
+    int rows;                    // grouped rows J
+    const Fp4ExpertDesc* experts;   // [expert_end - expert_begin]
+    int hidden, inter;
+    const float *dq_gu, *dq_dn;  // dequantised activations [2J][hidden] and [J][inter]
+    float *gate_out, *up_out, *grouped_out;
+    // exact projections (gu_jobs != null): a job per pass of at most pass_tokens tokens (<= Q4_PASS_TOKENS), or, with 0, per group
+    int pass_tokens;
+    Fp4Job *gu_jobs, *dn_jobs;   // [2 passes] gate, up, gate, ...; [passes]; passes <= local experts + J / pass_tokens
+    int* n_jobs;                 // [2] gate and up jobs, down jobs
+    // tensor-core projections (tc_gu != null): [2E] gate then up, [E]; groups of remote experts get ntok = 0
+    struct Fp4TcJob *tc_gu, *tc_dn;
+    float *ig_gu, *ig_dn;        // [2J], [J]; 0: a row of a remote expert
+};
+cudaError_t launch_nvfp4_moe_plan(const Fp4PlanArgs& args, cudaStream_t stream);
 // ---- nvfp4_gemm_tc.cu: block-scaled tensor-core form of a grouped NVFP4 projection (tolerance path) ----
 struct Fp4TcJob {
     float* y;                  // y[n * y_stride + m]
@@ -218,10 +229,9 @@ cudaError_t make_fp4_weight_map(CUtensorMap* out, const void* base, int C, int r
 cudaError_t make_fp4_act_maps(CUtensorMap* out3, const void* base, int C, int rows);
 cudaError_t launch_nvfp4_gemm_tc(const Fp4TcJob* jobs, int njobs, int R, int C, const Fp4TcMaps& maps, int* status,
                                  cudaStream_t stream);
-// live / n_live (optional, device): indices of the jobs that have tokens and their number; njobs is then the
-// largest number of such jobs the call can have, and the grid spans only that many
+// njobs_dev (optional, device): number of live jobs; njobs is then the most the call can have
 cudaError_t launch_nvfp4_jobs(const Fp4Job* jobs, int njobs, int max_rows, int max_tok, int C, bool aligned,
-                              cudaStream_t stream, const int* live = nullptr, const int* n_live = nullptr);
+                              cudaStream_t stream, const int* njobs_dev = nullptr);
 
 // ---- router_kernels.cu ---------------------------------------------------
 // Device-side error word: 0 = ok; set (never cleared) by kernels that meet a

@@ -82,7 +82,7 @@ struct Stack {
     uint8_t *fp4_packed = nullptr, *fp4_scales = nullptr;
     Fp4Job *fp4_gu_jobs = nullptr, *fp4_dn_jobs = nullptr;
     Fp4TcJob *fp4_tc_gu = nullptr, *fp4_tc_dn = nullptr;
-    int* fp4_live = nullptr;                   // [2 + 3E]: counts and indices of the projection jobs that have tokens
+    int* fp4_n_jobs = nullptr;                 // [2]: projection jobs of gate and up, of down
     CUtensorMap fp4_x_gu[3], fp4_x_dn[3];      // packed activations as [2J][H/2] and as [J][M/2]
     CUtensorMap fp4_xs_gu[3], fp4_xs_dn[3];    // their block scales as [2J][H/16] and as [J][M/16]
     bool fp4_maps_ok = false;
@@ -152,7 +152,7 @@ static void free_stack(Stack* s) {
     cudaFree(s->grouped_alt); cudaFree(s->weights_alt); cudaFree(s->layer_counters); cudaFree(s->d_layer_args);
     cudaFree(s->fp4_dq_gu); cudaFree(s->fp4_dq_dn); cudaFree(s->fp4_gate); cudaFree(s->fp4_up); cudaFree(s->fp4_ig_gu);
     cudaFree(s->fp4_ig_dn); cudaFree(s->fp4_packed); cudaFree(s->fp4_scales); cudaFree(s->fp4_gu_jobs); cudaFree(s->fp4_dn_jobs);
-    cudaFree(s->fp4_tc_gu); cudaFree(s->fp4_tc_dn); cudaFree(s->fp4_live);
+    cudaFree(s->fp4_tc_gu); cudaFree(s->fp4_tc_dn); cudaFree(s->fp4_n_jobs);
     cudaFree(s->xs_h); cudaFree(s->xs_l); cudaFree(s->cs_h); cudaFree(s->cs_l);
     cudaFree(s->xh); cudaFree(s->xl); cudaFree(s->chain_h); cudaFree(s->chain_l);
     cudaFree(s->tc_items_fused); cudaFree(s->tc_items_plain); cudaFree(s->tc_work);
@@ -309,9 +309,9 @@ int salt_b200_stack_add_nvfp4_layer(void* stack, const SaltB200Nvfp4LayerSpec* s
         !(dev_alloc(&s->fp4_dq_gu, 2 * J * s->hidden) && dev_alloc(&s->fp4_dq_dn, J * s->inter) &&
           dev_alloc(&s->fp4_gate, J * s->inter) && dev_alloc(&s->fp4_up, J * s->inter) && dev_alloc(&s->fp4_ig_gu, 2 * J) &&
           dev_alloc(&s->fp4_ig_dn, J) && dev_alloc(&s->fp4_packed, 2 * J * (size_t)s->hidden / 2) &&
-          dev_alloc(&s->fp4_scales, 2 * J * (size_t)s->hidden / 16) && dev_alloc(&s->fp4_gu_jobs, (size_t)2 * E) &&
-          dev_alloc(&s->fp4_dn_jobs, (size_t)E) && dev_alloc(&s->fp4_tc_gu, (size_t)2 * E) &&
-          dev_alloc(&s->fp4_tc_dn, (size_t)E) && dev_alloc(&s->fp4_live, (size_t)(2 + 3 * E))))
+          dev_alloc(&s->fp4_scales, 2 * J * (size_t)s->hidden / 16) && dev_alloc(&s->fp4_gu_jobs, 2 * (E + J / Q4_PASS_TOKENS)) &&
+          dev_alloc(&s->fp4_dn_jobs, E + J / Q4_PASS_TOKENS) && dev_alloc(&s->fp4_tc_gu, (size_t)2 * E) &&
+          dev_alloc(&s->fp4_tc_dn, (size_t)E) && dev_alloc(&s->fp4_n_jobs, 2)))
         return -1;
     if (!s->fp4_maps_ok)
         s->fp4_maps_ok = make_fp4_act_maps(s->fp4_x_gu, s->fp4_packed, s->hidden, (int)(2 * J)) == cudaSuccess &&
@@ -509,48 +509,52 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
         Timed t(s, KC_PLAN, st);
         if (!cuda_ok(launch_moe_plan(a, st), "plan")) return -1;
     }
-    if (l.nvfp4 && (flags & SB_EXPERTS_TENSOR_CORE)) {
-        // block-scaled tensor-core form (tolerance path): same plan, same bit-exact quantiser, the two
-        // projection batches as tcgen05.mma.kind::mxf4nvf4 GEMMs
-        if (!l.fp4_tc_ok) return -1;
-        Timed t(s, KC_GATE_UP, st);
-        Fp4TcMaps mg, md;
-        mg.w = l.fp4_w_gu; md.w = l.fp4_w_dn;
-        mg.ws = l.fp4_ws_gu; md.ws = l.fp4_ws_dn;
-        for (int v = 0; v < 3; v++) {
-            mg.x[v] = s->fp4_x_gu[v]; md.x[v] = s->fp4_x_dn[v];
-            mg.xs[v] = s->fp4_xs_gu[v]; md.xs[v] = s->fp4_xs_dn[v];
-        }
-        if (!cuda_ok(launch_nvfp4_moe_plan(s->group_offsets, E, s->expert_begin, s->expert_end, jobs, l.fp4_experts, H, M,
-                                           s->fp4_dq_gu, s->fp4_gate, s->fp4_up, s->fp4_dq_dn, s->grouped_out,
-                                           s->fp4_gu_jobs, s->fp4_dn_jobs, s->fp4_ig_gu, s->fp4_ig_dn, st, s->fp4_tc_gu,
-                                           s->fp4_tc_dn), "nvfp4 plan") ||
-            !cuda_ok(launch_nvfp4_qdq(d_x, 2 * jobs, H, s->fp4_ig_gu, s->fp4_packed, s->fp4_scales, nullptr,
-                                      s->status, st, s->g2c, jobs, K), "nvfp4 qdq x") ||
-            !cuda_ok(launch_nvfp4_gemm_tc(s->fp4_tc_gu, 2 * E, M, H, mg, s->status, st), "nvfp4 tc gate/up") ||
-            !cuda_ok(launch_nvfp4_qdq(s->fp4_gate, jobs, M, s->fp4_ig_dn, s->fp4_packed, s->fp4_scales, nullptr,
-                                      s->status, st, nullptr, 1, 1, s->fp4_up), "nvfp4 geglu + qdq") ||
-            !cuda_ok(launch_nvfp4_gemm_tc(s->fp4_tc_dn, E, H, M, md, s->status, st), "nvfp4 tc down"))
-            return -1;
-        return 0;
-    }
     if (l.nvfp4) {
-        if (flags & SB_EXPERTS_TENSOR_CORE_SINGLE) return -1;
+        const bool tc = (flags & SB_EXPERTS_TENSOR_CORE) != 0;
+        if (tc ? !l.fp4_tc_ok : (flags & SB_EXPERTS_TENSOR_CORE_SINGLE) != 0) return -1;
+        Fp4PlanArgs p;
+        memset(&p, 0, sizeof p);
+        p.group_offsets = s->group_offsets; p.n_experts = E; p.expert_begin = s->expert_begin; p.expert_end = s->expert_end;
+        p.rows = jobs; p.experts = l.fp4_experts; p.hidden = H; p.inter = M;
+        p.dq_gu = s->fp4_dq_gu; p.dq_dn = s->fp4_dq_dn;
+        p.gate_out = s->fp4_gate; p.up_out = s->fp4_up; p.grouped_out = s->grouped_out;
+        p.ig_gu = s->fp4_ig_gu; p.ig_dn = s->fp4_ig_dn;
         Timed t(s, KC_GATE_UP, st);
-        const int live_max = std::min(s->expert_end - s->expert_begin, jobs);   // experts that can have tokens
-        if (!cuda_ok(launch_nvfp4_moe_plan(s->group_offsets, E, s->expert_begin, s->expert_end, jobs, l.fp4_experts, H, M,
-                                           s->fp4_dq_gu, s->fp4_gate, s->fp4_up, s->fp4_dq_dn, s->grouped_out,
-                                           s->fp4_gu_jobs, s->fp4_dn_jobs, s->fp4_ig_gu, s->fp4_ig_dn, st, nullptr, nullptr,
-                                           s->fp4_live), "nvfp4 plan") ||
-            !cuda_ok(launch_nvfp4_qdq(d_x, 2 * jobs, H, s->fp4_ig_gu, s->fp4_packed, s->fp4_scales, s->fp4_dq_gu,
-                                      s->status, st, s->g2c, jobs, K), "nvfp4 qdq x") ||
-            !cuda_ok(launch_nvfp4_jobs(s->fp4_gu_jobs, 2 * live_max, M, B, H, true, st, s->fp4_live + 2, s->fp4_live), "nvfp4 gate/up") ||
-            !cuda_ok(launch_nvfp4_qdq(s->fp4_gate, jobs, M, s->fp4_ig_dn, s->fp4_packed, s->fp4_scales, s->fp4_dq_dn,
-                                      s->status, st, nullptr, 1, 1, s->fp4_up), "nvfp4 geglu + qdq") ||
-            !cuda_ok(launch_nvfp4_jobs(s->fp4_dn_jobs, live_max, H, B, M, true, st, s->fp4_live + 2 + 2 * E,
-                                       s->fp4_live + 1), "nvfp4 down"))
-            return -1;
-        return 0;
+        if (tc) {
+            // block-scaled tensor-core form (tolerance path): same plan, same bit-exact quantiser, the two
+            // projection batches as tcgen05.mma.kind::mxf4nvf4 GEMMs
+            Fp4TcMaps mg, md;
+            mg.w = l.fp4_w_gu; md.w = l.fp4_w_dn;
+            mg.ws = l.fp4_ws_gu; md.ws = l.fp4_ws_dn;
+            for (int v = 0; v < 3; v++) {
+                mg.x[v] = s->fp4_x_gu[v]; md.x[v] = s->fp4_x_dn[v];
+                mg.xs[v] = s->fp4_xs_gu[v]; md.xs[v] = s->fp4_xs_dn[v];
+            }
+            p.tc_gu = s->fp4_tc_gu; p.tc_dn = s->fp4_tc_dn;
+            return cuda_ok(launch_nvfp4_moe_plan(p, st), "nvfp4 plan") &&
+                   cuda_ok(launch_nvfp4_qdq(d_x, 2 * jobs, H, s->fp4_ig_gu, s->fp4_packed, s->fp4_scales, nullptr,
+                                            s->status, st, s->g2c, jobs, K), "nvfp4 qdq x") &&
+                   cuda_ok(launch_nvfp4_gemm_tc(s->fp4_tc_gu, 2 * E, M, H, mg, s->status, st), "nvfp4 tc gate/up") &&
+                   cuda_ok(launch_nvfp4_qdq(s->fp4_gate, jobs, M, s->fp4_ig_dn, s->fp4_packed, s->fp4_scales, nullptr,
+                                            s->status, st, nullptr, 1, 1, s->fp4_up), "nvfp4 geglu + qdq") &&
+                   cuda_ok(launch_nvfp4_gemm_tc(s->fp4_tc_dn, E, H, M, md, s->status, st), "nvfp4 tc down") ? 0 : -1;
+        }
+        // exact: jobs of a pass each while the grid's y extent holds them, else of a whole group
+        int passes_max = std::min(jobs, local + jobs / Q4_PASS_TOKENS);
+        p.pass_tokens = Q4_PASS_TOKENS;
+        if (2 * passes_max > 65535) {
+            p.pass_tokens = 0;
+            passes_max = std::min(jobs, local);
+        }
+        const int tok_max = p.pass_tokens ? std::min(B, p.pass_tokens) : B;
+        p.gu_jobs = s->fp4_gu_jobs; p.dn_jobs = s->fp4_dn_jobs; p.n_jobs = s->fp4_n_jobs;
+        return cuda_ok(launch_nvfp4_moe_plan(p, st), "nvfp4 plan") &&
+               cuda_ok(launch_nvfp4_qdq(d_x, 2 * jobs, H, s->fp4_ig_gu, s->fp4_packed, s->fp4_scales, s->fp4_dq_gu,
+                                        s->status, st, s->g2c, jobs, K), "nvfp4 qdq x") &&
+               cuda_ok(launch_nvfp4_jobs(s->fp4_gu_jobs, 2 * passes_max, M, tok_max, H, true, st, s->fp4_n_jobs), "nvfp4 gate/up") &&
+               cuda_ok(launch_nvfp4_qdq(s->fp4_gate, jobs, M, s->fp4_ig_dn, s->fp4_packed, s->fp4_scales, s->fp4_dq_dn,
+                                        s->status, st, nullptr, 1, 1, s->fp4_up), "nvfp4 geglu + qdq") &&
+               cuda_ok(launch_nvfp4_jobs(s->fp4_dn_jobs, passes_max, H, tok_max, M, true, st, s->fp4_n_jobs + 1), "nvfp4 down") ? 0 : -1;
     }
     if (fused) {
         FusedArgs f;

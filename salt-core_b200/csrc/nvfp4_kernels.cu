@@ -147,9 +147,9 @@ cudaError_t launch_nvfp4_qdq(const float* x, int rows, int C, const float* ig_ro
 // Any C (multiple of 16), any alignment: one warp per (row, token), lane l owns
 // accumulator l.
 __global__ void __launch_bounds__(128)
-nvfp4_generic_kernel(const Fp4Job* __restrict__ jobs, const int* __restrict__ live, const int* __restrict__ n_live) {
-    if (live != nullptr && (int)blockIdx.z >= *n_live) return;
-    const Fp4Job jb = jobs[live != nullptr ? live[blockIdx.z] : blockIdx.z];
+nvfp4_generic_kernel(const Fp4Job* __restrict__ jobs, const int* __restrict__ njobs_dev) {
+    if (njobs_dev != nullptr && (int)blockIdx.z >= *njobs_dev) return;
+    const Fp4Job jb = jobs[blockIdx.z];
     const int r = blockIdx.x * 4 + (threadIdx.x >> 5), tok = blockIdx.y;
     if (r >= jb.R || tok >= jb.ntok) return;
     const int lane = threadIdx.x & 31;
@@ -174,105 +174,100 @@ nvfp4_generic_kernel(const Fp4Job* __restrict__ jobs, const int* __restrict__ li
 
 // ---- a MoE layer of NVFP4 experts (reference caller: models/gemma4-26b-a4b/src/gemma4_text.c:8912-8945,
 // two projection batches with the GeGLU between them) ------------------------------------------------
-// One thread per expert: the projection jobs of its token group and the input global scale of every
-// grouped row (gate rows [0, J), up rows [J, 2J) of the gathered activations; down rows [0, J)).
-static __device__ __forceinline__ void
-nvfp4_plan_expert(int e, const int* __restrict__ group_offsets, int E, int expert_begin, int expert_end, int J,
-                  const Fp4ExpertDesc* __restrict__ experts, int H, int M, const float* dq_gu, float* gate_out,
-                  float* up_out, const float* dq_dn, float* grouped_out, Fp4Job* gu_jobs, Fp4Job* dn_jobs, float* ig_gu,
-                  float* ig_dn, Fp4TcJob* tc_gu, Fp4TcJob* tc_dn, int* live, int* n_gu, int* n_dn);
-
-__global__ void __launch_bounds__(128)
-nvfp4_moe_plan_kernel(const int* __restrict__ group_offsets, int E, int expert_begin, int expert_end, int J,
-                      const Fp4ExpertDesc* __restrict__ experts, int H, int M, const float* dq_gu, float* gate_out,
-                      float* up_out, const float* dq_dn, float* grouped_out, Fp4Job* gu_jobs, Fp4Job* dn_jobs,
-                      float* ig_gu, float* ig_dn, Fp4TcJob* tc_gu, Fp4TcJob* tc_dn, int* live) {
-    // live (optional): [0] / [1] = number of gate|up / down jobs with tokens, then their indices ([2, 2 + 2E)
-    // into gu_jobs, [2 + 2E, 2 + 3E) into dn_jobs) so the projection launches span only those
-    __shared__ int n_gu, n_dn;
-    if (threadIdx.x == 0) n_gu = n_dn = 0;
+// The input global scale of every grouped row (gate rows [0, J), up rows [J, 2J) of the gathered activations; down rows
+// [0, J)), and the projection jobs: one per pass of up to pass_tokens tokens of an expert, the largest passes first (gate and
+// up of pass i are gu_jobs[2 i] and [2 i + 1]), with their number; or, for the tensor cores, the jobs of whole groups.
+// (One job per expert in grids as deep as the batch left three of four blocks empty at 16 tokens and 180 000 of 196 000 at
+// 256, each with its shared memory until it had read its job.)
+__global__ void __launch_bounds__(128) nvfp4_moe_plan_kernel(Fp4PlanArgs a) {
+    __shared__ int s_class[Q4_PASS_TOKENS];       // passes by size, largest first; then the next slot of each size
+    const int E = a.n_experts, P = a.pass_tokens;
+    if (threadIdx.x < Q4_PASS_TOKENS) s_class[threadIdx.x] = 0;
     pdl_wait();                    // the group offsets come from the plan kernel before this one
     pdl_launch_dependents();
     __syncthreads();
-    for (int e = threadIdx.x; e < E; e += blockDim.x)
-        nvfp4_plan_expert(e, group_offsets, E, expert_begin, expert_end, J, experts, H, M, dq_gu, gate_out, up_out, dq_dn,
-                          grouped_out, gu_jobs, dn_jobs, ig_gu, ig_dn, tc_gu, tc_dn, live, &n_gu, &n_dn);
-    __syncthreads();
-    if (threadIdx.x == 0 && live != nullptr) {
-        live[0] = n_gu;
-        live[1] = n_dn;
+    // pass_tokens = 0: groups are not cut, and come in any order
+    const auto full = [&](int cnt) { return P ? cnt / P : 0; };
+    const auto rest = [&](int cnt) { return P ? cnt % P : cnt; };
+    const auto rest_class = [&](int cnt) { return P ? P - cnt % P : 0; };
+    if (a.gu_jobs != nullptr) {
+        for (int e = a.expert_begin + threadIdx.x; e < a.expert_end; e += blockDim.x) {
+            const int cnt = a.group_offsets[e + 1] - a.group_offsets[e];
+            if (full(cnt)) atomicAdd(&s_class[0], full(cnt));
+            if (rest(cnt)) atomicAdd(&s_class[rest_class(cnt)], 1);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int run = 0;
+            for (int k = 0; k < Q4_PASS_TOKENS; k++) { const int c = s_class[k]; s_class[k] = run; run += c; }
+            a.n_jobs[0] = 2 * run;
+            a.n_jobs[1] = run;
+        }
+        __syncthreads();
+    }
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+        const int g0 = a.group_offsets[e], cnt = a.group_offsets[e + 1] - g0;
+        const bool local = e >= a.expert_begin && e < a.expert_end;
+        Fp4ExpertDesc d;
+        if (local) d = a.experts[e - a.expert_begin];
+        if (local && a.gu_jobs != nullptr) {
+            const int nfull = full(cnt), first = nfull ? atomicAdd(&s_class[0], nfull) : 0;
+            for (int p = 0; p < nfull + (rest(cnt) ? 1 : 0); p++) {
+                const int slot = p < nfull ? first + p : atomicAdd(&s_class[rest_class(cnt)], 1);
+                const size_t row = (size_t)g0 + (size_t)p * P;
+                Fp4Job j;
+                j.ntok = p < nfull ? P : rest(cnt);
+                j.R = a.inter; j.C = a.hidden; j.x_stride = a.hidden; j.y_stride = a.inter;
+                j.codes = d.codes[0]; j.scales = d.scales[0]; j.wg = d.wg[0];
+                j.x = a.dq_gu + row * a.hidden; j.y = a.gate_out + row * a.inter;
+                a.gu_jobs[2 * slot] = j;
+                j.codes = d.codes[1]; j.scales = d.scales[1]; j.wg = d.wg[1];
+                j.x = a.dq_gu + (row + a.rows) * a.hidden; j.y = a.up_out + row * a.inter;
+                a.gu_jobs[2 * slot + 1] = j;
+                j.R = a.hidden; j.C = a.inter; j.x_stride = a.inter; j.y_stride = a.hidden;
+                j.codes = d.codes[2]; j.scales = d.scales[2]; j.wg = d.wg[2];
+                j.x = a.dq_dn + row * a.inter; j.y = a.grouped_out + row * a.hidden;
+                a.dn_jobs[slot] = j;
+            }
+        }
+        if (a.tc_gu != nullptr) {
+            // the up matrix follows the gate codes (M rows) and the gate scales (M / 8 rows of H / 2 bytes) in the expert's
+            // slot; the quantised activations' block scales use the rows of the packed codes (gate [0, J), up [J, 2J);
+            // down [0, J) after the second quantisation); scale rows are C / 16 bytes long: in those units the up scales
+            // start 9 M rows (one tensor) after the gate scales
+            const int M = a.inter;
+            Fp4TcJob t;
+            t.ntok = local ? cnt : 0; t.w_slice = local ? e - a.expert_begin : 0;
+            t.R = M; t.y_stride = M; t.w_row0 = 0; t.ws_row0 = 0; t.x_row0 = g0;
+            t.wg = local ? d.wg[0] : 0.0f; t.ig = local ? d.ig[0] : 1.0f; t.y = a.gate_out + (size_t)g0 * M;
+            a.tc_gu[e] = t;
+            t.w_row0 = M + (M >> 3); t.ws_row0 = 9 * M; t.x_row0 = a.rows + g0;
+            t.wg = local ? d.wg[1] : 0.0f; t.ig = local ? d.ig[1] : 1.0f; t.y = a.up_out + (size_t)g0 * M;
+            a.tc_gu[E + e] = t;
+            t.R = a.hidden; t.y_stride = a.hidden; t.w_row0 = 0; t.ws_row0 = 0; t.x_row0 = g0;
+            t.wg = local ? d.wg[2] : 0.0f; t.ig = local ? d.ig[2] : 1.0f; t.y = a.grouped_out + (size_t)g0 * a.hidden;
+            a.tc_dn[e] = t;
+        }
+        for (int t = 0; t < cnt; t++) {               // rows of remote experts are marked (scale 0) and skipped by the quantiser
+            a.ig_gu[g0 + t] = local ? d.ig[0] : 0.0f;
+            a.ig_gu[a.rows + g0 + t] = local ? d.ig[1] : 0.0f;
+            a.ig_dn[g0 + t] = local ? d.ig[2] : 0.0f;
+        }
     }
 }
 
-static __device__ __forceinline__ void
-nvfp4_plan_expert(int e, const int* __restrict__ group_offsets, int E, int expert_begin, int expert_end, int J,
-                  const Fp4ExpertDesc* __restrict__ experts, int H, int M, const float* dq_gu, float* gate_out,
-                  float* up_out, const float* dq_dn, float* grouped_out, Fp4Job* gu_jobs, Fp4Job* dn_jobs, float* ig_gu,
-                  float* ig_dn, Fp4TcJob* tc_gu, Fp4TcJob* tc_dn, int* live, int* n_gu, int* n_dn) {
-    const int g0 = group_offsets[e], cnt = group_offsets[e + 1] - g0;
-    const bool local = e >= expert_begin && e < expert_end;
-    Fp4ExpertDesc d;
-    if (local) d = experts[e - expert_begin];
-    Fp4Job j;
-    j.R = M; j.C = H; j.ntok = local ? cnt : 0; j.x_stride = H; j.y_stride = M;
-    j.codes = local ? d.codes[0] : nullptr; j.scales = local ? d.scales[0] : nullptr; j.wg = local ? d.wg[0] : 0.0f;
-    j.x = dq_gu + (size_t)g0 * H; j.y = gate_out + (size_t)g0 * M;
-    gu_jobs[e] = j;
-    j.codes = local ? d.codes[1] : nullptr; j.scales = local ? d.scales[1] : nullptr; j.wg = local ? d.wg[1] : 0.0f;
-    j.x = dq_gu + (size_t)(J + g0) * H; j.y = up_out + (size_t)g0 * M;
-    gu_jobs[E + e] = j;
-    j.R = H; j.C = M; j.x_stride = M; j.y_stride = H;
-    j.codes = local ? d.codes[2] : nullptr; j.scales = local ? d.scales[2] : nullptr; j.wg = local ? d.wg[2] : 0.0f;
-    j.x = dq_dn + (size_t)g0 * M; j.y = grouped_out + (size_t)g0 * H;
-    dn_jobs[e] = j;
-    if (live != nullptr && local && cnt > 0) {
-        const int i = atomicAdd(n_gu, 2);
-        live[2 + i] = e;
-        live[3 + i] = E + e;
-        live[2 + 2 * E + atomicAdd(n_dn, 1)] = e;
-    }
-    if (tc_gu) {
-        // the same jobs for the tensor-core kernel: the up matrix follows the gate codes (M rows) and the gate
-        // scales (M / 8 rows of H / 2 bytes) in the expert's slot; the quantised activations' block scales
-        // use the rows of the packed codes (gate [0, J), up [J, 2J); down [0, J) after the second quantisation);
-        // scale rows are C / 16 bytes long: in those units the up scales start 9 M rows (one tensor) after the
-        // gate scales
-        Fp4TcJob t;
-        t.ntok = local ? cnt : 0; t.w_slice = local ? e - expert_begin : 0;
-        t.R = M; t.y_stride = M; t.w_row0 = 0; t.ws_row0 = 0; t.x_row0 = g0;
-        t.wg = local ? d.wg[0] : 0.0f; t.ig = local ? d.ig[0] : 1.0f; t.y = gate_out + (size_t)g0 * M;
-        tc_gu[e] = t;
-        t.w_row0 = M + (M >> 3); t.ws_row0 = 9 * M; t.x_row0 = J + g0;
-        t.wg = local ? d.wg[1] : 0.0f; t.ig = local ? d.ig[1] : 1.0f; t.y = up_out + (size_t)g0 * M;
-        tc_gu[E + e] = t;
-        t.R = H; t.y_stride = H; t.w_row0 = 0; t.ws_row0 = 0; t.x_row0 = g0;
-        t.wg = local ? d.wg[2] : 0.0f; t.ig = local ? d.ig[2] : 1.0f; t.y = grouped_out + (size_t)g0 * H;
-        tc_dn[e] = t;
-    }
-    for (int t = 0; t < cnt; t++) {                   // rows of remote experts are marked (scale 0) and skipped by the quantiser
-        ig_gu[g0 + t] = local ? d.ig[0] : 0.0f;
-        ig_gu[J + g0 + t] = local ? d.ig[1] : 0.0f;
-        ig_dn[g0 + t] = local ? d.ig[2] : 0.0f;
-    }
-}
-
-cudaError_t launch_nvfp4_moe_plan(const int* group_offsets, int E, int expert_begin, int expert_end, int J,
-                                  const Fp4ExpertDesc* experts, int H, int M, const float* dq_gu, float* gate_out,
-                                  float* up_out, const float* dq_dn, float* grouped_out, Fp4Job* gu_jobs, Fp4Job* dn_jobs,
-                                  float* ig_gu, float* ig_dn, cudaStream_t stream, Fp4TcJob* tc_gu, Fp4TcJob* tc_dn,
-                                  int* live) {
-    return launch_pdl(nvfp4_moe_plan_kernel, dim3(1), dim3(128), 0, stream, group_offsets, E, expert_begin, expert_end, J,
-                      experts, H, M, dq_gu, gate_out, up_out, dq_dn, grouped_out, gu_jobs, dn_jobs, ig_gu, ig_dn, tc_gu,
-                      tc_dn, live);
+cudaError_t launch_nvfp4_moe_plan(const Fp4PlanArgs& a, cudaStream_t stream) {
+    if (a.pass_tokens < 0 || a.pass_tokens > Q4_PASS_TOKENS) return cudaErrorInvalidValue;
+    return launch_pdl(nvfp4_moe_plan_kernel, dim3(1), dim3(128), 0, stream, a);
 }
 
 cudaError_t launch_nvfp4_jobs(const Fp4Job* jobs, int njobs, int max_rows, int max_tok, int C, bool aligned,
-                              cudaStream_t stream, const int* live, const int* n_live) {
+                              cudaStream_t stream, const int* njobs_dev) {
     if (njobs < 1 || max_rows < 1 || max_tok < 1) return cudaSuccess;
-    if (aligned && fp4_batch_supported(C)) return launch_fp4_batch(jobs, njobs, live, n_live, max_rows, max_tok, C, stream);
+    if (aligned && fp4_batch_supported(C)) return launch_fp4_batch(jobs, njobs, njobs_dev, max_rows, max_tok, C, stream);
     dim3 grid((max_rows + 3) / 4, max_tok, njobs);
     if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
-    nvfp4_generic_kernel<<<grid, 128, 0, stream>>>(jobs, live, n_live);
+    nvfp4_generic_kernel<<<grid, 128, 0, stream>>>(jobs, njobs_dev);
     return launched();
 }
 

@@ -137,6 +137,11 @@ class ClockSampler:
                 "samples": len(sm), "reasons": sorted(reasons)}
 
 
+# What ran on the host cores: a ratio against the port is no comparison with the reference.
+CPU_KINDS = {"reference": "the reference's own functions (oracle/_ref)",
+             "port": "this repository's CPU port (oracle/salt_oracle.c; the reference's sources were not there to build)"}
+
+
 def make_layer(synth, fmt, seed):
     return synth.make_q4_moe_layer_bulk(seed) if fmt == "q4" else synth.make_nvfp4_moe_layer(seed)
 
@@ -202,8 +207,8 @@ def cpu_baseline(layers, B, seconds, threads, fmt="q4"):
             break
     return {"value": B * n / el, "unit": UNIT, "cores": used, "kind": kind,
             "sample": f"{n} single-layer passes at B={B} cycling {len(layers)} distinct layers "
-                      f"({el:.1f} s); reference functions on " +
-                      ("a persistent pthread pool" if fmt == "q4" else "the reference's own row threads, one projection at a time"),
+                      f"({el:.1f} s); " + CPU_KINDS[kind] +
+                      (" on a persistent pthread pool" if fmt == "q4" else " on row threads, one projection at a time"),
             "ms_per_layer": 1e3 * el / n}
 
 
@@ -285,7 +290,7 @@ def run_reference(args):
     ms = 1e3 * el / args.steps
     value = B * n_host / (ms * 1e-3)
     sample = (f"each step = {n_host} layers of the stack (of {args.layers}) at B={B}, RMSNorm between layers; "
-              f"reference CPU functions, {used} threads")
+              f"{CPU_KINDS[kind]}, {used} threads")
     print(json.dumps({
         "impl": "reference", "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": args.gpus,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,

@@ -428,7 +428,7 @@ int salt_b200_ffn_block_forward(void *stack, int layer, const float *d_residual,
 
 /* Phase A of one layer on `stream` (a cudaStream_t, NULL = default stream):
  * router input, logits, top-k, grouping, gate/up + GeGLU, down for the local
- * experts.  d_x is [B][hidden] in device memory.  flags:
+ * experts.  d_x is [B][hidden] in device memory, 16-byte aligned (else the call returns -1).  flags:
  *   SALT_B200_EXPERTS_ZERO_REMOTE         clear grouped_out first, so rows of remote experts read as +0
  *   SALT_B200_EXPERTS_ROUTER_INPUT_READY  the previous layer's combine already prepared the router input */
 #define SALT_B200_EXPERTS_ZERO_REMOTE 1
@@ -461,7 +461,8 @@ int salt_b200_layer_combine(void *stack, int layer, int B, float *d_y, int flags
  *                          softmax top-k of its B tokens -> d_selected [B][topk] (expert ids, ascending within a
  *                          token), d_weights [B][topk]; both caller-owned device memory
  *   _layer_experts_routed  owner rank: d_out[i] = expert d_experts[i] (one of THIS stack's experts) applied to
- *                          d_rows[i] (gate | up, GeGLU, down), i < n_rows <= max_tokens * topk, any order; the
+ *                          d_rows[i] (gate | up, GeGLU, down), i < n_rows <= max_tokens * topk, any order (d_rows and
+ *                          d_out 16-byte aligned, else -1); the
  *                          rows are grouped by expert as reference src/moe_group.c:83-182 groups them and every
  *                          row's result depends only on (expert weights, row), so it is the same whichever rank
  *                          computes it and whatever else is in the call.  flags: the TENSOR_CORE flags
@@ -516,7 +517,8 @@ int salt_b200_stack_ep_reset(void *stack);
 int salt_b200_stack_ep_disconnect(void *stack);
 
 /* Layers [first, first+count) back to back (phase A + B each), chained through
- * the layers' RMSNorm; d_x and d_y are device pointers and may alias. */
+ * the layers' RMSNorm; d_x and d_y are device pointers and may alias.  d_x must be 16-byte aligned (else -1, except
+ * for one token on one launch per layer, which takes any address). */
 int salt_b200_stack_forward_device(void *stack, int first, int count, const float *d_x, int B, float *d_y,
                                    void *stream);
 /* Same with HOST input/output: copies in, runs, copies out, synchronises, and

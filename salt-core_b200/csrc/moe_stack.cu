@@ -448,7 +448,8 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
 // d_router_src feeds the router input (unless it is already prepared), d_x the expert projections.
 static int layer_experts_impl(Stack* s, int layer, const float* d_router_src, const float* d_x, int B, int flags,
                               cudaStream_t st) {
-    if (!s || layer < 0 || layer >= (int)s->layers.size() || !d_x || !d_router_src || B < 1 || B > s->max_tokens)
+    if (!s || layer < 0 || layer >= (int)s->layers.size() || !d_x || !d_router_src || B < 1 || B > s->max_tokens ||
+        ((uintptr_t)d_x & 15))                              // every expert kernel moves rows in 16-byte pieces
         return -1;
     const Layer& l = s->layers[(size_t)layer];
     if ((flags & SB_EXPERTS_ZERO_REMOTE) &&
@@ -489,7 +490,7 @@ static int experts_run(Stack* s, const Layer& l, const float* d_x, int B, int K,
     const bool fused = !l.nvfp4 && s->fused_decode && !(flags & (SB_EXPERTS_TENSOR_CORE | SB_EXPERTS_TENSOR_CORE_SINGLE |
                                                      SB_EXPERTS_TWO_LAUNCHES)) &&
                        B == 1 && njobs_max <= FUSED_MAX_JOBS &&
-                       ((((uintptr_t)d_x) | ((uintptr_t)l.pool) | l.expert_stride) & 15) == 0 &&
+                       ((((uintptr_t)l.pool) | l.expert_stride) & 15) == 0 &&
                        q4_fused_plan(H, M, njobs_max, nullptr);
     if (fused) {
         a.fused_jobs = s->fused_jobs; a.fused_done = s->fused_done;
@@ -726,7 +727,7 @@ int salt_b200_layer_experts_routed(void* stack, int layer, const float* d_rows, 
         (s->hidden % 4) != 0)
         return -1;
     if (n_rows == 0) return 0;
-    if (!d_rows || !d_experts || !d_out || ((uintptr_t)d_out & 15)) return -1;
+    if (!d_rows || !d_experts || !d_out || (((uintptr_t)d_rows | (uintptr_t)d_out) & 15)) return -1;
     const Layer& l = s->layers[(size_t)layer];
     flags &= (SB_EXPERTS_TENSOR_CORE | SB_EXPERTS_TENSOR_CORE_SINGLE);
     if (experts_run(s, l, d_rows, n_rows, 1, d_experts, false, flags | SB_EXPERTS_TWO_LAUNCHES, st) != 0) return -1;

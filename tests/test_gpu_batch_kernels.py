@@ -30,7 +30,7 @@ def test_batch_projection_vs_oracle(orc, synth, R, C, B):
 
 
 def test_single_token_of_a_wide_row(orc, synth):
-    """More columns than the one-token kernel holds in shared memory."""
+    """12288 columns: scale tables of 192 words per row."""
     rng = np.random.default_rng(17)
     R, C = 70, 12288
     v, s, b = synth.make_q4(rng, R, C)

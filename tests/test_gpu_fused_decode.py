@@ -1,5 +1,6 @@
-"""The one-launch decode expert kernel (gate | up -> GeGLU -> down for all selected experts)
-against the two-launch form and the CPU oracle, bit for bit, through the C ABI."""
+"""The one-launch decode kernels (one token: gate | up -> GeGLU -> down for all selected experts, and the whole layer)
+against the two-launch form and the CPU oracle, bit for bit, through the C ABI; two to four tokens, which take the batch
+kernel either way, against the oracle."""
 import numpy as np
 import pytest
 
@@ -50,8 +51,8 @@ def test_fused_decode_repeated_tokens_share_groups(orc, synth):
 
 
 def test_fused_decode_sharded_expert_ranges(orc, synth):
-    """Expert-parallel ranges: each stack runs the fused kernel on its own groups only (some
-    ranges get none); the union over one shared grouped buffer equals the unsharded layer."""
+    """Expert-parallel ranges: each stack runs its own groups only (some ranges get none); the union over one shared
+    grouped buffer equals the unsharded layer.  (Two tokens: the batch kernel.)"""
     import torch
     H, M, E, K, B = 2816, 704, 128, 8, 2
     layer = synth.make_q4_moe_layer_bulk(330)

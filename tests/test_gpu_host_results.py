@@ -107,7 +107,7 @@ def _best_us(call):
 
 def test_large_results_of_single_floats_are_copied(synth):
     """131072 results: 207 to 229 us written one by one over the bus, 80 to 130 copied; the same results as whole lines take
-    40 to 50, which is the measure of this box here."""
+    40 to 50, which is the measure of the host at hand."""
     g, rng, R = gpu(), np.random.default_rng(1), 131072
     g.set_mapped_only(0)
     y = np.zeros(R, np.float32)

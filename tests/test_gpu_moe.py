@@ -408,8 +408,8 @@ def test_whole_ffn_block_vs_oracle(orc, synth, geom):
 
 @pytest.mark.parametrize("geom", [(320, 64, 24, 2, 300), (320, 64, 24, 2, 1030), (2816, 704, 128, 8, 1030)])
 def test_router_logits_prefill_sized_batches_vs_oracle(orc, synth, geom):
-    """Batches of several hundred rows take the large-tile logits kernels (32 experts x 16 or 32 rows
-    per block); ragged tiles in both directions, a last column slab shorter than the others."""
+    """Batches of several hundred rows: one block of few experts x few rows per SM, and two and four rows per lane of
+    the kernel for many rows; ragged tiles in both directions, a last column slab shorter than the others."""
     import torch
     H, M, E, K, B = geom
     make = synth.make_q4_moe_layer_bulk if H == 2816 else synth.make_q4_moe_layer
@@ -431,9 +431,8 @@ def test_router_logits_prefill_sized_batches_vs_oracle(orc, synth, geom):
 
 
 def test_stack_two_layers_prefill_sized_batch_vs_oracle(orc, synth):
-    """300 rows at the bench geometry: the reduce + RMSNorm + router-input glue runs one warp per row
-    (dependent-add chains handed from lane to lane), the logits take the large tiles; the second layer's
-    output depends on both."""
+    """300 rows at the bench geometry: the reduce + RMSNorm + router-input glue runs one warp per row (the sums of four
+    rows side by side in one warp), the logits take the kernel for many rows; the second layer's output depends on both."""
     B = 300
     layers = [synth.make_q4_moe_layer_bulk(95 + i) for i in range(2)]
     x = synth.make_tokens(97, B, 2816)
@@ -462,9 +461,9 @@ def test_stack_two_layers_prefill_sized_batch_hidden_5120_vs_oracle(orc, synth):
 
 
 def test_stack_wide_hidden_takes_any_shape_kernels_vs_oracle(orc, synth):
-    """hidden = 5696 is beyond what the tiled projection kernels hold in shared memory: the stack runs the
-    any-shape kernels, one grid row per token of a group.  Groups of more than four tokens must all be
-    computed (6 tokens over 4 experts, top-2: every group holds several tokens)."""
+    """hidden = 5696: 89 quantisation groups per row, more columns than a glue thread of the narrow form owns.  (An earlier
+    form of the tiled projection kernels could not hold such rows; tests/test_gpu_any_shape.py has the widths that take the
+    any-shape kernels now.)  Groups of more than four tokens must all be computed (6 tokens over 4 experts, top-2)."""
     H, M, E, K, B = 5696, 128, 4, 2, 6
     layers = [synth.make_q4_moe_layer(97 + i, hidden=H, inter=M, n_experts=E, topk=K) for i in range(2)]
     x = synth.make_tokens(99, B, H)

@@ -291,7 +291,7 @@ int salt_gpu_shared_buffer_alloc(SaltGpuSharedBuffer *buffer, size_t nbytes);
 int salt_gpu_shared_buffer_free(SaltGpuSharedBuffer *buffer);
 int salt_gpu_exact_cells(const SaltGpuExactCell *cells, int count);
 
-/* ---- present, fail closed: outside the MoE-FFN path -------------------- */
+/* ---- affine 8-bit and bf16 projections of routers and heads -------------- */
 int salt_gpu_q8_matvec(const uint32_t *vals, const uint16_t *scales, const uint16_t *biases, int R, int C,
                        const float *x, float *y);                           /* gpu.h:37 */
 int salt_gpu_q8_batch(const uint32_t *const *vals, const uint16_t *const *scales, const uint16_t *const *biases,
@@ -299,6 +299,7 @@ int salt_gpu_q8_batch(const uint32_t *const *vals, const uint16_t *const *scales
                       int njobs);                                            /* gpu.h:89 */
 int salt_gpu_bf16_matvec(const void *key, int R, int C, const float *input, float *output);        /* gpu.h:63 */
 int salt_gpu_bf16_matvec_batch(const void *key, int R, int C, int B, const float *inputs, float *outputs);
+/* ---- present, fail closed: outside the MoE-FFN path -------------------- */
 int salt_gpu_attention_batch(int full_attention, int n_heads, int n_kv_heads, int head_dim, int window,
                              const SaltGpuSharedBuffer *queries, size_t query_float_offset,
                              const SaltGpuSharedBuffer *kv, size_t key_float_offset, size_t value_float_offset,
@@ -329,7 +330,11 @@ int salt_gpu_attention_transform(int n_heads, int n_kv_heads, int head_dim, int 
  * n_experts slots of expert_stride bytes, each gate | up | down, each tensor
  * values | scales | biases (the slot order of the reference's expert pool,
  * tools/gemma4-mlx4-source.py:180-199).  norm_weight, when not NULL, is the
- * RMSNorm weight applied to this layer's output before the next layer. */
+ * RMSNorm weight applied to this layer's output before the next layer.
+ * Device memory of a layer beside the uploaded bytes: one 32-bit word (scale << 16) | bias per quantisation group (the
+ * same bytes again, 11 % of a layer) for the decode kernels and, where the TENSOR_CORE flags admit the geometry, these
+ * words once more in the order the tensor-core kernels read and two floats per weight row (12 %) - whether or not a
+ * flag is ever used: 104 MB beside 428 MB at 128 experts of 704 x 2816. */
 typedef struct SaltB200Q4LayerSpec {
     int hidden, inter, n_experts, topk;
     float eps;
@@ -396,8 +401,8 @@ int salt_b200_stack_nvfp4_buffers(void *stack, SaltB200Nvfp4Buffers *out);
  * A forward pass of ONE token over affine-Q4 layers goes further: level 1 (the default) runs each layer
  * (reduce, norm, router, top-k, experts) as one launch; level 2 runs ALL layers of the pass in one launch
  * whose blocks stay resident, a layer ending with an arrival counter instead of a kernel boundary (one
- * launch per pass for hosts where launches are the cost; on a B200 with graph replay it measured 49.1 us
- * per layer against 46.3 us for level 1, whose programmatic dependent launches overlap a layer's prologue
+ * launch per pass for hosts where launches are the cost; on a B200 with graph replay it measured 43.4 us
+ * per layer against 40.1 us for level 1, whose programmatic dependent launches overlap a layer's prologue
  * with the previous layer's tail).  enable = 0 makes every later forward pass of this stack use the phase
  * kernels instead; all levels produce the same bits. */
 int salt_b200_stack_set_fused_decode(void *stack, int enable);

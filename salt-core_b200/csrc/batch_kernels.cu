@@ -23,12 +23,15 @@
 //   * The canonical fold goes through a shared-memory area of the warp, two lanes per row, and the GeGLU of the
 //     pass' tokens is spread over the lanes, instead of running on one lane in sixteen.
 //
-// What bounds it now: issue cycles.  A packed or a logic operation holds a scheduler for two cycles; per row, lane and
-// 32-column step a token takes 16 of them, the dequantisation 20.  Measured (hidden 2816, inter 704, 128 experts,
-// top-8; gate/up + down of a layer): 64 tokens 698 -> 438 us, 16 tokens 274 -> 175 us, 6 tokens 140 -> 98 us against
-// two rows per lane and whole groups as blocks; 2 tokens 46 us, where one persistent launch for both phases took 51.
-// NVFP4 (hidden 5120, inter 1536, 64 experts, top-4; expert phase of a layer): 1 token 71 -> 51 us, 16 tokens 640 -> 291; whole layers
-// with jobs of passes instead of empty blocks: 16 tokens 338 -> 308 us, 64 tokens 875 -> 769, 256 tokens 3030 -> 2570.
+// What bounds it now: issue cycles.  Per row, lane and 32-column step a token takes four packed operations, each of which
+// holds a scheduler for two cycles.  At 64 tokens (gate/up) 63 of 196 M warp instructions are these: 43 % of the launch's
+// cycles; the others (dequantisation once per pass and row, activation loads, the blocks' tables, prologues and folds) are
+// another 45 %.  At 16 tokens, where nearly every pass holds one or two, the products are 16 of 67 M.  Measured
+// (hidden 2816, inter 704, 128 experts, top-8; gate/up + down of a layer, event pairs): 64 tokens 698 -> 423 us, 16 tokens
+// 274 -> 156 us, 6 tokens 140 -> 90 us against two rows per lane and whole groups as blocks; 2 tokens 45 us, where one
+// persistent launch for both phases took 51.
+// NVFP4 (hidden 5120, inter 1536, 64 experts, top-4; expert phase of a layer): 1 token 71 -> 51 us, 16 tokens 640 -> 291; whole
+// layers with jobs of passes instead of empty blocks: 16 tokens 338 -> 305 us, 64 tokens 867 -> 766, 256 tokens 3020 -> 2570.
 #include "fp4_core.cuh"
 #include "internal.h"
 #include "pdl.cuh"

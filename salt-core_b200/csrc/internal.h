@@ -145,7 +145,7 @@ cudaError_t launch_q4_tc_tables(const uint32_t* tables, int hidden, int inter, i
                                 float* unscale, cudaStream_t stream);
 cudaError_t make_q4_tc_weight_maps(TcWeightMaps* out, const uint8_t* pool, size_t expert_stride, const uint32_t* tables,
                                    const float* row_scale, const float* row_unscale, int hidden, int inter, int experts);
-// Can the tensor-core kernels take this geometry?  Sizes must be multiples of 64; a size that is no multiple of
+// Do the tensor-core calls admit this geometry?  Sizes must be multiples of 64; a size that is no multiple of
 // 256 must not exceed 3520 (single) / 960 (hi + lo halves).
 bool q4_tc_supported(int hidden, int inter, bool split);
 // What the tensor-core launches of a layer read: the tokens' rows in grouped order (fp16; split: residuals and group means

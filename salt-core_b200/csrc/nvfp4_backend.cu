@@ -56,7 +56,7 @@ static Tensor* fp4_tensor(const void* key, int R, int C, const Resource** res_ou
     for (auto& r : B.resources)
         if (r.kind == t.kind && r.id == t.id && r.active && r.dev) {
             if (!t.dv) {
-                // codes and scales must be 16-byte aligned for the tile kernel; copy if not
+                // codes and scales must be 16-byte aligned for the batch kernel; copy if not
                 const uint64_t offs[2] = {t.voff, t.soff};
                 const size_t sizes[2] = {t.vbytes, t.gbytes};
                 const uint8_t* out[2];

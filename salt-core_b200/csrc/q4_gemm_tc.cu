@@ -37,12 +37,13 @@
 //                     the columns), sixteen columns at a time to stay inside 96 registers: GeGLU (fused gate/up) or plain
 //                     store (down).  It runs after the group's second chunk of the NEXT unit, so that the tensor core
 //                     does not drain at a unit's end
-// Measured (B200, 1965 MHz, a whole expert layer: hidden 2816, inter 704, 128 experts,
-// top-8): 512 tokens in split precision 800 us with three MMAs per K step on split weights -> 515 with exact weights and
-// separate rings -> 473 with the delayed epilogue, four stages and the correction chunk's table words loaded at once (they
-// came in four serial batches, 9000 cycles a chunk) -> 430 with cheaper kernels around the GEMMs and tables by group.
-// 1999 tokens in single precision 780 -> 707 -> 694 -> 607.  In that
-// state the tensor pipe is busy 35 to 40 % of the time and the schedulers issue in 45 % of the cycles.
+// Measured (B200, 1965 MHz, a whole layer with its router: hidden 2816, inter 704, 128 experts, top-8): 512 tokens in split
+// precision 800 us with three MMAs per K step on split weights -> 515 with exact weights and separate rings -> 473 with the
+// delayed epilogue, four stages and the correction chunk's table words loaded at once (they came in four serial batches, 9000
+// cycles a chunk) -> 430 with cheaper kernels around the GEMMs and tables by group -> 420 with whole sectors per store and
+// half a stage for a last tile of 64 rows (gate/up 201, down 107).  1999 tokens in single precision 780 -> 707 -> 694 -> 607
+// -> 585 (gate/up 222, down 142).  The tensor pipe is busy 36 to 49 % of the time, the schedulers issue in 47 to 62 % of the
+// cycles: converters and tensor core still wait for one another.
 // What was measured on the way here: a register ring of global loads for the packed bytes does not prefetch - waiting for
 // the oldest load also waits for the younger ones that share its scoreboard (hence TMA); one mbarrier wait costs 150 to 250
 // cycles even when its phase is complete, so the phases needed next are tested ahead; a tcgen05.mma costs the issuing
@@ -287,7 +288,8 @@ __device__ __forceinline__ uint4 lds_v4(const uint8_t* p) {
 }
 
 // gelu_tanh(g) * u.  0.5 (1 + tanh i) = 1 / (1 + exp(-2 i)): a tenth of tanhf's instructions, and no cancellation for
-// large negative g (relative error a few 2^-23; the epilogue of a unit of 44 chunks took 10000 cycles with tanhf).
+// large negative g (the error of __expf grows with its argument: relative to the result a few 2^-23 near zero, |2 i| 2^-23 or
+// so far from it, where the result is tiny; the epilogue of a unit of 44 chunks took 10000 cycles with tanhf).
 __device__ __forceinline__ float geglu_fast(float g, float u) {
     const float inner = 0.7978845608028654f * (g + 0.044715f * g * g * g);
     return __fdividef(g * u, 1.0f + __expf(-2.0f * inner));
@@ -962,7 +964,8 @@ cudaError_t make_q4_tc_weight_maps(TcWeightMaps* out, const uint8_t* pool, size_
     return cudaSuccess;
 }
 
-// The documented limits of the two precisions (a size that is no multiple of 256 is bounded).
+// The limits of the two precisions are those the calls have always documented.  They come from tables that an earlier form
+// kept in shared memory for sizes that are no multiple of 256; nothing in this form needs them, and nothing was tested beyond.
 bool q4_tc_supported(int hidden, int inter, bool split) {
     if (hidden < TC_KC || inter < TC_KC || (hidden % TC_KC) || (inter % TC_KC)) return false;
     const int limit = split ? 960 : 3520;

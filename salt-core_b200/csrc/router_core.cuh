@@ -79,7 +79,7 @@ static __device__ __forceinline__ float serial_sum(const float* sq, int n) {
 //      binade's ends, and the term is not a half-way case; all other elements are "serial
 //      points".  Consecutive certain elements share one binade, so their integer increments
 //      add up exactly (64-bit scan);
-//   3. one thread walks the serial points in order: for the run of certain elements before
+//   3. one warp walks the serial points in order: for the run of certain elements before
 //      each point it CHECKS that the exact running sum really is in the predicted binade
 //      and stays there (else it adds that run element by element), adds the run's integer
 //      total, then performs the serial point's addition in floating point.
@@ -96,7 +96,7 @@ constexpr int POSSUM_SCRATCH = 8 + 32 + 32 + 64 + 32 + POSSUM_NS * 4 + 96;
 
 template <int V = POSSUM_V>
 static __device__ float block_sum_nonneg(const float* sq, int n, uint32_t* scratch) {
-    constexpr uint32_t ONE24 = 1u << 24, MARGIN = 1u << 13;
+    constexpr uint32_t MARGIN = 1u << 13;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
     float* fs = (float*)(scratch + 8);                 // [32] warp totals of the float scan
     float* flast = (float*)(scratch + 40);             // [32] last inclusive value of each warp

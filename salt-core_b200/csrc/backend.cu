@@ -874,7 +874,8 @@ int salt_gpu_proj_batch_indexed(const uint32_t* vals, const uint16_t* scales, co
         if (B.mapped_only) B.stats.mapped_only_misses++;
         return -1;
     }
-    const size_t need = (size_t)job_count * C;
+    // a whole number of 16-byte pieces: the next call's rows may be read in such pieces
+    const size_t need = ((size_t)job_count * C + 3) & ~(size_t)3;
     if (need > B.stage_floats) return -1;
     if (B.x_cursor + need > B.stage_floats) {
         if (!cuda_ok(cudaStreamSynchronize(B.stream), "stage wrap")) return -1;
@@ -883,7 +884,7 @@ int salt_gpu_proj_batch_indexed(const uint32_t* vals, const uint16_t* scales, co
     float* dx = B.d_x + B.x_cursor;
     B.x_cursor += need;
     B.in_flight = true;
-    if (!cuda_ok(cudaMemcpyAsync(dx, xs + (size_t)first_job * C, need * sizeof(float), cudaMemcpyHostToDevice,
+    if (!cuda_ok(cudaMemcpyAsync(dx, xs + (size_t)first_job * C, (size_t)job_count * C * sizeof(float), cudaMemcpyHostToDevice,
                                  B.stream), "x upload"))
         return -1;
     // descriptor ring: one slot per outstanding call

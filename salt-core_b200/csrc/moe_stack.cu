@@ -99,6 +99,7 @@ struct Stack {
     float *norm_a = nullptr, *norm_b = nullptr, *dense_chain = nullptr, *dense_out = nullptr;
     float *routed_out = nullptr, *combine_scratch = nullptr;
     int dense_cap = 0;
+    std::vector<void*> retired;                // buffers outgrown by later calls: layers and captured passes may still name them
     bool own_grouped = true;
     size_t grouped_bytes = 0;
     float *h_in = nullptr, *h_out = nullptr;  // pinned staging for the host entry point
@@ -143,6 +144,7 @@ static void free_stack(Stack* s) {
     }
     cudaFree(s->norm_a); cudaFree(s->norm_b); cudaFree(s->dense_chain); cudaFree(s->dense_out);
     cudaFree(s->routed_out); cudaFree(s->combine_scratch);
+    for (void* p : s->retired) cudaFree(p);
     cudaFree(s->rin); cudaFree(s->logits); cudaFree(s->weights); cudaFree(s->chain);
     if (s->own_grouped) cudaFree(s->grouped_out);
     cudaFree(s->reduced); cudaFree(s->act_a); cudaFree(s->act_b); cudaFree(s->io_in); cudaFree(s->io_out);
@@ -915,10 +917,11 @@ int salt_b200_stack_attach_ffn_block(void* stack, int layer, const SaltB200FfnBl
     if (l.ffn || l.nvfp4) return -1;
     const int H = s->hidden, D = spec->dense_inter;
     const size_t T = (size_t)s->max_tokens;
-    if (D > s->dense_cap) {
-        cudaFree(s->dense_chain);
-        s->dense_chain = nullptr;
-        if (!dev_alloc(&s->dense_chain, T * D)) return -1;
+    if (D > s->dense_cap) {                    // the jobs of layers attached before keep the buffer that they have
+        float* wider = nullptr;
+        if (!dev_alloc(&wider, T * D)) return -1;
+        if (s->dense_chain) s->retired.push_back(s->dense_chain);
+        s->dense_chain = wider;
         s->dense_cap = D;
     }
     if (!s->norm_a &&

@@ -1022,14 +1022,19 @@ static int forward_decode_layers(Stack* s, int first, int count, const float* d_
     // one "layer finished" counter per layer (the whole-stack launch)
     const int stride = FUSED_MAX_JOBS + 1;
     if (count > s->layers_cap) {       // set-up, not part of a captured pass: forward passes are not captured before one has run
-        cudaFree(s->layer_counters);
-        cudaFree(s->d_layer_args);
-        s->layer_counters = nullptr;
-        s->d_layer_args = nullptr;
-        if (!dev_alloc(&s->layer_counters, (size_t)count * (stride + 1)) || !dev_alloc(&s->d_layer_args, (size_t)count))
+        const int cap = (int)s->layers.size();                 // >= count
+        int32_t* counters = nullptr;
+        LayerDecodeArgs* args = nullptr;
+        if (!dev_alloc(&counters, (size_t)cap * (stride + 1)) || !dev_alloc(&args, (size_t)cap)) {
+            cudaFree(counters);
             return -1;
-        s->h_layer_args.reserve((size_t)count);
-        s->layers_cap = count;
+        }
+        if (s->layer_counters) s->retired.push_back(s->layer_counters);      // a captured pass may name them
+        if (s->d_layer_args) s->retired.push_back(s->d_layer_args);
+        s->layer_counters = counters;
+        s->d_layer_args = args;
+        s->h_layer_args.reserve((size_t)cap);
+        s->layers_cap = cap;
     }
     if (!cuda_ok(cudaMemsetAsync(s->layer_counters, 0, (size_t)count * (stride + 1) * sizeof(int32_t), st), "layer counters"))
         return -1;

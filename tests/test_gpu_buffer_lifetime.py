@@ -2,7 +2,7 @@
 import pytest
 
 from conftest import assert_bits_equal
-from gpu_util import stack_mod
+from gpu_util import oracle_stack, stack_mod
 from test_gpu_moe import _oracle_ffn_block
 
 pytestmark = pytest.mark.gpu
@@ -23,4 +23,35 @@ def test_wider_dense_branch_attached_later(orc, synth):
         assert st.ffn_block_forward(i, d_x.data_ptr(), B, d_y.data_ptr()) == 0
         assert st.status() == 0
         assert_bits_equal(d_y.cpu().numpy(), _oracle_ffn_block(orc, layers[i], blocks[i], x), f"layer {i}")
+    st.close()
+
+
+@pytest.mark.parametrize("level", [1, 2])
+def test_captured_pass_after_layers_were_added(orc, synth, level):
+    """A captured one-token pass replayed after a longer pass has run: the longer one needs more counters and arguments."""
+    import torch
+    H, M, E, K = 512, 128, 16, 4
+    layers = [synth.make_q4_moe_layer(890 + i, hidden=H, inter=M, n_experts=E, topk=K) for i in range(5)]
+    st, stream = stack_mod().MoeStack(4, H, M, E, K), torch.cuda.Stream()
+    st.set_fused_decode(level)
+    st.add_layer(layers[0])
+    st.add_layer(layers[1])
+    x, other = (torch.from_numpy(synth.make_tokens(s, 1, H)).cuda() for s in (895, 896))
+    y, z = torch.zeros(1, H, device="cuda"), torch.zeros(1, H, device="cuda")
+    assert st.graph_capture(x.data_ptr(), 1, y.data_ptr(), stream.cuda_stream) == 0
+    want, _ = oracle_stack(orc, layers[:2], x.cpu().numpy(), threads=4)
+    for layer in layers[2:]:
+        st.add_layer(layer)
+    assert st.forward_device(other.data_ptr(), 1, z.data_ptr(), stream=stream.cuda_stream) == 0
+    stream.synchronize()
+    full, _ = oracle_stack(orc, layers, other.cpu().numpy(), threads=4)
+    assert_bits_equal(z.cpu().numpy(), full, "all layers")
+    held = [torch.full((1 << 18,), 7, dtype=torch.int32, device="cuda") for _ in range(16)]     # where freed memory would go
+    if level == 1:
+        y.zero_()
+        torch.cuda.synchronize()
+        assert st.graph_launch(stream.cuda_stream) == 0
+        assert st.status(stream.cuda_stream) == 0
+        assert_bits_equal(y.cpu().numpy(), want, "replayed pass over the first two layers")
+    assert all(int(h.min()) == 7 and int(h.max()) == 7 for h in held)
     st.close()

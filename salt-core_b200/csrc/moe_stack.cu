@@ -15,6 +15,7 @@
 #include <string.h>
 
 #include <mutex>
+#include <new>
 #include <vector>
 
 #include "../../include/salt_gpu_b200.h"
@@ -1016,6 +1017,30 @@ static bool decode_layers_apply(Stack* s, int B) {
            q4_layer_decode_plan(s->hidden, s->inter, s->n_experts, s->topk, s->topk < local ? s->topk : local, nullptr);
 }
 
+static void CUDART_CB free_captured_args(void* p) { delete[] (LayerDecodeArgs*)p; }
+
+// Arguments that a copy on `st` may be made from: the vector itself or, while `st` captures, a copy that lives as long as the
+// graph does (later passes fill the vector anew).
+static const LayerDecodeArgs* capture_copy(const std::vector<LayerDecodeArgs>& args, cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    if (!cuda_ok(cudaStreamGetCaptureInfo_v2(st, &status, nullptr, &graph, nullptr, nullptr), "capture info")) return nullptr;
+    if (status != cudaStreamCaptureStatusActive) return args.data();
+    LayerDecodeArgs* own = new (std::nothrow) LayerDecodeArgs[args.size()];
+    if (!own) return nullptr;
+    memcpy(own, args.data(), args.size() * sizeof(LayerDecodeArgs));
+    cudaUserObject_t object = nullptr;
+    if (!cuda_ok(cudaUserObjectCreate(&object, own, free_captured_args, 1, cudaUserObjectNoDestructorSync), "captured arguments")) {
+        delete[] own;
+        return nullptr;
+    }
+    if (!cuda_ok(cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove), "captured arguments")) {
+        cudaUserObjectRelease(object, 1);
+        return nullptr;
+    }
+    return own;
+}
+
 static int forward_decode_layers(Stack* s, int first, int count, const float* d_x, float* d_y, cudaStream_t st) {
     const int H = s->hidden, M = s->inter, K = s->topk;
     // per layer: the logits arrival counter and FUSED_MAX_JOBS job counters; after all layers' blocks of those,
@@ -1077,10 +1102,10 @@ static int forward_decode_layers(Stack* s, int first, int count, const float* d_
         if (!cuda_ok(launch_q4_layer_decode(a, a.f.n_jobs_max, st), "decode layer")) return -1;
     }
     if (stacked) {
-        // the arguments travel with every pass (a captured pass replays the copy from this host vector, whose
-        // storage stays put while the capacity holds: set-up, like the counters above)
-        if (!cuda_ok(cudaMemcpyAsync(s->d_layer_args, s->h_layer_args.data(), (size_t)count * sizeof(LayerDecodeArgs),
-                                     cudaMemcpyHostToDevice, st), "layer arguments"))
+        // the arguments travel with every pass; a captured pass replays the copy from an array of its own
+        const LayerDecodeArgs* args = capture_copy(s->h_layer_args, st);
+        if (!args || !cuda_ok(cudaMemcpyAsync(s->d_layer_args, args, (size_t)count * sizeof(LayerDecodeArgs),
+                                              cudaMemcpyHostToDevice, st), "layer arguments"))
             return -1;
         Timed t(s, KC_GATE_UP, st);
         if (!cuda_ok(launch_q4_stack_decode(s->d_layer_args, count, s->layer_counters + (size_t)count * stride, H, M,

@@ -47,11 +47,35 @@ def test_captured_pass_after_layers_were_added(orc, synth, level):
     full, _ = oracle_stack(orc, layers, other.cpu().numpy(), threads=4)
     assert_bits_equal(z.cpu().numpy(), full, "all layers")
     held = [torch.full((1 << 18,), 7, dtype=torch.int32, device="cuda") for _ in range(16)]     # where freed memory would go
-    if level == 1:
+    y.zero_()
+    torch.cuda.synchronize()
+    assert st.graph_launch(stream.cuda_stream) == 0
+    assert st.status(stream.cuda_stream) == 0
+    assert_bits_equal(y.cpu().numpy(), want, "replayed pass over the first two layers")
+    assert all(int(h.min()) == 7 and int(h.max()) == 7 for h in held)
+    st.close()
+
+
+def test_captured_whole_pass_keeps_its_arguments(orc, synth):
+    """All layers in one launch: the arguments of a captured pass are its own, whatever passes run between its replays."""
+    import torch
+    H, M, E, K = 512, 128, 16, 4
+    layers = [synth.make_q4_moe_layer(900 + i, hidden=H, inter=M, n_experts=E, topk=K) for i in range(4)]
+    st, stream = stack_mod().MoeStack(4, H, M, E, K), torch.cuda.Stream()
+    for layer in layers:
+        st.add_layer(layer)
+    st.set_fused_decode(2)
+    x, other = (torch.from_numpy(synth.make_tokens(s, 1, H)).cuda() for s in (905, 906))
+    y, z = torch.zeros(1, H, device="cuda"), torch.zeros(1, H, device="cuda")
+    assert st.graph_capture(x.data_ptr(), 1, y.data_ptr(), stream.cuda_stream, first=0, count=2) == 0
+    want, _ = oracle_stack(orc, layers[:2], x.cpu().numpy(), threads=4)
+    between, _ = oracle_stack(orc, layers[1:], other.cpu().numpy(), threads=4)
+    for _ in range(2):
+        assert st.forward_device(other.data_ptr(), 1, z.data_ptr(), first=1, count=3, stream=stream.cuda_stream) == 0
         y.zero_()
         torch.cuda.synchronize()
         assert st.graph_launch(stream.cuda_stream) == 0
         assert st.status(stream.cuda_stream) == 0
-        assert_bits_equal(y.cpu().numpy(), want, "replayed pass over the first two layers")
-    assert all(int(h.min()) == 7 and int(h.max()) == 7 for h in held)
+        assert_bits_equal(y.cpu().numpy(), want, "replayed pass")
+        assert_bits_equal(z.cpu().numpy(), between, "pass between")
     st.close()

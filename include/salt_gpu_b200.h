@@ -407,7 +407,8 @@ int salt_b200_stack_nvfp4_buffers(void *stack, SaltB200Nvfp4Buffers *out);
  * kernels instead; all levels produce the same bits. */
 int salt_b200_stack_set_fused_decode(void *stack, int enable);
 /* Replace the grouped-output buffer by caller-owned device memory (for example
- * a buffer registered with a communication library). */
+ * a buffer registered with a communication library).  A pass captured before names the old buffer: the stack's own graph
+ * is dropped (salt_b200_stack_graph_launch returns -1 until the next capture), other captures must be made anew. */
 int salt_b200_stack_set_grouped_out(void *stack, void *device_buffer, size_t nbytes);
 
 /* The dense branch and the norms that make a MoE layer the reference model's whole feed-forward

@@ -409,6 +409,10 @@ int salt_b200_stack_nvfp4_buffers(void* stack, SaltB200Nvfp4Buffers* out) {
 int salt_b200_stack_set_grouped_out(void* stack, void* device_buffer, size_t nbytes) {
     Stack* s = (Stack*)stack;
     if (!s || !device_buffer || nbytes < s->grouped_bytes || ((uintptr_t)device_buffer & 15)) return -1;
+    if (s->graph) {                        // the captured pass names the buffer that goes
+        cudaGraphExecDestroy(s->graph);
+        s->graph = nullptr;
+    }
     if (s->own_grouped) cudaFree(s->grouped_out);
     s->grouped_out = (float*)device_buffer;
     s->own_grouped = false;

@@ -79,3 +79,23 @@ def test_captured_whole_pass_keeps_its_arguments(orc, synth):
         assert_bits_equal(y.cpu().numpy(), want, "replayed pass")
         assert_bits_equal(z.cpu().numpy(), between, "pass between")
     st.close()
+
+
+def test_captured_pass_is_dropped_with_the_grouped_buffer(orc, synth):
+    import torch
+    H, M, E, K, B = 512, 128, 16, 4, 3
+    layer = synth.make_q4_moe_layer(910, hidden=H, inter=M, n_experts=E, topk=K)
+    st, stream = stack_mod().MoeStack(4, H, M, E, K), torch.cuda.Stream()
+    st.add_layer(layer)
+    x = torch.from_numpy(synth.make_tokens(911, B, H)).cuda()
+    y, grouped = torch.zeros(B, H, device="cuda"), torch.zeros(4 * K * H, device="cuda")
+    assert st.graph_capture(x.data_ptr(), B, y.data_ptr(), stream.cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert st.set_grouped_out(grouped.data_ptr(), grouped.numel() * 4) == 0
+    assert st.graph_launch(stream.cuda_stream) == -1
+    assert st.graph_capture(x.data_ptr(), B, y.data_ptr(), stream.cuda_stream) == 0
+    y.zero_()
+    torch.cuda.synchronize()
+    assert st.graph_launch(stream.cuda_stream) == 0 and st.status(stream.cuda_stream) == 0
+    assert_bits_equal(y.cpu().numpy(), orc.moe_layer_q4(layer, x.cpu().numpy(), threads=4)[0], "captured anew")
+    st.close()

@@ -186,6 +186,10 @@ __global__ void __launch_bounds__(128) nvfp4_moe_plan_kernel(Fp4PlanArgs a) {
     pdl_wait();                    // the group offsets come from the plan kernel before this one
     pdl_launch_dependents();
     __syncthreads();
+    // rows past the last group (selections without an expert) are skipped by the quantiser too: their entries of the row
+    // table are an earlier batch's and may lie past this one's rows
+    for (int r = a.group_offsets[E] + (int)threadIdx.x; r < a.rows; r += blockDim.x)
+        a.ig_gu[r] = a.ig_gu[a.rows + r] = a.ig_dn[r] = 0.0f;
     // pass_tokens = 0: groups are not cut, and come in any order
     const auto full = [&](int cnt) { return P ? cnt / P : 0; };
     const auto rest = [&](int cnt) { return P ? cnt % P : cnt; };

@@ -687,7 +687,10 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(MoePlanArgs a) {
         const int i = i0 + lane;
         const bool live = i < s1;
         int e = live ? a.selected[i] : -1;
-        if (e < 0 || e >= E) e = -1;
+        if (e < 0 || e >= E) {
+            e = -1;
+            if (live) a.canonical_to_grouped[i] = -1;      // no row: what an earlier batch left there is another token's
+        }
         const unsigned peers = __match_any_sync(0xffffffffu, e);
         if (e >= 0) {
             const int before = __popc(peers & ((1u << lane) - 1u));
@@ -796,6 +799,8 @@ __global__ void __launch_bounds__(4 * TOPK_THREADS) moe_plan_small_kernel(MoePla
         if (e >= 0) {
             a.grouped_to_canonical[before] = lane;
             a.canonical_to_grouped[lane] = before;
+        } else if (lane < jobs) {
+            a.canonical_to_grouped[lane] = -1;             // no row: what an earlier batch left there is another token's
         }
         s_sel[lane] = e;
         s_first[lane] = (e >= 0 && first) ? 1 : 0;

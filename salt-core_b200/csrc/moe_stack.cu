@@ -171,7 +171,15 @@ static void free_stack(Stack* s) {
 
 template <typename T>
 static bool dev_alloc(T** p, size_t count) {
-    return cuda_ok(cudaMalloc((void**)p, count * sizeof(T) + 16), "stack alloc");
+    if (cuda_ok(cudaMalloc((void**)p, count * sizeof(T) + 16), "stack alloc")) return true;
+    *p = nullptr;
+    return false;
+}
+
+template <typename T>
+static void dev_free(T** p) {
+    cudaFree(*p);
+    *p = nullptr;
 }
 
 template <typename T>
@@ -308,14 +316,18 @@ int salt_b200_stack_add_nvfp4_layer(void* stack, const SaltB200Nvfp4LayerSpec* s
     if (spec->expert_stride < 3 * tensor_bytes || (spec->expert_stride % 16) != 0) return -1;
     const size_t T = (size_t)s->max_tokens, J = T * (size_t)s->topk;
     const int E = s->n_experts;
-    if (!s->fp4_dq_gu &&
+    if (!s->fp4_n_jobs &&                  // the last of them: all or none
         !(dev_alloc(&s->fp4_dq_gu, 2 * J * s->hidden) && dev_alloc(&s->fp4_dq_dn, J * s->inter) &&
           dev_alloc(&s->fp4_gate, J * s->inter) && dev_alloc(&s->fp4_up, J * s->inter) && dev_alloc(&s->fp4_ig_gu, 2 * J) &&
           dev_alloc(&s->fp4_ig_dn, J) && dev_alloc(&s->fp4_packed, 2 * J * (size_t)s->hidden / 2) &&
           dev_alloc(&s->fp4_scales, 2 * J * (size_t)s->hidden / 16) && dev_alloc(&s->fp4_gu_jobs, 2 * (E + J / Q4_PASS_TOKENS)) &&
           dev_alloc(&s->fp4_dn_jobs, E + J / Q4_PASS_TOKENS) && dev_alloc(&s->fp4_tc_gu, (size_t)2 * E) &&
-          dev_alloc(&s->fp4_tc_dn, (size_t)E) && dev_alloc(&s->fp4_n_jobs, 2)))
+          dev_alloc(&s->fp4_tc_dn, (size_t)E) && dev_alloc(&s->fp4_n_jobs, 2))) {
+        dev_free(&s->fp4_dq_gu); dev_free(&s->fp4_dq_dn); dev_free(&s->fp4_gate); dev_free(&s->fp4_up); dev_free(&s->fp4_ig_gu);
+        dev_free(&s->fp4_ig_dn); dev_free(&s->fp4_packed); dev_free(&s->fp4_scales); dev_free(&s->fp4_gu_jobs);
+        dev_free(&s->fp4_dn_jobs); dev_free(&s->fp4_tc_gu); dev_free(&s->fp4_tc_dn);
         return -1;
+    }
     if (!s->fp4_maps_ok)
         s->fp4_maps_ok = make_fp4_act_maps(s->fp4_x_gu, s->fp4_packed, s->hidden, (int)(2 * J)) == cudaSuccess &&
                          make_fp4_act_maps(s->fp4_x_dn, s->fp4_packed, s->inter, (int)J) == cudaSuccess &&
@@ -929,10 +941,12 @@ int salt_b200_stack_attach_ffn_block(void* stack, int layer, const SaltB200FfnBl
         s->dense_chain = wider;
         s->dense_cap = D;
     }
-    if (!s->norm_a &&
+    if (!s->combine_scratch &&             // the last of them: all or none
         !(dev_alloc(&s->norm_a, T * H) && dev_alloc(&s->norm_b, T * H) && dev_alloc(&s->dense_out, T * H) &&
-          dev_alloc(&s->routed_out, T * H) && dev_alloc(&s->combine_scratch, 2 * T * H)))
+          dev_alloc(&s->routed_out, T * H) && dev_alloc(&s->combine_scratch, 2 * T * H))) {
+        dev_free(&s->norm_a); dev_free(&s->norm_b); dev_free(&s->dense_out); dev_free(&s->routed_out);
         return -1;
+    }
     const size_t gu = q4_blob_bytes(D, H), dn = q4_blob_bytes(H, D);      // equal, kept apart for clarity
     bool ok = dev_alloc(&l.dense, 2 * gu + dn) &&
               cuda_ok(cudaMemcpy(l.dense, spec->dense_gate, gu, cudaMemcpyHostToDevice), "dense gate") &&
@@ -943,7 +957,12 @@ int salt_b200_stack_attach_ffn_block(void* stack, int layer, const SaltB200FfnBl
               upload(&l.post_ffn_norm_1, spec->post_ffn_norm_1, (size_t)H) &&
               upload(&l.post_ffn_norm_2, spec->post_ffn_norm_2, (size_t)H) &&
               upload(&l.post_ffn_norm, spec->post_ffn_norm, (size_t)H);
-    if (!ok) return -1;
+    const auto undo = [&l] {
+        dev_free(&l.dense); dev_free(&l.pre_ffn_norm); dev_free(&l.pre_ffn_norm_2); dev_free(&l.post_ffn_norm_1);
+        dev_free(&l.post_ffn_norm_2); dev_free(&l.post_ffn_norm); dev_free(&l.dense_jobs);
+        return -1;
+    };
+    if (!ok) return undo();
     const size_t vb = (size_t)D * H / 2, gb = (size_t)D * H / 64 * 2;
     Q4Job jobs[2];
     memset(jobs, 0, sizeof jobs);
@@ -956,7 +975,7 @@ int salt_b200_stack_attach_ffn_block(void* stack, int layer, const SaltB200FfnBl
     b.vals = l.dense + 2 * gu; b.scales = b.vals + vb; b.biases = b.scales + gb;
     b.x = s->dense_chain; b.y = s->dense_out; b.x_rows = nullptr; b.x_div = 1;
     b.R = H; b.C = D; b.ntok = 1; b.x_stride = D; b.y_stride = H;
-    if (!upload(&l.dense_jobs, jobs, (size_t)2)) return -1;
+    if (!upload(&l.dense_jobs, jobs, (size_t)2)) return undo();
     l.dense_inter = D;
     l.layer_scalar = spec->layer_scalar;
     l.ffn = true;

@@ -201,7 +201,7 @@ struct Fp4PlanArgs {
     int hidden, inter;
     const float *dq_gu, *dq_dn;  // dequantised activations [2J][hidden] and [J][inter]
     float *gate_out, *up_out, *grouped_out;
-    // exact projections (gu_jobs != null): a job per pass of at most pass_tokens tokens (<= Q4_PASS_TOKENS), or, with 0, per group
+    // exact projections (gu_jobs != null): a job per pass of pass_tokens = Q4_PASS_TOKENS tokens, or, with 0, per group
     int pass_tokens;
     Fp4Job *gu_jobs, *dn_jobs;   // [2 passes] gate, up, gate, ...; [passes]; passes <= local experts + J / pass_tokens
     int* n_jobs;                 // [2] gate and up jobs, down jobs

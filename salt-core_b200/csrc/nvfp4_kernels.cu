@@ -179,48 +179,48 @@ nvfp4_generic_kernel(const Fp4Job* __restrict__ jobs, const int* __restrict__ nj
 // up of pass i are gu_jobs[2 i] and [2 i + 1]), with their number; or, for the tensor cores, the jobs of whole groups.
 // (One job per expert in grids as deep as the batch left three of four blocks empty at 16 tokens and 180 000 of 196 000 at
 // 256, each with its shared memory until it had read its job.)
-__global__ void __launch_bounds__(128) nvfp4_moe_plan_kernel(Fp4PlanArgs a) {
-    __shared__ int s_class[Q4_PASS_TOKENS];       // passes by size, largest first; then the next slot of each size
-    const int E = a.n_experts, P = a.pass_tokens;
-    if (threadIdx.x < Q4_PASS_TOKENS) s_class[threadIdx.x] = 0;
+// A thread per expert.  The kernel is a link of a decode layer's chain of launches, so everything that does not depend on the
+// routing is read before the wait and the slots need one barrier: a class' base is the sum of the counts before it.
+__global__ void __launch_bounds__(1024) nvfp4_moe_plan_kernel(Fp4PlanArgs a) {
+    constexpr int P = Q4_PASS_TOKENS;
+    __shared__ int s_count[P], s_next[P];         // passes by size, largest first; those that have a slot
+    const int E = a.n_experts, e = threadIdx.x;
+    const bool local = e >= a.expert_begin && e < a.expert_end;
+    Fp4ExpertDesc d;
+    if (local) d = a.experts[e - a.expert_begin];
+    if (threadIdx.x < P) s_count[threadIdx.x] = s_next[threadIdx.x] = 0;
+    __syncthreads();
     pdl_wait();                    // the group offsets come from the plan kernel before this one
     pdl_launch_dependents();
-    __syncthreads();
+    const int g0 = e < E ? a.group_offsets[e] : 0, cnt = e < E ? a.group_offsets[e + 1] - g0 : 0;
     // rows past the last group (selections without an expert) are skipped by the quantiser too: their entries of the row
     // table are an earlier batch's and may lie past this one's rows
     for (int r = a.group_offsets[E] + (int)threadIdx.x; r < a.rows; r += blockDim.x)
         a.ig_gu[r] = a.ig_gu[a.rows + r] = a.ig_dn[r] = 0.0f;
     // pass_tokens = 0: groups are not cut, and come in any order
-    const auto full = [&](int cnt) { return P ? cnt / P : 0; };
-    const auto rest = [&](int cnt) { return P ? cnt % P : cnt; };
-    const auto rest_class = [&](int cnt) { return P ? P - cnt % P : 0; };
-    if (a.gu_jobs != nullptr) {
-        for (int e = a.expert_begin + threadIdx.x; e < a.expert_end; e += blockDim.x) {
-            const int cnt = a.group_offsets[e + 1] - a.group_offsets[e];
-            if (full(cnt)) atomicAdd(&s_class[0], full(cnt));
-            if (rest(cnt)) atomicAdd(&s_class[rest_class(cnt)], 1);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int run = 0;
-            for (int k = 0; k < Q4_PASS_TOKENS; k++) { const int c = s_class[k]; s_class[k] = run; run += c; }
-            a.n_jobs[0] = 2 * run;
-            a.n_jobs[1] = run;
-        }
-        __syncthreads();
+    const int nfull = a.pass_tokens ? cnt / P : 0, rest = a.pass_tokens ? cnt % P : cnt, k_rest = a.pass_tokens ? (P - rest) % P : 0;
+    const bool jobs = a.gu_jobs != nullptr && local && cnt > 0;
+    if (jobs) {
+        if (nfull) atomicAdd(&s_count[0], nfull);
+        if (rest) atomicAdd(&s_count[k_rest], 1);
     }
-    for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        const int g0 = a.group_offsets[e], cnt = a.group_offsets[e + 1] - g0;
-        const bool local = e >= a.expert_begin && e < a.expert_end;
-        Fp4ExpertDesc d;
-        if (local) d = a.experts[e - a.expert_begin];
-        if (local && a.gu_jobs != nullptr) {
-            const int nfull = full(cnt), first = nfull ? atomicAdd(&s_class[0], nfull) : 0;
-            for (int p = 0; p < nfull + (rest(cnt) ? 1 : 0); p++) {
-                const int slot = p < nfull ? first + p : atomicAdd(&s_class[rest_class(cnt)], 1);
+    __syncthreads();
+    if (threadIdx.x == 0 && a.gu_jobs != nullptr) {
+        int run = 0;
+        for (int k = 0; k < P; k++) run += s_count[k];
+        a.n_jobs[0] = 2 * run;
+        a.n_jobs[1] = run;
+    }
+    if (e < E) {
+        if (jobs) {
+            const int first = nfull ? atomicAdd(&s_next[0], nfull) : 0;
+            int last = rest ? atomicAdd(&s_next[k_rest], 1) : 0;
+            for (int k = 0; k < k_rest; k++) last += s_count[k];
+            for (int p = 0; p < nfull + (rest ? 1 : 0); p++) {
+                const int slot = p < nfull ? first + p : last;
                 const size_t row = (size_t)g0 + (size_t)p * P;
                 Fp4Job j;
-                j.ntok = p < nfull ? P : rest(cnt);
+                j.ntok = p < nfull ? P : rest;
                 j.R = a.inter; j.C = a.hidden; j.x_stride = a.hidden; j.y_stride = a.inter;
                 j.codes = d.codes[0]; j.scales = d.scales[0]; j.wg = d.wg[0];
                 j.x = a.dq_gu + row * a.hidden; j.y = a.gate_out + row * a.inter;
@@ -261,8 +261,8 @@ __global__ void __launch_bounds__(128) nvfp4_moe_plan_kernel(Fp4PlanArgs a) {
 }
 
 cudaError_t launch_nvfp4_moe_plan(const Fp4PlanArgs& a, cudaStream_t stream) {
-    if (a.pass_tokens < 0 || a.pass_tokens > Q4_PASS_TOKENS) return cudaErrorInvalidValue;
-    return launch_pdl(nvfp4_moe_plan_kernel, dim3(1), dim3(128), 0, stream, a);
+    if ((a.pass_tokens != 0 && a.pass_tokens != Q4_PASS_TOKENS) || a.n_experts < 1 || a.n_experts > 1024) return cudaErrorInvalidValue;
+    return launch_pdl(nvfp4_moe_plan_kernel, dim3(1), dim3((a.n_experts + 31) & ~31), 0, stream, a);
 }
 
 cudaError_t launch_nvfp4_jobs(const Fp4Job* jobs, int njobs, int max_rows, int max_tok, int C, bool aligned,

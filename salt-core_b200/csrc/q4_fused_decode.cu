@@ -463,14 +463,14 @@ static __host__ __device__ __forceinline__ LayerScratch layer_scratch(int H, int
     L.pes = 3 * h64;                             // the layer's per-expert scales ...
     L.lit = L.pes + ((E + 3) & ~3);              // ... and literal-dequantisation flags, fetched before the grid dependency
     L.topk = L.lit + ((E + 3) & ~3);
-    L.scan = L.topk + topk_scratch_floats(E, topk);
-    L.end = L.scan + POSSUM_SCRATCH;
+    L.scan = L.topk + topk_scratch_floats(E, topk);       // a multiple of four floats, as all before it
+    L.end = L.scan + ORDERED_SCRATCH;
     return L;
 }
 
-// one copy of the in-order sum for both of its uses (less code for the SM to fetch)
-static __device__ __noinline__ float layer_ordered_sum(const float* sq, int n, bool bad, uint32_t* scan) {
-    return ordered_sum_of_squares<LAYER_NV>(sq, n, bad, scan);
+// one copy of the in-order sum for its three uses (less code for the SM to fetch)
+static __device__ __noinline__ float layer_ordered_sum(float* p, int n, int rounds, uint32_t* scan) {
+    return block_sum_ordered(p, n, rounds, scan);
 }
 
 // One layer by the whole grid.  STACKED = false: the body of q4_layer_decode_kernel (one launch per layer; the
@@ -579,7 +579,7 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
                 bad |= !finite_f(v[j]) || !finite_f(nw[j]);
             }
         }
-        const float ss = layer_ordered_sum(sq, H, bad, scan);
+        const float ss = layer_ordered_sum(sq, H, 1, scan);
         if (tid == 0) {
             s_inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)H), a.eps_norm));
             if (!finite_f(s_inv)) flag(a.f.status, SB_ERR_NONFINITE);
@@ -611,7 +611,7 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
         }
     }
     {
-        const float ss = layer_ordered_sum(sq, H, bad, scan);
+        const float ss = layer_ordered_sum(sq, H, 1, scan);
         if (tid == 0) {
             s_inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)H), a.eps_router));
             if (!finite_f(s_inv) || !finite_f(s_root)) flag(a.f.status, SB_ERR_NONFINITE);
@@ -628,11 +628,8 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
     }
     if (bad) flag(a.f.status, SB_ERR_NONFINITE);
     // ---- router logits: expert e = cta, cta + grid, ...: acc = fl(acc + fl(W[c] * rin[c])), c ascending (reference
-    // src/kernels.c:98-106).  Every thread leaves the products of its columns, one warp adds them (a product of +0 past
-    // the last column changes nothing: a sum that starts at +0 is never -0).  The products in one warp's registers, the
-    // sum handed from lane to lane, took 16800 cycles where this takes 13700 ----
+    // src/kernels.c:98-106).  Every thread leaves the products of its columns, the block adds them as it adds squares ----
     uint32_t ph_w = 0;
-    const int H64 = (H + 63) & ~63;
     for (int e = cta; e < E; e += ncta) {
         if (e != cta) {
             __syncthreads();               // the row and the products of the expert before are no longer read
@@ -647,15 +644,12 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
 #pragma unroll
         for (int j = 0; j < NV; j++) {
             const int d = tid + j * NT;
-            if (d < H64) prod[d] = d < H ? __fmul_rn(wrow[d], v[j]) : 0.0f;
+            if (d < H) prod[d] = __fmul_rn(wrow[d], v[j]);
         }
-        __syncthreads();
-        if (warp == 0) {
-            const float acc = chain_sum(prod, H64);
-            if (lane == 0) {
-                a.logits[e] = acc;
-                asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(a.logits_count) : "memory");
-            }
+        const float acc = layer_ordered_sum(prod, H, 2, scan);
+        if (tid == 0) {
+            a.logits[e] = acc;
+            asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(a.logits_count) : "memory");
         }
     }
     // ---- all logits, then top-k and the job list, by every block for itself ----

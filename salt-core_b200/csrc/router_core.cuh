@@ -3,6 +3,7 @@
 #pragma once
 #include "bitmath.cuh"
 #include "internal.h"
+#include "q4_core.cuh"
 
 namespace sb {
 
@@ -63,231 +64,261 @@ static __device__ __forceinline__ float serial_sum(const float* sq, int n) {
     return ss;
 }
 
-// The same sum - S = 0; S = fl(S + sq[i]) for i = 0..n-1, bit for bit - by the whole
-// block, for terms that are all finite and >= +0 (squares).
+// The same sum - s = 0; s = fl(s + p[i]) for i = 0..n-1, bit for bit - by the whole block, for any terms.
 //
-// While the running sum stays inside one binade, every partial sum is a multiple of that
-// binade's ulp u, and fl(S + p) = S + (p rounded to a multiple of u): the roundings no
-// longer depend on S, so the increments are integers that can be added in any order.
-// Only two kinds of element need the real running sum: one whose addition may leave the
-// binade, and a term exactly half-way between two multiples of u (its rounding goes to
-// the even neighbour of the running sum).
+// The terms are cut into 32 segments.  A chain of additions cannot be cut, but what a segment makes of its starting value can
+// be tabulated: the segment's real additions are run from ORDERED_CANDS candidates, spaced by g around a predicted start,
+// and the exact running sum then only has to pick its candidate, segment after segment.
 //
-//   1. an approximate prefix sum A (parallel float scan) PREDICTS the binade of the running
-//      sum before and after every element;
-//   2. an element is "certain" when A stays inside one binade across it, away from the
-//      binade's ends, and the term is not a half-way case; all other elements are "serial
-//      points".  Consecutive certain elements share one binade, so their integer increments
-//      add up exactly (64-bit scan);
-//   3. one warp walks the serial points in order: for the run of certain elements before
-//      each point it CHECKS that the exact running sum really is in the predicted binade
-//      and stays there (else it adds that run element by element), adds the run's integer
-//      total, then performs the serial point's addition in floating point.
-// The prediction only decides how much work is parallel; every step of the exact sum is
-// either an integer identity that was checked or a real floating-point addition.  A typical
-// row of a few thousand squares has ~20 serial points.  The first 64 terms (where the sum
-// doubles every few steps) are added serially, and so is everything when the serial
-// points exceed the list (half-way cases everywhere, subnormal sums).
+//   1. sums in any order predict the running sum at every quarter of a segment.  In a second round the real additions of a
+//      quarter from there add up to better predictions, as they leave out what the chain's roundings leave out: sums with
+//      terms of both signs need them (half as many looks without an answer, below), squares do not;
+//   2. lane t of three warps runs segment t from five or six candidates each, with g = the larger of ulp(start) and u / 8 (u: the unit
+//      of the last place of the largest sum seen at the segment's quarters).  A fourth warp runs it from two sentinels well
+//      outside the candidates and sees whether the two stay in the same binades, step by step, and in which at most.  As
+//      additions are monotone, a path that starts between the sentinels then stays in those binades too;
+//   3. the running sum s is start + q g.  Where q is one of -8 .. 7 the candidate IS s.  Otherwise the candidate 16 k g away
+//      from s stands for it, if both lie between sentinels that stayed together and 16 g is an even number of units of the
+//      last place everywhere in the segment: both paths then round alike, half-way cases too, and stay 16 k g apart;
+//   4. one warp per four segments makes a table of them together (its candidates are the first one's, and so are its
+//      sentinels, which must pass between the sentinels of the others); one warp walks the eight tables from s = 0.  Where a
+//      table has no answer it takes the four segments one by one, and where a segment has none, term by term.
+// So the predictions decide only how much runs side by side: every result is a real addition of the chain, or one shifted
+// by an amount that is proven to pass through it.  Just under 1 % of the segments of a router row have no answer (mostly
+// where the sum passes zero and its binade changes with every step), hardly any of squares.
+// What bounds it: the additions of 2 (n / 32 dependent ones, six side by side, about 10 cycles each), those of segments
+// without an answer (600 cycles each with what it takes to get there), 60 to 130 cycles per look into a table, five or six barriers
+// with a scan or two between them.  Measured in a block of 640 threads (B200): 2816 squares 4000 cycles, where integer increments
+// between the points at which the sum changes its binade took 7500; 2816 products 5200 on average, where one warp's chain took
+// 13 700; 5120 of them 5800 (25 000).  32 candidates with more warps, or one segment per warp with a candidate per lane, were
+// slower: loads of the terms took the time.
 //
-// Needs blockDim.x * V >= n (V = elements per thread) and blockDim.x a multiple of 32.  scratch: POSSUM_SCRATCH words
-// of shared memory.  Every thread of the block must call; all return the sum.
-constexpr int POSSUM_V = 4, POSSUM_HEAD = 64, POSSUM_NS = 192;
-constexpr int POSSUM_SCRATCH = 8 + 32 + 32 + 64 + 32 + POSSUM_NS * 4 + 96;
+// p and scratch (ORDERED_SCRATCH words): shared memory, 16-byte aligned; p written by the block, no barrier needed before the
+// call.  At least 256 threads, whole warps; every thread of the block must call; all return the sum.
+constexpr int ORDERED_CANDS = 16;
+constexpr int ORDERED_PITCH = 20;                         // floats per table: candidates' ends, the sentinels', bank offset
+constexpr int ORDERED_GROUP = 4, ORDERED_GROUPS = 32 / ORDERED_GROUP;
+constexpr int ORDERED_SCRATCH = 8 + 2 * 4 * 32 + 4 * 32 + 2 * 32 + 32 + 2 * ORDERED_GROUPS + (32 + ORDERED_GROUPS) * ORDERED_PITCH;
 
-template <int V = POSSUM_V>
-static __device__ float block_sum_nonneg(const float* sq, int n, uint32_t* scratch) {
-    constexpr uint32_t MARGIN = 1u << 13;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-    float* fs = (float*)(scratch + 8);                 // [32] warp totals of the float scan
-    float* flast = (float*)(scratch + 40);             // [32] last inclusive value of each warp
-    unsigned long long* ws = (unsigned long long*)(scratch + 72);   // [32] warp totals of the integer scan
-    uint32_t* wc = scratch + 136;                      // [32] warp counts of serial points
-    uint32_t* sp_k = scratch + 168;                    // [NS] index of serial point
-    uint32_t* sp_e = sp_k + POSSUM_NS;                 // [NS] predicted exponent field after it
-    unsigned long long* sp_i = (unsigned long long*)(sp_e + POSSUM_NS);   // [NS] integer prefix at it
-    uint2* pt_run = (uint2*)(sp_i + POSSUM_NS);         // [32] runs of the batch being walked: bits to add, binade
-    float* pt_term = (float*)(pt_run + 32);            // [32] ... and the terms after them
-    const int base = tid * V;
-
-    // ---- 1. approximate inclusive prefix sums
-    float p[V], loc[V];
-    float run = 0.0f;
-#pragma unroll
-    for (int j = 0; j < V; j++) {
-        p[j] = base + j < n ? sq[base + j] : 0.0f;
-        run += p[j];
-        loc[j] = run;
-    }
-    float inc_s = run;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const float t = __shfl_up_sync(0xffffffffu, inc_s, off);
-        if (lane >= off) inc_s += t;
-    }
-    if (lane == 31) fs[warp] = inc_s;
-    __syncthreads();
-    float wt = lane < nw ? fs[lane] : 0.0f;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const float t = __shfl_up_sync(0xffffffffu, wt, off);
-        if (lane >= off) wt += t;
-    }
-    const float woff = warp ? __shfl_sync(0xffffffffu, wt, warp - 1) : 0.0f;
-    const float incl_t = woff + inc_s;                 // this thread's last inclusive value
-    if (lane == 31) flast[warp] = incl_t;
-    __syncthreads();
-    // value before this thread's first element = the previous thread's last inclusive value, bit for bit
-    float before = __shfl_up_sync(0xffffffffu, incl_t, 1);
-    if (lane == 0) before = warp ? flast[warp - 1] : 0.0f;
-
-    // ---- 2. classify, integer increments
-    unsigned long long isum = 0;        // increments of this thread's certain elements so far
-    uint32_t nser = 0, ser_mask = 0;
-    unsigned long long ser_i[V];
-    uint32_t ser_e[V];
-    float a_before = before;
-#pragma unroll
-    for (int j = 0; j < V; j++) {
-        const int k = base + j;
-        const float a_after = j == V - 1 ? incl_t : before + loc[j];
-        const uint32_t bb = __float_as_uint(a_before), ab = __float_as_uint(a_after);
-        ser_i[j] = 0; ser_e[j] = 0;
-        if (k >= POSSUM_HEAD && k < n) {
-            const uint32_t Eb = bb >> 23, Ea = ab >> 23;
-            const uint32_t pb = __float_as_uint(p[j]);
-            const uint32_t Ep = max(pb >> 23, 1u);
-            const uint32_t m = (pb & 0x7fffffu) | ((pb >> 23) ? 0x800000u : 0u);
-            bool certain = Eb == Ea && Eb >= 1u && Eb < 255u && (bb & 0x7fffffu) >= MARGIN &&
-                           (ab & 0x7fffffu) <= 0x7fffffu - MARGIN && Ep <= Eb;
-            uint32_t inc = 0;
-            if (certain) {
-                const uint32_t sh = Eb - Ep;
-                if (sh == 0) {
-                    inc = m;
-                } else if (sh <= 24) {
-                    const uint32_t rem = m & ((1u << sh) - 1u), half = 1u << (sh - 1);
-                    inc = (m >> sh) + (rem > half ? 1u : 0u);
-                    certain = rem != half;
-                }                                    // sh > 24: below half an ulp, adds nothing
-            }
-            if (certain) {
-                isum += inc;
-            } else {
-                ser_mask |= 1u << j;
-                ser_i[j] = isum;
-                ser_e[j] = Ea;
-                nser++;
-            }
-        }
-        if (k == POSSUM_HEAD - 1) scratch[2] = ab >> 23;   // predicted exponent field after the serial head
-        a_before = a_after;
-    }
-
-    // ---- 3. scan of (integer increments, serial point count)
-    unsigned long long si = isum;
-    uint32_t sc = nser;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const unsigned long long ti = __shfl_up_sync(0xffffffffu, si, off);
-        const uint32_t tc = __shfl_up_sync(0xffffffffu, sc, off);
-        if (lane >= off) { si += ti; sc += tc; }
-    }
-    if (lane == 31) { ws[warp] = si; wc[warp] = sc; }
-    __syncthreads();
-    unsigned long long wi = lane < nw ? ws[lane] : 0ull;
-    uint32_t wcn = lane < nw ? wc[lane] : 0u;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const unsigned long long ti = __shfl_up_sync(0xffffffffu, wi, off);
-        const uint32_t tc = __shfl_up_sync(0xffffffffu, wcn, off);
-        if (lane >= off) { wi += ti; wcn += tc; }
-    }
-    const unsigned long long ioff = (warp ? __shfl_sync(0xffffffffu, wi, warp - 1) : 0ull) + (si - isum);
-    uint32_t slot = (warp ? __shfl_sync(0xffffffffu, wcn, warp - 1) : 0u) + (sc - nser);
-    const uint32_t ns = __shfl_sync(0xffffffffu, wcn, nw - 1);
-    const unsigned long long itotal = __shfl_sync(0xffffffffu, wi, nw - 1);
-#pragma unroll
-    for (int j = 0; j < V; j++)
-        if (ser_mask & (1u << j)) {
-            if (slot < (uint32_t)POSSUM_NS) {
-                sp_k[slot] = (uint32_t)(base + j);
-                sp_e[slot] = ser_e[j];
-                sp_i[slot] = ioff + ser_i[j];
-            }
-            slot++;
-        }
-    __syncthreads();
-
-    // ---- 4. the exact walk, by warp 0.  Lane j of a batch of 32 points prepares point j: the run of certain elements before
-    // it as ONE integer to add to the bits of the running sum (adding units of the last place is adding to the bits while
-    // the binade lasts), with the binade it needs, and the point's own term.  The chain, which all lanes run alike, is then
-    // one integer and one floating-point addition per point; the binades are checked beside it, and a batch with a wrong
-    // prediction is walked again, run by run.  (The points go through shared memory: a shuffle in a loop whose length the
-    // compiler does not know to be the same for all lanes took up to 240 cycles, three of them per point.)
-    if (warp == 0) {
-        float S;
-        if (ns > (uint32_t)POSSUM_NS || n <= POSSUM_HEAD) {
-            S = serial_sum(sq, n);
-        } else {
-            S = (((uintptr_t)sq) & 15) == 0 ? chain_sum(sq, POSSUM_HEAD) : serial_sum(sq, POSSUM_HEAD);
-            const uint32_t E0 = scratch[2];
-            for (uint32_t base0 = 0; base0 <= ns; base0 += 32) {
-                const uint32_t mine = base0 + (uint32_t)lane;
-                if (mine <= ns) {
-                    const int idx = mine < ns ? (int)sp_k[mine] : n, from = mine ? (int)sp_k[mine - 1] + 1 : POSSUM_HEAD;
-                    const unsigned long long tot = (mine < ns ? sp_i[mine] : itotal) - (mine ? sp_i[mine - 1] : 0ull);
-                    const uint32_t bin = (mine ? sp_e[mine - 1] : E0) << 23;
-                    const bool some = idx > from;
-                    pt_run[lane] = make_uint2(some ? (uint32_t)(tot < 0xffffffull ? tot : 0xffffffull) : 0u, some ? bin : 0xffffffffu);
-                    pt_term[lane] = mine < ns ? sq[idx] : 0.0f;              // past the last point: + 0
-                }
-                __syncwarp();
-                const int cnt = (int)min(32u, ns + 1u - base0);
-                float F = S;
-                uint32_t off = 0;                        // bits in which a run's ends differ from its predicted binade
-#pragma unroll 4
-                for (int j = 0; j < cnt; j++) {
-                    const uint2 r = pt_run[j];
-                    const uint32_t b0 = __float_as_uint(F), b1 = b0 + r.x;
-                    off |= r.y != 0xffffffffu ? (b0 ^ r.y) | (b1 ^ r.y) : 0u;
-                    F = __fadd_rn(__uint_as_float(b1), pt_term[j]);
-                }
-                if (off < 0x800000u) {
-                    S = F;
-                } else {
-                    for (int j = 0; j < cnt; j++) {
-                        const uint2 r = pt_run[j];
-                        const uint32_t b0 = __float_as_uint(S), b1 = b0 + r.x, jx = base0 + (uint32_t)j;
-                        if (((b0 ^ r.y) | (b1 ^ r.y)) < 0x800000u) {
-                            S = __uint_as_float(b1);
-                        } else {                                             // no run, or the prediction missed
-                            const int idx = jx < ns ? (int)sp_k[jx] : n;
-                            for (int i = jx ? (int)sp_k[jx - 1] + 1 : POSSUM_HEAD; i < idx; i++) S = __fadd_rn(S, sq[i]);
-                        }
-                        S = __fadd_rn(S, pt_term[j]);
-                    }
-                }
-                __syncwarp();
-            }
-        }
-        if (lane == 0) scratch[0] = __float_as_uint(S);
-    }
-    __syncthreads();
-    return __uint_as_float(scratch[0]);
+static __device__ __forceinline__ uint32_t shared_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+static __device__ __forceinline__ float4 shared_f4(uint32_t at) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+    return v;
+}
+static __device__ __forceinline__ float2 shared_f2(uint32_t at) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at));
+    return v;
+}
+static __device__ __forceinline__ float shared_f(uint32_t at) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at));
+    return v;
 }
 
-// Sum of the squares in sq[0..n) in element order.  `bad` = this thread saw a non-finite
-// input; then (for any thread) the serial chain runs so that NaN / Inf propagate as in
-// the reference.  Every thread of the block must call; all return the sum.
-template <int V = POSSUM_V>
-static __device__ __forceinline__ float ordered_sum_of_squares(const float* sq, int n, bool bad, uint32_t* scratch) {
-    const bool serial = (int)blockDim.x * V < n || (blockDim.x & 31u);
-    if (__syncthreads_or(bad) || serial) {   // the barrier also orders the writes of sq before the reads below
-        if (threadIdx.x == 0) scratch[0] = __float_as_uint(serial_sum(sq, n));
-        __syncthreads();
-        return __uint_as_float(scratch[0]);
+// term(v.x), term(v.y), ... for the `mine` pieces of four floats at `at` and zeros up to a multiple of four of `pieces` or
+// more: four pieces are loaded while the four before them are used.  The same trips for all lanes and no branch inside: lanes
+// that part company in a loop are slow to meet again, and one by one they take 32 times as long.
+template <class Term>
+static __device__ __forceinline__ void for_terms(uint32_t at, uint32_t zeros, int mine, int pieces, Term term) {
+    float4 a[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) a[j] = shared_f4(j < mine ? at + 16 * j : zeros);
+#pragma unroll 2
+    for (int i = 0; i < pieces; i += 4) {
+        float4 b[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) b[j] = shared_f4(i + 4 + j < mine ? at + 16 * (i + 4 + j) : zeros);
+#pragma unroll
+        for (int j = 0; j < 4; j++) { term(a[j].x); term(a[j].y); term(a[j].z); term(a[j].w); }
+#pragma unroll
+        for (int j = 0; j < 4; j++) a[j] = b[j];
     }
-    return block_sum_nonneg<V>(sq, n, scratch);
+}
+
+// ulp of a float with these exponent bits (0x7f800000 & bits); 0 where that is no normal number
+static __device__ __forceinline__ float ulp_of(uint32_t exponent) {
+    return exponent > (23u << 23) ? __uint_as_float(exponent - (23u << 23)) : 0.0f;
+}
+static __device__ __forceinline__ uint32_t exponent_of(float v) { return __float_as_uint(v) & 0x7f800000u; }
+
+// A look into one table: seg = start, g, 1 / g; between = sentinels (none: empty).  s becomes the sum behind the segment.
+// inside: s has to lie between the sentinels even where it is a candidate.  No branches.
+static __device__ __forceinline__ bool ordered_step(float& s, const float4& seg, const float2& between, uint32_t ends, bool inside) {
+    constexpr float MAGIC = 12582912.0f + ORDERED_CANDS / 2;          // q + MAGIC has q + CANDS / 2 in its low bits
+    const float d = __fsub_rn(s, seg.x), m = __fmaf_rn(d, seg.z, MAGIC);
+    const uint32_t k = __float_as_uint(m) & (ORDERED_CANDS - 1);
+    const float end = shared_f(ends + 4 * k);
+    const float from = __fmaf_rn(__fsub_rn(__uint_as_float(0x4b000000u | k), 8388608.0f + ORDERED_CANDS / 2), seg.y, seg.x);
+    const float shift = __fsub_rn(s, from);
+    const int in = (int)(between.x <= s) & (int)(s <= between.y);
+    const int whole = (int)(__fsub_rn(m, MAGIC) == __fmul_rn(d, seg.z));
+    s = __fadd_rn(end, shift);
+    return ((int)(shift == 0.0f) | (in & whole)) & (in | (int)!inside) & (int)(s == s);
+}
+
+static __device__ __forceinline__ float block_sum_ordered(float* p, int n, int rounds, uint32_t* scratch) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // words of scratch: zeros [4], result [4], sums of the segments' quarters [2][4][32], seg [32] (start, g, 1 / g, first piece << 16 | pieces), sentinels
+    // [32][2], largest unit of the last place [32], sentinels of the groups [GROUPS][2], ends [32][PITCH], of groups [GROUPS][PITCH]
+    constexpr int RESULT = 4, QUARTER = 8, SEG = QUARTER + 2 * 4 * 32, BETWEEN = SEG + 4 * 32, UNIT = BETWEEN + 2 * 32, GBETWEEN = UNIT + 32,
+                  ENDS = GBETWEEN + 2 * ORDERED_GROUPS, GENDS = ENDS + 32 * ORDERED_PITCH;
+    static_assert(GENDS + ORDERED_GROUPS * ORDERED_PITCH == ORDERED_SCRATCH && ENDS % 4 == 0 && SEG % 4 == 0, "scratch");
+    float* const sf = (float*)scratch;
+    const uint32_t base = shared_at(scratch), zeros = base, terms = shared_at(p);
+    // segments of an odd number of 16-byte pieces: the lanes read other banks
+    const int pieces = ((n + 127) >> 7) | 1, all = (n + 3) >> 2;
+    if (threadIdx.x < 4) {
+        sf[threadIdx.x] = 0.0f;
+        if (n + (int)threadIdx.x < 4 * all) p[n + threadIdx.x] = 0.0f;
+    }
+    __syncthreads();
+    // ---- 1. predictions: sums of the segments' quarters, from zero and then from where those predict them to start
+    float q0, q1, q2, q3, start;                          // the segment's quarters, summed up; its start
+    auto predict = [&](int table) {
+        const float* q = sf + QUARTER + 128 * table + lane;
+        q0 = q[0]; q1 = q0 + q[32]; q2 = q1 + q[64]; q3 = q2 + q[96];
+        start = q3;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float t = __shfl_up_sync(0xffffffffu, start, o);
+            start += lane >= o ? t : 0.0f;
+        }
+        start = __shfl_up_sync(0xffffffffu, start, 1);
+        start = lane == 0 ? 0.0f : start;
+    };
+    const int quarter = (pieces + 3) >> 2;
+#pragma unroll 1
+    for (int table = 0; table < rounds; table++) {
+        if (warp < 4) {
+            float r0 = 0.0f;
+            if (table != 0) {
+                predict(0);
+                r0 = start + (warp < 2 ? (warp == 0 ? 0.0f : q0) : (warp == 2 ? q1 : q2));
+            }
+            const int first = lane * pieces + warp * quarter;
+            float r = r0;
+            for_terms(terms + 16 * first, zeros, min(all - first, min(quarter, pieces - warp * quarter)), quarter, [&](float t) { r = __fadd_rn(r, t); });
+            sf[QUARTER + 128 * table + 32 * warp + lane] = r - r0;
+        }
+        __syncthreads();
+    }
+    // ---- 2. candidates and sentinels
+    if (warp < 4) {
+        predict(rounds - 1);
+        // a segment that would start far below the values it reaches has no good candidates: it starts a quarter later
+        const float inner = fmaxf(fmaxf(fabsf(start + q0), fabsf(start + q1)), fmaxf(fabsf(start + q2), fabsf(start + q3)));
+        const bool late = lane > 0 && fabsf(start) < 0.125f * inner && fabsf(start) < fabsf(start + q0);
+        const uint32_t lates = __ballot_sync(0xffffffffu, late) >> lane;
+        const int begin = lane * pieces + (lates & 1u ? quarter : 0);
+        const int count = min(lane * pieces + pieces + (lates & 2u ? quarter : 0), all) - begin, trips = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(count, 0));
+        start = late ? start + q0 : start;
+        const float next = __shfl_down_sync(0xffffffffu, start, 1);
+        const float u = ulp_of(exponent_of(fmaxf(inner, fmaxf(fabsf(start), lane < 31 ? fabsf(next) : 0.0f))));
+        const uint32_t from = terms + 16 * begin;
+        float g = fmaxf(ulp_of(exponent_of(start)), u * (2.0f / ORDERED_CANDS));
+        g = g >= 1.0e-36f && g <= 1.0e36f ? g : 0.0f;     // 1 / g is exact: g is a power of two
+        if (warp < 3) {
+            static_assert(ORDERED_CANDS == 16, "candidates 0..5, 5..10, 10..15: a scheduler each, the sentinels on the fourth");
+            float s[6];
+#pragma unroll
+            for (int i = 0; i < 6; i++) s[i] = __fmaf_rn((float)(5 * warp + i - ORDERED_CANDS / 2), g, start);
+            for_terms(from, zeros, count, trips, [&](float t) {
+#pragma unroll
+                for (int i = 0; i < 6; i++) s[i] = __fadd_rn(s[i], t);
+            });
+#pragma unroll
+            for (int i = 0; i < 6; i++) sf[ENDS + lane * ORDERED_PITCH + 5 * warp + i] = s[i];
+        } else {
+            // 128 u: several times what the roundings of a few thousand terms add up to, a small part of a binade.  Those that
+            // have to pass between the sentinels of the segments behind start closer.
+            const float w = lane % ORDERED_GROUP == 0 ? (rounds == 1 ? 64.0f : 32.0f) : 128.0f, lo0 = start - w * u, hi0 = start + w * u;
+            float lo = lo0, hi = hi0, top = fabsf(hi0);
+            uint32_t differ = __float_as_uint(lo) ^ __float_as_uint(hi);
+            for_terms(from, zeros, count, trips, [&](float t) {
+                lo = __fadd_rn(lo, t);
+                hi = __fadd_rn(hi, t);
+                differ |= __float_as_uint(lo) ^ __float_as_uint(hi);
+                top = fmaxf(top, fabsf(hi));
+            });
+            const float most = ulp_of(exponent_of(top));
+            const bool together = (differ & 0xff800000u) == 0u && exponent_of(top) != 0x7f800000u && most > 0.0f && g * ORDERED_CANDS >= 2.0f * most;
+            *(float4*)(sf + SEG + 4 * lane) = make_float4(start, g, g > 0.0f ? __uint_as_float(0x7f000000u - __float_as_uint(g)) : 0.0f, __int_as_float(begin << 16 | max(count, 0)));
+            *(float2*)(sf + BETWEEN + 2 * lane) = together ? make_float2(lo0, hi0) : make_float2(1.0f, -1.0f);
+            sf[UNIT + lane] = together ? most : __uint_as_float(0x7f800000u);
+            *(float2*)(sf + ENDS + lane * ORDERED_PITCH + ORDERED_CANDS) = make_float2(lo, hi);
+        }
+    }
+    __syncthreads();
+    // ---- 3. tables of four segments
+    if (warp < ORDERED_GROUPS) {
+        const int t0 = warp * ORDERED_GROUP, k = min(lane, ORDERED_CANDS + 1);
+        const bool sentinel = lane >= ORDERED_CANDS;
+        const uint32_t at = base + 4 * (SEG + 4 * t0), bt = base + 4 * (BETWEEN + 2 * t0), et = base + 4 * (ENDS + t0 * ORDERED_PITCH);
+        float s = shared_f(et + 4 * k);
+        float4 seg[ORDERED_GROUP];
+        float2 between[ORDERED_GROUP];
+#pragma unroll
+        for (int i = 0; i < ORDERED_GROUP; i++) {
+            seg[i] = shared_f4(at + 16 * i);
+            between[i] = shared_f2(bt + 8 * i);
+        }
+        const float4 unit = shared_f4(base + 4 * (UNIT + t0));
+        int ok = (int)!sentinel | (int)(between[0].x <= between[0].y);
+#pragma unroll
+        for (int i = 1; i < ORDERED_GROUP; i++) ok &= (int)ordered_step(s, seg[i], between[i], et + 4 * ORDERED_PITCH * i, sentinel);
+        const float most = fmaxf(fmaxf(unit.x, unit.y), fmaxf(unit.z, unit.w));
+        const bool together = __all_sync(0xffffffffu, ok | (int)!sentinel) && seg[0].y * ORDERED_CANDS >= 2.0f * most;
+        if (lane < ORDERED_CANDS) sf[GENDS + warp * ORDERED_PITCH + lane] = ok ? s : __uint_as_float(0x7fffffffu);
+        if (lane == 0) *(float2*)(sf + GBETWEEN + 2 * warp) = together ? between[0] : make_float2(1.0f, -1.0f);
+    }
+    __syncthreads();
+    // ---- 4. the walk.  Squares: as if every look had its answer.  Else, and if one has not: what the next look needs is loaded
+    // while this one waits for its table
+    if (threadIdx.x == 0) {
+        float s = 0.0f;
+        bool all_known = rounds == 1;
+        if (rounds == 1) {
+#pragma unroll
+            for (int i = 0; i < ORDERED_GROUPS; i++)
+                all_known &= ordered_step(s, shared_f4(base + 4 * (SEG + 4 * ORDERED_GROUP * i)), shared_f2(base + 4 * (GBETWEEN + 2 * i)),
+                                          base + 4 * (GENDS + i * ORDERED_PITCH), false);
+            if (!all_known) s = 0.0f;
+        }
+        float4 seg = shared_f4(base + 4 * SEG);
+        float2 lohi = shared_f2(base + 4 * GBETWEEN);
+#pragma unroll 1
+        for (int i = all_known ? ORDERED_GROUPS : 0; i < ORDERED_GROUPS; i++) {
+            const int t0 = ORDERED_GROUP * i, n0 = min(t0 + ORDERED_GROUP, 31), ni = min(i + 1, ORDERED_GROUPS - 1);
+            const float4 next_seg = shared_f4(base + 4 * (SEG + 4 * n0));
+            const float2 next_lohi = shared_f2(base + 4 * (GBETWEEN + 2 * ni));
+            float after = s;
+            if (!ordered_step(after, seg, lohi, base + 4 * (GENDS + i * ORDERED_PITCH), false)) {
+                float2 own = shared_f2(base + 4 * (BETWEEN + 2 * t0));
+#pragma unroll 1
+                for (int t = t0; t < t0 + ORDERED_GROUP; t++) {
+                    const float4 one_seg = shared_f4(base + 4 * (SEG + 4 * min(t + 1, 31)));
+                    const float2 one_own = shared_f2(base + 4 * (BETWEEN + 2 * min(t + 1, 31)));
+                    after = s;
+                    if (!ordered_step(after, seg, own, base + 4 * (ENDS + t * ORDERED_PITCH), false)) {
+                        after = s;
+                        const int at = __float_as_int(seg.w), count = at & 0xffff;
+                        for_terms(terms + 16 * (at >> 16), zeros, count, count, [&](float v) { after = __fadd_rn(after, v); });
+                    }
+                    s = after;
+                    seg = one_seg;
+                    own = one_own;
+                }
+            }
+            s = after;
+            seg = next_seg;
+            lohi = next_lohi;
+        }
+        sf[RESULT] = s;
+    }
+    __syncthreads();
+    return sf[RESULT];
 }
 
 // Softmax top-k (gemma4.c:132-186) + ascending-expert ordering of the selected

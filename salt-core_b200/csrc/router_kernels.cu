@@ -2,16 +2,17 @@
 //
 // Everything here is bit-exact against the reference CPU functions; the reference arithmetic
 // contains several chains that are serial by definition (sums of squares, router logits,
-// softmax denominators).  Signed chains (logits, denominators) are kept serial per row / expert,
-// with the independent products formed ahead by other lanes and many chains running side by
-// side; the sums of squares are reproduced by a predict-and-verify scheme (block_sum_nonneg)
-// that does most of the additions as order-free integer increments.
+// softmax denominators).  Many chains run side by side, each added by a lane; where few are asked for, the whole block
+// adds one (block_sum_ordered).
 #include "internal.h"
 #include "pdl.cuh"
 #include "q4_core.cuh"
 #include "router_core.cuh"
 
 namespace sb {
+
+// one copy of the in-order sum per kernel: its instructions are fetched cold, and the second sum finds them there
+static __device__ __noinline__ float row_sum_of_squares(float* p, int n, uint32_t* scratch) { return block_sum_ordered(p, n, 1, scratch); }
 
 // mode 0: RMSNorm  y = (x*inv) [* weight]             (gemma4.c:85-101)
 // mode 1: router input  y = ((x*inv)*scale)*root      (gemma4.c:103-130)
@@ -22,7 +23,7 @@ norm_rows_kernel(const float* __restrict__ x, const float* __restrict__ weight, 
     extern __shared__ __align__(16) float srow[];   // [n] row, then [n (padded to 4)] squares
     float* ssq = srow + ((n + 3) & ~3);
     __shared__ float s_inv, s_root;
-    __shared__ __align__(8) uint32_t s_scan[POSSUM_SCRATCH];
+    __shared__ __align__(16) uint32_t s_scan[ORDERED_SCRATCH];
     const float* xr = x + (size_t)blockIdx.x * n;
     float* yr = y + (size_t)blockIdx.x * n;
     bool bad = false;
@@ -33,7 +34,7 @@ norm_rows_kernel(const float* __restrict__ x, const float* __restrict__ weight, 
         bad |= !finite_f(v);
         if (MODE == 1 || with_scale) bad |= !finite_f(weight[i]);
     }
-    const float ss = ordered_sum_of_squares(ssq, n, bad, s_scan);
+    const float ss = row_sum_of_squares(ssq, n, s_scan);
     if (threadIdx.x == 0) {
         {
             const float mean = __fadd_rn(__fdiv_rn(ss, (float)n), eps);
@@ -68,7 +69,7 @@ norm_rows_kernel(const float* __restrict__ x, const float* __restrict__ weight, 
 //   [norm]    v = RMSNorm(v) * norm_w                      (gemma4.c:85-101)
 //             y_out = v  (written whenever reduce or norm ran)
 //   [router]  rin = ((v * inv) * scale) * (1/sqrt(n))      (gemma4.c:103-130)
-// The two sums of squares are formed in element order by block_sum_nonneg over
+// The two sums of squares are formed in element order by block_sum_ordered over
 // squares computed in parallel.
 // ---- affine 8-bit matvec (router projections of packages that quantise the router) -----------
 // src/kernels.c:343-369: one byte per element, bf16 scale / bias per 64 consecutive elements of
@@ -115,7 +116,7 @@ static __device__ void norm_row_block(const float* x, const float* w, float* y, 
         sq[i] = __fmul_rn(v, v);
         bad |= !finite_f(v) || !finite_f(w[i]);
     }
-    const float ss = ordered_sum_of_squares(sq, n, bad, scan);
+    const float ss = row_sum_of_squares(sq, n, scan);
     if (threadIdx.x == 0) {
         *s_inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)n), eps));
         if (!finite_f(*s_inv)) flag(status, SB_ERR_NONFINITE);
@@ -137,7 +138,7 @@ residual_postnorm_rows_kernel(const float* __restrict__ residual, const float* _
                               int* status) {
     extern __shared__ __align__(16) float cell_sm[];     // [n] squares, [n] normalised branch
     __shared__ float s_inv;
-    __shared__ __align__(8) uint32_t s_scan[POSSUM_SCRATCH];
+    __shared__ __align__(16) uint32_t s_scan[ORDERED_SCRATCH];
     const size_t row = blockIdx.x;
     float* normed = cell_sm + ((n + 3) & ~3);
     bool bad = false;
@@ -160,7 +161,7 @@ parallel_combine_rows_kernel(const float* __restrict__ residual, const float* __
                              float* scratch_b, float* __restrict__ out, int n, float eps, float scalar, int* status) {
     extern __shared__ __align__(16) float cell_sm[];     // [n] squares
     __shared__ float s_inv;
-    __shared__ __align__(8) uint32_t s_scan[POSSUM_SCRATCH];
+    __shared__ __align__(16) uint32_t s_scan[ORDERED_SCRATCH];
     const size_t row = blockIdx.x;
     float* sum = scratch_a + row * n;
     float* fin = scratch_b + row * n;
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(GLUE_NV == 4 ? 1024 : 512) glue_rows_kernel(Gl
     const int n = a.n;
     float* sq = gsm;                       // [n] squares for the ordered sums
     __shared__ float s_inv, s_root;
-    __shared__ __align__(8) uint32_t s_scan[POSSUM_SCRATCH];
+    __shared__ __align__(16) uint32_t s_scan[ORDERED_SCRATCH];
     __shared__ int s_g[64];
     __shared__ float s_w[64];
     const int row = blockIdx.x, T = blockDim.x, tid = threadIdx.x;
@@ -315,7 +316,7 @@ __global__ void __launch_bounds__(GLUE_NV == 4 ? 1024 : 512) glue_rows_kernel(Gl
                 bad |= !finite_f(v[j]) || !finite_f(nw[j]);
             }
         }
-        const float ss = ordered_sum_of_squares<GLUE_NV>(sq, n, bad, s_scan);
+        const float ss = row_sum_of_squares(sq, n, s_scan);
         if (tid == 0) {
             s_inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)n), a.eps_norm));
             if (!finite_f(s_inv)) flag(a.status, SB_ERR_NONFINITE);
@@ -345,7 +346,7 @@ __global__ void __launch_bounds__(GLUE_NV == 4 ? 1024 : 512) glue_rows_kernel(Gl
                 bad |= !finite_f(v[j]) || !finite_f(rs[j]);
             }
         }
-        const float ss = ordered_sum_of_squares<GLUE_NV>(sq, n, bad, s_scan);
+        const float ss = row_sum_of_squares(sq, n, s_scan);
         if (tid == 0) {
             s_inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)n), a.eps_router));
             if (!finite_f(s_inv) || !finite_f(s_root)) flag(a.status, SB_ERR_NONFINITE);

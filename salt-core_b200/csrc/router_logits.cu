@@ -1,11 +1,12 @@
 // Router logits, bit-exact: logits[row][e] = the reference's chain acc = fl(acc + fl(W[e][c] * x[row][c])), columns
 // ascending from +0 (reference src/kernels.c:98-106).
 //
-// A logit is a chain of H dependent adds: at 4.4 cycles each 2816 columns take 6.5 us whatever the machine, and rows x
-// experts chains are all the parallelism there is.  A warp alone on its scheduler issues in order and every shared load
+// A logit is a chain of H dependent adds: at 4.4 cycles each 2816 columns take 6.5 us, and rows x experts chains are all the
+// parallelism there is unless a chain is added in pieces, which takes several times the additions.  A warp alone on its scheduler issues in order and every shared load
 // holds it for about four cycles (measured: 4.5 cycles per column for add + multiply from registers, 8.8 with a 4-byte
 // load per column), so a lane owns whole chains and reads 16 bytes at a time:
-//   * up to four rows (router_logits_chain_kernel): a block per chain, products in shared memory, one warp adds.
+//   * few chains (router_logits_chain_kernel): a block per chain, products in shared memory, added by the block in pieces
+//     (block_sum_ordered), about 4500 cycles for 2816 columns where one warp's chain took 13 000.
 //   * few rows (router_logits_few_kernel): eight experts x eight rows per block.  Helper warps form the products of a slab
 //     of 128 columns and leave them in shared memory, a chain per row; a lane of an adding warp reads four products and
 //     does four adds, nothing else.  Few experts per block because a block's weights all come through one SM.
@@ -326,14 +327,14 @@ cudaError_t launch_many(const float* W, const float* x, float* logits, int rows,
     return launch_pdl(router_logits_many_kernel<NSL, R>, grid, dim3(192), (size_t)G::SMEM, stream, W, x, logits, rows, E, H, status);
 }
 
-// ---- up to four rows: a block per (expert, row).  All its threads form the products, coalesced, in shared memory; one
-// warp adds them.  (A warp per chain with the products in its lanes' registers, handed from lane to lane, paid for
-// strided loads of the weights and for a shuffle and a branch in every turn.)
-constexpr int CHAIN_THREADS = 128;
+// ---- few chains: a block per (expert, row).  All its threads form the products, coalesced, in shared memory and add
+// them together (block_sum_ordered).
+constexpr int CHAIN_THREADS = 256;
 template <int N4>                             // 16-byte pieces per thread
 __global__ void __launch_bounds__(CHAIN_THREADS)
-router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict__ x, float* __restrict__ logits, int E, int H, int sms) {
+router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict__ x, float* __restrict__ logits, int E, int H) {
     extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ __align__(16) uint32_t scratch[ORDERED_SCRATCH];
     const int e = blockIdx.x, r = blockIdx.y, n4 = H >> 2;
     const float4* w4 = (const float4*)(W + (size_t)e * H);
     const float4* x4 = (const float4*)(x + (size_t)r * H);
@@ -357,11 +358,8 @@ router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict_
             ((float4*)smem)[k] = make_float4(__fmul_rn(w[i].x, v[i].x), __fmul_rn(w[i].y, v[i].y), __fmul_rn(w[i].z, v[i].z),
                                              __fmul_rn(w[i].w, v[i].w));
     }
-    __syncthreads();
-    // blocks that share an SM add on different schedulers
-    if ((threadIdx.x >> 5) != (((blockIdx.y * gridDim.x + blockIdx.x) / sms) & 3)) return;
-    const float acc = chain_sum((const float*)smem, H);
-    if ((threadIdx.x & 31) == 0) logits[(size_t)r * E + e] = __fadd_rn(acc, 0.0f);
+    const float acc = block_sum_ordered((float*)smem, H, 2, scratch);
+    if (threadIdx.x == 0) logits[(size_t)r * E + e] = __fadd_rn(acc, 0.0f);
 }
 
 }  // namespace
@@ -371,13 +369,16 @@ cudaError_t launch_router_logits(const float* W, const float* x, float* logits, 
     if (rows < 1) return cudaSuccess;
     if ((H % 64) != 0 || ((((uintptr_t)W) | ((uintptr_t)x)) & 15) != 0) return cudaErrorInvalidValue;
     const int sms = device_sms();
-    // a block per chain while that is a few blocks per SM (more rows share the weights, below)
-    if (rows <= 4 && H <= 10 * 4 * CHAIN_THREADS) {
+    // A block per chain up to six blocks per SM: adding a chain in pieces keeps four schedulers busy for some 1500 cycles, a
+    // chain per lane (below) takes its 13 000 for any number of them.  Decode layers, one chain per lane / a block per chain:
+    // 128 experts x 2816: 5 rows 103 / 100 us, 6 rows 115 / 113, 8 rows 135.5 / 135.3, 12 rows 167 / 171; 64 experts x 2048: 8 rows
+    // 103 / 101, 16 rows 142 / 144; NVFP4, 64 x 5120: 5 rows 156 / 143, 8 rows 198 / 186, 16 rows 292 / 287.
+    if ((long)E * rows <= 6L * sms && H <= 5 * 4 * CHAIN_THREADS) {
         const dim3 grid(E, rows);
         const size_t smem = (size_t)H * 4;
-        if (H <= 6 * 4 * CHAIN_THREADS)
-            return launch_pdl(router_logits_chain_kernel<6>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H, sms);
-        return launch_pdl(router_logits_chain_kernel<10>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H, sms);
+        if (H <= 3 * 4 * CHAIN_THREADS)
+            return launch_pdl(router_logits_chain_kernel<3>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H);
+        return launch_pdl(router_logits_chain_kernel<5>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H);
     }
     // one chain per lane while one round of blocks holds them all, then as many per lane as keep it to one round
     const long few = (long)((E + FEW_E - 1) / FEW_E) * ((rows + FEW_ROWS - 1) / FEW_ROWS);

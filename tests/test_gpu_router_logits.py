@@ -31,7 +31,7 @@ def test_router_logits_ragged_vs_oracle(orc, synth, H, E, B):
     st.close()
 
 
-# The chain-per-block form (one to four rows, both piece counts, a column remainder) and the top-k behind it: experts that
+# The block-per-chain form (both piece counts, a column remainder) and the top-k behind it: experts that
 # share a router row tie (the lower one wins), one, several and more than four keys per lane, top-k up to all experts.
 @pytest.mark.parametrize("H,E,K,B", [(64, 2, 2, 1), (2816, 33, 8, 2), (3136, 128, 8, 4), (192, 129, 6, 3), (256, 128, 32, 1),
                                      (128, 64, 4, 20)])
@@ -58,4 +58,63 @@ def test_router_topk_ties_vs_oracle(orc, synth, H, E, K, B):
         assert rc == 0
         assert_bits_equal(sel[t], want_sel, f"selected of row {t}")
         assert_bits_equal(wts[t], want_w, f"weights of row {t}")
+    st.close()
+
+
+def _hard_rows(rng, E, H):
+    """Router rows whose running sums do what a block that adds a chain in pieces has to survive."""
+    w = np.empty((E, H), np.float32)
+    for e in range(E):
+        g = rng.standard_normal(H)
+        kind = e % 12
+        if kind == 1:
+            g *= 10.0 ** rng.uniform(-16, 16, H)                   # most terms vanish, a few decide
+        elif kind == 2:
+            g = rng.integers(-8, 9, H) * 0.25                      # half-way cases, exact zeros on the way
+        elif kind == 3:
+            g[1::2] = -g[0::2]                                     # pairs that nearly cancel
+        elif kind == 4:
+            g[H // 2:] = -g[:H - H // 2]
+        elif kind == 5:
+            g = np.sin(np.arange(H) * 0.01) * 3.0                  # passes zero and comes back
+        elif kind == 6:
+            g *= 1e-38                                             # subnormal terms and sums
+        elif kind == 7:
+            g = np.sign(g) * 2.0 ** rng.integers(-12, 12, H)
+        elif kind == 8:
+            g = np.where(np.arange(H) < H - 3, 0.0, g)             # zeros, then the only terms
+        elif kind == 9:
+            g[0], g[-1] = 1e30, -1e30                              # everything between is lost
+        elif kind == 10:
+            g = np.abs(g)
+        elif kind == 11:
+            g[H // 3] = -np.abs(g).sum()                           # from far below zero back up
+        w[e] = g
+    return w
+
+
+# One launch per layer (one token) and a block per chain (up to four rows): widths of less than a piece per segment, of odd and
+# even numbers of pieces, and the widest of each kernel.
+@pytest.mark.parametrize("H,B,fused", [(64, 1, True), (192, 1, True), (2816, 1, True), (3200, 1, True), (64, 4, False), (704, 3, False),
+                                       (2816, 2, False), (5120, 1, False), (5120, 4, False)])
+def test_router_chains_with_hard_rows_vs_oracle(orc, synth, H, B, fused):
+    import torch
+    E, K = 48, 4
+    layer = synth.make_q4_moe_layer(670 + H, hidden=H, inter=64, n_experts=E, topk=K)
+    layer.router_w[:] = _hard_rows(np.random.default_rng(671 + H + B), E, H)
+    st = stack_mod().MoeStack(B, H, 64, E, K)
+    st.add_layer(layer)
+    x = synth.make_tokens(672 + B, B, H)
+    d_x = torch.from_numpy(x).cuda()
+    d_y = torch.zeros_like(d_x)
+    if fused:
+        assert st.forward_device(d_x.data_ptr(), B, d_y.data_ptr()) == 0
+    else:
+        assert st.layer_experts(0, d_x.data_ptr(), B) == 0
+    st.status()                                                    # a selection among huge logits may be refused: not the point here
+    got = d2h(st.workspace().logits, B * E, np.float32).reshape(B, E)
+    for t in range(B):
+        rc, rin = orc.router_input(x[t], layer.router_scale, layer.eps)
+        assert rc == 0
+        assert_bits_equal(got[t], orc.router_scores(layer.router_w, None, rin), f"logits of row {t} over {H} columns")
     st.close()

@@ -27,8 +27,8 @@
 // holds a scheduler for two cycles.  At 64 tokens (gate/up) 63 of 196 M warp instructions are these: 43 % of the launch's
 // cycles; the others (dequantisation once per pass and row, activation loads, the blocks' tables, prologues and folds) are
 // another 45 %.  At 16 tokens, where nearly every pass holds one or two, the products are 16 of 67 M.  Measured
-// (hidden 2816, inter 704, 128 experts, top-8; gate/up + down of a layer, event pairs): 64 tokens 698 -> 423 us, 16 tokens
-// 274 -> 156 us, 6 tokens 140 -> 90 us against two rows per lane and whole groups as blocks; 2 tokens 45 us, where one
+// (hidden 2816, inter 704, 128 experts, top-8; gate/up + down of a layer, event pairs): 64 tokens 698 -> 409 us, 16 tokens
+// 274 -> 150 us, 6 tokens 140 -> 87 us against two rows per lane and whole groups as blocks; 2 tokens 44 us, where one
 // persistent launch for both phases took 51.
 // NVFP4 (hidden 5120, inter 1536, 64 experts, top-4; expert phase of a layer): 1 token 71 -> 51 us, 16 tokens 640 -> 291; whole
 // layers with jobs of passes instead of empty blocks: 16 tokens 338 -> 305 us, 64 tokens 867 -> 766, 256 tokens 3020 -> 2570.
@@ -339,10 +339,12 @@ __device__ __forceinline__ void run_pass(const Q4Job& jb, Loader<NMAT, RL>& ld, 
         const uint8_t* w = stage + sr0 * CH_BYTES + 2 * u;
         const float* x = (const float*)(stage + G.x_off) + 4 * u;
         const int live = min(CH_STEPS, steps - ch * CH_STEPS);
-        // (one quantisation group per iteration: the four pass sizes of a layer's groups run side by side on an SM, and
-        // with whole chunks unrolled their code did not fit the instruction cache)
+        // One quantisation group per iteration: the four pass sizes of a layer's groups run side by side on an SM, and their code
+        // has to come through the instruction cache.  Two Q4 groups: 16 tokens 1167 -> 1125 us in six layers, 64 tokens 2761 -> 2680,
+        // two tokens 365 -> 357; one 32-column step: 1125 and 2787.  An NVFP4 group is shorter, two are better there (136 / 139 us for
+        // one token).
         const uint32_t r16 = (uint32_t)r7 << 4;
-#pragma unroll 2
+#pragma unroll (STEP == STEP_FP4 ? 2 : 1)
         for (int g = 0; g < live / 2; g++) {
             const uint32_t o = ((uint32_t)g << 5) ^ r16;
             if constexpr (STEP == STEP_FP4)

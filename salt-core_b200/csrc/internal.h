@@ -80,6 +80,7 @@ cudaError_t launch_q4_fused(const FusedArgs& args, cudaStream_t stream);
 
 // One decode layer (one token) in one launch: [reduce + RMSNorm of the previous layer] -> router
 // input -> logits -> top-k -> experts.
+constexpr int LOGIT_COPIES = 16;         // a block reads one of them
 struct alignas(16) LayerDecodeArgs {
     FusedArgs f;                   // H, M, chain, out (this layer's grouped rows), done (this layer's counters), status
     const float* x_in;             // [H] the stack input, used when prev_grouped is null
@@ -93,7 +94,7 @@ struct alignas(16) LayerDecodeArgs {
     const float* router_w;         // [E][H]
     const float* per_expert_scale; // [E]
     float* logits;                 // [E]
-    int* logits_count;             // arrival counter of this layer, zero at launch
+    uint32_t* logit_slots;         // [LOGIT_COPIES][E up to 4] inverted bits of this layer's logits, zero at launch (no logit yet)
     int E, topk, expert_begin, expert_end;
     int32_t* selected;             // [topk] outputs of block 0 ...
     float* weights_out;            // [topk] (a different buffer than prev_weights)

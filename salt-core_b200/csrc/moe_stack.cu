@@ -70,7 +70,7 @@ struct Stack {
     int32_t* fused_done = nullptr;
     // one-launch decode layers (one token): buffers of the other parity and per-layer arrival counters
     float *grouped_alt = nullptr, *weights_alt = nullptr;
-    int32_t* layer_counters = nullptr;         // [layers_cap][FUSED_MAX_JOBS + 1], then [layers_cap] "layer finished" counters
+    int32_t* layer_counters = nullptr;         // [layers_cap] logit slots and job counters (forward_decode_layers), then [layers_cap] "layer finished" counters
     LayerDecodeArgs* d_layer_args = nullptr;   // [layers_cap] arguments of the whole-stack decode launch
     std::vector<LayerDecodeArgs> h_layer_args;
     int layers_cap = 0;
@@ -1066,9 +1066,9 @@ static const LayerDecodeArgs* capture_copy(const std::vector<LayerDecodeArgs>& a
 
 static int forward_decode_layers(Stack* s, int first, int count, const float* d_x, float* d_y, cudaStream_t st) {
     const int H = s->hidden, M = s->inter, K = s->topk;
-    // per layer: the logits arrival counter and FUSED_MAX_JOBS job counters; after all layers' blocks of those,
-    // one "layer finished" counter per layer (the whole-stack launch)
-    const int stride = FUSED_MAX_JOBS + 1;
+    // per layer: slots of the logits and FUSED_MAX_JOBS job counters, all zero at the start of a pass; after all layers' blocks
+    // of those, one "layer finished" counter per layer (the whole-stack launch)
+    const size_t slots = (size_t)LOGIT_COPIES * ((s->n_experts + 3) & ~3), stride = slots + FUSED_MAX_JOBS;
     if (count > s->layers_cap) {       // set-up, not part of a captured pass: forward passes are not captured before one has run
         const int cap = (int)s->layers.size();                 // >= count
         int32_t* counters = nullptr;
@@ -1098,9 +1098,9 @@ static int forward_decode_layers(Stack* s, int first, int count, const float* d_
         LayerDecodeArgs a;
         memset(&a, 0, sizeof a);
         a.f.H = H; a.f.M = M; a.f.chain = s->chain; a.f.out = gbuf[i & 1];
-        a.f.done = s->layer_counters + (size_t)i * stride + 1; a.f.status = s->status;
+        a.f.done = s->layer_counters + (size_t)i * stride + slots; a.f.status = s->status;
         a.f.n_jobs_max = n_jobs_max;
-        a.logits_count = s->layer_counters + (size_t)i * stride;
+        a.logit_slots = (uint32_t*)(s->layer_counters + (size_t)i * stride);
         if (i == 0) {
             a.x_in = d_x;
         } else {

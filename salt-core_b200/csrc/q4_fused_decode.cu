@@ -309,14 +309,16 @@ __device__ __forceinline__ bool fused_expert_rounds(const FusedArgs& a, const Fu
     // order of the requests: the small ones first (scales, biases, activations: the tables are built
     // from them while the weights stream in), then every warp's gate/up rows, then the down rows
     Round R = round_of(0);
-    if (warp == 0) issue_scales(R);
+    if (warp == 0) {
+        issue_scales(R);               // publishes s_rg and s_rd with its arrivals on bar_sc
+        __syncwarp();
+    }
     if (tid == 0) {
         if (!x_resident) {
             mbar_expect_tx(bar_x, (uint32_t)(H * 4));
             bulk_g2s(sX, a.x, (uint32_t)(H * 4), bar_x);
         }
     }
-    __syncthreads();               // s_rg / s_rd are published, the small requests are queued
     issue_gu(R);
     if (tid == 0) issue_dn(R);
     if (!x_resident && !fused_mbar_wait(bar_x, 0)) timeout = true;
@@ -442,8 +444,7 @@ __global__ void __launch_bounds__(16 * SLOTS, 1) q4_fused_expert_kernel(FusedArg
 //     block for itself: its results (the experts' activation row, the router input) stay in the
 //     block's shared memory and nothing is waited for;
 //   * block e forms the logit of expert e (reference src/kernels.c:98-106: one dependent-add chain
-//     over the hidden size, handed from lane to lane of one warp), stores it and bumps an arrival
-//     counter; every block polls the counter (bounded), reads the logits and repeats the top-k
+//     over the hidden size, added in pieces) and stores it; every block polls the logits (bounded) and repeats the top-k
 //     (gemma4.c:132-186) and the job list for itself;
 //   * block 0 also leaves selections, weights and the (trivial, one token) grouping in global
 //     memory for the next layer's reduce and for the caller.
@@ -540,12 +541,8 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
 
     // ---- the layer's input row: ordered weighted reduce of the previous layer, or the stack input ----
     if (a.prev_grouped != nullptr) {
-        if (tid < K) {
-            const float w = __ldcg(a.prev_weights + tid);
-            if (!finite_f(w)) flag(a.f.status, SB_ERR_NONFINITE);
-            s_w[tid] = w;
-        }
-        __syncthreads();
+        float w_own = 0.0f;
+        if (tid < K) w_own = __ldcg(a.prev_weights + tid);
         for (int r0 = 0; r0 < K; r0 += 8) {
             float o[NV][8];
 #pragma unroll
@@ -555,6 +552,13 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
                     const int d = tid + j * NT;
                     o[j][i] = (r0 + i < K && d < H) ? __ldcg(a.prev_grouped + (size_t)(r0 + i) * H + d) : 0.0f;
                 }
+            if (r0 == 0) {                     // the first rows are on their way
+                if (tid < K) {
+                    if (!finite_f(w_own)) flag(a.f.status, SB_ERR_NONFINITE);
+                    s_w[tid] = w_own;
+                }
+                __syncthreads();
+            }
 #pragma unroll
             for (int i = 0; i < 8; i++)
                 if (r0 + i < K && finite_f(s_w[r0 + i])) {
@@ -647,20 +651,36 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
             if (d < H) prod[d] = __fmul_rn(wrow[d], v[j]);
         }
         const float acc = layer_ordered_sum(prod, H, 2, scan);
-        if (tid == 0) {
-            a.logits[e] = acc;
-            asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(a.logits_count) : "memory");
+        if (tid < LOGIT_COPIES)
+            asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(a.logit_slots + tid * ((E + 3) & ~3) + e), "r"(~__float_as_uint(acc)) : "memory");
+        if (tid == 0) a.logits[e] = acc;
+        __syncwarp();                      // before the other lanes start to poll
+    }
+    // ---- all logits, then top-k and the job list, by every block for itself.  A logit is its own arrival mark: its inverted
+    // bits, or zero (no sum has all bits set); a counter cost its release and a second trip to the L2.  Copies, because one
+    // copy that all blocks read, sixteen sectors each, kept its slices of the L2 busy for 2000 to 4000 cycles ----
+    float* const s_logits = tk;                  // where the top-k keeps them if it needs a copy
+    if (warp == 0) {
+        const uint32_t* slots = a.logit_slots + cta % LOGIT_COPIES * ((E + 3) & ~3);
+        for (int e = 4 * lane; e < E; e += 128) {
+            uint4 b;
+            uint32_t i = 0;
+            do {
+                asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w) : "l"(slots + e) : "memory");
+                if (e + 1 >= E) b.y = 1u;
+                if (e + 2 >= E) b.z = 1u;
+                if (e + 3 >= E) b.w = 1u;
+            } while ((b.x == 0u || b.y == 0u || b.z == 0u || b.w == 0u) && ++i < FUSED_SPIN_LIMIT);
+            if (i >= FUSED_SPIN_LIMIT) timeout = true;
+            const uint32_t w[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (e + k < E) s_logits[e + k] = __uint_as_float(~w[k]);
         }
     }
-    // ---- all logits, then top-k and the job list, by every block for itself ----
-    if (tid == 0) {
-        uint32_t i = 0;
-        while (ld_acquire_gpu(a.logits_count) < E && i < FUSED_SPIN_LIMIT) i++;
-        if (i >= FUSED_SPIN_LIMIT) timeout = true;
-    }
     __syncthreads();
-    topk_group(tid < 160, a.logits, s_pes, s_sel, s_wts, E, K, 1, cta == 0 ? a.f.status : nullptr, tk,
-               tk + topk_scratch_floats(E, K) - 4, tid, 160);
+    topk_group(tid < 160, [&](int e) { return s_logits[e]; }, s_pes, s_sel, s_wts, E, K, 1, cta == 0 ? a.f.status : nullptr, tk,
+               tk + topk_scratch_floats(E, K) - 4, tid, 160, 1);
     __syncthreads();
     // job list: thread j takes selection j (its slot = the local selections before it; the list keeps rank order)
     if (tid < K) {

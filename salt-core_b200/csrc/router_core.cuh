@@ -327,17 +327,21 @@ static __device__ __forceinline__ float block_sum_ordered(float* p, int n, int r
 // the renormalisation sum are serial chains in expert / rank order.
 //
 // Executed by a group of `gsize` >= 64 consecutive threads (ltid = index in group, whole warps) on one row; every thread of
-// the block must call it (block-wide barriers inside), groups without a row pass active = false.  lr: the row's logits in
-// global memory.  sm = this group's scratch of 2E + 2*topk floats (16-byte aligned), sc = 4 floats of per-group scalars.
+// the block must call it (block-wide barriers inside), groups without a row pass active = false.  logit(e): the row's logit of
+// expert e, the same at every call.  sm = this group's scratch of 2E + 2*topk floats (16-byte aligned), sc = 4 floats of
+// per-group scalars, bar: number of a barrier of the group's own (1 and up).
 //
 // Nothing but latencies: up to 128 experts the group's first warp picks the selections, the largest of four keys per lane
-// at a time, while the other warps evaluate the exponentials; it then does all the rest without another barrier (the
-// divisions side by side, the two serial sums by all lanes alike).  Ranking every expert against all others, and one
-// thread dividing by the sum rank after rank, took 6800 cycles of a decode layer; this takes about half.
-static __device__ __forceinline__ void topk_group(bool active, const float* lr, const float* per_expert_scale,
-                                                  int32_t* sel_out, float* w_out, int E, int topk,
-                                                  int sort_by_expert, int* status, float* sm, float* sc,
-                                                  int ltid, int gsize) {
+// at a time, while the other warps evaluate the exponentials and the second one adds them in order; then the first warp does
+// the rest, a selection per lane (the divisions side by side, the sum of the selected ones by all lanes alike).
+// Measured in a decode layer (128 experts, top-8): from the logits in the block to the weights 3500 cycles, 5000 with the sum after
+// the selections and one thread reading each selection back; the exponentials and their 128 ordered additions take 1600 of them.
+static __device__ __forceinline__ void group_barrier(int bar, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory"); }
+
+template <class Logit>
+static __device__ __forceinline__ void topk_group(bool active, Logit logit, const float* per_expert_scale, int32_t* sel_out, float* w_out,
+                                                  int E, int topk, int sort_by_expert, int* status, float* sm, float* sc,
+                                                  int ltid, int gsize, int bar) {
     constexpr int KEYS = 4;          // experts per lane of the first warp
     float* sl = sm;                  // [E] logits (more than 32 * KEYS experts)
     float* se = sm + E;              // [E] exp(l - max)
@@ -346,8 +350,9 @@ static __device__ __forceinline__ void topk_group(bool active, const float* lr, 
     int* s_bad = (int*)(sc + 3);
     const bool few = E <= 32 * KEYS;
     float own = 0.0f;                // the first expert whose exponential this thread evaluates
-    if (active && few && ltid >= 32 && ltid - 32 < E) own = __ldcg(lr + ltid - 32);
+    if (active && few && ltid >= 32 && ltid - 32 < E) own = logit(ltid - 32);
     uint32_t key[KEYS];
+    int mine = 0;                    // first warp: selection number ltid
     if (active && ltid < 32) {
         float m = __int_as_float(0xff800000);
         bool bad = false;
@@ -357,7 +362,7 @@ static __device__ __forceinline__ void topk_group(bool active, const float* lr, 
                 const int e = ltid + 32 * i;
                 key[i] = 0u;                                     // below every finite logit's key
                 if (e < E) {
-                    const float v = __ldcg(lr + e);
+                    const float v = logit(e);
                     bad |= !finite_f(v) || (per_expert_scale && !finite_f(per_expert_scale[e]));
                     m = fmaxf(m, v);
                     const uint32_t b = __float_as_uint(__fadd_rn(v, 0.0f));      // -0 ranks like +0
@@ -366,7 +371,7 @@ static __device__ __forceinline__ void topk_group(bool active, const float* lr, 
             }
         } else {
             for (int e = ltid; e < E; e += 32) {
-                const float v = __ldcg(lr + e);
+                const float v = logit(e);
                 bad |= !finite_f(v) || (per_expert_scale && !finite_f(per_expert_scale[e]));
                 m = fmaxf(m, v);
                 sl[e] = v;
@@ -379,6 +384,7 @@ static __device__ __forceinline__ void topk_group(bool active, const float* lr, 
             sc[0] = m;
             *s_bad = bad ? 1 : 0;
         }
+        __syncwarp();
     }
     __syncthreads();
     // the reference rejects non-finite logits before ranking (gemma4.c:149-152)
@@ -398,46 +404,72 @@ static __device__ __forceinline__ void topk_group(bool active, const float* lr, 
     } else if (go && ltid >= 32) {
         const float mx = sc[0];
         for (int e = ltid - 32; e < E; e += gsize - 32)
-            se[e] = expf_exact(__fsub_rn(e == ltid - 32 ? own : __ldcg(lr + e), mx));
+            se[e] = expf_exact(__fsub_rn(e == ltid - 32 ? own : logit(e), mx));
+        group_barrier(bar, gsize - 32);
+        if (ltid < 64) {
+            const float all = (E & 63) == 0 && (((uintptr_t)se) & 15) == 0 ? chain_sum(se, E) : serial_sum(se, E);
+            if (ltid == 32) sc[1] = all;
+        }
     } else if (go) {
+#pragma unroll 1
         for (int j = 0; j < topk; j++) {
             uint32_t best = key[0];
 #pragma unroll
             for (int i = 1; i < KEYS; i++) best = max(best, key[i]);
             best = __reduce_max_sync(0xffffffffu, best);
-            uint32_t e = 0xffffffffu;                            // the lowest expert of those that tie
+            int e = 0;                                           // the lowest expert of those that tie
 #pragma unroll
-            for (int i = KEYS - 1; i >= 0; i--)
-                if (key[i] == best) e = (uint32_t)(ltid + 32 * i);
-            e = __reduce_min_sync(0xffffffffu, e);
+            for (int i = KEYS - 1; i >= 0; i--) {
+                const uint32_t tied = __ballot_sync(0xffffffffu, key[i] == best);
+                e = tied ? 32 * i + __ffs(tied) - 1 : e;
+            }
 #pragma unroll
-            for (int i = 0; i < KEYS; i++)
-                if (e == (uint32_t)(ltid + 32 * i)) key[i] = 0u;
-            if (ltid == 0) ssel[j] = (int)e;
+            for (int i = 0; i < KEYS; i++) key[i] = e == ltid + 32 * i ? 0u : key[i];
+            mine = j == ltid ? e : mine;
+            if (topk > 32 && ltid == 0) ssel[j] = e;
         }
     }
     __syncthreads();
     if (go && ltid < 32) {
-        const float all = (E & 63) == 0 && (((uintptr_t)se) & 15) == 0 ? chain_sum(se, E) : serial_sum(se, E);
+        float all;
+        if (few) all = sc[1];
+        else all = (E & 63) == 0 && (((uintptr_t)se) & 15) == 0 ? chain_sum(se, E) : serial_sum(se, E);
         bool bad = !(all > 0.0f) || !finite_f(all);
-        for (int j = ltid; j < topk; j += 32) sw[j] = __fdiv_rn(se[ssel[j]], all);
-        __syncwarp();
-        float selsum = 0.0f;
-#pragma unroll 8
-        for (int j = 0; j < topk; j++) selsum = __fadd_rn(selsum, sw[j]);
-        if (!(selsum > 0.0f) || !finite_f(selsum)) bad = true;
-        for (int j = ltid; j < topk; j += 32) {
-            const int e = ssel[j];
-            const float nrm = __fdiv_rn(sw[j], selsum);
-            const float w = __fmul_rn(nrm, per_expert_scale ? per_expert_scale[e] : 1.0f);
-            int pos = j;
-            if (sort_by_expert) {
-                pos = 0;
-#pragma unroll 8
-                for (int i = 0; i < topk; i++) pos += (ssel[i] < e) ? 1 : 0;
+        if (few && topk <= 32) {
+            const float w = __fdiv_rn(se[mine], all);
+            float selsum = 0.0f;
+            int before = 0;
+#pragma unroll 4
+            for (int j = 0; j < topk; j++) {
+                selsum = __fadd_rn(selsum, __shfl_sync(0xffffffffu, w, j));
+                before += __shfl_sync(0xffffffffu, mine, j) < mine ? 1 : 0;
             }
-            sel_out[pos] = e;
-            w_out[pos] = w;
+            if (!(selsum > 0.0f) || !finite_f(selsum)) bad = true;
+            if (ltid < topk) {
+                const int pos = sort_by_expert ? before : ltid;
+                sel_out[pos] = mine;
+                w_out[pos] = __fmul_rn(__fdiv_rn(w, selsum), per_expert_scale ? per_expert_scale[mine] : 1.0f);
+            }
+        } else {
+            for (int j = ltid; j < topk; j += 32) sw[j] = __fdiv_rn(se[ssel[j]], all);
+            __syncwarp();
+            float selsum = 0.0f;
+#pragma unroll 8
+            for (int j = 0; j < topk; j++) selsum = __fadd_rn(selsum, sw[j]);
+            if (!(selsum > 0.0f) || !finite_f(selsum)) bad = true;
+            for (int j = ltid; j < topk; j += 32) {
+                const int e = ssel[j];
+                const float nrm = __fdiv_rn(sw[j], selsum);
+                const float w = __fmul_rn(nrm, per_expert_scale ? per_expert_scale[e] : 1.0f);
+                int pos = j;
+                if (sort_by_expert) {
+                    pos = 0;
+#pragma unroll 8
+                    for (int i = 0; i < topk; i++) pos += (ssel[i] < e) ? 1 : 0;
+                }
+                sel_out[pos] = e;
+                w_out[pos] = w;
+            }
         }
         if (ltid == 0 && bad) *s_bad = 1;
     }

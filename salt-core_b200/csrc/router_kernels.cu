@@ -556,9 +556,10 @@ router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ p
     pdl_wait();                    // the logits come from the previous kernel
     pdl_launch_dependents();
     float* sc = tk_sm + topk_scratch_floats(E, topk) - 4;
-    topk_group(true, logits + (size_t)blockIdx.x * E, per_expert_scale, selected + (size_t)blockIdx.x * topk,
+    const float* lr = logits + (size_t)blockIdx.x * E;
+    topk_group(true, [&](int e) { return __ldcg(lr + e); }, per_expert_scale, selected + (size_t)blockIdx.x * topk,
                weights + (size_t)blockIdx.x * topk, E, topk, sort_by_expert, status, tk_sm, sc, threadIdx.x,
-               blockDim.x);
+               blockDim.x, 1);
 }
 
 cudaError_t launch_router_topk(const float* logits, const float* per_expert_scale, int32_t* selected, float* weights,
@@ -612,8 +613,9 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(MoePlanArgs a) {
         float* mine = tk + grp * per;
         const bool active = grp < a.rows;
         const int row = active ? grp : 0;
-        topk_group(active, a.logits + (size_t)row * E, a.per_expert_scale, a.selected_out + (size_t)row * a.topk,
-                   a.weights_out + (size_t)row * a.topk, E, a.topk, 1, a.status, mine, mine + per - 4, ltid, 128);
+        const float* lr = a.logits + (size_t)row * E;
+        topk_group(active, [&](int e) { return __ldcg(lr + e); }, a.per_expert_scale, a.selected_out + (size_t)row * a.topk,
+                   a.weights_out + (size_t)row * a.topk, E, a.topk, 1, a.status, mine, mine + per - 4, ltid, 128, grp + 1);
         __syncthreads();   // selections written by this block are read back below
     }
     int* hist = sp;               // [32][E]
@@ -781,8 +783,9 @@ __global__ void __launch_bounds__(4 * TOPK_THREADS) moe_plan_small_kernel(MoePla
         float* mine = tk + grp * per;
         const bool active = grp < a.rows;
         const int row = active ? grp : 0;
-        topk_group(active, a.logits + (size_t)row * E, a.per_expert_scale, a.selected_out + (size_t)row * a.topk,
-                   a.weights_out + (size_t)row * a.topk, E, a.topk, 1, a.status, mine, mine + per - 4, ltid, TOPK_THREADS);
+        const float* lr = a.logits + (size_t)row * E;
+        topk_group(active, [&](int e) { return __ldcg(lr + e); }, a.per_expert_scale, a.selected_out + (size_t)row * a.topk,
+                   a.weights_out + (size_t)row * a.topk, E, a.topk, 1, a.status, mine, mine + per - 4, ltid, TOPK_THREADS, grp + 1);
         __syncthreads();   // selections written by this block are read back below
     }
     const int jobs = a.rows * a.topk;

@@ -10,10 +10,10 @@
 //   * few rows (router_logits_few_kernel): eight experts x eight rows per block.  Helper warps form the products of a slab
 //     of 128 columns and leave them in shared memory, a chain per row; a lane of an adding warp reads four products and
 //     does four adds, nothing else.  Few experts per block because a block's weights all come through one SM.
-//   * many rows (router_logits_many_kernel): 64 experts x 4 R rows per block, NSL x R chains per lane, so that a 16-byte
+//   * many rows (router_logits_many_kernel): 64 experts x CW R rows per block, NSL x R chains per lane, so that a 16-byte
 //     load of weights serves R chains and one of activations NSL.
 // Slabs of weights and activations are fetched by warps of their own.  Between events, 128 experts x 2816 columns: 64 rows
-// 39 -> 19 us, 512 rows 47 -> 36, 2048 rows 100 -> 87 against tiles of 8 x 8 to 32 x 32 chains, one or four per lane, with a
+// 39 -> 19 us, 512 rows 47 -> 36, 2048 rows 100 -> 76 against tiles of 8 x 8 to 32 x 32 chains, one or four per lane, with a
 // barrier per slab.
 #include "internal.h"
 #include "mbar.cuh"
@@ -222,10 +222,10 @@ router_logits_few_kernel(const float* __restrict__ W, const float* __restrict__ 
     if (!ok) flag(status, SB_ERR_TIMEOUT);
 }
 
-// ---- many rows: 32 NSL experts x 4 R rows per block -------------------------------------------------------
-template <int NSL, int R>
+// ---- many rows: 32 NSL experts x CW R rows per block ------------------------------------------------------
+template <int NSL, int R, int CW>
 struct ManyTile {
-    static constexpr int WE = 32 * NSL, ROWS = 4 * R;
+    static constexpr int WE = 32 * NSL, ROWS = CW * R, THREADS = 32 * (CW + 2);
     static constexpr uint32_t STAGE_BYTES = (WE + ROWS) * ROW_BYTES;
     static constexpr int STAGES = 3;
     static constexpr uint32_t SMEM = STAGES * STAGE_BYTES + 2 * STAGES * 8;
@@ -262,12 +262,12 @@ __device__ __forceinline__ void add_columns(const float* w, const float* x, floa
     }
 }
 
-// warps 0..3: R rows each, lane = expert; 4, 5: copies
-template <int NSL, int R>
-__global__ void __launch_bounds__(192, 1)
+// CW warps: R rows each, lane = expert; two more: copies
+template <int NSL, int R, int CW>
+__global__ void __launch_bounds__(32 * (CW + 2), 1)
 router_logits_many_kernel(const float* __restrict__ W, const float* __restrict__ x, float* __restrict__ logits, int rows, int E,
                           int H, int* status) {
-    using G = ManyTile<NSL, R>;
+    using G = ManyTile<NSL, R, CW>;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t* full = (uint64_t*)(smem + G::STAGES * G::STAGE_BYTES);
     uint64_t* empty = full + G::STAGES;
@@ -276,15 +276,15 @@ router_logits_many_kernel(const float* __restrict__ W, const float* __restrict__
     if (threadIdx.x == 0) {
         for (int i = 0; i < G::STAGES; i++) {
             mbar_init(full + i, 64);
-            mbar_init(empty + i, 4);
+            mbar_init(empty + i, CW);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     bool ok = true;
-    if (warp == 4) {
+    if (warp == CW) {
         ok = fetch_slabs(smem, full, empty, G::STAGES, G::STAGE_BYTES, 0, G::WE, W, e0, E - 1, H, G::STAGES);
-    } else if (warp == 5) {
+    } else if (warp == CW + 1) {
         ok = fetch_slabs(smem, full, empty, G::STAGES, G::STAGE_BYTES, G::WE, min(G::ROWS, rows - row0), x, row0, rows - 1, H, 0);
     } else {
         pdl_wait();
@@ -318,13 +318,13 @@ router_logits_many_kernel(const float* __restrict__ W, const float* __restrict__
     if (!ok) flag(status, SB_ERR_TIMEOUT);
 }
 
-template <int NSL, int R>
+template <int NSL, int R, int CW>
 cudaError_t launch_many(const float* W, const float* x, float* logits, int rows, int E, int H, int* status, cudaStream_t stream) {
-    using G = ManyTile<NSL, R>;
-    cudaError_t e = ensure_dynamic_smem((const void*)router_logits_many_kernel<NSL, R>, G::SMEM);
+    using G = ManyTile<NSL, R, CW>;
+    cudaError_t e = ensure_dynamic_smem((const void*)router_logits_many_kernel<NSL, R, CW>, G::SMEM);
     if (e != cudaSuccess) return e;
     const dim3 grid((E + G::WE - 1) / G::WE, (rows + G::ROWS - 1) / G::ROWS);
-    return launch_pdl(router_logits_many_kernel<NSL, R>, grid, dim3(192), (size_t)G::SMEM, stream, W, x, logits, rows, E, H, status);
+    return launch_pdl(router_logits_many_kernel<NSL, R, CW>, grid, dim3(G::THREADS), (size_t)G::SMEM, stream, W, x, logits, rows, E, H, status);
 }
 
 // ---- few chains: a block per (expert, row).  All its threads form the products, coalesced, in shared memory and add
@@ -389,11 +389,19 @@ cudaError_t launch_router_logits(const float* W, const float* x, float* logits, 
                           (size_t)FEW_SMEM, stream, W, x, logits, rows, E, H, status);
     }
     const long lanes = (long)((E + 31) / 32) * ((rows + 3) / 4);                 // blocks of one chain per lane
-    if (lanes <= sms) return launch_many<1, 1>(W, x, logits, rows, E, H, status, stream);
-    if (lanes <= 2 * sms) return launch_many<1, 2>(W, x, logits, rows, E, H, status, stream);
-    if (lanes <= 4 * sms) return launch_many<2, 2>(W, x, logits, rows, E, H, status, stream);
-    if (lanes <= 8 * sms) return launch_many<2, 4>(W, x, logits, rows, E, H, status, stream);
-    return launch_many<2, 8>(W, x, logits, rows, E, H, status, stream);
+    if (lanes <= sms) return launch_many<1, 1, 4>(W, x, logits, rows, E, H, status, stream);
+    if (lanes <= 2 * sms) return launch_many<1, 2, 4>(W, x, logits, rows, E, H, status, stream);
+    if (lanes <= 4 * sms) return launch_many<2, 2, 4>(W, x, logits, rows, E, H, status, stream);
+    // Two adding warps per scheduler: one alone issues an addition or a product every 1.5 to 1.8 cycles, two together one every 1.1
+    // to 1.3.  Seven warps where their smaller tiles take no more time in all: 1999 rows 88.5 -> 77.1 us (eight warps 81.8), 1024 rows 49.4
+    // -> 45.7 (50.4); 512 rows 34.6 with four warps of four chains per lane, 35.2 with seven of two.
+    const auto rounds = [&](int tile) { return ((long)((E + 63) / 64) * ((rows + tile - 1) / tile) + sms - 1) / sms; };
+    if (lanes <= 8 * sms) {
+        if (7 * rounds(14) <= 8 * rounds(16)) return launch_many<2, 2, 7>(W, x, logits, rows, E, H, status, stream);
+        return launch_many<2, 2, 8>(W, x, logits, rows, E, H, status, stream);
+    }
+    if (7 * rounds(28) <= 8 * rounds(32)) return launch_many<2, 4, 7>(W, x, logits, rows, E, H, status, stream);
+    return launch_many<2, 4, 8>(W, x, logits, rows, E, H, status, stream);
 }
 
 }  // namespace sb

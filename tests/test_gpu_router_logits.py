@@ -118,3 +118,9 @@ def test_router_chains_with_hard_rows_vs_oracle(orc, synth, H, B, fused):
         assert rc == 0
         assert_bits_equal(got[t], orc.router_scores(layer.router_w, None, rin), f"logits of row {t} over {H} columns")
     st.close()
+
+
+# The tiles of many rows with seven and with eight adding warps, of two and of four rows each, and their last, partial rows.
+@pytest.mark.parametrize("H,E,B", [(192, 128, 900), (128, 130, 1190), (64, 128, 2073), (192, 64, 2400), (64, 128, 2100)])
+def test_router_logits_adding_warps_vs_oracle(orc, synth, H, E, B):
+    test_router_logits_ragged_vs_oracle(orc, synth, H, E, B)

@@ -369,10 +369,10 @@ __device__ __forceinline__ void run_tokens(const Q4Job& jb, Loader<NMAT, RL>& ld
     else run_pass<NMAT, RL, 1, STEP>(jb, ld, G, smem, r0, nvalid, tb);
 }
 
-// blockIdx: row tile, job, pass of the job's tokens
+// blockIdx: row tile, job, pass of `pass` of the job's tokens
 template <int FMT, int NMAT, int RL>
 __global__ void __launch_bounds__(NT, RL == 4 ? 4 : 6)
-batch_kernel(const void* __restrict__ jobs, const int* __restrict__ njobs_dev, int C, int jobs_early) {
+batch_kernel(const void* __restrict__ jobs, const int* __restrict__ njobs_dev, int C, int jobs_early, int pass) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int ROWS = 4 * RL * WARPS, ROWS_A = ROWS / NMAT;
     // jobs_early: the job table was written at least two launches back, so everything except the activation rows
@@ -386,22 +386,25 @@ batch_kernel(const void* __restrict__ jobs, const int* __restrict__ njobs_dev, i
     __shared__ __align__(16) Q4Job jb;
     float wg = 0.0f;
     if (FMT == FMT_FP4) {                                   // the same descriptor in the shared form
-        const Fp4Job& f = ((const Fp4Job*)jobs)[blockIdx.y];
-        wg = f.wg;
+        const Fp4Job* f = (const Fp4Job*)jobs + blockIdx.y;      // through L2: this SM's L1 may hold an earlier pass' jobs
+        wg = __ldcg(&f->wg);
         if (threadIdx.x == 0) {
-            jb.vals = f.codes; jb.scales = f.scales; jb.x = f.x; jb.y = f.y; jb.x_rows = nullptr;
-            jb.R = f.R; jb.ntok = f.ntok; jb.x_stride = f.x_stride; jb.y_stride = f.y_stride;
+            static_assert(sizeof(void*) == 8, "pointers as 64-bit words");
+            const auto pointer = [](const void* at) { return (void*)__ldcg((const unsigned long long*)at); };
+            jb.vals = (const uint8_t*)pointer(&f->codes); jb.scales = (const uint8_t*)pointer(&f->scales);
+            jb.x = (const float*)pointer(&f->x); jb.y = (float*)pointer(&f->y); jb.x_rows = nullptr;
+            jb.R = __ldcg(&f->R); jb.ntok = __ldcg(&f->ntok); jb.x_stride = __ldcg(&f->x_stride); jb.y_stride = __ldcg(&f->y_stride);
         }
     } else if (threadIdx.x < sizeof(Q4Job) / 16) {
         ((uint4*)&jb)[threadIdx.x] = __ldcg((const uint4*)((const Q4Job*)jobs + blockIdx.y) + threadIdx.x);
     }
     __syncthreads();
-    const int r0 = blockIdx.x * ROWS_A, tb = blockIdx.z * MAX_T;
+    const int r0 = blockIdx.x * ROWS_A, tb = blockIdx.z * pass;
     if (r0 >= jb.R || tb >= jb.ntok) return;
     const int nvalid = min(ROWS_A, jb.R - r0), tid = threadIdx.x;
     const BatchGeom G = batch_geom(FMT, C, NMAT, RL);
     __shared__ const float* x_row[MAX_T];
-    Loader<NMAT, RL> ld(jb, x_row, r0, C, min(MAX_T, jb.ntok - tb));
+    Loader<NMAT, RL> ld(jb, x_row, r0, C, min(pass, jb.ntok - tb));
 
     // first stages: weights and scales, then (after the dependency) activations
     ld.weights(smem);
@@ -483,16 +486,16 @@ batch_kernel(const void* __restrict__ jobs, const int* __restrict__ njobs_dev, i
 
 template <int FMT, int NMAT, int RL>
 cudaError_t launch_batch(const void* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
-                         cudaStream_t stream, int pdl) {
+                         cudaStream_t stream, int pdl, int pass = MAX_T) {
     const BatchGeom G = batch_geom(FMT, C, NMAT, RL);
     cudaError_t e = ensure_dynamic_smem((const void*)batch_kernel<FMT, NMAT, RL>, G.smem);
     if (e != cudaSuccess) return e;
     constexpr int ROWS_A = 4 * RL * WARPS / NMAT;
-    const dim3 grid((max_rows + ROWS_A - 1) / ROWS_A, njobs_max, (max_tok + MAX_T - 1) / MAX_T);
+    const dim3 grid((max_rows + ROWS_A - 1) / ROWS_A, njobs_max, (max_tok + pass - 1) / pass);
     if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
     if (pdl >= 0)
-        return launch_pdl(batch_kernel<FMT, NMAT, RL>, grid, dim3(NT), (size_t)G.smem, stream, jobs, njobs_dev, C, pdl);
-    batch_kernel<FMT, NMAT, RL><<<grid, NT, G.smem, stream>>>(jobs, njobs_dev, C, 0);
+        return launch_pdl(batch_kernel<FMT, NMAT, RL>, grid, dim3(NT), (size_t)G.smem, stream, jobs, njobs_dev, C, pdl, pass);
+    batch_kernel<FMT, NMAT, RL><<<grid, NT, G.smem, stream>>>(jobs, njobs_dev, C, 0, pass);
     return launched();
 }
 
@@ -523,9 +526,12 @@ bool fp4_batch_supported(int C) { return C >= 256 && (C % 256) == 0; }
 cudaError_t launch_fp4_batch(const Fp4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
                              cudaStream_t stream) {
     const long blocks = (long)((max_rows + 63) / 64) * njobs_max * ((max_tok + MAX_T - 1) / MAX_T);
-    return two_rows_per_lane(FMT_FP4, blocks)
-               ? launch_batch<FMT_FP4, 1, 2>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, 0)
-               : launch_batch<FMT_FP4, 1, 4>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, 0);
+    if (!two_rows_per_lane(FMT_FP4, blocks)) return launch_batch<FMT_FP4, 1, 4>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, 1);
+    // Host calls (jobs of a stack are passes already): two tokens a pass where even that leaves room for two blocks per SM: a block's products are a chain of chunks, shorter with
+    // fewer tokens.  From the host, four / two tokens a pass: 1536 rows x 5120, 4 tokens 49.3 / 43.8 us, 7 tokens 52.8 / 51.2; 200 x
+    // 5120, 16 tokens 60.8 / 55.5; 6000 x 2048, 7 tokens (five blocks per SM) 46.8 / 49.5.
+    const bool two = njobs_dev == nullptr && (long)((max_rows + 31) / 32) * njobs_max * ((max_tok + 1) / 2) <= 2L * device_sms();
+    return launch_batch<FMT_FP4, 1, 2>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, 1, two ? 2 : MAX_T);
 }
 
 }  // namespace sb

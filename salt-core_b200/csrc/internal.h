@@ -44,6 +44,8 @@ bool q4_batch_supported(int C, int nmat);
 cudaError_t launch_q4_batch(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
                             int nmat, cudaStream_t stream, int pdl);
 bool fp4_batch_supported(int C);
+// Programmatic dependent launch of the kernel before it, which writes the activations; jobs and njobs_dev were written at least two
+// launches back.
 cudaError_t launch_fp4_batch(const Fp4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
                              cudaStream_t stream);
 
@@ -230,7 +232,8 @@ cudaError_t make_fp4_weight_map(CUtensorMap* out, const void* base, int C, int r
 cudaError_t make_fp4_act_maps(CUtensorMap* out3, const void* base, int C, int rows);
 cudaError_t launch_nvfp4_gemm_tc(const Fp4TcJob* jobs, int njobs, int R, int C, const Fp4TcMaps& maps, int* status,
                                  cudaStream_t stream);
-// njobs_dev (optional, device): number of live jobs; njobs is then the most the call can have
+// njobs_dev (optional, device): number of live jobs; njobs is then the most the call can have.  Between the writer of jobs and
+// njobs_dev and this launch there is the quantiser's.
 cudaError_t launch_nvfp4_jobs(const Fp4Job* jobs, int njobs, int max_rows, int max_tok, int C, bool aligned,
                               cudaStream_t stream, const int* njobs_dev = nullptr);
 

@@ -500,15 +500,18 @@ static cudaError_t launch_glue_warps(const GlueArgs& a, int rows, int sms, cudaS
 
 // Most rows for which the block-per-row form is the faster one.  It takes a full round of the chip for every `at_once` rows
 // (one block per SM; four of 256 threads for narrow rows), the warp form about as long for one row as for several hundred.
-// Measured with 148 SMs, two sums (one launch, us, block / warp form): 1024 columns 592 rows 13.2 / 12.5, 768 rows 19 / 14;
-// 2048 columns 148 rows 12 / 21, 296 rows 23.5 / 20.7, 320 rows 34 / 21, 2048 rows 167 / 45; 4096 columns 296 rows 26 / 33, 320
-// rows 38 / 33; 5120 columns 148 rows 24 / 39, 192 rows 45 / 39; 6144 columns 192 rows 48 / 51, 320 rows 72 / 53.  One sum lies
-// alike.  Without a sum the block form's rounds are three times shorter: 2816 columns 320 rows 10.4 / 12.4, 512 rows 13.8 /
-// 12.4; 5120 columns 192 rows 12.4 / 10.4.
+// Measured with 148 SMs and four selections (one launch, us, block / warp form, one sum and two): 1024 columns 296 rows 5.5 / 8.6 and
+// 8.5 / 11.2, 592 rows 8.7 / 8.8 and 12.2 / 11.7; 2048 columns 148 rows 7.7 / 12.7 and 10.3 / 18.9, 256 rows 13.2 / 12.6 and
+// 18.8 / 18.8; 2816 columns 296 rows 13.8 / 16.7 and 19.5 / 26.7, 320 rows 19.2 / 16.8 and 27.7 / 27.0; 5120 columns 256 rows
+// 17.6 / 22.9 and 25.5 / 37.1, 320 rows 24.2 / 23.0 and 35.8 / 37.3; 6144 columns 444 rows 27.0 / 29.2 and 41.8 / 47.4, 512 rows
+// 33.3 / 29.1 and 51.6 / 47.5.  Without a sum the block form's rounds are three times shorter: 2816 columns and eight selections, 320
+// rows 10.4 / 12.4, 512 rows 13.8 / 12.4.
 static int glue_block_rows(const GlueArgs& a, int sms) {
     const int at_once = a.n <= 1024 ? 4 * sms : sms;
+    const int sums = (a.norm_w != nullptr) + (a.router_scale != nullptr);
     int rounds = a.n <= 1024 || (a.n > 4096 && a.n <= 5120) ? 1 : 2;
-    if (a.norm_w == nullptr && a.router_scale == nullptr && a.n <= 4096) rounds++;
+    if (sums == 1) rounds = a.n <= 2048 ? 1 : (a.n <= 5120 ? 2 : 3);
+    if (sums == 0 && a.n <= 4096) rounds++;
     return rounds * at_once;
 }
 

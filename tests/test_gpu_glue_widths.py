@@ -85,3 +85,27 @@ def test_flagged_rows(synth):
     keep = [t for t in range(rows) if t != 7]
     assert torch.equal(y[0][keep], y[1][keep])
     st.close()
+
+
+@pytest.mark.parametrize("n,rounds", [(1024, 4), (1088, 1), (2048, 1), (2112, 2), (5120, 2), (5184, 3), (6144, 3)])
+def test_form_of_one_sum(orc, synth, n, rounds):
+    """With one in-order sum (a prompt's router input, a last layer's norm) the line lies elsewhere; both sides of it."""
+    import torch
+    line = rounds * SMS
+    st, layers = _stack(synth, n, line + 1)
+    for rows, blocks in ((line, line), (line + 1, (line + 4) // 4)):
+        x = synth.make_tokens(830 + n, rows, n)
+        d_x, y = torch.from_numpy(x).cuda(), torch.zeros(rows, n, device="cuda")
+        assert st.layer_experts(0, d_x.data_ptr(), rows) == 0
+        torch.cuda.synchronize()
+
+        def call(stream):
+            assert st.layer_combine(0, rows, y.data_ptr(), apply_norm=True, stream=stream) == 0
+        (name, grid), = captured_kernels(call)
+        assert grid == (blocks, 1, 1), (name, n, rows)
+        call(torch.cuda.current_stream().cuda_stream)
+        assert st.status() == 0
+        for t in (0, rows // 2, rows - 1):
+            want, _, _ = orc.moe_layer_q4(layers[0], x[t:t + 1], threads=4)
+            assert_bits_equal(y[t].cpu().numpy(), orc.rmsnorm(want[0], layers[0].norm_weight, layers[0].eps, True)[1], f"row {t} of {rows} x {n}")
+    st.close()

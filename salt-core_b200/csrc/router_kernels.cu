@@ -4,6 +4,7 @@
 // contains several chains that are serial by definition (sums of squares, router logits,
 // softmax denominators).  Many chains run side by side, each added by a lane; where few are asked for, the whole block
 // adds one (block_sum_ordered).
+#include <cooperative_groups.h>
 #include "internal.h"
 #include "pdl.cuh"
 #include "q4_core.cuh"
@@ -603,9 +604,14 @@ static __device__ __forceinline__ void write_expert_jobs(const MoePlanArgs& a, i
 // warp then walks its segment in order, ranking equal experts inside a 32-wide
 // step with match_any.  Experts outside [expert_begin, expert_end) keep their
 // slots in the global order but get no job descriptor.
+// NB blocks, a cluster if more than one: each takes a contiguous part of the selections and learns the others' counts through
+// distributed shared memory; the first one writes what there is one of.  A lone block is bound by latencies that grow with the
+// selections (a load, a match and a store for every 1024 of them): 1999 rows x 8.
+template <int NB>
 __global__ void __launch_bounds__(1024) moe_plan_kernel(MoePlanArgs a) {
     extern __shared__ __align__(16) int sp[];
     const int E = a.n_experts;
+    const int part = NB > 1 ? (int)blockIdx.x : 0;
     pdl_wait();                    // the logits or the selections come from the previous kernel
     pdl_launch_dependents();
     if (a.logits != nullptr) {
@@ -624,10 +630,12 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(MoePlanArgs a) {
     int* hist = sp;               // [32][E]
     int* offs = sp + 32 * E;      // [E+1]
     int* act = offs + (E + 1);    // [E] active prefix
+    int* own = act + E;           // [E] this block's selections of an expert (NB > 1)
     const int jobs = a.rows * a.topk;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int seg = (jobs + 31) / 32;
-    const int s0 = min(jobs, warp * seg), s1 = min(jobs, s0 + seg);
+    const int j0 = NB > 1 ? min(jobs, part * ((jobs + NB - 1) / NB)) : 0, j1 = NB > 1 ? min(jobs, j0 + (jobs + NB - 1) / NB) : jobs;
+    const int seg = (j1 - j0 + 31) / 32;
+    const int s0 = min(j1, j0 + warp * seg), s1 = min(j1, s0 + seg);
     for (int i = threadIdx.x; i < 32 * E; i += blockDim.x) hist[i] = 0;
     __syncthreads();
     for (int i = s0 + lane; i < s1; i += 32) {
@@ -636,15 +644,34 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(MoePlanArgs a) {
         else atomicAdd(&hist[warp * E + e], 1);
     }
     __syncthreads();
-    // per expert: exclusive scan over segments, total count left in offs[e]
+    if constexpr (NB > 1) {
+        for (int e = threadIdx.x; e < E; e += blockDim.x) {
+            int sum = 0;
+#pragma unroll 8
+            for (int w = 0; w < 32; w++) sum += hist[w * E + e];
+            own[e] = sum;
+        }
+        cooperative_groups::this_cluster().sync();
+    }
+    // per expert: exclusive scan over segments (of all blocks), total count left in offs[e]
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        int run = 0;
+        int run = 0, after = 0;
+        if constexpr (NB > 1) {
+            int theirs[NB];
+#pragma unroll
+            for (int b = 0; b < NB; b++) theirs[b] = *cooperative_groups::this_cluster().map_shared_rank(own + e, b);
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                run += b < part ? theirs[b] : 0;
+                after += b > part ? theirs[b] : 0;
+            }
+        }
         for (int w = 0; w < 32; w++) {
             const int c = hist[w * E + e];
             hist[w * E + e] = run;
             run += c;
         }
-        offs[e] = run;
+        offs[e] = run + after;
     }
     __syncthreads();
     // exclusive scans over experts (E <= 1024 = one expert per thread): group
@@ -677,8 +704,11 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(MoePlanArgs a) {
             }
             warp_cnt[lane] = wc - tot_c;     // exclusive prefix of the warp totals
             warp_act[lane] = wa - tot_a;
-            if (lane == 31) { offs[E] = wc; *a.n_active = wa; }
-            if (lane == 0) *a.max_group = wm;
+            if (lane == 31) {
+                offs[E] = wc;
+                if (part == 0) *a.n_active = wa;
+            }
+            if (lane == 0 && part == 0) *a.max_group = wm;
         }
         __syncthreads();
         if (e < E) {
@@ -687,7 +717,8 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(MoePlanArgs a) {
         }
     }
     __syncthreads();
-    for (int e = threadIdx.x; e <= E; e += blockDim.x) a.group_offsets[e] = offs[e];
+    if (part == 0)
+        for (int e = threadIdx.x; e <= E; e += blockDim.x) a.group_offsets[e] = offs[e];
     // ordered placement
     for (int i0 = s0; i0 < s1; i0 += 32) {
         const int i = i0 + lane;
@@ -709,8 +740,12 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(MoePlanArgs a) {
             hist[warp * E + e] += __popc(peers);
         __syncwarp();
     }
+    if constexpr (NB > 1) {
+        cooperative_groups::this_cluster().sync();         // no block leaves while another may read its counts
+        if (part != 0) return;
+    }
     if (a.fused_done != nullptr && threadIdx.x < FUSED_MAX_JOBS) a.fused_done[threadIdx.x] = 0;
-    __syncthreads();               // the placement is complete: the descriptors below read it back
+    __syncthreads();               // the placement is complete: the descriptors below reuse its tables
     if (a.pass_tokens > 0) {
         // one job per pass of up to pass_tokens tokens, the largest passes first: their cost is proportional to
         // their tokens, and with whole groups as jobs the SMs that drew the popular experts finished last (B = 64:
@@ -852,6 +887,11 @@ __global__ void __launch_bounds__(4 * TOPK_THREADS) moe_plan_small_kernel(MoePla
     }
 }
 
+// One block / a cluster of eight, top-8 (event pairs, us): 128 rows 10.7 / 12.6, 192 rows 12.7 / 12.6, 256 rows 12.7 / 12.7, 384 rows
+// 14.7 / 12.7, 512 rows 16.2 / 12.7, 1024 rows 21.2 / 13.4, 1999 rows 33.2 / 14.9.
+constexpr int PLAN_BLOCKS = 8;             // the portable cluster size
+constexpr long PLAN_CLUSTER_JOBS = 2048;   // selections
+
 cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream) {
     if (a.logits != nullptr && a.rows >= 1 && a.rows <= 4 && a.rows * a.topk <= 32) {
         const size_t small = (size_t)a.rows * topk_scratch_floats(a.n_experts, a.topk) * sizeof(float);
@@ -864,12 +904,18 @@ cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream) {
         if (a.rows > 8) return cudaErrorInvalidValue;
         smem += (size_t)8 * topk_scratch_floats(a.n_experts, a.topk) * sizeof(float);
     }
+    if (smem > 160 * 1024) return cudaErrorInvalidValue;
+    if (a.logits == nullptr && (long)a.rows * a.topk >= PLAN_CLUSTER_JOBS) {
+        smem += (size_t)a.n_experts * sizeof(int);
+        cudaError_t e = ensure_dynamic_smem((const void*)moe_plan_kernel<PLAN_BLOCKS>, (size_t)(164 * 1024));
+        if (e != cudaSuccess) return e;
+        return launch_pdl_cluster(moe_plan_kernel<PLAN_BLOCKS>, PLAN_BLOCKS, dim3(1024), smem, stream, a);
+    }
     if (smem > 48 * 1024) {
-        cudaError_t e = ensure_dynamic_smem((const void*)moe_plan_kernel, (size_t)(160 * 1024));
+        cudaError_t e = ensure_dynamic_smem((const void*)moe_plan_kernel<1>, (size_t)(160 * 1024));
         if (e != cudaSuccess) return e;
     }
-    if (smem > 160 * 1024) return cudaErrorInvalidValue;
-    return launch_pdl(moe_plan_kernel, dim3(1), dim3(1024), smem, stream, a);
+    return launch_pdl(moe_plan_kernel<1>, dim3(1), dim3(1024), smem, stream, a);
 }
 
 }  // namespace sb

@@ -315,7 +315,7 @@ __device__ __forceinline__ void load_chunk(Loader<NMAT, RL>& ld, const BatchGeom
     cp_async_commit();
 }
 
-template <int NMAT, int RL, int T, int STEP>
+template <int NMAT, int RL, int T, int STEP, int UNROLL>
 __device__ __forceinline__ void run_pass(const Q4Job& jb, Loader<NMAT, RL>& ld, const BatchGeom& G, uint8_t* smem,
                                          int r0, int nvalid, int tb) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, u = lane & 7, lrow = lane >> 3;
@@ -339,12 +339,12 @@ __device__ __forceinline__ void run_pass(const Q4Job& jb, Loader<NMAT, RL>& ld, 
         const uint8_t* w = stage + sr0 * CH_BYTES + 2 * u;
         const float* x = (const float*)(stage + G.x_off) + 4 * u;
         const int live = min(CH_STEPS, steps - ch * CH_STEPS);
-        // One quantisation group per iteration: the four pass sizes of a layer's groups run side by side on an SM, and their code
+        // One Q4 quantisation group per iteration in a layer: the four pass sizes of a layer's groups run side by side on an SM, and their code
         // has to come through the instruction cache.  Two Q4 groups: 16 tokens 1167 -> 1125 us in six layers, 64 tokens 2761 -> 2680,
         // two tokens 365 -> 357; one 32-column step: 1125 and 2787.  An NVFP4 group is shorter, two are better there (136 / 139 us for
         // one token).
         const uint32_t r16 = (uint32_t)r7 << 4;
-#pragma unroll (STEP == STEP_FP4 ? 2 : 1)
+#pragma unroll UNROLL
         for (int g = 0; g < live / 2; g++) {
             const uint32_t o = ((uint32_t)g << 5) ^ r16;
             if constexpr (STEP == STEP_FP4)
@@ -360,17 +360,17 @@ __device__ __forceinline__ void run_pass(const Q4Job& jb, Loader<NMAT, RL>& ld, 
                              (float*)(smem + G.table_off), sr0, acc);
 }
 
-template <int NMAT, int RL, int STEP>
+template <int NMAT, int RL, int STEP, int UNROLL>
 __device__ __forceinline__ void run_tokens(const Q4Job& jb, Loader<NMAT, RL>& ld, const BatchGeom& G, uint8_t* smem,
                                            int r0, int nvalid, int tb) {
-    if (ld.ntok == 4) run_pass<NMAT, RL, 4, STEP>(jb, ld, G, smem, r0, nvalid, tb);
-    else if (ld.ntok == 3) run_pass<NMAT, RL, 3, STEP>(jb, ld, G, smem, r0, nvalid, tb);
-    else if (ld.ntok == 2) run_pass<NMAT, RL, 2, STEP>(jb, ld, G, smem, r0, nvalid, tb);
-    else run_pass<NMAT, RL, 1, STEP>(jb, ld, G, smem, r0, nvalid, tb);
+    if (ld.ntok == 4) run_pass<NMAT, RL, 4, STEP, UNROLL>(jb, ld, G, smem, r0, nvalid, tb);
+    else if (ld.ntok == 3) run_pass<NMAT, RL, 3, STEP, UNROLL>(jb, ld, G, smem, r0, nvalid, tb);
+    else if (ld.ntok == 2) run_pass<NMAT, RL, 2, STEP, UNROLL>(jb, ld, G, smem, r0, nvalid, tb);
+    else run_pass<NMAT, RL, 1, STEP, UNROLL>(jb, ld, G, smem, r0, nvalid, tb);
 }
 
 // blockIdx: row tile, job, pass of `pass` of the job's tokens
-template <int FMT, int NMAT, int RL>
+template <int FMT, int NMAT, int RL, int UNROLL>
 __global__ void __launch_bounds__(NT, RL == 4 ? 4 : 6)
 batch_kernel(const void* __restrict__ jobs, const int* __restrict__ njobs_dev, int C, int jobs_early, int pass) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -447,7 +447,7 @@ batch_kernel(const void* __restrict__ jobs, const int* __restrict__ njobs_dev, i
 #pragma unroll
     for (int k = 1; k < STAGES - 1; k++) load_chunk<FMT, NMAT, RL>(ld, G, smem + k * G.stage_bytes);
     if constexpr (FMT == FMT_FP4) {
-        run_tokens<NMAT, RL, STEP_FP4>(jb, ld, G, smem, r0, nvalid, tb);
+        run_tokens<NMAT, RL, STEP_FP4, UNROLL>(jb, ld, G, smem, r0, nvalid, tb);
     } else {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
         __syncthreads();
@@ -479,23 +479,23 @@ batch_kernel(const void* __restrict__ jobs, const int* __restrict__ njobs_dev, i
                 }
             lit = __syncthreads_or(lit);
         }
-        if (lit) run_tokens<NMAT, RL, STEP_Q4_LITERAL>(jb, ld, G, smem, r0, nvalid, tb);
-        else run_tokens<NMAT, RL, STEP_Q4>(jb, ld, G, smem, r0, nvalid, tb);
+        if (lit) run_tokens<NMAT, RL, STEP_Q4_LITERAL, UNROLL>(jb, ld, G, smem, r0, nvalid, tb);
+        else run_tokens<NMAT, RL, STEP_Q4, UNROLL>(jb, ld, G, smem, r0, nvalid, tb);
     }
 }
 
-template <int FMT, int NMAT, int RL>
+template <int FMT, int NMAT, int RL, int UNROLL = FMT == FMT_FP4 ? 2 : 1>
 cudaError_t launch_batch(const void* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
                          cudaStream_t stream, int pdl, int pass = MAX_T) {
     const BatchGeom G = batch_geom(FMT, C, NMAT, RL);
-    cudaError_t e = ensure_dynamic_smem((const void*)batch_kernel<FMT, NMAT, RL>, G.smem);
+    cudaError_t e = ensure_dynamic_smem((const void*)batch_kernel<FMT, NMAT, RL, UNROLL>, G.smem);
     if (e != cudaSuccess) return e;
     constexpr int ROWS_A = 4 * RL * WARPS / NMAT;
     const dim3 grid((max_rows + ROWS_A - 1) / ROWS_A, njobs_max, (max_tok + pass - 1) / pass);
     if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
     if (pdl >= 0)
-        return launch_pdl(batch_kernel<FMT, NMAT, RL>, grid, dim3(NT), (size_t)G.smem, stream, jobs, njobs_dev, C, pdl, pass);
-    batch_kernel<FMT, NMAT, RL><<<grid, NT, G.smem, stream>>>(jobs, njobs_dev, C, 0, pass);
+        return launch_pdl(batch_kernel<FMT, NMAT, RL, UNROLL>, grid, dim3(NT), (size_t)G.smem, stream, jobs, njobs_dev, C, pdl, pass);
+    batch_kernel<FMT, NMAT, RL, UNROLL><<<grid, NT, G.smem, stream>>>(jobs, njobs_dev, C, 0, pass);
     return launched();
 }
 
@@ -516,6 +516,9 @@ cudaError_t launch_q4_batch(const Q4Job* jobs, int njobs_max, const int* njobs_d
     const long blocks = (long)((max_rows + 64 / nmat - 1) / (64 / nmat)) * njobs_max * ((max_tok + MAX_T - 1) / MAX_T);
     const bool two = two_rows_per_lane(FMT_Q4, blocks);
 #define SB_BATCH(NM, RL) launch_batch<FMT_Q4, NM, RL>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, pdl)
+    // one matrix for a host call, few blocks: nothing else is in the instruction cache
+    if (nmat == 1 && two && njobs_dev == nullptr)
+        return launch_batch<FMT_Q4, 1, 2, 2>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, pdl);
     if (nmat == 2) return two ? SB_BATCH(2, 2) : SB_BATCH(2, 4);
     return two ? SB_BATCH(1, 2) : SB_BATCH(1, 4);
 #undef SB_BATCH

@@ -74,7 +74,7 @@ struct FusedArgs {
     int jobs_per_round;          // filled in by the launcher
     int* status;
 };
-struct FusedLaunch { int grid, jobs_per_round; size_t smem; };
+struct FusedLaunch { int grid, slots, jobs_per_round; size_t smem; };
 // Whether the fused kernel serves this geometry on the current device (and how it would be launched).
 bool q4_fused_plan(int H, int M, int n_jobs_max, FusedLaunch* out);
 // Launched as a programmatic dependent launch; jobs, counters and x come from the previous kernel.

@@ -452,7 +452,8 @@ __global__ void __launch_bounds__(16 * SLOTS, 1) q4_fused_expert_kernel(FusedArg
 // list exists.  The previous layer's grouped outputs and weights are read from the buffers of the
 // OTHER parity, so a block that is late in its glue never sees rows of this layer.
 constexpr int LAYER_NV = 5;                 // columns per thread of the row-wise glue
-constexpr int LAYER_SLOTS = 40;
+// Row slots of a block: 40, or 42 where that saves a round (q4_fused_plan).
+constexpr int LAYER_SLOTS = 40, LAYER_SLOTS_MORE = 42;
 
 struct LayerScratch {                        // offsets in floats from the start of shared memory
     int sq, prod, wrow, pes, lit, topk, scan, end;
@@ -478,10 +479,10 @@ static __device__ __noinline__ float layer_ordered_sum(float* p, int n, int roun
 // previous layer is the previous kernel).  STACKED = true: layer `li` of q4_stack_decode_kernel, whose blocks
 // stay resident over all layers: the previous layer is complete when every block has bumped its counter
 // (prev_done reaches the grid size; bounded wait), and the block's barriers are re-initialised.
-template <bool STACKED>
+template <bool STACKED, int SLOTS>
 __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint8_t* smem, int li, const int* prev_done,
                                                   int* my_done) {
-    constexpr int SLOTS = LAYER_SLOTS, NT = 16 * SLOTS, NV = LAYER_NV;
+    constexpr int NT = 16 * SLOTS, NV = LAYER_NV;
     const int H = a.f.H, M = a.f.M, E = a.E, K = a.topk;
     const FusedGeom G = fused_geom(H, M, SLOTS);
     FusedSmem<SLOTS> S(smem, G);
@@ -732,16 +733,18 @@ __device__ __forceinline__ void layer_decode_body(const LayerDecodeArgs& a, uint
     }
 }
 
-__global__ void __launch_bounds__(16 * LAYER_SLOTS, 1) q4_layer_decode_kernel(LayerDecodeArgs a) {
+template <int SLOTS>
+__global__ void __launch_bounds__(16 * SLOTS, 1) q4_layer_decode_kernel(LayerDecodeArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
-    layer_decode_body<false>(a, smem, 0, nullptr, nullptr);
+    layer_decode_body<false, SLOTS>(a, smem, 0, nullptr, nullptr);
     if (a.last) pdl_launch_dependents();
 }
 
 // All layers of a decode step in ONE launch: the blocks (one per SM) stay resident, so the code of a layer is
 // fetched once per step instead of once per layer, and a layer ends with one arrival counter instead of a kernel
 // boundary.  layers[li] are the per-layer arguments (device memory), done[li] the arrival counters (zero at launch).
-__global__ void __launch_bounds__(16 * LAYER_SLOTS, 1)
+template <int SLOTS>
+__global__ void __launch_bounds__(16 * SLOTS, 1)
 q4_stack_decode_kernel(const LayerDecodeArgs* __restrict__ layers, int n_layers, int* done) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(16) LayerDecodeArgs s_args;
@@ -752,7 +755,7 @@ q4_stack_decode_kernel(const LayerDecodeArgs* __restrict__ layers, int n_layers,
         for (int i = threadIdx.x; i < (int)(sizeof(LayerDecodeArgs) / 16); i += blockDim.x)
             ((uint4*)&s_args)[i] = __ldg((const uint4*)(layers + li) + i);
         __syncthreads();
-        layer_decode_body<true>(s_args, smem, li, li > 0 ? done + li - 1 : nullptr, done + li);
+        layer_decode_body<true, SLOTS>(s_args, smem, li, li > 0 ? done + li - 1 : nullptr, done + li);
     }
     pdl_launch_dependents();
 }
@@ -806,21 +809,40 @@ bool q4_fused_plan(int H, int M, int n_jobs_max, FusedLaunch* out) {
     DeviceInfo* d = device_info();
     if (!d || H < 64 || M < 64 || (H & 63) || (M & 63) || n_jobs_max < 1 || n_jobs_max > FUSED_MAX_JOBS)
         return false;
-    const int slots = LAYER_SLOTS;
-    const FusedGeom g = fused_geom(H, M, slots);
-    if (g.total > FUSED_SMEM_LIMIT) return false;
     const int grid = d->sms;
     // most jobs per round whose shares fit the block: ceil(J*M/grid) <= slots, ceil(J*H/grid) <= dn_cap
-    int jmax = 0;
-    for (int J = 1; J <= grid && J <= FUSED_MAX_JOBS; J++) {
-        const int P = (J * M + grid - 1) / grid;
-        int Q = (J * H + grid - 1) / grid;
-        Q += Q & 1;
-        if (P > slots || Q > g.dn_cap || P > M || Q > H) break;
-        jmax = J;
-    }
+    const auto most = [&](int slots) {
+        const FusedGeom g = fused_geom(H, M, slots);
+        int jmax = 0;
+        if (g.total > FUSED_SMEM_LIMIT) return jmax;
+        for (int J = 1; J <= grid && J <= FUSED_MAX_JOBS; J++) {
+            const int P = (J * M + grid - 1) / grid;
+            int Q = (J * H + grid - 1) / grid;
+            Q += Q & 1;
+            if (P > slots || Q > g.dn_cap || P > M || Q > H) break;
+            jmax = J;
+        }
+        return jmax;
+    };
+    const auto rounds = [&](int jmax) { return (n_jobs_max + jmax - 1) / jmax; };
+    int slots = LAYER_SLOTS, jmax = most(slots);
     if (jmax < 1) return false;
-    if (out) { out->grid = grid; out->jobs_per_round = jmax; out->smem = g.total; }
+    // Two more slots cost a decode layer 1.6 us (2816 x 704, eight jobs in one round of 40: 36.4 us with 40, 38.1 with 42), a second
+    // round takes more (2048 x 768: 38.0 with two rounds of 40, 34.5 with one of 42).
+    if (rounds(jmax) > 1) {
+        const int more = most(LAYER_SLOTS_MORE);
+        if (more > 0 && rounds(more) < rounds(jmax)) {
+            slots = LAYER_SLOTS_MORE;
+            jmax = more;
+        }
+    }
+    // rounds of equal size: 4 + 4 jobs of 2048 x 768 take 38.0 us, 7 + 1 38.8 (a round of one job has few warps at work)
+    if (out) {
+        out->grid = grid;
+        out->slots = slots;
+        out->jobs_per_round = (n_jobs_max + rounds(jmax) - 1) / rounds(jmax);
+        out->smem = fused_geom(H, M, slots).total;
+    }
     return true;
 }
 
@@ -830,9 +852,10 @@ cudaError_t launch_q4_fused(const FusedArgs& args, cudaStream_t stream) {
     if (((uintptr_t)args.x) & 15) return cudaErrorInvalidValue;
     FusedArgs a = args;
     a.jobs_per_round = L.jobs_per_round;
-    cudaError_t e = ensure_dynamic_smem((const void*)q4_fused_expert_kernel<LAYER_SLOTS>, FUSED_SMEM_LIMIT);
+    const auto kernel = L.slots == LAYER_SLOTS ? q4_fused_expert_kernel<LAYER_SLOTS> : q4_fused_expert_kernel<LAYER_SLOTS_MORE>;
+    cudaError_t e = ensure_dynamic_smem((const void*)kernel, FUSED_SMEM_LIMIT);
     if (e != cudaSuccess) return e;
-    return launch_pdl(q4_fused_expert_kernel<LAYER_SLOTS>, dim3(L.grid), dim3(16 * LAYER_SLOTS), L.smem, stream, a);
+    return launch_pdl(kernel, dim3(L.grid), dim3(16 * L.slots), L.smem, stream, a);
 }
 
 bool q4_layer_decode_plan(int H, int M, int E, int topk, int n_jobs_max, FusedLaunch* out) {
@@ -840,7 +863,7 @@ bool q4_layer_decode_plan(int H, int M, int E, int topk, int n_jobs_max, FusedLa
     if (!q4_fused_plan(H, M, n_jobs_max, &L) || H > 16 * LAYER_SLOTS * LAYER_NV || (H & 3) || E < 1 ||
         E > 1024 || topk < 1 || topk > 64 || topk > E)
         return false;
-    const FusedGeom g = fused_geom(H, M, LAYER_SLOTS);
+    const FusedGeom g = fused_geom(H, M, L.slots);
     if ((size_t)layer_scratch(H, E, topk).end * 4 > g.off_sgu) return false;    // the scratch overlays the weight rows only
     if (out) *out = L;
     return true;
@@ -850,9 +873,10 @@ cudaError_t launch_q4_stack_decode(const LayerDecodeArgs* d_layers, int n_layers
                                    int n_jobs_max, cudaStream_t stream) {
     FusedLaunch L;
     if (n_layers < 1 || !q4_layer_decode_plan(H, M, E, topk, n_jobs_max, &L)) return cudaErrorInvalidValue;
-    cudaError_t e = ensure_dynamic_smem((const void*)q4_stack_decode_kernel, FUSED_SMEM_LIMIT);
+    const auto kernel = L.slots == LAYER_SLOTS ? q4_stack_decode_kernel<LAYER_SLOTS> : q4_stack_decode_kernel<LAYER_SLOTS_MORE>;
+    cudaError_t e = ensure_dynamic_smem((const void*)kernel, FUSED_SMEM_LIMIT);
     if (e != cudaSuccess) return e;
-    return launch_pdl(q4_stack_decode_kernel, dim3(L.grid), dim3(16 * LAYER_SLOTS), L.smem, stream, d_layers, n_layers, d_done);
+    return launch_pdl(kernel, dim3(L.grid), dim3(16 * L.slots), L.smem, stream, d_layers, n_layers, d_done);
 }
 
 // jobs_per_round of a layer's arguments (what launch_q4_layer_decode fills in for a single launch)
@@ -864,11 +888,12 @@ int q4_layer_decode_jobs_per_round(int H, int M, int E, int topk, int n_jobs_max
 cudaError_t launch_q4_layer_decode(const LayerDecodeArgs& args, int n_jobs_max, cudaStream_t stream) {
     FusedLaunch L;
     if (!q4_layer_decode_plan(args.f.H, args.f.M, args.E, args.topk, n_jobs_max, &L)) return cudaErrorInvalidValue;
-    cudaError_t e = ensure_dynamic_smem((const void*)q4_layer_decode_kernel, FUSED_SMEM_LIMIT);
+    const auto kernel = L.slots == LAYER_SLOTS ? q4_layer_decode_kernel<LAYER_SLOTS> : q4_layer_decode_kernel<LAYER_SLOTS_MORE>;
+    cudaError_t e = ensure_dynamic_smem((const void*)kernel, FUSED_SMEM_LIMIT);
     if (e != cudaSuccess) return e;
     LayerDecodeArgs a = args;
     a.f.jobs_per_round = L.jobs_per_round;
-    return launch_pdl(q4_layer_decode_kernel, dim3(L.grid), dim3(16 * LAYER_SLOTS), L.smem, stream, a);
+    return launch_pdl(kernel, dim3(L.grid), dim3(16 * L.slots), L.smem, stream, a);
 }
 
 }  // namespace sb

@@ -116,3 +116,10 @@ def test_whole_pass_in_one_launch_equals_per_layer_launches_and_oracle(orc, synt
     got = st.forward_host(mid_n.reshape(1, H), first=1)
     assert_bits_equal(got, want, "layers 1.. from the normalised output of layer 0")
     st.close()
+
+
+# One round of 42 slots where 40 take two, two rounds of 42 where 40 take three, and two rounds of 40 (3 + 2 jobs).
+@pytest.mark.parametrize("geom", [(2048, 768, 16, 8, 2), (1024, 1536, 12, 8, 2), (512, 1600, 12, 5, 2)])
+def test_rounds_and_slots(orc, synth, geom):
+    test_whole_pass_in_one_launch_equals_per_layer_launches_and_oracle(orc, synth, geom)
+    test_fused_decode_equals_two_launch_form_and_oracle(orc, synth, geom[:4], 1)

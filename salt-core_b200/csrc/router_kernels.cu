@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(GLUE_NV == 4 ? 1024 : 512) glue_rows_kernel(Gl
 // l + 32, ... of its row in registers.  The squares of the four rows go to shared memory and ONE warp runs the four
 // in-order sums side by side, a row per lane (the reference's order: columns ascending from +0).  A chain of 2816 costs about
 // 6 us, but the rows of a few blocks per SM run side by side, where the block-per-row form above keeps a whole SM busy for
-// 12 us per row with two sums.  (Rows in lane-contiguous pieces, the sum handed from lane to lane, loaded 32 lines per
+// 10 us per row with two sums.  (Rows in lane-contiguous pieces, the sum handed from lane to lane, loaded 32 lines per
 // instruction: 1999 rows took 68 us for reduce and two sums, this takes 56.)
 // P: pieces per lane, an even number, for rows of more than 128 (P - 2) and at most 128 P columns; FULL: exactly 128 P.  The
 // row takes 4 P registers of a lane and what is left of its share holds the loads in flight, and pieces that may lie outside

@@ -23,6 +23,9 @@ int device_sms();
 // Raises a kernel's dynamic shared memory limit to at least `bytes` on the CURRENT device (the limit
 // is a per-device attribute of the function; remembered per device and kernel, safe from any thread).
 cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes);
+// Dynamic shared memory of a launch that needs no such call: a block has 48 KB without one, and the kernel's static
+// variables (at most 6 KB in this library) count too.
+constexpr size_t PLAIN_DYNAMIC_SMEM = 42 * 1024;
 
 // ---- q4_kernels.cu -------------------------------------------------------
 // Runs every job (all share C and nmat).  njobs_dev (device int, may be null)

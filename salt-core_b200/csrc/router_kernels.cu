@@ -197,15 +197,19 @@ __global__ void __launch_bounds__(256) softcap_kernel(float* __restrict__ logits
     logits[i] = __fmul_rn(cap, tanhf_exact(__fdiv_rn(v, cap)));
 }
 
+// Shared memory of the kernels that hold whole rows of any width, up to 200 KB of them.
+static cudaError_t allow_row_smem(const void* kernel, size_t smem) {
+    constexpr size_t most = 200 * 1024;
+    if (smem > most) return cudaErrorInvalidValue;
+    return smem > PLAIN_DYNAMIC_SMEM ? ensure_dynamic_smem(kernel, most) : cudaSuccess;
+}
+
 cudaError_t launch_residual_postnorm(const float* residual, const float* branch, const float* weight, float* out,
                                      int rows, int n, float eps, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
     const size_t smem = (size_t)(2 * ((n + 3) & ~3) + 8) * sizeof(float);
-    if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    if (smem > 48 * 1024) {
-        cudaError_t e = ensure_dynamic_smem((const void*)residual_postnorm_rows_kernel, (size_t)(200 * 1024));
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_row_smem((const void*)residual_postnorm_rows_kernel, smem);
+    if (e != cudaSuccess) return e;
     residual_postnorm_rows_kernel<<<rows, 1024, smem, stream>>>(residual, branch, weight, out, n, eps, status);
     return launched();
 }
@@ -215,11 +219,8 @@ cudaError_t launch_parallel_combine(const float* residual, const float* dense, c
                                     int rows, int n, float eps, float scalar, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
     const size_t smem = (size_t)(n + 8) * sizeof(float);
-    if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    if (smem > 48 * 1024) {
-        cudaError_t e = ensure_dynamic_smem((const void*)parallel_combine_rows_kernel, (size_t)(200 * 1024));
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_row_smem((const void*)parallel_combine_rows_kernel, smem);
+    if (e != cudaSuccess) return e;
     parallel_combine_rows_kernel<<<rows, 1024, smem, stream>>>(residual, dense, routed, wd, wr, wf, scratch_a, scratch_b,
                                                                out, n, eps, scalar, status);
     return launched();
@@ -537,8 +538,10 @@ cudaError_t launch_glue(const GlueArgs& a, int rows, cudaStream_t stream) {
 cudaError_t launch_rmsnorm(const float* x, const float* weight, float* y, int rows, int n, float eps, int with_scale,
                            int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
-    norm_rows_kernel<0><<<rows, 256, (size_t)(2 * n + 8) * sizeof(float), stream>>>(x, weight, y, n, eps, with_scale, 0.0f,
-                                                                           status);
+    const size_t smem = (size_t)(2 * n + 8) * sizeof(float);
+    const cudaError_t e = allow_row_smem((const void*)norm_rows_kernel<0>, smem);
+    if (e != cudaSuccess) return e;
+    norm_rows_kernel<0><<<rows, 256, smem, stream>>>(x, weight, y, n, eps, with_scale, 0.0f, status);
     return launched();
 }
 
@@ -548,7 +551,10 @@ constexpr int TOPK_THREADS = 160;
 cudaError_t launch_router_input(const float* x, const float* scale, float* out, int rows, int n, float eps,
                                 float root, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
-    norm_rows_kernel<1><<<rows, 256, (size_t)(2 * n + 8) * sizeof(float), stream>>>(x, scale, out, n, eps, 1, root, status);
+    const size_t smem = (size_t)(2 * n + 8) * sizeof(float);
+    const cudaError_t e = allow_row_smem((const void*)norm_rows_kernel<1>, smem);
+    if (e != cudaSuccess) return e;
+    norm_rows_kernel<1><<<rows, 256, smem, stream>>>(x, scale, out, n, eps, 1, root, status);
     return launched();
 }
 

@@ -917,7 +917,7 @@ cudaError_t launch_moe_plan(const MoePlanArgs& a, cudaStream_t stream) {
         if (e != cudaSuccess) return e;
         return launch_pdl_cluster(moe_plan_kernel<PLAN_BLOCKS>, PLAN_BLOCKS, dim3(1024), smem, stream, a);
     }
-    if (smem > 48 * 1024) {
+    if (smem > PLAIN_DYNAMIC_SMEM) {
         cudaError_t e = ensure_dynamic_smem((const void*)moe_plan_kernel<1>, (size_t)(160 * 1024));
         if (e != cudaSuccess) return e;
     }

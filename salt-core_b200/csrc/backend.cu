@@ -66,6 +66,7 @@ uint64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
 bool cuda_ok(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return true;
     if (getenv("SALT_GPU_DIAG")) fprintf(stderr, "salt-b200: %s: %s\n", what, cudaGetErrorString(e));
+    cudaGetLastError();            // reported here: the next launch of this thread is not to find it (launched() in internal.h)
     return false;
 }
 

@@ -158,6 +158,24 @@ static __device__ __forceinline__ bool ordered_step(float& s, const float4& seg,
     return ((int)(shift == 0.0f) | (in & whole)) & (in | (int)!inside) & (int)(s == s);
 }
 
+// The same sum, in one chain, by warp `who` (blocks of an SM that take different warps add on different schedulers).
+static __device__ __forceinline__ float block_sum_chain(const float* p, int n, uint32_t* scratch, int who) {
+    float* const result = (float*)scratch + 4;              // where the pieces leave theirs, too
+    __syncthreads();
+    if ((int)(threadIdx.x >> 5) == who) {
+        float s = n >= 64 ? chain_sum(p, n & ~63) : 0.0f;
+        for (int i = n & ~63; i < n; i++) s = __fadd_rn(s, p[i]);
+        if ((threadIdx.x & 31) == 0) *result = s;
+    }
+    __syncthreads();
+    return *result;
+}
+
+// Terms up to which that is the shorter way for a block by itself: the pieces cost 2800 (squares) or 3700 cycles (products)
+// whatever their length, a chain 460 and 4.15 a term.  Block of 640 threads, chain / pieces: 576 squares 2860 / 2990, 640 3120 /
+// 2990; 768 products 3650 / 4370, 832 3910 / 4010, 896 4180 / 4140.
+static __device__ __forceinline__ bool sum_in_chain(int n, int rounds) { return n <= (rounds == 1 ? 576 : 832); }
+
 static __device__ __forceinline__ float block_sum_ordered(float* p, int n, int rounds, uint32_t* scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // words of scratch: zeros [4], result [4], sums of the segments' quarters [2][4][32], seg [32] (start, g, 1 / g, first piece << 16 | pieces), sentinels

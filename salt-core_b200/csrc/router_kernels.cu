@@ -13,7 +13,9 @@
 namespace sb {
 
 // one copy of the in-order sum per kernel: its instructions are fetched cold, and the second sum finds them there
-static __device__ __noinline__ float row_sum_of_squares(float* p, int n, uint32_t* scratch) { return block_sum_ordered(p, n, 1, scratch); }
+static __device__ __noinline__ float row_sum_of_squares(float* p, int n, uint32_t* scratch) {
+    return sum_in_chain(n, 1) ? block_sum_chain(p, n, scratch, 0) : block_sum_ordered(p, n, 1, scratch);
+}
 
 // mode 0: RMSNorm  y = (x*inv) [* weight]             (gemma4.c:85-101)
 // mode 1: router input  y = ((x*inv)*scale)*root      (gemma4.c:103-130)

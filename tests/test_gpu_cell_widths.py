@@ -67,6 +67,14 @@ def test_parallel_combine(orc, n):
     assert g.shared_buffer_free(buf) == 0
 
 
+@pytest.mark.parametrize("n", [3, 64, 127, 128, 319, 575, 576, 577, 580, 640])
+def test_sums_of_few_squares(orc, n):
+    """One warp adds up to 576 squares in a row, with a tail of less than 64; above that the block adds them in pieces."""
+    test_norms(orc, n)
+    test_residual_postnorm(orc, n)
+    test_parallel_combine(orc, n)
+
+
 def test_wider_rows_are_refused():
     g, bm = gpu(), backend_mod()
     n = 51200

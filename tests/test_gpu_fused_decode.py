@@ -13,7 +13,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("geom", [
     # (hidden, inter, experts, topk): the bench layer; a layer whose rows need no padding; one
     # with many small experts (all 32 groups in one round); odd multiples of 64
-    (2816, 704, 128, 8), (256, 128, 32, 8), (512, 128, 32, 4), (1344, 320, 16, 2)])
+    (2816, 704, 128, 8), (256, 128, 32, 8), (512, 128, 32, 4), (1344, 320, 16, 2),
+    # sums by one warp end at 576 squares and 832 products
+    (576, 64, 8, 2), (640, 64, 8, 2), (832, 64, 8, 2), (896, 64, 8, 2)])
 @pytest.mark.parametrize("B", [1, 2, 3, 4])
 def test_fused_decode_equals_two_launch_form_and_oracle(orc, synth, geom, B):
     H, M, E, K = geom

@@ -6,7 +6,7 @@
 // holds it for about four cycles (measured: 4.5 cycles per column for add + multiply from registers, 8.8 with a 4-byte
 // load per column), so a lane owns whole chains and reads 16 bytes at a time:
 //   * few chains (router_logits_chain_kernel): a block per chain, products in shared memory, added by the block in pieces
-//     (block_sum_ordered), about 4500 cycles for 2816 columns where one warp's chain took 13 000.
+//     (block_sum_ordered), about 4500 cycles for 2816 columns where one warp's chain took 13 000, or, short ones, by one warp.
 //   * few rows (router_logits_few_kernel): eight experts x eight rows per block.  Helper warps form the products of a slab
 //     of 128 columns and leave them in shared memory, a chain per row; a lane of an adding warp reads four products and
 //     does four adds, nothing else.  Few experts per block because a block's weights all come through one SM.
@@ -328,11 +328,11 @@ cudaError_t launch_many(const float* W, const float* x, float* logits, int rows,
 }
 
 // ---- few chains: a block per (expert, row).  All its threads form the products, coalesced, in shared memory and add
-// them together (block_sum_ordered).
+// them together (block_sum_ordered) or, in_chains = the number of SMs, one of its warps does, another one in each round of blocks.
 constexpr int CHAIN_THREADS = 256;
 template <int N4>                             // 16-byte pieces per thread
 __global__ void __launch_bounds__(CHAIN_THREADS)
-router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict__ x, float* __restrict__ logits, int E, int H) {
+router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict__ x, float* __restrict__ logits, int E, int H, int in_chains) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ __align__(16) uint32_t scratch[ORDERED_SCRATCH];
     const int e = blockIdx.x, r = blockIdx.y, n4 = H >> 2;
@@ -358,7 +358,9 @@ router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict_
             ((float4*)smem)[k] = make_float4(__fmul_rn(w[i].x, v[i].x), __fmul_rn(w[i].y, v[i].y), __fmul_rn(w[i].z, v[i].z),
                                              __fmul_rn(w[i].w, v[i].w));
     }
-    const float acc = block_sum_ordered((float*)smem, H, 2, scratch);
+    float acc;
+    if (in_chains > 0) acc = block_sum_chain((const float*)smem, H, scratch, (int)((blockIdx.y * gridDim.x + blockIdx.x) / in_chains) & 3);
+    else acc = block_sum_ordered((float*)smem, H, 2, scratch);
     if (threadIdx.x == 0) logits[(size_t)r * E + e] = __fadd_rn(acc, 0.0f);
 }
 
@@ -369,16 +371,23 @@ cudaError_t launch_router_logits(const float* W, const float* x, float* logits, 
     if (rows < 1) return cudaSuccess;
     if ((H % 64) != 0 || ((((uintptr_t)W) | ((uintptr_t)x)) & 15) != 0) return cudaErrorInvalidValue;
     const int sms = device_sms();
-    // A block per chain up to six blocks per SM: adding a chain in pieces keeps four schedulers busy for some 1500 cycles, a
-    // chain per lane (below) takes its 13 000 for any number of them.  Decode layers, one chain per lane / a block per chain:
-    // 128 experts x 2816: 5 rows 103 / 100 us, 6 rows 115 / 113, 8 rows 135.5 / 135.3, 12 rows 167 / 171; 64 experts x 2048: 8 rows
-    // 103 / 101, 16 rows 142 / 144; NVFP4, 64 x 5120: 5 rows 156 / 143, 8 rows 198 / 186, 16 rows 292 / 287.
-    if ((long)E * rows <= 6L * sms && H <= 5 * 4 * CHAIN_THREADS) {
+    // A block per chain up to five chains per SM, and up to 2.3 + H / 600 of long ones.  The kernel with a chain per lane takes
+    // about as long for one chain as for many (logits and top-k of 1024 / 2816 / 5120 columns: 9 / 16 / 25 us).  A block per chain / that
+    // kernel (us, chains per SM): 512 columns 4.3: 6.8 / 7.7, 5.2: 8.3 / 7.8; 1024 columns 4.3: 7.9 / 9.0, 5.2: 10.1 / 9.0; 2048 columns
+    // 5.2: 12.3 / 13.0, 6.1: 13.2 / 13.1; 2816 columns 6.9: 15.6 / 16.1, 8.6: 17.5 / 16.2; 4096 columns 8.6: 20.4 / 21.2, 10.4:
+    // 23.1 / 21.2; 5120 columns 8.6: 22.5 / 25.3, 10.4: 25.3 / 25.4, 12.1: 27.8 / 25.3.
+    const long chains = (long)E * rows;
+    if (600 * chains <= (long)sms * (H < 1620 ? 3000 : 1380 + H) && H <= 5 * 4 * CHAIN_THREADS) {
+        // One warp's chain leaves the schedulers to the other blocks of the SM, pieces need them: chains are the shorter way up to
+        // 832 columns, or 700 and 330 more per chain and SM, while all blocks fit at once.  In pieces / as chains (us, chains per
+        // SM): 1024 columns 0.9: 7.2 / 7.4, 2.6: 8.2 / 7.2, 4.3: 9.1 / 7.9; 1536 columns 1.7: 8.0 / 8.4, 2.6: 8.6 / 8.5, 4.3: 10.9 / 10.2;
+        // 2048 columns 2.6: 9.1 / 9.9, 3.5: 10.0 / 10.0, 4.3: 10.9 / 10.7, 5.2: 12.3 / 14.8; 2816 columns 4.3: 11.7 / 13.0.
+        const int in_chains = chains <= 5L * sms && (H <= 832 || (H - 700) * (long)sms <= 330 * chains) ? sms : 0;
         const dim3 grid(E, rows);
         const size_t smem = (size_t)H * 4;
         if (H <= 3 * 4 * CHAIN_THREADS)
-            return launch_pdl(router_logits_chain_kernel<3>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H);
-        return launch_pdl(router_logits_chain_kernel<5>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H);
+            return launch_pdl(router_logits_chain_kernel<3>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H, in_chains);
+        return launch_pdl(router_logits_chain_kernel<5>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H, in_chains);
     }
     // one chain per lane while one round of blocks holds them all, then as many per lane as keep it to one round
     const long few = (long)((E + FEW_E - 1) / FEW_E) * ((rows + FEW_ROWS - 1) / FEW_ROWS);

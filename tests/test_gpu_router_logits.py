@@ -5,6 +5,7 @@ import pytest
 
 from conftest import assert_bits_equal
 from gpu_util import d2h, stack_mod
+from graph_util import captured_kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -117,6 +118,32 @@ def test_router_chains_with_hard_rows_vs_oracle(orc, synth, H, B, fused):
         rc, rin = orc.router_input(x[t], layer.router_scale, layer.eps)
         assert rc == 0
         assert_bits_equal(got[t], orc.router_scores(layer.router_w, None, rin), f"logits of row {t} over {H} columns")
+    st.close()
+
+
+# Both sides of the lines (148 SMs): one warp adds a chain of up to 832 columns (squares: 576), of more where more chains share an SM;
+# a block per chain up to so many chains, the kernel of a chain per lane above.
+@pytest.mark.parametrize("H,B", [(512, 15), (512, 16), (576, 1), (640, 1), (832, 2), (896, 2), (1024, 3), (1024, 4), (1024, 16), (1536, 7), (1536, 8),
+                                 (2048, 12), (2048, 13), (2048, 17), (2048, 18), (2816, 21), (2816, 22), (5120, 33), (5120, 34)])
+def test_router_chains_at_the_lines(orc, synth, H, B):
+    test_router_chains_with_hard_rows_vs_oracle(orc, synth, H, B, False)
+
+
+@pytest.mark.parametrize("H,most", [(64, 15), (512, 15), (1600, 15), (2048, 17), (2816, 21), (5120, 33), (5184, 0)])
+def test_form_follows_from_chains_and_length(synth, H, most):
+    import torch
+    assert torch.cuda.get_device_properties(0).multi_processor_count == 148
+    E, K, B = 48, 4, most + 1
+    st = stack_mod().MoeStack(B, H, 64, E, K)
+    st.add_layer(synth.make_q4_moe_layer(690 + H, hidden=H, inter=64, n_experts=E, topk=K))
+    x = torch.randn(B, H, device="cuda")
+    sel, w = torch.zeros(B * K, dtype=torch.int32, device="cuda"), torch.zeros(B * K, device="cuda")
+    assert st.layer_route(0, x.data_ptr(), B, sel.data_ptr(), w.data_ptr()) == 0
+    for rows in range(max(1, most), B + 1):
+        def call(stream):
+            assert st.layer_route(0, x.data_ptr(), rows, sel.data_ptr(), w.data_ptr(), router_input_ready=True, stream=stream) == 0
+        grids = [grid for _, grid in captured_kernels(call)]
+        assert ((E, rows, 1) in grids) == (rows <= most), (H, rows, grids)
     st.close()
 
 

@@ -502,21 +502,34 @@ static cudaError_t launch_glue_warps(const GlueArgs& a, int rows, int sms, cudaS
     return launched();
 }
 
-// Most rows for which the block-per-row form is the faster one.  It takes a full round of the chip for every `at_once` rows
-// (one block per SM; four of 256 threads for narrow rows), the warp form about as long for one row as for several hundred.
-// Measured with 148 SMs and four selections (one launch, us, block / warp form, one sum and two): 1024 columns 296 rows 5.5 / 8.6 and
-// 8.5 / 11.2, 592 rows 8.7 / 8.8 and 12.2 / 11.7; 2048 columns 148 rows 7.7 / 12.7 and 10.3 / 18.9, 256 rows 13.2 / 12.6 and
-// 18.8 / 18.8; 2816 columns 296 rows 13.8 / 16.7 and 19.5 / 26.7, 320 rows 19.2 / 16.8 and 27.7 / 27.0; 5120 columns 256 rows
-// 17.6 / 22.9 and 25.5 / 37.1, 320 rows 24.2 / 23.0 and 35.8 / 37.3; 6144 columns 444 rows 27.0 / 29.2 and 41.8 / 47.4, 512 rows
-// 33.3 / 29.1 and 51.6 / 47.5.  Without a sum the block form's rounds are three times shorter: 2816 columns and eight selections, 320
-// rows 10.4 / 12.4, 512 rows 13.8 / 12.4.
+// Most rows for which the block-per-row form is the faster one.  It takes a full round of the chip for every round of blocks (one
+// per SM; four of 256 threads for rows up to 1024 columns), the warp form about as long for one row as for several hundred.
+// Measured with 148 SMs, four / eight selections (one launch, us, block against warp form):
+//   two sums: 64 columns 592 rows 6.3 against 6.7 / 6.5 against 6.7, 740 rows 8.8 against 6.8; 1024 columns 592 rows 12.4 against
+//   11.6 / 12.7 against 12.6; 1536 columns 160 rows 16.8 against 14.7 / 18.3 against 16.7; 1792 columns 160 rows - / 17.4 against 18.8;
+//   2816 columns 296 rows 19.2 against 26.3 / 20.2 against 29.0, 320 rows 27.3 against 26.8 / 28.4 against 29.3; 4096 columns 444
+//   rows 30.8 against 31.1 / 33.1 against 35.1; 4160 columns 296 rows 25.4 against 31.1, 320 rows 34.4 against 31.0; 5120 columns 296
+//   rows 25.8 against 37.2 / 31.5 against 39.3, 320 rows 35.9 against 37.1 / 43.2 against 39.3; 6144 columns 444 rows 40.7 against 47.1 /
+//   54.8 against 66.0, 480 rows 50.9 against 47.5 / 69.1 against 70.0;
+//   one sum: 1024 columns 592 rows 8.7 against 8.5 / 8.4 against 10.3; 2048 columns 160 rows 12.1 against 12.6 / 12.9 against 14.6,
+//   256 rows 13.3 against 12.6 / 13.9 against 14.6; 2816 columns 296 rows 13.8 against 16.7 / 14.8 against 20.8, 320 rows 19.2 against
+//   16.8 / 19.6 against 20.8; 5120 columns 296 rows 17.7 against 22.9 / 22.3 against 24.9; 6144 columns 444 rows 27.0 against 29.0 /
+//   39.4 against 43.3;
+//   no sum: 1024 columns 592 rows 4.4 against 4.5 / 4.9 against 6.5, 888 rows 5.9 against 6.2 / 6.5 against 6.6, 1184 rows 7.2 against
+//   6.4 / 8.1 against 6.7; 1088 columns 160 rows 6.6 against 6.3 / 7.1 against 6.4; 2048 columns 296 rows 7.0 against 6.4 / 7.7 against
+//   8.5; 2816 columns 296 rows 7.1 against 8.4 / 8.0 against 12.5, 444 rows 10.2 against 8.5 / 11.6 against 12.5; 5120 columns 160
+//   rows 8.2 against 8.4 / 12.6 against 10.6; 6144 columns 296 rows 9.0 against 10.6 / 14.4 against 16.7.
 static int glue_block_rows(const GlueArgs& a, int sms) {
-    const int at_once = a.n <= 1024 ? 4 * sms : sms;
     const int sums = (a.norm_w != nullptr) + (a.router_scale != nullptr);
-    int rounds = a.n <= 1024 || (a.n > 4096 && a.n <= 5120) ? 1 : 2;
-    if (sums == 1) rounds = a.n <= 2048 ? 1 : (a.n <= 5120 ? 2 : 3);
-    if (sums == 0 && a.n <= 4096) rounds++;
-    return rounds * at_once;
+    if (sums == 0) {
+        const bool many = a.topk > 4;
+        if (a.n <= 1024) return (many ? 6 : 4) * sms;
+        if (many && a.n > 2048 && a.n <= 2816) return 3 * sms;      // above 2816 columns fewer warp-form blocks share an SM
+        return (a.n < 2048 || (a.n == 2048 && !many) || (a.n > 4096 && a.n <= 5120) ? 1 : 2) * sms;
+    }
+    if (a.n <= 1024) return 4 * sms;
+    const int rounds = a.n <= (sums == 2 ? 1664 : 2048) ? 1 : (a.n <= 5120 ? 2 : 3);
+    return rounds * sms;
 }
 
 cudaError_t launch_glue(const GlueArgs& a, int rows, cudaStream_t stream) {

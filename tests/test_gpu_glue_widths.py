@@ -12,9 +12,15 @@ pytestmark = pytest.mark.gpu
 SMS = 148
 
 
-def _stack(synth, n, rows, norm=True):
-    st = stack_mod().MoeStack(rows, n, 64, 4, 2)
-    layers = [synth.make_q4_moe_layer(800 + n + i, hidden=n, inter=64, n_experts=4, topk=2) for i in range(2)]
+def _line(n):
+    """Most rows that the block form takes with two in-order sums."""
+    return (4 if n <= 1024 else 1 if n <= 1664 else 2 if n <= 5120 else 3) * SMS
+
+
+def _stack(synth, n, rows, norm=True, topk=2):
+    experts = max(4, topk)
+    st = stack_mod().MoeStack(rows, n, 64, experts, topk)
+    layers = [synth.make_q4_moe_layer(800 + n + i, hidden=n, inter=64, n_experts=experts, topk=topk) for i in range(2)]
     for layer in layers:
         layer.router_scale[:] = 1.0 + 0.01 * np.arange(n) / n
         st.add_layer(layer, with_norm=norm)
@@ -24,7 +30,7 @@ def _stack(synth, n, rows, norm=True):
 @pytest.mark.parametrize("n", [64, 192, 256, 320, 1024, 1088, 2048, 2816, 2880, 3072, 3328, 4096, 5056, 6144])
 @pytest.mark.parametrize("extra", [0, 1, 6])
 def test_rows_vs_oracle(orc, synth, n, extra):
-    rows = (4 if n <= 1024 else 1 if 4096 < n <= 5120 else 2) * SMS + extra       # the line, and row remainders above it
+    rows = _line(n) + extra                                  # the line, and row remainders above it
     st, layers = _stack(synth, n, rows)
     import torch
     x = synth.make_tokens(801 + n, rows, n)
@@ -46,10 +52,10 @@ def test_rows_vs_oracle(orc, synth, n, extra):
     st.close()
 
 
-@pytest.mark.parametrize("n", [64, 1024, 1088, 2048, 2816, 3072, 4096, 4160, 5120, 6080])
+@pytest.mark.parametrize("n", [64, 1024, 1088, 1664, 1728, 2048, 2816, 3072, 4096, 4160, 5120, 5184, 6080])
 def test_form_follows_from_sizes(synth, n):
     import torch
-    line = (4 if n <= 1024 else 1 if 4096 < n <= 5120 else 2) * SMS
+    line = _line(n)
     assert torch.cuda.get_device_properties(0).multi_processor_count == SMS
     st, _ = _stack(synth, n, line + 1)
     for rows, blocks in ((line, line), (line + 1, (line + 4) // 4)):
@@ -108,4 +114,30 @@ def test_form_of_one_sum(orc, synth, n, rounds):
         for t in (0, rows // 2, rows - 1):
             want, _, _ = orc.moe_layer_q4(layers[0], x[t:t + 1], threads=4)
             assert_bits_equal(y[t].cpu().numpy(), orc.rmsnorm(want[0], layers[0].norm_weight, layers[0].eps, True)[1], f"row {t} of {rows} x {n}")
+    st.close()
+
+
+@pytest.mark.parametrize("n,topk,rounds", [(64, 2, 4), (1024, 2, 4), (1088, 2, 1), (2048, 2, 1), (2112, 2, 2), (4096, 2, 2), (4160, 2, 1), (5120, 2, 1),
+                                           (5184, 2, 2), (6144, 2, 2), (1024, 5, 6), (1088, 5, 1), (2048, 5, 2), (2112, 5, 3), (2816, 5, 3),
+                                           (2880, 5, 2), (5120, 5, 1)])
+def test_form_without_a_sum(orc, synth, n, topk, rounds):
+    """The reduce alone: both sides of its line."""
+    import torch
+    line = rounds * SMS
+    st, layers = _stack(synth, n, line + 1, topk=topk)
+    for rows, blocks in ((line, line), (line + 1, (line + 4) // 4)):
+        x = synth.make_tokens(840 + n, rows, n)
+        d_x, y = torch.from_numpy(x).cuda(), torch.zeros(rows, n, device="cuda")
+        assert st.layer_experts(0, d_x.data_ptr(), rows) == 0
+        torch.cuda.synchronize()
+
+        def call(stream):
+            assert st.layer_combine(0, rows, y.data_ptr(), apply_norm=False, stream=stream) == 0
+        (name, grid), = captured_kernels(call)
+        assert grid == (blocks, 1, 1), (name, n, rows)
+        call(torch.cuda.current_stream().cuda_stream)
+        assert st.status() == 0
+        for t in (0, rows // 2, rows - 1):
+            want, _, _ = orc.moe_layer_q4(layers[0], x[t:t + 1], threads=4)
+            assert_bits_equal(y[t].cpu().numpy(), want[0], f"row {t} of {rows} x {n}")
     st.close()

@@ -85,7 +85,9 @@ static __device__ __forceinline__ float serial_sum(const float* sq, int n) {
 //      table has no answer it takes the four segments one by one, and where a segment has none, term by term.
 // So the predictions decide only how much runs side by side: every result is a real addition of the chain, or one shifted
 // by an amount that is proven to pass through it.  Just under 1 % of the segments of a router row have no answer (mostly
-// where the sum passes zero and its binade changes with every step), hardly any of squares.
+// where the sum passes zero and its binade changes with every step), hardly any of squares.  The sixth such segment takes the
+// rest of the chain with it, so that terms of which nothing can be tabulated (pairs that cancel) take at most half as long again
+// as a chain: 2816 of them 17 400 cycles, 26 500 without that limit, 12 100 as a chain by one warp.
 // What bounds it: the additions of 2 (n / 32 dependent ones, six side by side, about 10 cycles each), those of segments
 // without an answer (600 cycles each with what it takes to get there), 60 to 130 cycles per look into a table, five or six barriers
 // with a scan or two between them.  Measured in a block of 640 threads (B200): 2816 squares 4000 cycles, where integer increments
@@ -96,6 +98,7 @@ static __device__ __forceinline__ float serial_sum(const float* sq, int n) {
 // p and scratch (ORDERED_SCRATCH words): shared memory, 16-byte aligned; p written by the block, no barrier needed before the
 // call.  At least 256 threads, whole warps; every thread of the block must call; all return the sum.
 constexpr int ORDERED_CANDS = 16;
+constexpr int ORDERED_MISSES = 6;                         // segments without an answer, the last of them with all that follow
 constexpr int ORDERED_PITCH = 20;                         // floats per table: candidates' ends, the sentinels', bank offset
 constexpr int ORDERED_GROUP = 4, ORDERED_GROUPS = 32 / ORDERED_GROUP;
 constexpr int ORDERED_SCRATCH = 8 + 2 * 4 * 32 + 4 * 32 + 2 * 32 + 32 + 2 * ORDERED_GROUPS + (32 + ORDERED_GROUPS) * ORDERED_PITCH;
@@ -306,6 +309,7 @@ static __device__ __forceinline__ float block_sum_ordered(float* p, int n, int r
         }
         float4 seg = shared_f4(base + 4 * SEG);
         float2 lohi = shared_f2(base + 4 * GBETWEEN);
+        int missed = 0;
 #pragma unroll 1
         for (int i = all_known ? ORDERED_GROUPS : 0; i < ORDERED_GROUPS; i++) {
             const int t0 = ORDERED_GROUP * i, n0 = min(t0 + ORDERED_GROUP, 31), ni = min(i + 1, ORDERED_GROUPS - 1);
@@ -321,8 +325,15 @@ static __device__ __forceinline__ float block_sum_ordered(float* p, int n, int r
                     after = s;
                     if (!ordered_step(after, seg, own, base + 4 * (ENDS + t * ORDERED_PITCH), false)) {
                         after = s;
-                        const int at = __float_as_int(seg.w), count = at & 0xffff;
-                        for_terms(terms + 16 * (at >> 16), zeros, count, count, [&](float v) { after = __fadd_rn(after, v); });
+                        missed++;
+                        const int at = __float_as_int(seg.w), first = at >> 16;
+                        int count = at & 0xffff;
+                        if (missed >= ORDERED_MISSES) {              // the rest of the chain
+                            count = all - first;
+                            t = 31;
+                            i = ORDERED_GROUPS;
+                        }
+                        for_terms(terms + 16 * first, zeros, count, count, [&](float v) { after = __fadd_rn(after, v); });
                     }
                     s = after;
                     seg = one_seg;

@@ -121,6 +121,37 @@ def test_router_chains_with_hard_rows_vs_oracle(orc, synth, H, B, fused):
     st.close()
 
 
+# Every pair of products nearly cancels (from the first, from the middle or but for the last columns): segments without an answer up to their limit and past it.
+@pytest.mark.parametrize("H,B,fused", [(896, 1, True), (2816, 1, True), (960, 2, False), (2816, 3, False), (5120, 2, False)])
+def test_router_chains_of_cancelling_pairs_vs_oracle(orc, synth, H, B, fused):
+    import torch
+    E, K = 12, 4
+    layer = synth.make_q4_moe_layer(700 + H, hidden=H, inter=64, n_experts=E, topk=K)
+    rng = np.random.default_rng(701 + H)
+    w = rng.standard_normal((E, H))
+    for e in range(E):
+        lo, hi = [(0, H), (H // 2 + 2 * (e // 3), H), (0, H - 64 * (e // 3 + 1))][e % 3]
+        w[e, lo + 1:hi:2] = -w[e, lo:hi - 1:2] * (1.0 + 1e-6 * rng.standard_normal((hi - lo) // 2))
+    layer.router_w[:] = w.astype(np.float32)
+    layer.router_scale[:] = 1.0
+    st = stack_mod().MoeStack(B, H, 64, E, K)
+    st.add_layer(layer)
+    d_x = torch.ones(B, H, device="cuda")
+    d_y = torch.zeros_like(d_x)
+    if fused:
+        assert st.forward_device(d_x.data_ptr(), B, d_y.data_ptr()) == 0
+    else:
+        assert st.layer_experts(0, d_x.data_ptr(), B) == 0
+    assert st.status() == 0
+    got = d2h(st.workspace().logits, B * E, np.float32).reshape(B, E)
+    rc, rin = orc.router_input(np.ones(H, np.float32), layer.router_scale, layer.eps)
+    assert rc == 0
+    want = orc.router_scores(layer.router_w, None, rin)
+    for t in range(B):
+        assert_bits_equal(got[t], want, f"logits of row {t} over {H} columns")
+    st.close()
+
+
 # Both sides of the lines (148 SMs): one warp adds a chain of up to 832 columns (squares: 576), of more where more chains share an SM;
 # a block per chain up to so many chains, the kernel of a chain per lane above.
 @pytest.mark.parametrize("H,B", [(512, 15), (512, 16), (576, 1), (640, 1), (832, 2), (896, 2), (1024, 3), (1024, 4), (1024, 16), (1536, 7), (1536, 8),

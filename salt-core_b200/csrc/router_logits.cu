@@ -328,11 +328,11 @@ cudaError_t launch_many(const float* W, const float* x, float* logits, int rows,
 }
 
 // ---- few chains: a block per (expert, row).  All its threads form the products, coalesced, in shared memory and add
-// them together (block_sum_ordered) or, in_chains = the number of SMs, one of its warps does, another one in each round of blocks.
+// them together (block_sum_ordered) or, WARP, one of its warps does, another one in each round of blocks (of `sms`).
 constexpr int CHAIN_THREADS = 256;
-template <int N4>                             // 16-byte pieces per thread
+template <int N4, bool WARP>                  // N4: 16-byte pieces per thread
 __global__ void __launch_bounds__(CHAIN_THREADS)
-router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict__ x, float* __restrict__ logits, int E, int H, int in_chains) {
+router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict__ x, float* __restrict__ logits, int E, int H, int sms) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ __align__(16) uint32_t scratch[ORDERED_SCRATCH];
     const int e = blockIdx.x, r = blockIdx.y, n4 = H >> 2;
@@ -359,7 +359,7 @@ router_logits_chain_kernel(const float* __restrict__ W, const float* __restrict_
                                              __fmul_rn(w[i].w, v[i].w));
     }
     float acc;
-    if (in_chains > 0) acc = block_sum_chain((const float*)smem, H, scratch, (int)((blockIdx.y * gridDim.x + blockIdx.x) / in_chains) & 3);
+    if constexpr (WARP) acc = block_sum_chain((const float*)smem, H, scratch, (int)((blockIdx.y * gridDim.x + blockIdx.x) / sms) & 3);
     else acc = block_sum_ordered((float*)smem, H, 2, scratch);
     if (threadIdx.x == 0) logits[(size_t)r * E + e] = __fadd_rn(acc, 0.0f);
 }
@@ -382,12 +382,11 @@ cudaError_t launch_router_logits(const float* W, const float* x, float* logits, 
         // 832 columns, or 700 and 330 more per chain and SM, while all blocks fit at once.  In pieces / as chains (us, chains per
         // SM): 1024 columns 0.9: 7.2 / 7.4, 2.6: 8.2 / 7.2, 4.3: 9.1 / 7.9; 1536 columns 1.7: 8.0 / 8.4, 2.6: 8.6 / 8.5, 4.3: 10.9 / 10.2;
         // 2048 columns 2.6: 9.1 / 9.9, 3.5: 10.0 / 10.0, 4.3: 10.9 / 10.7, 5.2: 12.3 / 14.8; 2816 columns 4.3: 11.7 / 13.0.
-        const int in_chains = chains <= 5L * sms && (H <= 832 || (H - 700) * (long)sms <= 330 * chains) ? sms : 0;
-        const dim3 grid(E, rows);
-        const size_t smem = (size_t)H * 4;
-        if (H <= 3 * 4 * CHAIN_THREADS)
-            return launch_pdl(router_logits_chain_kernel<3>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H, in_chains);
-        return launch_pdl(router_logits_chain_kernel<5>, grid, dim3(CHAIN_THREADS), smem, stream, W, x, logits, E, H, in_chains);
+        static_assert(3 * 4 * CHAIN_THREADS >= 700 + 5 * 330, "chains by one warp: three pieces per thread");
+        const bool warp = chains <= 5L * sms && (H <= 832 || (H - 700) * (long)sms <= 330 * chains);
+        const auto kernel = warp ? router_logits_chain_kernel<3, true>
+                                 : (H <= 3 * 4 * CHAIN_THREADS ? router_logits_chain_kernel<3, false> : router_logits_chain_kernel<5, false>);
+        return launch_pdl(kernel, dim3(E, rows), dim3(CHAIN_THREADS), (size_t)H * 4, stream, W, x, logits, E, H, sms);
     }
     // one chain per lane while one round of blocks holds them all, then as many per lane as keep it to one round
     const long few = (long)((E + FEW_E - 1) / FEW_E) * ((rows + FEW_ROWS - 1) / FEW_ROWS);

@@ -231,7 +231,7 @@ static bool run_jobs(int n, int njobs, size_t x_bytes, int max_rows, int max_tok
     if (!stage_upload((size_t)n * sizeof(Q4Job), x_bytes, "job and x upload")) return false;
     if (bits == 8) {
         if (!cuda_ok(launch_q8_jobs(dj, njobs, max_rows, max_tok, C, B.stream), "q8 launch")) return false;
-    } else if (!cuda_ok(launch_q4_jobs(dj, njobs, nullptr, max_rows, max_tok, C, nmat, aligned, B.stream), "q4 launch"))
+    } else if (!cuda_ok(launch_q4_jobs(dj, njobs, nullptr, max_rows, max_tok, C, nmat, aligned, B.stream, -1, true), "q4 launch"))
         return false;
     return true;
 }
@@ -899,7 +899,7 @@ int salt_gpu_proj_batch_indexed(const uint32_t* vals, const uint16_t* scales, co
     B.in_flight = true;
     fill_job(*hj, *t, dx, (float*)output->backend + y_float_offset + (size_t)first_job * R, job_count, C, R);
     if (!cuda_ok(cudaMemcpyAsync(dj, hj, sizeof(Q4Job), cudaMemcpyHostToDevice, B.stream), "job upload") ||
-        !cuda_ok(launch_q4_jobs(dj, 1, nullptr, R, job_count, C, 1, (C % 64) == 0, B.stream), "launch"))
+        !cuda_ok(launch_q4_jobs(dj, 1, nullptr, R, job_count, C, 1, (C % 64) == 0, B.stream, -1, true), "launch"))
         return -1;
     count_kinds(kind == SALT_GPU_RESOURCE_TRUNK, kind == SALT_GPU_RESOURCE_EXPERT_LAYER,
                 kind == SALT_GPU_RESOURCE_ARENA);
@@ -1073,7 +1073,7 @@ int salt_gpu_q4_selected_shared(const SaltGpuSelectedProjectionJob* jobs, int jo
             aligned = aligned && aligned_by_desc[(size_t)n1];
             n1++;
         }
-        if (!cuda_ok(launch_q4_jobs(dj + n0, n1 - n0, nullptr, max_rows, max_tok, C, 1, aligned, B.stream),
+        if (!cuda_ok(launch_q4_jobs(dj + n0, n1 - n0, nullptr, max_rows, max_tok, C, 1, aligned, B.stream, -1, true),
                      "selected launch"))
             return -1;
         n0 = n1;

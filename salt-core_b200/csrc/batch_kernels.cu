@@ -512,12 +512,14 @@ bool two_rows_per_lane(int fmt, long blocks) { return blocks < (fmt == FMT_Q4 ? 
 bool q4_batch_supported(int C, int nmat) { return C >= 64 && (C % 64) == 0 && batch_geom(FMT_Q4, C, nmat, 4).smem <= 225 * 1024; }
 
 cudaError_t launch_q4_batch(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
-                            int nmat, cudaStream_t stream, int pdl) {
+                            int nmat, cudaStream_t stream, int pdl, bool alone) {
     const long blocks = (long)((max_rows + 64 / nmat - 1) / (64 / nmat)) * njobs_max * ((max_tok + MAX_T - 1) / MAX_T);
     const bool two = two_rows_per_lane(FMT_Q4, blocks);
 #define SB_BATCH(NM, RL) launch_batch<FMT_Q4, NM, RL>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, pdl)
-    // one matrix for a host call, few blocks: nothing else is in the instruction cache
-    if (nmat == 1 && two && njobs_dev == nullptr)
+    // One projection by itself, few blocks: its code does not share the instruction cache with another variant's, two groups per
+    // iteration are the shorter loop (from the host, one / two groups: 4096 x 4096 1 token 29.6 / 29.1 us, 4 tokens 61.9 / 60.2, 16 tokens
+    // 119 / 118).  Behind a gate/up launch they are not: chain of four one-token experts 40.9 / 42.3, whole block of 4 tokens 149.0 / 150.7.
+    if (nmat == 1 && two && alone)
         return launch_batch<FMT_Q4, 1, 2, 2>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, pdl);
     if (nmat == 2) return two ? SB_BATCH(2, 2) : SB_BATCH(2, 4);
     return two ? SB_BATCH(1, 2) : SB_BATCH(1, 4);
@@ -530,9 +532,10 @@ cudaError_t launch_fp4_batch(const Fp4Job* jobs, int njobs_max, const int* njobs
                              cudaStream_t stream) {
     const long blocks = (long)((max_rows + 63) / 64) * njobs_max * ((max_tok + MAX_T - 1) / MAX_T);
     if (!two_rows_per_lane(FMT_FP4, blocks)) return launch_batch<FMT_FP4, 1, 4>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, 1);
-    // Host calls (jobs of a stack are passes already): two tokens a pass where even that leaves room for two blocks per SM: a block's products are a chain of chunks, shorter with
-    // fewer tokens.  From the host, four / two tokens a pass: 1536 rows x 5120, 4 tokens 49.3 / 43.8 us, 7 tokens 52.8 / 51.2; 200 x
-    // 5120, 16 tokens 60.8 / 55.5; 6000 x 2048, 7 tokens (five blocks per SM) 46.8 / 49.5.
+    // Jobs of whole groups (their number is the host's): two tokens a pass where even that leaves room for two blocks per SM: a
+    // block's products are a chain of chunks, shorter with fewer tokens.  Jobs numbered on the device are passes already.  From the
+    // host, four / two tokens a pass: 1536 rows x 5120, 4 tokens 49.3 / 43.8 us, 7 tokens 52.8 / 51.2; 200 x 5120, 16 tokens 60.8 /
+    // 55.5; 6000 x 2048, 7 tokens (five blocks per SM) 46.8 / 49.5.
     const bool two = njobs_dev == nullptr && (long)((max_rows + 31) / 32) * njobs_max * ((max_tok + 1) / 2) <= 2L * device_sms();
     return launch_batch<FMT_FP4, 1, 2>(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, stream, 1, two ? 2 : MAX_T);
 }

@@ -34,8 +34,9 @@ constexpr size_t PLAIN_DYNAMIC_SMEM = 42 * 1024;
 // pdl: -1 ordinary launch; 0 programmatic dependent launch, the jobs come from the previous
 // kernel; 1 the same but the jobs (and njobs_dev) were written at least two launches back, so
 // the weights are prefetched while the previous kernel is still running.
+// alone: a call's only projection launch, with none of another kind right before or after it.
 cudaError_t launch_q4_jobs(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
-                           int nmat, bool aligned, cudaStream_t stream, int pdl = -1);
+                           int nmat, bool aligned, cudaStream_t stream, int pdl = -1, bool alone = false);
 // Do these jobs run on a kernel whose results leave the chip as whole lines?
 bool q4_stores_lines(int C, int nmat, bool aligned);
 
@@ -45,7 +46,7 @@ struct Fp4Job;
 constexpr int Q4_PASS_TOKENS = 4;        // tokens that share one dequantisation
 bool q4_batch_supported(int C, int nmat);
 cudaError_t launch_q4_batch(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
-                            int nmat, cudaStream_t stream, int pdl);
+                            int nmat, cudaStream_t stream, int pdl, bool alone);
 bool fp4_batch_supported(int C);
 // Programmatic dependent launch of the kernel before it, which writes the activations; jobs and njobs_dev were written at least two
 // launches back.

@@ -1290,7 +1290,7 @@ int salt_b200_q4_matvec_device(const void* d_vals, const void* d_scales, const v
     const bool aligned = (C % 64) == 0 &&
                          ((((uintptr_t)d_vals | (uintptr_t)d_scales | (uintptr_t)d_biases | (uintptr_t)d_x) & 15) == 0);
     if (!cuda_ok(cudaMemcpyAsync(d_job, &j, sizeof j, cudaMemcpyHostToDevice, (cudaStream_t)stream), "job upload") ||
-        !cuda_ok(launch_q4_jobs(d_job, 1, nullptr, R, B, C, 1, aligned, (cudaStream_t)stream), "launch"))
+        !cuda_ok(launch_q4_jobs(d_job, 1, nullptr, R, B, C, 1, aligned, (cudaStream_t)stream, -1, true), "launch"))
         return -1;
     return 0;
 }

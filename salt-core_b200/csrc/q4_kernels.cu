@@ -56,10 +56,10 @@ q4_generic_kernel(const Q4Job* __restrict__ jobs, const int* __restrict__ njobs_
 bool q4_stores_lines(int C, int nmat, bool aligned) { return aligned && q4_batch_supported(C, nmat); }
 
 cudaError_t launch_q4_jobs(const Q4Job* jobs, int njobs_max, const int* njobs_dev, int max_rows, int max_tok, int C,
-                           int nmat, bool aligned, cudaStream_t stream, int pdl) {
+                           int nmat, bool aligned, cudaStream_t stream, int pdl, bool alone) {
     if (njobs_max < 1 || max_rows < 1 || max_tok < 1) return cudaSuccess;
     if (q4_stores_lines(C, nmat, aligned))
-        return launch_q4_batch(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, nmat, stream, pdl);
+        return launch_q4_batch(jobs, njobs_max, njobs_dev, max_rows, max_tok, C, nmat, stream, pdl, alone);
     dim3 grid((max_rows + 3) / 4, max_tok, njobs_max);
     if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
     if (nmat == 2) q4_generic_kernel<2><<<grid, 128, 0, stream>>>(jobs, njobs_dev);

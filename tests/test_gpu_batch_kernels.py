@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 
 from conftest import assert_bits_equal
-from gpu_util import backend_mod, gpu
+from gpu_util import backend_mod, gpu, stack_mod
+from graph_util import captured_kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -61,3 +62,21 @@ def test_nvfp4_batch_projection_vs_oracle(orc, synth, R, C):
             assert rc == 0
             assert_bits_equal(ys[t], want, f"nvfp4 {R}x{C} token {t} of {B}")
     assert g.weight_resource_unbind(bm.RESOURCE_EXPERT_LAYER, 97) == 0
+
+
+def test_down_of_a_whole_block_shares_the_layers_kernel(synth):
+    """The dense down product of a block runs the kernel of the routed one, not the one for a projection by itself (the last template
+    argument: groups per iteration)."""
+    import torch
+    H, M, E, K, B = 256, 64, 8, 2, 2
+    st = stack_mod().MoeStack(B, H, M, E, K)
+    st.add_layer(synth.make_q4_moe_layer(91, hidden=H, inter=M, n_experts=E, topk=K))
+    assert st.attach_ffn_block(0, synth.make_ffn_block(92, hidden=H, dense_inter=128)) == 0
+    x = torch.randn(B, H, device="cuda")
+    y = torch.zeros_like(x)
+
+    def call(stream):
+        assert st.ffn_block_forward(0, x.data_ptr(), B, y.data_ptr(), stream=stream) == 0
+    names = [name for name, _ in captured_kernels(call) if "batch_kernel" in name]
+    assert len(names) == 4 and names[1] == names[3] and "ILi0ELi1ELi2ELi1E" in names[1], names
+    st.close()

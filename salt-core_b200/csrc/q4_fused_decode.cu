@@ -466,7 +466,7 @@ static __host__ __device__ __forceinline__ LayerScratch layer_scratch(int H, int
     L.lit = L.pes + ((E + 3) & ~3);              // ... and literal-dequantisation flags, fetched before the grid dependency
     L.topk = L.lit + ((E + 3) & ~3);
     L.scan = L.topk + topk_scratch_floats(E, topk);       // a multiple of four floats, as all before it
-    L.end = L.scan + ORDERED_SCRATCH;
+    L.end = L.scan + (sum_in_chain(H, 1) ? CHAIN_SCRATCH : ORDERED_SCRATCH);
     return L;
 }
 

@@ -161,7 +161,9 @@ static __device__ __forceinline__ bool ordered_step(float& s, const float4& seg,
     return ((int)(shift == 0.0f) | (in & whole)) & (in | (int)!inside) & (int)(s == s);
 }
 
-// The same sum, in one chain, by warp `who` (blocks of an SM that take different warps add on different schedulers).
+// The same sum, in one chain, by warp `who` (blocks of an SM that take different warps add on different schedulers).  scratch:
+// CHAIN_SCRATCH words are enough.
+constexpr int CHAIN_SCRATCH = 8;
 static __device__ __forceinline__ float block_sum_chain(const float* p, int n, uint32_t* scratch, int who) {
     float* const result = (float*)scratch + 4;              // where the pieces leave theirs, too
     __syncthreads();
@@ -177,7 +179,7 @@ static __device__ __forceinline__ float block_sum_chain(const float* p, int n, u
 // Terms up to which that is the shorter way for a block by itself: the pieces cost 2800 (squares) or 3700 cycles (products)
 // whatever their length, a chain 460 and 4.15 a term.  Block of 640 threads, chain / pieces: 576 squares 2860 / 2990, 640 3120 /
 // 2990; 768 products 3650 / 4370, 832 3910 / 4010, 896 4180 / 4140.
-static __device__ __forceinline__ bool sum_in_chain(int n, int rounds) { return n <= (rounds == 1 ? 576 : 832); }
+static __host__ __device__ __forceinline__ bool sum_in_chain(int n, int rounds) { return n <= (rounds == 1 ? 576 : 832); }
 
 static __device__ __forceinline__ float block_sum_ordered(float* p, int n, int rounds, uint32_t* scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -6,6 +6,7 @@ import pytest
 
 from conftest import assert_bits_equal
 from gpu_util import oracle_stack, stack_mod
+from graph_util import captured_kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -125,3 +126,25 @@ def test_whole_pass_in_one_launch_equals_per_layer_launches_and_oracle(orc, synt
 def test_rounds_and_slots(orc, synth, geom):
     test_whole_pass_in_one_launch_equals_per_layer_launches_and_oracle(orc, synth, geom)
     test_fused_decode_equals_two_launch_form_and_oracle(orc, synth, geom[:4], 1)
+
+
+@pytest.mark.parametrize("E", [8, 140, 170, 230])
+def test_narrow_layers_of_many_experts_are_one_launch(orc, synth, E):
+    """The scratch of a layer's first phases has to fit where its weight rows will be, which is little at 64 columns."""
+    import torch
+    H, M, K = 64, 64, 4
+    layer = synth.make_q4_moe_layer(360 + E, hidden=H, inter=M, n_experts=E, topk=K)
+    st = stack_mod().MoeStack(1, H, M, E, K)
+    st.add_layer(layer)
+    x = synth.make_tokens(361 + E, 1, H)
+    d_x = torch.from_numpy(x).cuda()
+    d_y = torch.zeros_like(d_x)
+
+    def call(stream):
+        assert st.forward_device(d_x.data_ptr(), 1, d_y.data_ptr(), stream=stream) == 0
+    names = [name for name, _ in captured_kernels(call)]
+    assert any("q4_layer_decode_kernel" in name for name in names), names
+    call(torch.cuda.current_stream().cuda_stream)
+    want, _, _ = orc.moe_layer_q4(layer, x, threads=4)
+    assert_bits_equal(d_y.cpu().numpy(), want, f"{E} experts")
+    st.close()

@@ -24,9 +24,9 @@
 //     pass' tokens is spread over the lanes, instead of running on one lane in sixteen.
 //
 // What bounds it now: issue cycles.  Per row, lane and 32-column step a token takes four packed operations, each of which
-// holds a scheduler for two cycles.  At 64 tokens (gate/up) 63 of 196 M warp instructions are these: 43 % of the launch's
+// holds a scheduler for two cycles.  At 64 tokens (gate/up) 63 of 193 M warp instructions are these: 43 % of the launch's
 // cycles; the others (dequantisation once per pass and row, activation loads, the blocks' tables, prologues and folds) are
-// another 45 %.  At 16 tokens, where nearly every pass holds one or two, the products are 16 of 67 M.  Measured
+// another 44 %.  At 16 tokens, where nearly every pass holds one or two, the products are 16 of 65 M.  Measured
 // (hidden 2816, inter 704, 128 experts, top-8; gate/up + down of a layer, event pairs): 64 tokens 698 -> 409 us, 16 tokens
 // 274 -> 150 us, 6 tokens 140 -> 87 us against two rows per lane and whole groups as blocks; 2 tokens 44 us, where one
 // persistent launch for both phases took 51.

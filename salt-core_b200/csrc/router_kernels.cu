@@ -3,7 +3,7 @@
 // Everything here is bit-exact against the reference CPU functions; the reference arithmetic
 // contains several chains that are serial by definition (sums of squares, router logits,
 // softmax denominators).  Many chains run side by side, each added by a lane; where few are asked for, the whole block
-// adds one (block_sum_ordered).
+// adds one (block_sum_ordered) or, a short one, one of its warps does.
 #include <cooperative_groups.h>
 #include "internal.h"
 #include "pdl.cuh"
@@ -72,8 +72,8 @@ norm_rows_kernel(const float* __restrict__ x, const float* __restrict__ weight, 
 //   [norm]    v = RMSNorm(v) * norm_w                      (gemma4.c:85-101)
 //             y_out = v  (written whenever reduce or norm ran)
 //   [router]  rin = ((v * inv) * scale) * (1/sqrt(n))      (gemma4.c:103-130)
-// The two sums of squares are formed in element order by block_sum_ordered over
-// squares computed in parallel.
+// The two sums of squares are formed in element order over squares computed in
+// parallel (row_sum_of_squares).
 // ---- affine 8-bit matvec (router projections of packages that quantise the router) -----------
 // src/kernels.c:343-369: one byte per element, bf16 scale / bias per 64 consecutive elements of
 // the flattened matrix (rows may straddle groups), ONE serial chain per row:

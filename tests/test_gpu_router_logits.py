@@ -94,8 +94,8 @@ def _hard_rows(rng, E, H):
     return w
 
 
-# One launch per layer (one token) and a block per chain (up to four rows): widths of less than a piece per segment, of odd and
-# even numbers of pieces, and the widest of each kernel.
+# One launch per layer (one token) and a block per chain: widths that one warp adds, of odd and even numbers of pieces, and the
+# widest of each kernel.
 @pytest.mark.parametrize("H,B,fused", [(64, 1, True), (192, 1, True), (2816, 1, True), (3200, 1, True), (64, 4, False), (704, 3, False),
                                        (2816, 2, False), (5120, 1, False), (5120, 4, False)])
 def test_router_chains_with_hard_rows_vs_oracle(orc, synth, H, B, fused):

@@ -11,6 +11,7 @@
 // returns -1.
 #include <cuda_runtime.h>
 #include <atomic>
+#include <climits>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -1131,7 +1132,7 @@ int salt_gpu_exact_cells(const SaltGpuExactCell* cells, int count) {
     for (int i = 0; i < count; i++) {
         const SaltGpuExactCell& c = cells[i];
         void* v[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-        if (c.n == 0) return -1;
+        if (c.n == 0 || c.n > (uint32_t)INT_MAX) return -1;         // the kernels count in int
         switch (c.kind) {
             case SALT_GPU_EXACT_RMSNORM:
                 if (c.aux > 1u || !cell_view(c.views[0], c.offsets[0], c.n, &v[0]) ||

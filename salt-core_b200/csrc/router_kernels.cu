@@ -209,7 +209,7 @@ static cudaError_t allow_row_smem(const void* kernel, size_t smem) {
 cudaError_t launch_residual_postnorm(const float* residual, const float* branch, const float* weight, float* out,
                                      int rows, int n, float eps, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
-    const size_t smem = (size_t)(2 * ((n + 3) & ~3) + 8) * sizeof(float);
+    const size_t smem = (2 * (((size_t)n + 3) & ~(size_t)3) + 8) * sizeof(float);
     const cudaError_t e = allow_row_smem((const void*)residual_postnorm_rows_kernel, smem);
     if (e != cudaSuccess) return e;
     residual_postnorm_rows_kernel<<<rows, 1024, smem, stream>>>(residual, branch, weight, out, n, eps, status);
@@ -220,7 +220,7 @@ cudaError_t launch_parallel_combine(const float* residual, const float* dense, c
                                     const float* wr, const float* wf, float* scratch_a, float* scratch_b, float* out,
                                     int rows, int n, float eps, float scalar, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
-    const size_t smem = (size_t)(n + 8) * sizeof(float);
+    const size_t smem = ((size_t)n + 8) * sizeof(float);
     const cudaError_t e = allow_row_smem((const void*)parallel_combine_rows_kernel, smem);
     if (e != cudaSuccess) return e;
     parallel_combine_rows_kernel<<<rows, 1024, smem, stream>>>(residual, dense, routed, wd, wr, wf, scratch_a, scratch_b,
@@ -553,7 +553,7 @@ cudaError_t launch_glue(const GlueArgs& a, int rows, cudaStream_t stream) {
 cudaError_t launch_rmsnorm(const float* x, const float* weight, float* y, int rows, int n, float eps, int with_scale,
                            int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
-    const size_t smem = (size_t)(2 * n + 8) * sizeof(float);
+    const size_t smem = (2 * (size_t)n + 8) * sizeof(float);
     const cudaError_t e = allow_row_smem((const void*)norm_rows_kernel<0>, smem);
     if (e != cudaSuccess) return e;
     norm_rows_kernel<0><<<rows, 256, smem, stream>>>(x, weight, y, n, eps, with_scale, 0.0f, status);
@@ -566,7 +566,7 @@ constexpr int TOPK_THREADS = 160;
 cudaError_t launch_router_input(const float* x, const float* scale, float* out, int rows, int n, float eps,
                                 float root, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
-    const size_t smem = (size_t)(2 * n + 8) * sizeof(float);
+    const size_t smem = (2 * (size_t)n + 8) * sizeof(float);
     const cudaError_t e = allow_row_smem((const void*)norm_rows_kernel<1>, smem);
     if (e != cudaSuccess) return e;
     norm_rows_kernel<1><<<rows, 256, smem, stream>>>(x, scale, out, n, eps, 1, root, status);
@@ -590,6 +590,7 @@ router_topk_kernel(const float* __restrict__ logits, const float* __restrict__ p
 cudaError_t launch_router_topk(const float* logits, const float* per_expert_scale, int32_t* selected, float* weights,
                                int rows, int E, int topk, int sort_by_expert, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
+    if (E < 1 || topk < 1 || (size_t)E + (size_t)topk > 6 * 1024) return cudaErrorInvalidValue;     // 48 KB, counted without overflow
     size_t smem = (size_t)topk_scratch_floats(E, topk) * sizeof(float);
     return launch_pdl(router_topk_kernel, dim3(rows), dim3(TOPK_THREADS), smem, stream, logits, per_expert_scale, selected, weights, E,
                       topk, sort_by_expert, status);

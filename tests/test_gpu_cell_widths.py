@@ -87,3 +87,19 @@ def test_wider_rows_are_refused():
     cell = bm.exact_cell(bm.EXACT_PARALLEL_COMBINE, [buf] * 8, [k * n for k in range(7)] + [8 * n], n, eps=1e-6, scalar=0.75)
     assert g.exact_cells([cell]) == -1
     assert g.shared_buffer_free(buf) == 0
+
+
+def test_counts_beyond_int_are_refused_on_the_host():
+    """Cells whose element counts wrap around in 32 bits, over views that claim to be large enough: no launch, no access."""
+    g, bm = gpu(), backend_mod()
+    rc, buf = g.shared_buffer_alloc(4096)
+    assert rc == 0
+    claim = bm.SharedBuffer(buf.contents, 1 << 40, buf.backend)
+    for kind in (bm.EXACT_RMSNORM, bm.EXACT_ROUTER_INPUT, bm.EXACT_RESIDUAL_POSTNORM, bm.EXACT_PARALLEL_COMBINE, bm.EXACT_SOFTCAP, bm.EXACT_TOPK):
+        for n in (0x80000000, 0x80000004, 0xfffffffc, 0xffffffff):
+            assert g.exact_cells([bm.exact_cell(kind, [claim] * 8, [0] * 8, n, aux=1, eps=1e-6, scalar=1.0)]) == -1, (kind, n)
+    for kind in (bm.EXACT_RMSNORM, bm.EXACT_ROUTER_INPUT, bm.EXACT_RESIDUAL_POSTNORM, bm.EXACT_PARALLEL_COMBINE):
+        for n in (0x40000000, 0x7ffffffd, 0x7fffffff):
+            assert g.exact_cells([bm.exact_cell(kind, [claim] * 8, [0] * 8, n, aux=1, eps=1e-6, scalar=1.0)]) == -1, (kind, n)
+    assert g.exact_cells([bm.exact_cell(bm.EXACT_TOPK, [claim] * 4, [0] * 4, (1 << 30) + 8, aux=1 << 30)]) == -1
+    assert g.shared_buffer_free(buf) == 0

@@ -12,14 +12,17 @@
 
 namespace sb {
 
-// one copy of the in-order sum per kernel: its instructions are fetched cold, and the second sum finds them there
+// One copy of the in-order sum per kernel: its instructions are fetched cold, and the second sum finds them there.  SHORT: rows
+// that one warp adds, kernels of their own: with both ways in one function the launches of a one-token block took 0.5 us longer.
+template <bool SHORT>
 static __device__ __noinline__ float row_sum_of_squares(float* p, int n, uint32_t* scratch) {
-    return sum_in_chain(n, 1) ? block_sum_chain(p, n, scratch, 0) : block_sum_ordered(p, n, 1, scratch);
+    if constexpr (SHORT) return block_sum_chain(p, n, scratch, 0);
+    else return block_sum_ordered(p, n, 1, scratch);
 }
 
 // mode 0: RMSNorm  y = (x*inv) [* weight]             (gemma4.c:85-101)
 // mode 1: router input  y = ((x*inv)*scale)*root      (gemma4.c:103-130)
-template <int MODE>
+template <int MODE, bool SHORT>
 __global__ void __launch_bounds__(256)
 norm_rows_kernel(const float* __restrict__ x, const float* __restrict__ weight, float* __restrict__ y, int n,
                  float eps, int with_scale, float root_in, int* status) {
@@ -37,7 +40,7 @@ norm_rows_kernel(const float* __restrict__ x, const float* __restrict__ weight, 
         bad |= !finite_f(v);
         if (MODE == 1 || with_scale) bad |= !finite_f(weight[i]);
     }
-    const float ss = row_sum_of_squares(ssq, n, s_scan);
+    const float ss = row_sum_of_squares<SHORT>(ssq, n, s_scan);
     if (threadIdx.x == 0) {
         {
             const float mean = __fadd_rn(__fdiv_rn(ss, (float)n), eps);
@@ -112,6 +115,7 @@ cudaError_t launch_q8_jobs(const Q4Job* jobs, int njobs, int max_rows, int max_t
 // ---- consumers of the routed-expert output (exact cells) -------------------------------------
 // y = (x * inv) * w with inv = (mean(x^2) + eps)^-1/2, one row per block; sq = n floats of shared
 // memory.  Returns with y complete and visible to the whole block.
+template <bool SHORT>
 static __device__ void norm_row_block(const float* x, const float* w, float* y, int n, float eps, float* sq,
                                       uint32_t* scan, float* s_inv, bool& bad, int* status) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -119,7 +123,7 @@ static __device__ void norm_row_block(const float* x, const float* w, float* y, 
         sq[i] = __fmul_rn(v, v);
         bad |= !finite_f(v) || !finite_f(w[i]);
     }
-    const float ss = row_sum_of_squares(sq, n, scan);
+    const float ss = row_sum_of_squares<SHORT>(sq, n, scan);
     if (threadIdx.x == 0) {
         *s_inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)n), eps));
         if (!finite_f(*s_inv)) flag(status, SB_ERR_NONFINITE);
@@ -135,6 +139,7 @@ static __device__ void norm_row_block(const float* x, const float* w, float* y, 
 }
 
 // out = residual + RMSNorm(branch) * weight   (models/gemma4-26b-a4b/src/gemma4.c:188-213)
+template <bool SHORT>
 __global__ void __launch_bounds__(1024)
 residual_postnorm_rows_kernel(const float* __restrict__ residual, const float* __restrict__ branch,
                               const float* __restrict__ weight, float* __restrict__ out, int n, float eps,
@@ -145,7 +150,7 @@ residual_postnorm_rows_kernel(const float* __restrict__ residual, const float* _
     const size_t row = blockIdx.x;
     float* normed = cell_sm + ((n + 3) & ~3);
     bool bad = false;
-    norm_row_block(branch + row * n, weight, normed, n, eps, cell_sm, s_scan, &s_inv, bad, status);
+    norm_row_block<SHORT>(branch + row * n, weight, normed, n, eps, cell_sm, s_scan, &s_inv, bad, status);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const float r = residual[row * n + i];
         const float y = __fadd_rn(r, normed[i]);
@@ -157,6 +162,7 @@ residual_postnorm_rows_kernel(const float* __restrict__ residual, const float* _
 
 // sum = RMSNorm(dense)*wd + RMSNorm(routed)*wr; fin = RMSNorm(sum)*wf; out = (residual + fin) * scalar
 // (gemma4.c:215-276).  scratch_a / scratch_b receive sum / fin as the reference leaves them.
+template <bool SHORT>
 __global__ void __launch_bounds__(1024)
 parallel_combine_rows_kernel(const float* __restrict__ residual, const float* __restrict__ dense,
                              const float* __restrict__ routed, const float* __restrict__ wd,
@@ -169,15 +175,15 @@ parallel_combine_rows_kernel(const float* __restrict__ residual, const float* __
     float* sum = scratch_a + row * n;
     float* fin = scratch_b + row * n;
     bool bad = !finite_f(scalar);
-    norm_row_block(dense + row * n, wd, sum, n, eps, cell_sm, s_scan, &s_inv, bad, status);
-    norm_row_block(routed + row * n, wr, fin, n, eps, cell_sm, s_scan, &s_inv, bad, status);
+    norm_row_block<SHORT>(dense + row * n, wd, sum, n, eps, cell_sm, s_scan, &s_inv, bad, status);
+    norm_row_block<SHORT>(routed + row * n, wr, fin, n, eps, cell_sm, s_scan, &s_inv, bad, status);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const float c = __fadd_rn(sum[i], fin[i]);
         bad |= !finite_f(c);
         sum[i] = c;
     }
     __syncthreads();
-    norm_row_block(sum, wf, fin, n, eps, cell_sm, s_scan, &s_inv, bad, status);
+    norm_row_block<SHORT>(sum, wf, fin, n, eps, cell_sm, s_scan, &s_inv, bad, status);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const float r = residual[row * n + i];
         const float y = __fmul_rn(__fadd_rn(r, fin[i]), scalar);
@@ -210,9 +216,10 @@ cudaError_t launch_residual_postnorm(const float* residual, const float* branch,
                                      int rows, int n, float eps, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
     const size_t smem = (2 * (((size_t)n + 3) & ~(size_t)3) + 8) * sizeof(float);
-    const cudaError_t e = allow_row_smem((const void*)residual_postnorm_rows_kernel, smem);
+    const auto kernel = sum_in_chain(n, 1) ? residual_postnorm_rows_kernel<true> : residual_postnorm_rows_kernel<false>;
+    const cudaError_t e = allow_row_smem((const void*)kernel, smem);
     if (e != cudaSuccess) return e;
-    residual_postnorm_rows_kernel<<<rows, 1024, smem, stream>>>(residual, branch, weight, out, n, eps, status);
+    kernel<<<rows, 1024, smem, stream>>>(residual, branch, weight, out, n, eps, status);
     return launched();
 }
 
@@ -221,10 +228,10 @@ cudaError_t launch_parallel_combine(const float* residual, const float* dense, c
                                     int rows, int n, float eps, float scalar, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
     const size_t smem = ((size_t)n + 8) * sizeof(float);
-    const cudaError_t e = allow_row_smem((const void*)parallel_combine_rows_kernel, smem);
+    const auto kernel = sum_in_chain(n, 1) ? parallel_combine_rows_kernel<true> : parallel_combine_rows_kernel<false>;
+    const cudaError_t e = allow_row_smem((const void*)kernel, smem);
     if (e != cudaSuccess) return e;
-    parallel_combine_rows_kernel<<<rows, 1024, smem, stream>>>(residual, dense, routed, wd, wr, wf, scratch_a, scratch_b,
-                                                               out, n, eps, scalar, status);
+    kernel<<<rows, 1024, smem, stream>>>(residual, dense, routed, wd, wr, wf, scratch_a, scratch_b, out, n, eps, scalar, status);
     return launched();
 }
 
@@ -239,7 +246,7 @@ cudaError_t launch_softcap(float* logits, int n, float cap, int* status, cudaStr
 // weights and router scales right at the start, the rows of the expert outputs as soon as
 // the rank table is known.
 // <4, 8> with 1024 threads serves rows up to 4096 columns; <16, 2> with 512 threads up to 8192.
-template <int GLUE_NV, int GLUE_RB>
+template <int GLUE_NV, int GLUE_RB, bool SHORT>
 __global__ void __launch_bounds__(GLUE_NV == 4 ? 1024 : 512) glue_rows_kernel(GlueArgs a) {
     extern __shared__ __align__(16) float gsm[];
     const int n = a.n;
@@ -320,7 +327,7 @@ __global__ void __launch_bounds__(GLUE_NV == 4 ? 1024 : 512) glue_rows_kernel(Gl
                 bad |= !finite_f(v[j]) || !finite_f(nw[j]);
             }
         }
-        const float ss = row_sum_of_squares(sq, n, s_scan);
+        const float ss = row_sum_of_squares<SHORT>(sq, n, s_scan);
         if (tid == 0) {
             s_inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)n), a.eps_norm));
             if (!finite_f(s_inv)) flag(a.status, SB_ERR_NONFINITE);
@@ -350,7 +357,7 @@ __global__ void __launch_bounds__(GLUE_NV == 4 ? 1024 : 512) glue_rows_kernel(Gl
                 bad |= !finite_f(v[j]) || !finite_f(rs[j]);
             }
         }
-        const float ss = row_sum_of_squares(sq, n, s_scan);
+        const float ss = row_sum_of_squares<SHORT>(sq, n, s_scan);
         if (tid == 0) {
             s_inv = pow_neg_half(__fadd_rn(__fdiv_rn(ss, (float)n), a.eps_router));
             if (!finite_f(s_inv) || !finite_f(s_root)) flag(a.status, SB_ERR_NONFINITE);
@@ -544,9 +551,9 @@ cudaError_t launch_glue(const GlueArgs& a, int rows, cudaStream_t stream) {
     if (a.n <= 4096) {
         // every thread owns 4 columns: wide rows and small batches get the largest block
         const int threads = (rows <= 16 || a.n > 1024) ? 1024 : 256;
-        return launch_pdl(glue_rows_kernel<4, 8>, dim3(rows), dim3(threads), smem, stream, a);
+        return launch_pdl(sum_in_chain(a.n, 1) ? glue_rows_kernel<4, 8, true> : glue_rows_kernel<4, 8, false>, dim3(rows), dim3(threads), smem, stream, a);
     }
-    if (a.n <= 8192) return launch_pdl(glue_rows_kernel<16, 2>, dim3(rows), dim3(512), smem, stream, a);
+    if (a.n <= 8192) return launch_pdl(glue_rows_kernel<16, 2, false>, dim3(rows), dim3(512), smem, stream, a);
     return cudaErrorInvalidValue;
 }
 
@@ -554,9 +561,10 @@ cudaError_t launch_rmsnorm(const float* x, const float* weight, float* y, int ro
                            int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
     const size_t smem = (2 * (size_t)n + 8) * sizeof(float);
-    const cudaError_t e = allow_row_smem((const void*)norm_rows_kernel<0>, smem);
+    const auto kernel = sum_in_chain(n, 1) ? norm_rows_kernel<0, true> : norm_rows_kernel<0, false>;
+    const cudaError_t e = allow_row_smem((const void*)kernel, smem);
     if (e != cudaSuccess) return e;
-    norm_rows_kernel<0><<<rows, 256, smem, stream>>>(x, weight, y, n, eps, with_scale, 0.0f, status);
+    kernel<<<rows, 256, smem, stream>>>(x, weight, y, n, eps, with_scale, 0.0f, status);
     return launched();
 }
 
@@ -567,9 +575,10 @@ cudaError_t launch_router_input(const float* x, const float* scale, float* out, 
                                 float root, int* status, cudaStream_t stream) {
     if (rows < 1) return cudaSuccess;
     const size_t smem = (2 * (size_t)n + 8) * sizeof(float);
-    const cudaError_t e = allow_row_smem((const void*)norm_rows_kernel<1>, smem);
+    const auto kernel = sum_in_chain(n, 1) ? norm_rows_kernel<1, true> : norm_rows_kernel<1, false>;
+    const cudaError_t e = allow_row_smem((const void*)kernel, smem);
     if (e != cudaSuccess) return e;
-    norm_rows_kernel<1><<<rows, 256, smem, stream>>>(x, scale, out, n, eps, 1, root, status);
+    kernel<<<rows, 256, smem, stream>>>(x, scale, out, n, eps, 1, root, status);
     return launched();
 }
 
